@@ -346,7 +346,7 @@ extern "C" int64_t nfc_composite_codes(const int32_t* a, uint32_t a_flip, const 
   NFC_CUDA(cudaGetLastError());
   uint64_t* ws = nullptr;
   uint32_t* is = nullptr;
-  int rc = radix_sort_u64(w0, w1, i0, i1, nv, std::max(1, wa + wb), true, s, sc, d_err, &ws, &is);
+  int rc = radix_sort_u64(w0, w1, i0, i1, nv, std::max(1, wa + wb), true, s, sc, &ws, &is);
   if (rc) return rc;
   const int64_t ntiles = (nv + kCcTile - 1) / kCcTile;
   uint64_t* lb = nullptr;

@@ -251,7 +251,7 @@ extern "C" int64_t nfc_group_count_distinct(const int32_t* keys, const uint8_t* 
   NFC_CUDA(cudaGetLastError());
   uint64_t* sorted = nullptr;
   uint32_t* unused = nullptr;
-  int rc = radix_sort_u64(p0, p1, nullptr, nullptr, n, bits, false, s, sc, d_err, &sorted, &unused);
+  int rc = radix_sort_u64(p0, p1, nullptr, nullptr, n, bits, false, s, sc, &sorted, &unused);
   if (rc) return rc;
   const int64_t ntiles = (nv + kCdTile - 1) / kCdTile;
   uint64_t* lb = nullptr;

@@ -120,22 +120,22 @@ int sketch_launch(const int32_t* keys, const uint8_t* key_validity, int64_t n, f
                   cudaStream_t s, const MlpRef* mlp = nullptr);
 size_t sketch_scratch_bytes();
 
-// Radix sort (radix.cu).  Sorts (key, value) pairs ascending by the key's
+// Radix sort (radix_sort.cu).  Sorts (key, value) pairs ascending by the key's
 // unsigned bit pattern over bits [0, key_bits); stable.  keys/vals are
 // overwritten with the sorted sequence; alt buffers are scratch of n.
 // vals may be null (keys only); if iota_vals is set, vals_in is ignored and
 // the payload of element i is i.
 int radix_sort_u32(uint32_t* keys, uint32_t* keys_alt, uint32_t* vals, uint32_t* vals_alt, int64_t n,
-                   int key_bits, bool iota_vals, cudaStream_t s, Scratch& sc, int32_t* d_err,
+                   int key_bits, bool iota_vals, cudaStream_t s, Scratch& sc,
                    uint32_t** keys_result, uint32_t** vals_result);
 int radix_sort_u64(uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt, int64_t n,
-                   int key_bits, bool iota_vals, cudaStream_t s, Scratch& sc, int32_t* d_err,
+                   int key_bits, bool iota_vals, cudaStream_t s, Scratch& sc,
                    uint64_t** keys_result, uint32_t** vals_result);
 // The same over the keys src[i] ^ in_xor of a read-only column (e.g. the
 // sign flip that orders int32 as unsigned): no separate transform pass;
 // keys / keys_alt are scratch of n and the result is in one of them.
 int radix_sort_u32_from(const uint32_t* src, uint32_t in_xor, uint32_t* keys, uint32_t* keys_alt, uint32_t* vals,
                         uint32_t* vals_alt, int64_t n, int key_bits, bool iota_vals, cudaStream_t s, Scratch& sc,
-                        int32_t* d_err, uint32_t** keys_result, uint32_t** vals_result);
+                        uint32_t** keys_result, uint32_t** vals_result);
 
 }  // namespace nfc

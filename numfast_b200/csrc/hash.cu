@@ -151,7 +151,7 @@ int hash_finish(const ColSet& cs, const OutSet& o, const StateRef& st, const uin
     return NFC_ERR_RANGE;
   }
   uint32_t *kr = nullptr, *vr = nullptr;
-  int rc = radix_sort_u32(k0, k1, v0, v1, ng, 32, false, s, sc, d_err, &kr, &vr);
+  int rc = radix_sort_u32(k0, k1, v0, v1, ng, 32, false, s, sc, &kr, &vr);
   if (rc) return rc;
   if (ng > 0) {
     k_hash_emit<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((ng + 255) / 256, (int64_t)num_sms() * 8)), 256, 0,

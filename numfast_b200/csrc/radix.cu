@@ -1,6 +1,6 @@
-// Onesweep LSD radix sort (8-bit digits) with decoupled look-back, and the
-// entry points built on it: stable argsort (ir_sort), sorted unique with
-// first-occurrence rows and counts (ir_unique_inverse), and gather.
+// Entry points built on the radix sort (radix_sort.cu): stable argsort
+// (ir_sort), sorted unique with first-occurrence rows and counts
+// (ir_unique_inverse), and gather.
 //
 // Semantics follow the reference:
 //   * ascending argsort == np.argsort(kind="stable")  (sort.rs:55-118);
@@ -11,424 +11,11 @@
 //     reverse input order (what _stable_desc_idx yields, since NaN != NaN);
 //   * invalid rows go last in input order (_sort_perm, cpu.py:1174-1225);
 //   * unique: uniq ascending, inverse with uniq[inv] == keys (unique.rs:30-91).
-//
-// Pass structure: one histogram kernel computes every pass's digit counts;
-// passes whose digit is constant over all keys are skipped; each remaining
-// pass is ONE kernel: tiles of 8192 keys rank locally (per-warp digit peers
-// from eight ballots), publish per-digit tile counts, look back over predecessor tiles
-// for their global offset, stage the tile in shared memory in digit order
-// and write it out in runs.
 #include <algorithm>
 
 #include "groupby_host.h"
 
 namespace nfc {
-
-constexpr int kSortThreads = 512;
-constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = 16;
-constexpr int kSortTile = kSortThreads * kSortItems;  // 8192
-constexpr uint32_t kStAgg = 1u << 30;
-constexpr uint32_t kStInc = 2u << 30;
-constexpr uint32_t kStVal = (1u << 30) - 1u;
-
-template <class K>
-__global__ void __launch_bounds__(256) k_radix_hist(const K* __restrict__ keys, int64_t n, int npasses,
-                                                    uint32_t* __restrict__ ghist, K xr) {
-  __shared__ uint32_t h[8][256];
-  for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) (&h[0][0])[i] = 0u;
-  __syncthreads();
-  // 16-byte vector loads, U of them in flight per thread, when the keys are
-  // 16-byte aligned; the scalar loop takes the rest.
-  constexpr int VEC = 16 / sizeof(K);
-  constexpr int U = 4;
-  int64_t done = 0;
-  if ((reinterpret_cast<uintptr_t>(keys) & 15u) == 0) {
-    const int64_t nvec = n / VEC;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t v0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v0 < nvec; v0 += stride * U) {
-      K kk[U][VEC];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int64_t v = v0 + u * stride;
-        if (v < nvec) {
-          if constexpr (sizeof(K) == 4) {
-            const uint4 q = __ldcs(reinterpret_cast<const uint4*>(keys) + v);
-            kk[u][0] = q.x ^ xr; kk[u][1] = q.y ^ xr; kk[u][2] = q.z ^ xr; kk[u][3] = q.w ^ xr;
-          } else {
-            const ulonglong2 q = __ldcs(reinterpret_cast<const ulonglong2*>(keys) + v);
-            kk[u][0] = q.x ^ xr; kk[u][1] = q.y ^ xr;
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (v0 + u * stride < nvec)
-#pragma unroll
-          for (int e = 0; e < VEC; ++e)
-            for (int p = 0; p < npasses; ++p) atomicAdd(&h[p][(uint32_t)(kk[u][e] >> (8 * p)) & 255u], 1u);
-    }
-    done = nvec * VEC;
-  }
-  for (int64_t i = done + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const K k = keys[i] ^ xr;
-    for (int p = 0; p < npasses; ++p) atomicAdd(&h[p][(uint32_t)(k >> (8 * p)) & 255u], 1u);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < npasses * 256; i += blockDim.x)
-    if ((&h[0][0])[i]) atomicAdd(&ghist[i], (&h[0][0])[i]);
-}
-
-// Exclusive scan of each pass's 256 bins (one block of 256 per pass).
-__global__ void k_radix_scan(const uint32_t* ghist, uint32_t* base) {
-  __shared__ uint32_t s_scan[33];
-  const int p = blockIdx.x;
-  uint32_t total;
-  const uint32_t v = ghist[p * 256 + threadIdx.x];
-  base[p * 256 + threadIdx.x] = block_excl_scan(v, s_scan, &total);
-}
-
-// The per-warp digit counters are dead once every element knows its tile
-// position, so the staging arrays overlay them: u64 keys with u32 values fit
-// in ~98 KB and two CTAs stay resident per SM.
-template <class K>
-struct SortSmem {
-  uint32_t dstart[256];
-  uint32_t gofs[256];
-  uint32_t scan[33];
-  uint32_t tile;
-  union {
-    uint32_t wh[kSortWarps][256];
-    struct {
-      K keys[kSortTile];
-      uint32_t vals[kSortTile];
-    } st;
-  } u;
-};
-
-// Lanes holding the same 8-bit digit as this lane (and the same validity):
-// one ballot per digit bit.  __match_any_sync serialises over the distinct
-// values in the warp, which for random digits is most of the 32 lanes; eight
-// ballots cost the same for any distribution.
-NFC_DEV unsigned match_digit8(uint32_t d, bool ok) {
-  const unsigned v = __ballot_sync(0xffffffffu, ok);
-  unsigned m = ok ? v : ~v;
-#pragma unroll
-  for (int b = 0; b < 8; ++b) {
-    const bool p = (d >> b) & 1u;
-    const unsigned bb = __ballot_sync(0xffffffffu, p);
-    m &= p ? bb : ~bb;
-  }
-  return m;
-}
-
-// Keys are read as kin[i] ^ xr (the first pass of a sort from a caller's
-// column applies an order-preserving flip on the way in) and written flipped.
-template <class K, bool HAS_VALS, bool IOTA>
-__global__ void __launch_bounds__(kSortThreads, 2) k_onesweep(const K* __restrict__ kin, K* __restrict__ kout,
-                                                           const uint32_t* __restrict__ vin,
-                                                           uint32_t* __restrict__ vout, int64_t n, int shift,
-                                                           const uint32_t* __restrict__ digit_base,
-                                                           uint32_t* __restrict__ status, uint32_t* ticket,
-                                                           int32_t* err, K xr) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  SortSmem<K>& S = *reinterpret_cast<SortSmem<K>*>(smem_raw);
-  const int lane = lane_id(), warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) S.tile = atomicAdd(ticket, 1u);
-  for (int i = threadIdx.x; i < kSortWarps * 256; i += kSortThreads) (&S.u.wh[0][0])[i] = 0u;
-  __syncthreads();
-  const int64_t tile = S.tile;
-  const int64_t base = tile * kSortTile;
-  // Digits are recomputed from the keys and IOTA values from the index
-  // instead of being held, which keeps two CTAs resident per SM.
-  K key[kSortItems];
-  uint32_t val[(HAS_VALS && !IOTA) ? kSortItems : 1];
-  uint32_t rank[kSortItems];
-  const int64_t wbase = base + warp * (32 * kSortItems) + lane;
-#pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
-    const int64_t idx = wbase + j * 32;
-    const bool ok = idx < n;
-    key[j] = ok ? kin[idx] ^ xr : (K)0;
-    if (HAS_VALS && !IOTA) val[j] = ok ? vin[idx] : 0u;
-  }
-#pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
-    const bool ok = wbase + j * 32 < n;
-    const uint32_t d = (uint32_t)(key[j] >> shift) & 255u;
-    const unsigned peers = match_digit8(d, ok);
-    const int leader = __ffs(peers) - 1;
-    uint32_t b = 0;
-    if (lane == leader && ok) {
-      b = S.u.wh[warp][d];
-      S.u.wh[warp][d] = b + (uint32_t)__popc(peers);
-    }
-    b = __shfl_sync(0xffffffffu, b, leader);
-    rank[j] = b + (uint32_t)__popc(peers & lanemask_lt());
-    __syncwarp();
-  }
-  __syncthreads();
-  uint32_t tile_cnt = 0;
-  if (threadIdx.x < 256) {
-    uint32_t run = 0;
-#pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) {
-      const uint32_t c = S.u.wh[w][threadIdx.x];
-      S.u.wh[w][threadIdx.x] = run;
-      run += c;
-    }
-    tile_cnt = run;
-  }
-  uint32_t total;
-  const uint32_t dstart = block_excl_scan(threadIdx.x < 256 ? tile_cnt : 0u, S.scan, &total);
-  if (threadIdx.x < 256) {
-    const int d = threadIdx.x;
-    S.dstart[d] = dstart;
-    uint32_t excl = 0;
-    uint32_t* st = status + (size_t)tile * 256 + d;
-    if (tile == 0) {
-      __threadfence();
-      atomicExch(st, kStInc | tile_cnt);
-    } else {
-      __threadfence();
-      atomicExch(st, kStAgg | tile_cnt);
-      // Windowed walk: kLbWin independent loads per round (tiles j .. j-7),
-      // consumed in order up to the first inclusive or unpublished status.
-      constexpr int kLbWin = 8;
-      int64_t j = tile - 1;
-      uint32_t spins = 0;
-      bool done = false;
-      while (!done) {
-        uint32_t w[kLbWin];
-#pragma unroll
-        for (int k = 0; k < kLbWin; ++k)
-          w[k] = j - k >= 0 ? ld_volatile_u32(status + (size_t)(j - k) * 256 + d) : kStInc;  // past tile 0: end
-        int take = 0;
-#pragma unroll
-        for (int k = 0; k < kLbWin; ++k) {
-          if (done) break;
-          const uint32_t flag = w[k] & ~kStVal;
-          if (flag == 0) break;
-          excl += w[k] & kStVal;
-          ++take;
-          if (flag == kStInc) done = true;
-        }
-        if (done) break;
-        if (take == 0 && ++spins > kSpinLimit) {
-          atomicExch(err, NFC_ERR_TIMEOUT);
-          break;
-        }
-        j -= take;
-      }
-      __threadfence();
-      atomicExch(st, kStInc | (excl + tile_cnt));
-    }
-    S.gofs[d] = digit_base[d] + excl - dstart;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
-    const uint32_t d = (uint32_t)(key[j] >> shift) & 255u;
-    rank[j] += S.dstart[d] + S.u.wh[warp][d];
-  }
-  __syncthreads();  // the counters are overwritten by the staged tile below
-#pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
-    const int64_t idx = wbase + j * 32;
-    if (idx < n) {
-      const uint32_t p = rank[j];
-      S.u.st.keys[p] = key[j];
-      if (HAS_VALS) S.u.st.vals[p] = IOTA ? (uint32_t)idx : val[(HAS_VALS && !IOTA) ? j : 0];
-    }
-  }
-  __syncthreads();
-  const int tile_n = (int)std::min<int64_t>(kSortTile, n - base);
-  for (int i = threadIdx.x; i < tile_n; i += kSortThreads) {
-    const K k = S.u.st.keys[i];
-    const uint32_t d = (uint32_t)(k >> shift) & 255u;
-    const uint32_t dst = S.gofs[d] + (uint32_t)i;
-    kout[dst] = k;
-    if (HAS_VALS) vout[dst] = S.u.st.vals[i];
-  }
-}
-
-// Inputs of at most kSmallSort keys (the distinct keys of a low-cardinality
-// hash group-by, small argsorts) are sorted by one CTA: a bitonic network in
-// shared memory over (masked key, input index) pairs, which makes it stable,
-// then a gather of the full keys and values.  One launch and no host round
-// trip, where the multi-pass sort costs a histogram read-back and up to
-// eight more launches.
-constexpr int kSmallSort = 2048;
-
-template <class K>
-__global__ void __launch_bounds__(1024) k_sort_small(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
-                                                     bool iota, int n, K mask, K xr, K* __restrict__ kout,
-                                                     uint32_t* __restrict__ vout) {
-  __shared__ K sk[kSmallSort];
-  __shared__ uint32_t si[kSmallSort];
-  int m = 1;
-  while (m < n) m <<= 1;
-  // Padding (index >= n) holds the largest key and sorts after every real key.
-  for (int i = threadIdx.x; i < m; i += blockDim.x) {
-    sk[i] = i < n ? ((kin[i] ^ xr) & mask) : ~(K)0;
-    si[i] = (uint32_t)i;
-  }
-  __syncthreads();
-  for (int size = 2; size <= m; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int t = threadIdx.x; t < (m >> 1); t += blockDim.x) {
-        const int lo = 2 * t - (t & (stride - 1));  // pair (lo, lo + stride), bit 'stride' of lo clear
-        const int hi = lo + stride;
-        const K a = sk[lo], b = sk[hi];
-        const uint32_t ia = si[lo], ib = si[hi];
-        const bool gt = a > b || (a == b && ia > ib);
-        if (gt == ((lo & size) == 0)) {  // ascending where bit 'size' of lo is clear
-          sk[lo] = b;
-          sk[hi] = a;
-          si[lo] = ib;
-          si[hi] = ia;
-        }
-      }
-      __syncthreads();
-    }
-  }
-  for (int r = threadIdx.x; r < n; r += blockDim.x) {
-    const uint32_t i = si[r];
-    kout[r] = kin[i] ^ xr;
-    if (vout) vout[r] = iota ? i : vin[i];
-  }
-}
-
-template <class K>
-__global__ void k_xor_copy(const K* __restrict__ in, K xr, int64_t n, K* __restrict__ out) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = in[i] ^ xr;
-}
-
-__global__ void k_iota(uint32_t* v, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    v[i] = (uint32_t)i;
-}
-
-// src (when not null) is a read-only key column that the histogram and the
-// first pass read as src[i] ^ in_xor; keys / keys_alt are then only the
-// ping-pong buffers, and the result never aliases src.
-template <class K>
-static int radix_sort_impl(K* keys, K* keys_alt, uint32_t* vals, uint32_t* vals_alt, int64_t n, int key_bits,
-                           bool iota_vals, cudaStream_t s, Scratch& sc, int32_t* d_err, K** keys_result,
-                           uint32_t** vals_result, const K* src = nullptr, K in_xor = 0) {
-  if (!src) {
-    src = keys;
-    in_xor = 0;
-  }
-  *keys_result = keys;
-  *vals_result = vals;
-  if (n <= 0) return NFC_OK;
-  const bool has_vals = vals != nullptr;
-  if (n <= kSmallSort) {
-    const K mask = key_bits >= (int)(8 * sizeof(K)) ? ~(K)0 : (K)(((K)1 << key_bits) - 1);
-    k_sort_small<K><<<1, 1024, 0, s>>>(src, vals, iota_vals, (int)n, mask, in_xor, keys_alt,
-                                       has_vals ? vals_alt : nullptr);
-    NFC_CUDA(cudaGetLastError());
-    *keys_result = keys_alt;
-    if (has_vals) *vals_result = vals_alt;
-    return NFC_OK;
-  }
-  if (n >= (1ll << 30)) {
-    set_last_error("radix sort: n=%lld >= 2^30", (long long)n);
-    return NFC_ERR_UNSUPPORTED;
-  }
-  const int npasses = (key_bits + 7) / 8;
-  uint32_t* hist = nullptr;
-  uint32_t* dbase = nullptr;
-  NFC_CUDA(sc.alloc(&hist, 2 * 8 * 256));
-  dbase = hist + 8 * 256;
-  NFC_CUDA(cudaMemsetAsync(hist, 0, 8 * 256 * sizeof(uint32_t), s));
-  {
-    int64_t g = std::min<int64_t>((n + 4095) / 4096, (int64_t)num_sms() * 4);
-    k_radix_hist<K><<<(unsigned)std::max<int64_t>(g, 1), 256, 0, s>>>(src, n, npasses, hist, in_xor);
-    NFC_CUDA(cudaGetLastError());
-  }
-  k_radix_scan<<<npasses, 256, 0, s>>>(hist, dbase);
-  NFC_CUDA(cudaGetLastError());
-  uint32_t hh[8 * 256];
-  NFC_CUDA(readback(hh, hist, sizeof(uint32_t) * 256 * npasses, s));
-  const int64_t ntiles = (n + kSortTile - 1) / kSortTile;
-  uint32_t* status = nullptr;
-  uint32_t* ticket = nullptr;
-  NFC_CUDA(sc.alloc(&status, (size_t)ntiles * 256 + 64));
-  ticket = status + (size_t)ntiles * 256;
-  const size_t smem = sizeof(SortSmem<K>);
-  if (has_vals) {
-    NFC_CUDA(cudaFuncSetAttribute(k_onesweep<K, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    NFC_CUDA(cudaFuncSetAttribute(k_onesweep<K, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  } else {
-    NFC_CUDA(cudaFuncSetAttribute(k_onesweep<K, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  }
-  const K* kin = src;
-  K* kout = src == keys ? keys_alt : keys;
-  K xr = in_xor;
-  uint32_t* vin = vals;
-  uint32_t* vout = vals_alt;
-  bool need_iota = has_vals && iota_vals;
-  for (int p = 0; p < npasses; ++p) {
-    bool trivial = false;
-    for (int d = 0; d < 256; ++d)
-      if ((int64_t)hh[p * 256 + d] == n) trivial = true;
-    if (trivial) continue;
-    NFC_CUDA(cudaMemsetAsync(status, 0, ((size_t)ntiles * 256 + 64) * sizeof(uint32_t), s));
-    if (has_vals && need_iota)
-      k_onesweep<K, true, true><<<(unsigned)ntiles, kSortThreads, smem, s>>>(kin, kout, vin, vout, n, 8 * p,
-                                                                             dbase + 256 * p, status, ticket, d_err,
-                                                                             xr);
-    else if (has_vals)
-      k_onesweep<K, true, false><<<(unsigned)ntiles, kSortThreads, smem, s>>>(kin, kout, vin, vout, n, 8 * p,
-                                                                              dbase + 256 * p, status, ticket, d_err,
-                                                                              xr);
-    else
-      k_onesweep<K, false, false><<<(unsigned)ntiles, kSortThreads, smem, s>>>(kin, kout, vin, vout, n, 8 * p,
-                                                                               dbase + 256 * p, status, ticket,
-                                                                               d_err, xr);
-    NFC_CUDA(cudaGetLastError());
-    need_iota = false;
-    xr = 0;
-    K* written = kout;
-    kout = written == keys ? keys_alt : keys;
-    kin = written;
-    std::swap(vin, vout);
-  }
-  const unsigned g1 = (unsigned)std::min<int64_t>((n + 255) / 256, (int64_t)num_sms() * 8);
-  if (kin == src && src != keys) {
-    // Every pass was trivial (all keys equal in the sorted bits): the result
-    // is the source itself, flipped into the first buffer.
-    k_xor_copy<K><<<g1, 256, 0, s>>>(src, in_xor, n, keys);
-    NFC_CUDA(cudaGetLastError());
-    kin = keys;
-  }
-  if (need_iota) {
-    // Every pass was trivial: the input order is already sorted.
-    k_iota<<<g1, 256, 0, s>>>(vin, n);
-    NFC_CUDA(cudaGetLastError());
-  }
-  *keys_result = const_cast<K*>(kin);
-  *vals_result = vin;
-  return NFC_OK;
-}
-
-int radix_sort_u32(uint32_t* keys, uint32_t* keys_alt, uint32_t* vals, uint32_t* vals_alt, int64_t n, int key_bits,
-                   bool iota_vals, cudaStream_t s, Scratch& sc, int32_t* d_err, uint32_t** kr, uint32_t** vr) {
-  return radix_sort_impl<uint32_t>(keys, keys_alt, vals, vals_alt, n, key_bits, iota_vals, s, sc, d_err, kr, vr);
-}
-int radix_sort_u32_from(const uint32_t* src, uint32_t in_xor, uint32_t* keys, uint32_t* keys_alt, uint32_t* vals,
-                        uint32_t* vals_alt, int64_t n, int key_bits, bool iota_vals, cudaStream_t s, Scratch& sc,
-                        int32_t* d_err, uint32_t** kr, uint32_t** vr) {
-  return radix_sort_impl<uint32_t>(keys, keys_alt, vals, vals_alt, n, key_bits, iota_vals, s, sc, d_err, kr, vr, src,
-                                   in_xor);
-}
-int radix_sort_u64(uint64_t* keys, uint64_t* keys_alt, uint32_t* vals, uint32_t* vals_alt, int64_t n, int key_bits,
-                   bool iota_vals, cudaStream_t s, Scratch& sc, int32_t* d_err, uint64_t** kr, uint32_t** vr) {
-  return radix_sort_impl<uint64_t>(keys, keys_alt, vals, vals_alt, n, key_bits, iota_vals, s, sc, d_err, kr, vr);
-}
 
 // ---------------------------------------------------------------------
 // Key transforms (order-preserving maps to unsigned).
@@ -590,7 +177,7 @@ static int argsort_core(int32_t dtype, const void* keys, uint32_t* pos, int64_t 
     NFC_CUDA(sc.alloc(&k1, (size_t)n));
     k_xform_i32<<<grid1d(n), 256, 0, s>>>(static_cast<const int32_t*>(keys), pos, n, desc, k0);
     NFC_CUDA(cudaGetLastError());
-    int rc = radix_sort_u32(k0, k1, vals, vals_alt, n, 32, iota, s, sc, d_err, &kres, &vres);
+    int rc = radix_sort_u32(k0, k1, vals, vals_alt, n, 32, iota, s, sc, &kres, &vres);
     if (rc) return rc;
   } else {
     uint64_t *k0 = nullptr, *k1 = nullptr, *kres = nullptr;
@@ -605,7 +192,7 @@ static int argsort_core(int32_t dtype, const void* keys, uint32_t* pos, int64_t 
       nan_fix = desc;
     }
     NFC_CUDA(cudaGetLastError());
-    int rc = radix_sort_u64(k0, k1, vals, vals_alt, n, 64, iota, s, sc, d_err, &kres, &vres);
+    int rc = radix_sort_u64(k0, k1, vals, vals_alt, n, 64, iota, s, sc, &kres, &vres);
     if (rc) return rc;
   }
   if (vres != perm_out) NFC_CUDA(cudaMemcpyAsync(perm_out, vres, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
@@ -1088,7 +675,7 @@ extern "C" int64_t nfc_unique(const int32_t* keys, int64_t n, int32_t* uniq_out,
   NFC_CUDA(sc.alloc(&v1, (size_t)n));
   // int32 keys sort as unsigned after a sign flip, applied as the keys are read.
   int rc = radix_sort_u32_from(reinterpret_cast<const uint32_t*>(keys), 0x80000000u, k0, k1, v0, v1, n, 32, true, s,
-                               sc, d_err, &kres, &vres);
+                               sc, &kres, &vres);
   if (rc) return rc;
   const int64_t ntiles = (n + kRunTile - 1) / kRunTile;
   uint64_t* lb = nullptr;

@@ -489,9 +489,9 @@ int topk_impl(const void* keys, const uint8_t* validity, int64_t n, bool desc, i
     uint32_t* cvr = nullptr;
     int rc;
     if constexpr (DT == NFC_I32)
-      rc = radix_sort_u32(c_img, c_img_alt, c_row, c_row_alt, on_prefix, 32, false, s, sc, d_err, &ckr, &cvr);
+      rc = radix_sort_u32(c_img, c_img_alt, c_row, c_row_alt, on_prefix, 32, false, s, sc, &ckr, &cvr);
     else
-      rc = radix_sort_u64(c_img, c_img_alt, c_row, c_row_alt, on_prefix, 64, false, s, sc, d_err, &ckr, &cvr);
+      rc = radix_sort_u64(c_img, c_img_alt, c_row, c_row_alt, on_prefix, 64, false, s, sc, &ckr, &cvr);
     if (rc) return rc;
     int64_t off = 0;
     if (DT == NFC_F64 && desc && prefix == 0) {
@@ -513,9 +513,9 @@ int topk_impl(const void* keys, const uint8_t* validity, int64_t n, bool desc, i
     uint32_t* vr = nullptr;
     int rc;
     if constexpr (DT == NFC_I32)
-      rc = radix_sort_u32(img, img_alt, row, row_alt, ksel, 32, false, s, sc, d_err, &kr, &vr);
+      rc = radix_sort_u32(img, img_alt, row, row_alt, ksel, 32, false, s, sc, &kr, &vr);
     else
-      rc = radix_sort_u64(img, img_alt, row, row_alt, ksel, 64, false, s, sc, d_err, &kr, &vr);
+      rc = radix_sort_u64(img, img_alt, row, row_alt, ksel, 64, false, s, sc, &kr, &vr);
     if (rc) return rc;
     NFC_CUDA(cudaMemcpyAsync(perm_out, vr, sizeof(int32_t) * ksel, cudaMemcpyDeviceToDevice, s));
   }
