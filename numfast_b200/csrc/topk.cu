@@ -30,14 +30,20 @@
 //                  for k <= 2,048), which is the argsort's order of them.
 //
 // Full passes over the column in the usual case: one histogram (more only
-// while the prefix group exceeds the buffer) and the split.  100M float64
-// keys, k = 1,000: 0.82 ms against 8.9 ms for the full argsort.
+// while the prefix group exceeds the buffer) and the split.
+//
+// Small k (topk_sampled) needs one pass over the column: the histograms run on
+// a sample of the rows, the rows up to a threshold that holds the k-th smallest
+// image with near certainty are collected in any order, and one CTA sorts them
+// by (image, row).  If the count shows the threshold too low, or too many rows
+// are on it (ties), the passes above run instead.
 //
 // Descending float64: every NaN is its own group in the reference's
 // _stable_desc_idx, so the NaN block comes first in REVERSE input order: the
 // selection takes the last `need` NaN rows and the sorted NaN prefix is
 // reversed.  For k above n / 8 the full argsort is cheaper and is used.
 #include <algorithm>
+#include <cmath>
 
 #include "groupby_core.cuh"
 #include "groupby_host.h"
@@ -367,6 +373,257 @@ __global__ void k_tk_reverse(int32_t* p, int64_t m) {
   }
 }
 
+// ---------------------------------------------------------------- sampled threshold
+// Bound of the exact form: 557 us of 100M float64 keys go into one histogram
+// and one ordered split, both over the whole column, and 50,000 candidates are
+// then sorted.  A threshold from a sample costs two small histograms; what is
+// left is one pass that reads the column and writes a few thousand rows.
+constexpr int kTkCap = 8192;          // rows one CTA sorts
+constexpr int64_t kTkExpect = 5000;   // most rows expected under the threshold
+
+constexpr int kTkFinalThreads = 512;
+constexpr int kTkLevels = 4;          // digits of the threshold at most
+
+struct TkSample {
+  uint64_t prefix, mask;  // threshold: rows with (image & mask) <= prefix
+  uint32_t target;        // rank in the sample still to find on the prefix
+  uint32_t below;         // sampled rows under the prefix
+  uint32_t ready;         // the threshold lets few enough rows through
+  uint32_t count;         // rows collected
+  uint32_t status;        // 1: the exact passes have to run
+  uint32_t pad;
+  uint32_t done[kTkLevels];  // CTAs that have finished each level
+  uint32_t hist[kTkLevels][kTkBins];
+};
+
+// Histogram of one 11-bit digit of the sampled rows on the prefix; the last
+// CTA to finish moves the prefix on to the digit that holds the target rank.
+// The sample is one group of four rows out of every `step`, at a hashed place:
+// short groups, so that sorted or clustered columns are sampled evenly too.
+template <int DT>
+__global__ void __launch_bounds__(kTkThreads) k_tk_sample(const void* __restrict__ keys,
+                                                         const uint8_t* __restrict__ validity, int64_t n, bool vec,
+                                                         bool desc, int level, int shift, uint32_t dmask,
+                                                         uint32_t step, uint32_t target, TkSample* st) {
+  __shared__ uint32_t h[2][kTkBins];
+  __shared__ uint32_t s_scan[33];
+  __shared__ int s_last;
+  if (level && st->ready) return;
+  const uint64_t prefix = level ? st->prefix : 0ull, mask = level ? st->mask : 0ull;
+  uint32_t* hs = h[(threadIdx.x >> 5) & 1];
+  for (int i = threadIdx.x; i < 2 * kTkBins; i += kTkThreads) (&h[0][0])[i] = 0u;
+  __syncthreads();
+  const int64_t ngroups = (n + 3) / 4;
+  const int64_t npick = (ngroups + step - 1) / step;
+  const int64_t stride = (int64_t)gridDim.x * kTkThreads;
+  constexpr int U = 4;
+  for (int64_t p0 = blockIdx.x * (int64_t)kTkThreads + threadIdx.x; p0 < npick; p0 += U * stride) {
+    uint64_t img[U][4];
+    uint32_t ok[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t p = p0 + u * stride;
+      const int64_t g = p * step + (step > 1 ? ((uint32_t)p * 0x9E3779B1u >> 8) % step : 0u);
+      ok[u] = p < npick && g < ngroups ? tk_load4<DT>(keys, validity, g * 4, n, vec, desc, img[u]) : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (((ok[u] >> r) & 1u) && (img[u][r] & mask) == prefix)
+          atomicAdd(&hs[(uint32_t)(img[u][r] >> shift) & dmask], 1u);
+  }
+  __syncthreads();
+  uint32_t* gh = st->hist[level];
+  for (int i = threadIdx.x; i < kTkBins; i += kTkThreads) {
+    const uint32_t c = h[0][i] + h[1][i];
+    if (c) atomicAdd(&gh[i], c);
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&st->done[level], 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  constexpr int kPer = kTkBins / kTkThreads;
+  uint32_t c[kPer], sum = 0;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    c[j] = __ldcg(&gh[threadIdx.x * kPer + j]);
+    sum += c[j];
+  }
+  uint32_t total;
+  uint32_t x = block_excl_scan(sum, s_scan, &total);
+  const uint32_t want = level ? st->target : target;
+  // Fewer sampled valid rows than the target: no digit holds it, and the
+  // levels that follow find nothing to count.
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    if (x < want && want <= x + c[j]) {
+      st->prefix = prefix | ((uint64_t)(threadIdx.x * kPer + j) << shift);
+      st->mask = mask | ((uint64_t)dmask << shift);
+      st->target = want - x;
+      const uint32_t below = (level ? st->below : 0u) + x;
+      st->below = below;
+      if ((uint64_t)(below + c[j]) * step <= (uint64_t)(kTkExpect + kTkExpect / 4)) st->ready = 1u;
+    }
+    x += c[j];
+  }
+}
+
+// Whether a key's image is at most `top`, on the key itself: one comparison
+// with the key at the threshold instead of building every row's image.
+template <int DT>
+struct TkUnder;
+template <>
+struct TkUnder<NFC_I32> {
+  int32_t t;
+  bool desc;
+  NFC_DEV TkUnder(uint64_t top, bool d)
+      : t((int32_t)((d ? ~(uint32_t)top : (uint32_t)top) ^ 0x80000000u)), desc(d) {}
+  NFC_DEV bool operator()(uint32_t raw) const { return desc ? (int32_t)raw >= t : (int32_t)raw <= t; }
+};
+template <>
+struct TkUnder<NFC_I64> {
+  int64_t t;
+  bool desc;
+  NFC_DEV TkUnder(uint64_t top, bool d) : t((int64_t)((d ? ~top : top) ^ 0x8000000000000000ull)), desc(d) {}
+  NFC_DEV bool operator()(uint64_t raw) const { return desc ? (int64_t)raw >= t : (int64_t)raw <= t; }
+};
+// float64: the zeros compare equal, as their images do.  Descending, NaN rows
+// come first (image 0) and pass as "not below"; ascending they come last and
+// fail "at most" (only a threshold on the NaN image itself lets them in).
+// Thresholds outside the images of numbers become the infinity on that side.
+template <>
+struct TkUnder<NFC_F64> {
+  double t;
+  bool desc, all;
+  NFC_DEV TkUnder(uint64_t top, bool d) : desc(d), all(top == ~0ull) {
+    const uint64_t inf = f64_ord(0x7FF0000000000000ull), ninf = f64_ord(0xFFF0000000000000ull);
+    const uint64_t u = min(max(d ? ~top : top, ninf), inf);
+    t = __longlong_as_double((long long)f64_unord(u));
+  }
+  NFC_DEV bool operator()(uint64_t raw) const {
+    const double v = __longlong_as_double((long long)raw);
+    return desc ? !(v < t) : (v <= t || all);
+  }
+};
+
+// Every valid row up to the threshold, in any order.
+template <int DT>
+__global__ void __launch_bounds__(kTkThreads, 4) k_tk_collect(const void* __restrict__ keys,
+                                                             const uint8_t* __restrict__ validity, int64_t n,
+                                                             bool vec, bool desc, TkSample* st,
+                                                             uint64_t* __restrict__ c_img,
+                                                             uint32_t* __restrict__ c_row) {
+  using R = typename std::conditional<DT == NFC_I32, uint32_t, uint64_t>::type;
+  if (!st->ready) return;
+  const uint64_t image_bits = DT == NFC_I32 ? 0xFFFFFFFFull : ~0ull;
+  const TkUnder<DT> under((st->prefix | ~st->mask) & image_bits, desc);
+  const R* col = static_cast<const R*>(keys);
+  const int lane = lane_id();
+  const int64_t ngroups = (n + 3) / 4;
+  const int64_t stride = (int64_t)gridDim.x * kTkThreads;
+  constexpr int U = 4;
+  for (int64_t g0 = blockIdx.x * (int64_t)kTkThreads + (threadIdx.x & ~31u); g0 < ngroups; g0 += U * stride) {
+    R raw[U][4];
+    uint32_t ok[U], hit = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t i0 = (g0 + u * stride + lane) * 4;
+      ok[u] = i0 + 4 <= n ? 0xFu : (i0 < n ? (1u << (uint32_t)(n - i0)) - 1u : 0u);
+      if (vec && i0 + 4 <= n) {
+        if constexpr (DT == NFC_I32) {
+          const uint4 q = __ldcs(reinterpret_cast<const uint4*>(col + i0));
+          raw[u][0] = q.x; raw[u][1] = q.y; raw[u][2] = q.z; raw[u][3] = q.w;
+        } else {
+          const ulonglong2* p = reinterpret_cast<const ulonglong2*>(col + i0);
+          const ulonglong2 x = __ldcs(p), y = __ldcs(p + 1);
+          raw[u][0] = x.x; raw[u][1] = x.y; raw[u][2] = y.x; raw[u][3] = y.y;
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) raw[u][r] = i0 + r < n ? col[i0 + r] : (R)0;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t i0 = (g0 + u * stride + lane) * 4;
+      if (validity && ok[u]) ok[u] &= (uint32_t)(__ldg(validity + (i0 >> 3)) >> (i0 & 7)) & 0xFu;
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (((ok[u] >> r) & 1u) && under(raw[u][r])) hit |= 1u << (4 * u + r);
+    }
+    if (!__any_sync(0xffffffffu, hit != 0u)) continue;
+    // Rare: one reservation per warp.  Once the buffer is full the exact
+    // passes will run, so the rest of the column does not matter.
+    const uint32_t mine = (uint32_t)__popc(hit);
+    uint32_t incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    uint32_t base = 0;
+    if (lane == 31) base = atomicAdd(&st->count, incl);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    if (base >= (uint32_t)kTkCap) return;
+    uint32_t pos = base + incl - mine;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if ((hit >> (4 * u + r)) & 1u) {
+          if (pos < (uint32_t)kTkCap) {
+            c_img[pos] = tk_image_bits<DT>(raw[u][r], desc);
+            c_row[pos] = (uint32_t)((g0 + u * stride + lane) * 4 + r);
+          }
+          ++pos;
+        }
+  }
+}
+
+// The collected rows in order of (image, row) -- descending float64 NaN rows
+// (image 0) by descending row -- first k rows out.  A row's place is the number
+// of rows before it, counted by a warp against all of them: the ~20 M
+// comparisons of 5,000 rows are microseconds over the whole chip, where one
+// CTA's bitonic sort took 114 us.
+__global__ void __launch_bounds__(kTkFinalThreads) k_tk_final(TkSample* st, bool nan_last_first, uint32_t k,
+                                                        const uint64_t* __restrict__ c_img,
+                                                        const uint32_t* __restrict__ c_row,
+                                                        int32_t* __restrict__ perm) {
+  extern __shared__ __align__(16) unsigned char tk_smem[];
+  const uint32_t cnt = st->count;
+  if (!st->ready || cnt < k || cnt > (uint32_t)kTkCap) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->status = 1u;
+    return;
+  }
+  uint64_t* si = reinterpret_cast<uint64_t*>(tk_smem);
+  uint32_t* sr = reinterpret_cast<uint32_t*>(si + kTkCap);
+#pragma unroll 4
+  for (uint32_t i = threadIdx.x; i < cnt; i += kTkFinalThreads) {
+    const uint64_t v = c_img[i];
+    const uint32_t r = c_row[i];
+    si[i] = v;
+    sr[i] = nan_last_first && v == 0ull ? ~r : r;
+  }
+  __syncthreads();
+  const uint32_t lane = lane_id();
+  for (uint32_t i = blockIdx.x + gridDim.x * (threadIdx.x >> 5); i < cnt;
+       i += gridDim.x * (kTkFinalThreads / 32)) {
+    const uint64_t v = si[i];
+    const uint32_t r = sr[i];
+    uint32_t before = 0;
+#pragma unroll 8
+    for (uint32_t j = lane; j < cnt; j += 32) {
+      const uint64_t w = si[j];
+      before += (w < v || (w == v && sr[j] < r)) ? 1u : 0u;
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0 && before < k) perm[before] = (int32_t)(nan_last_first && v == 0ull ? ~r : r);
+  }
+}
+
 unsigned tk_grid(int64_t n) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + kTkThreads - 1) / kTkThreads, (int64_t)num_sms() * 8));
 }
@@ -384,10 +641,69 @@ int tk_status(cudaStream_t s, const int32_t* d_err) {
   return h;
 }
 
+// Sample rank of the threshold when one group in `step` is sampled: it gets six standard deviations and 16 rows more
+// than k / step, so that the k-th row is missed about once in 1e8 calls on
+// rows that the sample represents (and the exact passes then run).
+int64_t tk_target(int64_t k, int64_t step) {
+  if (step == 1) return k;
+  const double q = (double)k / (double)step;
+  return (int64_t)(q + 6.0 * std::sqrt(q) + 16.0) + 1;
+}
+
+// The sampled form, for k small enough that its rows fit one CTA's sort.
+// *done = 0: not tried, or the threshold did not hold.
+template <int DT>
+int topk_sampled(const void* keys, const uint8_t* validity, int64_t n, bool desc, int64_t k, int32_t* perm_out,
+                 cudaStream_t s, int* done) {
+  *done = 0;
+  // About a million sampled rows at 64M (their histograms take a tenth of the
+  // pass), fewer groups skipped where k needs a sharper threshold.
+  int64_t step = std::min<int64_t>(64, std::max<int64_t>(1, n >> 20));
+  while (step > 1 && tk_target(k, step) * step > kTkExpect) step = step / 2;
+  if (tk_target(k, step) * step > kTkExpect || (step < 8 && n >= (1 << 24))) return NFC_OK;
+  Scratch sc(s);
+  TkSample* st = nullptr;
+  uint64_t* c_img = nullptr;
+  uint32_t* c_row = nullptr;
+  NFC_CUDA(sc.alloc(&st, 1));
+  NFC_CUDA(sc.alloc(&c_img, (size_t)kTkCap));
+  NFC_CUDA(sc.alloc(&c_row, (size_t)kTkCap));
+  NFC_CUDA(cudaMemsetAsync(st, 0, sizeof(TkSample), s));
+  const bool vec = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0;
+  const int bits = DT == NFC_I32 ? 32 : 64;
+  const unsigned gs = (unsigned)std::max<int64_t>(
+      1, std::min<int64_t>((n / 4 / step + 1023) / 1024, (int64_t)num_sms() * 4));
+  const uint32_t target = (uint32_t)tk_target(k, step);
+  for (int level = 0, shift = bits; level < kTkLevels && shift > 0; ++level) {
+    const int dbits = std::min(kTkDigitBits, shift);
+    shift -= dbits;
+    k_tk_sample<DT><<<gs, kTkThreads, 0, s>>>(keys, validity, n, vec, desc, level, shift, (1u << dbits) - 1u,
+                                              (uint32_t)step, target, st);
+    NFC_CUDA(cudaGetLastError());
+  }
+  const unsigned gc =
+      (unsigned)std::max<int64_t>(1, std::min<int64_t>((n / 16 + 255) / 256, (int64_t)num_sms() * 4));
+  k_tk_collect<DT><<<gc, kTkThreads, 0, s>>>(keys, validity, n, vec, desc, st, c_img, c_row);
+  NFC_CUDA(cudaGetLastError());
+  constexpr int smem = kTkCap * 12;
+  NFC_CUDA(cudaFuncSetAttribute(k_tk_final, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  k_tk_final<<<(unsigned)num_sms(), kTkFinalThreads, smem, s>>>(st, DT == NFC_F64 && desc, (uint32_t)k, c_img, c_row, perm_out);
+  NFC_CUDA(cudaGetLastError());
+  uint32_t status = 0;
+  NFC_CUDA(readback(&status, &st->status, sizeof(status), s));
+  *done = status == 0;
+  return NFC_OK;
+}
+
 template <int DT>
 int topk_impl(const void* keys, const uint8_t* validity, int64_t n, bool desc, int64_t k, int32_t* perm_out,
               cudaStream_t s) {
   using K = typename std::conditional<DT == NFC_I32, uint32_t, uint64_t>::type;
+  {
+    int done = 0;
+    const int rc = topk_sampled<DT>(keys, validity, n, desc, k, perm_out, s, &done);
+    if (rc || done) return rc;
+  }
   Scratch sc(s);
   int32_t* d_err = nullptr;
   uint32_t* hist = nullptr;
