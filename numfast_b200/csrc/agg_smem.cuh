@@ -221,4 +221,131 @@ NFC_DEV void agg_emit(const ColSet& cs, const AggState<NC>& st, int g, const Out
   }
 }
 
+// ---------------------------------------------------------------- hot keys
+// Rows of a key that takes a large share of a CTA's rows meet on one address:
+// every float64 sum and 64-bit min/max is then a serial chain.  Such a key
+// gets accumulators in every thread's registers instead (a compare and, on a
+// hit, plain arithmetic), reduced per warp and folded into its slot once.
+template <int NC>
+struct HotAcc {
+  uint32_t cnt;
+  uint64_t sum[NC > 0 ? NC : 1];
+  int32_t mn32[NC > 0 ? NC : 1], mx32[NC > 0 ? NC : 1];
+  uint64_t mn64[NC > 0 ? NC : 1], mx64[NC > 0 ? NC : 1];  // int64 as is, float64 as the ordered encodings
+};
+
+// Keys held in registers: as many as leave a 512-thread CTA its registers
+// (run-time column types need room for every type).
+template <int NC, uint32_t SIG>
+constexpr int hot_keys() { return SIG != 0 || NC <= 1 ? 4 : NC == 2 ? 2 : 1; }
+
+template <int NC, uint32_t SIG>
+NFC_DEV void hot_init(const ColSet& cs, HotAcc<NC>& a) {
+  a.cnt = 0u;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const bool i64 = col_dt<SIG>(cs, c) == NFC_I64;
+    a.sum[c] = 0ull;
+    a.mn32[c] = INT_MAX;
+    a.mx32[c] = INT_MIN;
+    a.mn64[c] = i64 ? (uint64_t)LLONG_MAX : ~0ull;
+    a.mx64[c] = i64 ? (uint64_t)LLONG_MIN : 0ull;
+  }
+}
+
+template <int NC, uint32_t SIG>
+NFC_DEV void hot_add(const ColSet& cs, HotAcc<NC>& a, const uint64_t* raw) {
+  ++a.cnt;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int dt = col_dt<SIG>(cs, c), ag = col_ag<SIG>(cs, c);
+    const uint64_t r = raw[c];
+    if (dt == NFC_I32) {
+      const int32_t v = (int32_t)(uint32_t)r;
+      if (ag & NFC_AGG_SUM) a.sum[c] += (uint64_t)(int64_t)v;
+      if (ag & NFC_AGG_MIN) a.mn32[c] = min(a.mn32[c], v);
+      if (ag & NFC_AGG_MAX) a.mx32[c] = max(a.mx32[c], v);
+    } else if (dt == NFC_I64) {
+      if (ag & NFC_AGG_SUM) a.sum[c] += r;
+      if (ag & NFC_AGG_MIN) a.mn64[c] = (uint64_t)min((long long)a.mn64[c], (long long)r);
+      if (ag & NFC_AGG_MAX) a.mx64[c] = (uint64_t)max((long long)a.mx64[c], (long long)r);
+    } else {
+      if (ag & NFC_AGG_SUM)
+        a.sum[c] = (uint64_t)__double_as_longlong(__longlong_as_double((long long)a.sum[c]) +
+                                                  __longlong_as_double((long long)r));
+      if (ag & NFC_AGG_MIN) a.mn64[c] = min(a.mn64[c], f64_min_enc(r));
+      if (ag & NFC_AGG_MAX) a.mx64[c] = max(a.mx64[c], f64_max_enc(r));
+    }
+  }
+}
+
+// Reduce one hot key over the warp and fold it into slot g (whole warp).
+template <int NC, uint32_t SIG>
+NFC_DEV void hot_flush(const ColSet& cs, const AggState<NC>& st, uint32_t g, const HotAcc<NC>& a) {
+  const uint32_t k = __reduce_add_sync(0xffffffffu, a.cnt);
+  if (k == 0u) return;
+  uint64_t sum[NC > 0 ? NC : 1], mn[NC > 0 ? NC : 1], mx[NC > 0 ? NC : 1];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int dt = col_dt<SIG>(cs, c), ag = col_ag<SIG>(cs, c);
+    uint64_t s = a.sum[c];
+    if (ag & NFC_AGG_SUM) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const uint64_t t = __shfl_xor_sync(0xffffffffu, s, o);
+        s = dt == NFC_F64 ? (uint64_t)__double_as_longlong(__longlong_as_double((long long)s) +
+                                                           __longlong_as_double((long long)t))
+                          : s + t;
+      }
+    }
+    sum[c] = s;
+    if (dt == NFC_I32) {
+      mn[c] = (uint64_t)(int64_t)__reduce_min_sync(0xffffffffu, a.mn32[c]);
+      mx[c] = (uint64_t)(int64_t)__reduce_max_sync(0xffffffffu, a.mx32[c]);
+    } else {
+      uint64_t lo = a.mn64[c], hi = a.mx64[c];
+      if (ag & (NFC_AGG_MIN | NFC_AGG_MAX)) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const uint64_t l2 = __shfl_xor_sync(0xffffffffu, lo, o), h2 = __shfl_xor_sync(0xffffffffu, hi, o);
+          if (dt == NFC_I64) {
+            lo = (uint64_t)min((long long)lo, (long long)l2);
+            hi = (uint64_t)max((long long)hi, (long long)h2);
+          } else {
+            lo = min(lo, l2);
+            hi = max(hi, h2);
+          }
+        }
+      }
+      mn[c] = lo;
+      mx[c] = hi;
+    }
+  }
+  if (lane_id() == 0) agg_apply_group<NC, SIG>(cs, st, g, k, sum, mn, mx);
+}
+
+// The up to H slots of [0, w) with the most rows counted so far, at least
+// `floor` rows each; 0xFFFFFFFF in the rest.  Whole block; red[33] is shared.
+// Slots below 2^16 and counts below 2^16.
+template <int H>
+NFC_DEV void pick_hot(const uint32_t* cnt, int w, uint32_t floor, uint32_t* red, uint32_t (&hot)[H]) {
+  uint32_t last = 0xFFFFFFFFu;
+#pragma unroll
+  for (int h = 0; h < H; ++h) {
+    uint32_t best = 0u;
+    for (int g = threadIdx.x; g < w; g += blockDim.x) {
+      const uint32_t v = (cnt[g] << 16) | (uint32_t)g;
+      if (v < last) best = max(best, v);
+    }
+    best = __reduce_max_sync(0xffffffffu, best);
+    if (lane_id() == 0) red[threadIdx.x >> 5] = best;
+    __syncthreads();
+    best = red[lane_id() < (blockDim.x >> 5) ? lane_id() : 0];
+    best = __reduce_max_sync(0xffffffffu, best);
+    __syncthreads();
+    hot[h] = (best >> 16) >= floor ? best & 0xFFFFu : 0xFFFFFFFFu;
+    last = best;
+  }
+}
+
 }  // namespace nfc
