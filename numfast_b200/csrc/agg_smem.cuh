@@ -79,6 +79,37 @@ NFC_DEV void agg_init(const ColSet& cs, const AggState<NC>& st, int g) {
   }
 }
 
+NFC_DEV void block_fill16(void* p, int vecs, uint64_t v) {
+  ulonglong2* q = static_cast<ulonglong2*>(p);
+  for (int i = threadIdx.x; i < vecs; i += blockDim.x) q[i] = make_ulonglong2(v, v);
+}
+
+// Identities of all w slots with 16-byte stores (whole block; w a multiple of
+// 4 and the state 16-byte aligned).  Slot by slot, eight 4- or 8-byte stores
+// per slot, the initialisation is a third of a bucket with a few hundred rows.
+template <int NC, uint32_t SIG>
+NFC_DEV void agg_init_all(const ColSet& cs, const AggState<NC>& st, int w) {
+  constexpr uint64_t kMax32 = 0x7FFFFFFF7FFFFFFFull, kMin32 = 0x8000000080000000ull;
+  block_fill16(st.cnt, w / 4, 0ull);
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int dt = col_dt<SIG>(cs, c), ag = col_ag<SIG>(cs, c);
+    if (dt == NFC_I32) {
+      if (ag & NFC_AGG_SUM) {
+        block_fill16(st.slo[c], w / 4, 0ull);
+        block_fill16(st.shi[c], w / 4, 0ull);
+      }
+      if (ag & NFC_AGG_MIN) block_fill16(st.mn[c], w / 4, kMax32);
+      if (ag & NFC_AGG_MAX) block_fill16(st.mx[c], w / 4, kMin32);
+    } else {
+      const bool i64 = dt == NFC_I64;
+      if (ag & NFC_AGG_SUM) block_fill16(st.s64[c], w / 2, 0ull);
+      if (ag & NFC_AGG_MIN) block_fill16(st.mn[c], w / 2, i64 ? (uint64_t)LLONG_MAX : ~0ull);
+      if (ag & NFC_AGG_MAX) block_fill16(st.mx[c], w / 2, i64 ? (uint64_t)LLONG_MIN : 0ull);
+    }
+  }
+}
+
 // READ_FIRST: min/max read the slot first and skip the atomic when the value
 // cannot win (the stored extreme only moves one way, so a value that does
 // not beat it now can never beat the final one).  That pays when slots see
@@ -234,10 +265,12 @@ struct HotAcc {
   uint64_t mn64[NC > 0 ? NC : 1], mx64[NC > 0 ? NC : 1];  // int64 as is, float64 as the ordered encodings
 };
 
-// Keys held in registers: as many as leave a 512-thread CTA its registers
-// (run-time column types need room for every type).
+// Keys held in registers: what two 512-thread CTAs per SM leave room for (the
+// slices of 69M Zipf(1.1) rows: four keys at one CTA per SM 1.04 ms, two keys at
+// two CTAs 0.76, four keys at two CTAs, spilled, 1.17).  Run-time column types
+// need room for every type.
 template <int NC, uint32_t SIG>
-constexpr int hot_keys() { return SIG != 0 || NC <= 1 ? 4 : NC == 2 ? 2 : 1; }
+constexpr int hot_keys() { return SIG != 0 || NC <= 1 ? 2 : 1; }
 
 template <int NC, uint32_t SIG>
 NFC_DEV void hot_init(const ColSet& cs, HotAcc<NC>& a) {

@@ -54,6 +54,11 @@ NFC_DEV void bulk_g2s_hint(void* dst, const void* src, uint32_t bytes, uint64_t*
       : "memory");
 }
 
+// Bring [p, p + bytes) into L2 (p and bytes multiples of 16).
+NFC_DEV void prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // 16- and 8-byte global stores with an L2 eviction policy.
 NFC_DEV void st_v2_u64_hint(uint64_t* p, uint64_t a, uint64_t b, uint64_t policy) {
   asm volatile("st.global.L2::cache_hint.v2.u64 [%0], {%1, %2}, %3;" ::"l"(p), "l"(a), "l"(b), "l"(policy) : "memory");

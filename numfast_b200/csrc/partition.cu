@@ -7,7 +7,7 @@
 //                  records, merge slots
 //   3. scatter     rows -> packed records in bucket order.  Aligned inputs:
 //                  pass 1 sends TMA-staged row tiles to coarse buckets of 64
-//                  fine ones, the refine pass splits the coarse buckets into
+//                  or 128 fine ones, the refine pass splits the coarse buckets into
 //                  fine ones; each tile is ranked by bucket in shared memory
 //                  and written as contiguous runs, one global reservation per
 //                  bucket and tile.  Otherwise one plain scatter pass (two
@@ -154,46 +154,73 @@ struct PartPlan {
   int64_t* offs;        // [nb+1] record offsets
   uint32_t* cursor;     // [nb]   scatter cursors
   int32_t* merge_slot;  // [nb]   merge-state slot of a bucket of several slices, else -1
-  int32_t* n_merge;     // [2]    merge slots, slices
+  int32_t* n_merge;     // [3]    merge slots, slices, skew (1: slices hold over a quarter of the records)
+  int2* multi;          // [max slices] per merge slot: its bucket, its first slice
   int2* slices;         // [max slices] (bucket, slice number)
 };
 
-__global__ void __launch_bounds__(1024) k_part_plan(const uint32_t* ghist, int32_t nb, int64_t slice,
-                                                    PartPlan pl) {
+// One CTA, counts staged in shared memory (nb words): global reads and writes
+// are coalesced and the whole plan is two block scans, thread t taking `per`
+// consecutive buckets.  (24,415 buckets: 66 us with a scan per 1,024 of them,
+// 54 us without the staging.)  Scanned together: records, then
+// slices << 15 | multi (n < 2^31: fewer than 2^16 slices, 2^15 buckets of
+// several).
+__global__ void __launch_bounds__(1024) k_part_plan(const uint32_t* __restrict__ ghist, int32_t nb, int64_t slice,
+                                                    int cshift, uint32_t* __restrict__ ccursor, PartPlan pl) {
+  extern __shared__ uint32_t s_off[];  // counts, then offsets
   __shared__ uint32_t s_scan[33];
-  __shared__ int64_t s_carry_off;
-  __shared__ int32_t s_carry_item, s_carry_merge;
-  if (threadIdx.x == 0) { s_carry_off = 0; s_carry_item = 0; s_carry_merge = 0; }
-  __syncthreads();
-  for (int64_t base = 0; base < nb; base += blockDim.x) {
-    const int64_t b = base + threadIdx.x;
-    const uint32_t h = b < nb ? ghist[b] : 0u;
-    const uint32_t items = h > slice ? (uint32_t)((h + slice - 1) / slice) : 0u;
-    const uint32_t multi = items > 0 ? 1u : 0u;
-    uint32_t t_off, t_items, t_multi;
-    const uint32_t e_off = block_excl_scan(h, s_scan, &t_off);
-    const uint32_t e_items = block_excl_scan(items, s_scan, &t_items);
-    const uint32_t e_multi = block_excl_scan(multi, s_scan, &t_multi);
-    if (b < nb) {
-      const int64_t off = s_carry_off + e_off;
-      pl.offs[b] = off;
-      pl.cursor[b] = (uint32_t)off;
-      pl.merge_slot[b] = multi ? s_carry_merge + (int32_t)e_multi : -1;
-      for (uint32_t i = 0; i < items; ++i)
-        pl.slices[s_carry_item + (int32_t)(e_items + i)] = make_int2((int32_t)b, (int32_t)i);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      s_carry_off += t_off;
-      s_carry_item += (int32_t)t_items;
-      s_carry_merge += (int32_t)t_multi;
-    }
-    __syncthreads();
+  const int32_t per = ((nb + (int32_t)blockDim.x - 1) / (int32_t)blockDim.x) | 1;  // odd: no bank conflicts
+  const int32_t b0 = min(nb, (int32_t)threadIdx.x * per), b1 = min(nb, b0 + per);
+  auto slices_of = [&](uint32_t h) { return h > slice ? (uint32_t)((h + slice - 1) / slice) : 0u; };
+#pragma unroll 4
+  for (int32_t b = threadIdx.x; b < nb; b += blockDim.x) {
+    s_off[b] = __ldg(ghist + b);
+    pl.merge_slot[b] = -1;
   }
+  __syncthreads();
+  uint32_t rows = 0, packed = 0, sliced = 0;
+  for (int32_t b = b0; b < b1; ++b) {
+    const uint32_t h = s_off[b], k = slices_of(h);
+    rows += h;
+    if (k) {
+      packed += k << 15 | 1u;
+      sliced += h;
+    }
+  }
+  uint32_t t_rows, t_packed, t_sliced;
+  uint32_t off = block_excl_scan(rows, s_scan, &t_rows);
+  uint32_t x = block_excl_scan(packed, s_scan, &t_packed);
+  block_excl_scan(sliced, s_scan, &t_sliced);
+  for (int32_t b = b0; b < b1; ++b) {
+    const uint32_t h = s_off[b], k = slices_of(h);
+    s_off[b] = off;
+    off += h;
+    if (k) {
+      pl.merge_slot[b] = (int32_t)(x & 0x7FFFu);
+      pl.multi[x & 0x7FFFu] = make_int2(b, (int32_t)(x >> 15));
+      x += k << 15 | 1u;
+    }
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int32_t b = threadIdx.x; b < nb; b += blockDim.x) {
+    const uint32_t o = s_off[b];
+    pl.offs[b] = o;
+    pl.cursor[b] = o;
+    if (ccursor && (b & ((1 << cshift) - 1)) == 0) ccursor[b >> cshift] = o;
+  }
+  const int32_t n_multi = (int32_t)(t_packed & 0x7FFFu), n_slices = (int32_t)(t_packed >> 15);
   if (threadIdx.x == 0) {
-    pl.offs[nb] = s_carry_off;
-    pl.n_merge[0] = s_carry_merge;
-    pl.n_merge[1] = s_carry_item;
+    pl.offs[nb] = t_rows;
+    pl.n_merge[0] = n_multi;
+    pl.n_merge[1] = n_slices;
+    pl.n_merge[2] = t_sliced > t_rows / 4 ? 1 : 0;
+  }
+  // The slices of each large bucket, a warp per bucket.
+  for (int32_t i = threadIdx.x >> 5; i < n_multi; i += blockDim.x >> 5) {
+    const int2 m = pl.multi[i];
+    const int32_t end = i + 1 < n_multi ? pl.multi[i + 1].y : n_slices;
+    for (int32_t j = m.y + (int32_t)lane_id(); j < end; j += 32) pl.slices[j] = make_int2(m.x, j - m.y);
   }
 }
 
@@ -352,11 +379,10 @@ __global__ void __launch_bounds__(kPartThreads, 2) k_part_scatter(const int32_t*
 // by bytes, so both scatter passes sort each tile by destination bucket in
 // shared memory and write the tile out in contiguous runs.  To keep runs
 // long the fan-out per pass stays <= 256: pass 1 sends rows to coarse
-// buckets (64 fine buckets each), pass 2 splits every coarse bucket into its
+// buckets (64 or 128 fine buckets each), pass 2 splits every coarse bucket into its
 // fine buckets.  Spans of at most 128 fine buckets need pass 1 only.
 // Each pass reserves a tile's range of a bucket with one global atomic.
 constexpr int kBulkTile = 2048;     // pass-1 rows per tile (TMA-staged)
-constexpr int kCoarseShift = 6;     // 64 fine buckets per coarse bucket
 constexpr int kMaxPassBins = 256;
 
 struct BulkLayout {
@@ -390,6 +416,29 @@ NFC_DEV uint32_t tile_reserve(const uint32_t* s_cnt, uint32_t* s_start, uint32_t
   return total;
 }
 
+// Rank of this lane's row in bucket `bin` of the tile (order within a bucket is
+// free); whole warp.  Under skewed keys most of a tile falls into one bucket
+// and its atomics run one after the other, so the rows of the warp that share
+// the first row's bucket take their places with one atomic.  That costs votes
+// and a shuffle on every row, hence the switch (100M rows, two passes: uniform
+// keys 1.15 ms without, 1.22 with; Zipf(1.1) keys 1.48 without, 1.32 with).
+NFC_DEV uint32_t tile_rank_skewed(uint32_t* s_cnt, uint32_t bin, bool ok) {
+  const unsigned act = __ballot_sync(0xffffffffu, ok);
+  const int first = act ? __ffs(act) - 1 : 0;
+  const uint32_t lead = __shfl_sync(0xffffffffu, bin, first);
+  const unsigned same = __ballot_sync(0xffffffffu, ok && bin == lead);
+  uint32_t r = 0;
+  if (__popc(same) >= 4) {  // the same for the whole warp
+    const bool mine = (same >> lane_id()) & 1u;
+    if ((int)lane_id() == first) r = atomicAdd(&s_cnt[bin], (uint32_t)__popc(same));
+    r = __shfl_sync(0xffffffffu, r, first) + (uint32_t)__popc(same & lanemask_lt());
+    if (ok && !mine) r = atomicAdd(&s_cnt[bin], 1u);
+  } else if (ok) {
+    r = atomicAdd(&s_cnt[bin], 1u);
+  }
+  return r;
+}
+
 // Pass 1: full tiles of kBulkTile rows, TMA-staged through a ring of
 // L.stages copies.  Each tile is ranked by bucket in shared memory as an
 // index permutation (no copy of the rows), reserves one range per bucket
@@ -404,7 +453,8 @@ __global__ void __launch_bounds__(kPartThreads, 2) k_part_pass1(const int32_t* _
                                                                int nbins, uint32_t keep_mask,
                                                                uint32_t* __restrict__ gcursor,
                                                                uint64_t* __restrict__ out, int32_t* err,
-                                                               uint32_t* gwide) {
+                                                               uint32_t* gwide, const int32_t* __restrict__ skew) {
+  const bool skewed = __ldg(skew) != 0;
   constexpr int NW = Rec<NC, PACK0>::NW;
   constexpr int kIter = kBulkTile / (4 * kPartThreads);
   uint32_t wide = 0;
@@ -465,9 +515,14 @@ __global__ void __launch_bounds__(kPartThreads, 2) k_part_pass1(const int32_t* _
       bin[j][0] = (uint32_t)((int64_t)kv.x - kmin) >> shift; bin[j][1] = (uint32_t)((int64_t)kv.y - kmin) >> shift;
       bin[j][2] = (uint32_t)((int64_t)kv.z - kmin) >> shift; bin[j][3] = (uint32_t)((int64_t)kv.w - kmin) >> shift;
       valid[j] = vmask ? (sv[i0 >> 5] >> (i0 & 31)) & 0xFu : 0xFu;
+      if (skewed) {
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
-        if (valid[j] & (1u << r)) rank[j][r] = atomicAdd(&s_cnt[bin[j][r]], 1u);
+        for (int r = 0; r < 4; ++r) rank[j][r] = tile_rank_skewed(s_cnt, bin[j][r], (valid[j] >> r) & 1u);
+      } else {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          if (valid[j] & (1u << r)) rank[j][r] = atomicAdd(&s_cnt[bin[j][r]], 1u);
+      }
     }
     __syncthreads();
     const uint32_t nvalid = tile_reserve(s_cnt, s_start, s_gbase, nbins, gcursor, s_scan);
@@ -537,22 +592,12 @@ __global__ void __launch_bounds__(kPartThreads) k_part_pass1_tail(const int32_t*
   publish_wide(wide, gwide);
 }
 
-// Pass-1 cursors and offsets of the coarse buckets (64 fine buckets each)
-// from the fine offsets.
-__global__ void k_part_plan2(const int64_t* offs, int32_t nb, int32_t nc, uint32_t* ccursor, int64_t* coffs) {
-  for (int32_t c = threadIdx.x; c <= nc; c += blockDim.x) {
-    const int64_t lo = offs[min((int64_t)c << kCoarseShift, (int64_t)nb)];
-    coffs[c] = lo;
-    if (c < nc) ccursor[c] = (uint32_t)lo;
-  }
-}
-
 // Pass 2, persistent form: the pass-1 output is cut into fixed tiles of
 // refine2_tile<NW>() records that stream into shared memory through a ring
 // of bulk-copy stages (the next tiles are in flight while one is split).
 // Pass 1 leaves the records in coarse-bucket order and a coarse bucket
-// covers 64 fine buckets, so a tile that touches at most four coarse
-// buckets spans at most 256 fine buckets: it is ranked by fine bucket in
+// covers 64 (128) fine buckets, so a tile that touches at most four (two)
+// coarse buckets spans at most 256 fine buckets: it is ranked by fine bucket in
 // shared memory (an index permutation, not a copy of the records), reserves
 // one range per fine bucket with one global atomic and writes each bucket's
 // records as a contiguous run.  A tile spanning more fine buckets (only when
@@ -570,7 +615,9 @@ constexpr size_t refine2_smem() {
 template <int NW>
 __global__ void __launch_bounds__(kPartThreads, 2) k_part_refine(const uint64_t* __restrict__ in, int64_t nv, int wb,
                                                                 uint32_t* __restrict__ fcursor,
-                                                                uint64_t* __restrict__ out, int32_t* err) {
+                                                                uint64_t* __restrict__ out, int32_t* err,
+                                                                const int32_t* __restrict__ skew) {
+  const bool skewed = __ldg(skew) != 0;
   constexpr int T = refine2_tile<NW>();
   constexpr int PER = T / kPartThreads;
   constexpr uint32_t kStageBytes = (uint32_t)T * NW * 8;
@@ -641,9 +688,15 @@ __global__ void __launch_bounds__(kPartThreads, 2) k_part_refine(const uint64_t*
     const uint32_t tlo = s_lo, thi = s_hi;
     if (thi - tlo < (uint32_t)kMaxPassBins) {
       uint32_t rank[PER];
+      if (skewed) {
 #pragma unroll
-      for (int u = 0; u < PER; ++u)
-        if (u * kPartThreads + tid < nrec) rank[u] = atomicAdd(&s_cnt[fb[u] - tlo], 1u);
+        for (int u = 0; u < PER; ++u)
+          rank[u] = tile_rank_skewed(s_cnt, fb[u] - tlo, u * kPartThreads + tid < nrec);
+      } else {
+#pragma unroll
+        for (int u = 0; u < PER; ++u)
+          if (u * kPartThreads + tid < nrec) rank[u] = atomicAdd(&s_cnt[fb[u] - tlo], 1u);
+      }
       __syncthreads();
       tile_reserve(s_cnt, s_start, s_gbase, (int)(thi - tlo + 1), fcursor + tlo, s_scan);
       __syncthreads();
@@ -730,32 +783,38 @@ struct PartAggArgs {
 };
 
 // Emit the present groups (count > 0) of bucket b in ascending key order.
-// Pass 1 counts them and places the bucket after its predecessors (decoupled
-// look-back); pass 2 walks the groups in rounds of blockDim, so consecutive
-// threads write consecutive output rows.
-template <int NC, uint32_t SIG, class CountF, class EmitF>
-NFC_DEV void part_emit(const PartAggArgs& a, int32_t b, int32_t wbk, int64_t key0, CountF cnt_of, EmitF emit,
-                       uint32_t* s_scan, int64_t* s_base) {
+// Warp w owns a run of consecutive slots and walks it in steps of 32, a step's
+// ballot giving each present group its place: two barriers per bucket (a block
+// scan per 512 slots took three each).  The bucket comes after its
+// predecessors by a decoupled look-back.
+template <class CountF, class EmitF>
+NFC_DEV void part_emit(const PartAggArgs& a, int32_t b, int32_t wbk, CountF cnt_of, EmitF emit, uint32_t* s_warp,
+                       int64_t* s_base) {
+  constexpr int kWarps = kPartThreads / 32;
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  const int per = ((wbk + kWarps - 1) / kWarps + 31) & ~31;
+  const int g0 = min(wbk, warp * per), g1 = min(wbk, g0 + per);
   uint32_t c = 0;
-  for (int g = threadIdx.x; g < wbk; g += blockDim.x) c += cnt_of(g) != 0u ? 1u : 0u;
-  uint32_t total;
-  block_excl_scan(c, s_scan, &total);
-  if (threadIdx.x < 32) {
+  for (int g = g0; g < g1; g += 32) c += __popc(__ballot_sync(0xffffffffu, g + lane < g1 && cnt_of(g + lane) != 0u));
+  if (lane == 0) s_warp[warp] = c;
+  __syncthreads();
+  if (warp == 0) {
+    const uint32_t total = __reduce_add_sync(0xffffffffu, lane < kWarps ? s_warp[lane] : 0u);
     const int64_t lbx = lookback_exclusive(a.lb, b, total, a.err);  // whole warp
-    if (threadIdx.x == 0) {
+    if (lane == 0) {
       *s_base = lbx;
-      if (b == a.nb - 1) *a.ng_out = *s_base + total;
+      if (b == a.nb - 1) *a.ng_out = lbx + total;
     }
   }
   __syncthreads();
-  int64_t base = *s_base;
-  for (int g0 = 0; g0 < wbk; g0 += blockDim.x) {
-    const int g = g0 + threadIdx.x;
-    const uint32_t pres = (g < wbk && cnt_of(g) != 0u) ? 1u : 0u;
-    uint32_t round_total;
-    const uint32_t excl = block_excl_scan(pres, s_scan, &round_total);
-    if (pres) emit(g, base + excl);
-    base += round_total;
+  int64_t pos = *s_base;
+  for (int w = 0; w < warp; ++w) pos += s_warp[w];
+  const unsigned lt = lanemask_lt();
+  for (int g = g0; g < g1; g += 32) {
+    const bool pres = g + lane < g1 && cnt_of(g + lane) != 0u;
+    const unsigned bal = __ballot_sync(0xffffffffu, pres);
+    if (pres) emit(g + lane, pos + __popc(bal & lt));
+    pos += __popc(bal);
   }
 }
 
@@ -800,10 +859,9 @@ NFC_DEV void for_records(const uint64_t* __restrict__ rp, int64_t i_lo, int64_t 
 // 50M domain the shared atomics on those keys made the aggregate 2.51 ms,
 // against 0.80 ms for the same rows of uniform keys.  The first records are
 // counted into the state, the keys with the largest counts then collect in
-// registers: 1.05 ms for these slices (69M of the rows) and 0.96 ms for the
-// other buckets.
+// registers.
 template <int NC, bool PACK0, uint32_t SIG>
-__global__ void __launch_bounds__(kPartThreads, 1) k_part_slices(PartAggArgs a) {
+__global__ void __launch_bounds__(kPartThreads, 2) k_part_slices(PartAggArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ uint32_t s_red[33];
   const int32_t W = 1 << a.wb;
@@ -818,7 +876,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) k_part_slices(PartAggArgs a) 
     const int32_t wbk = (int32_t)min((int64_t)W, a.m - ((int64_t)b << a.wb));
     const int64_t r_lo = a.offs[b] + (int64_t)sl.y * a.slice;
     const int64_t r_hi = min(a.offs[b + 1], r_lo + a.slice);
-    for (int g = threadIdx.x; g < wbk; g += blockDim.x) agg_init<NC, SIG>(a.cs, st, g);
+    agg_init_all<NC, SIG>(a.cs, st, W);
     __syncthreads();
     const uint64_t* rp = a.rec + (size_t)r_lo * NW;
     const int64_t nrec = r_hi - r_lo;
@@ -851,10 +909,14 @@ __global__ void __launch_bounds__(kPartThreads, 1) k_part_slices(PartAggArgs a) 
   }
 }
 
+// One CTA per bucket, claimed in order.  A persistent form that fetched its next
+// ticket and bounds ahead was slower on skewed keys (1.0-1.2 against 0.81 ms):
+// a CTA that holds a ticket while it works on a large bucket delays the
+// look-back of every bucket after it.
 template <int NC, bool PACK0, uint32_t SIG>
 __global__ void __launch_bounds__(kPartThreads, 2) k_part_agg(PartAggArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ uint32_t s_scan[33];
+  __shared__ uint32_t s_warp[kPartThreads / 32];
   __shared__ int64_t s_base;
   __shared__ int32_t s_bucket;
   if (threadIdx.x == 0) s_bucket = (int32_t)atomicAdd(a.ticket, 1u);
@@ -868,21 +930,19 @@ __global__ void __launch_bounds__(kPartThreads, 2) k_part_agg(PartAggArgs a) {
   const int32_t ms = a.merge_slot[b];
   if (ms >= 0) {  // its slices are merged in the global state
     const int64_t m0 = (int64_t)ms * W;
-    part_emit<NC, SIG>(a, b, wbk, key0, [&](int g) { return a.gm.cnt[m0 + g]; },
-                       [&](int g, int64_t pos) { state_emit(a.cs, a.gm, m0 + g, a.o, pos, key0 + g); }, s_scan,
-                       &s_base);
+    part_emit(a, b, wbk, [&](int g) { return a.gm.cnt[m0 + g]; },
+              [&](int g, int64_t pos) { state_emit(a.cs, a.gm, m0 + g, a.o, pos, key0 + g); }, s_warp, &s_base);
     return;
   }
   const int64_t r_lo = a.offs[b];
   const AggState<NC> st = carve_agg<NC, SIG>(a.cs, smem_raw, W, ~__ldg(a.wide));
-  for (int g = threadIdx.x; g < wbk; g += blockDim.x) agg_init<NC, SIG>(a.cs, st, g);
+  agg_init_all<NC, SIG>(a.cs, st, W);
   __syncthreads();
   for_records<NC, PACK0, U>(a.rec + (size_t)r_lo * NW, 0, a.offs[b + 1] - r_lo,
                             [&](uint32_t g, const uint64_t* raw) { agg_apply<NC, SIG, false>(a.cs, st, g, raw); });
   __syncthreads();
-  part_emit<NC, SIG>(a, b, wbk, key0, [&](int g) { return st.cnt[g]; },
-                     [&](int g, int64_t pos) { agg_emit<NC, SIG>(a.cs, st, g, a.o, pos, key0 + g); }, s_scan,
-                     &s_base);
+  part_emit(a, b, wbk, [&](int g) { return st.cnt[g]; },
+            [&](int g, int64_t pos) { agg_emit<NC, SIG>(a.cs, st, g, a.o, pos, key0 + g); }, s_warp, &s_base);
 }
 
 __global__ void k_merge_init(ColSet cs, StateRef gm, const int32_t* n_merge, int64_t w) {
@@ -892,13 +952,16 @@ __global__ void k_merge_init(ColSet cs, StateRef gm, const int32_t* n_merge, int
 }
 
 // ---------------------------------------------------------------- host
-constexpr int64_t kMaxBuckets = 16384;
+constexpr int64_t kMaxBuckets = 28672;  // two shared 32-bit tables of them in the plain scatter
+constexpr int64_t kMaxWideBuckets = 16384;
 constexpr int64_t kSlice = 65536;  // <= 65536 keeps the 16-bit-split int32 sums exact
 constexpr size_t kAggSmemBudget = 200 * 1024;
 
 // Bucket width: the widest whose shared-memory state leaves room for two
 // aggregate CTAs per SM (twice the warps to hide shared-atomic latency); if
-// that needs more than kMaxBuckets buckets, the widest one CTA can hold.
+// that needs more than kMaxBuckets buckets, the widest one CTA can hold, up to
+// kMaxWideBuckets of them.  (Zipf keys over a 50M domain, 100M rows: 24,415
+// buckets of 2,048 keys against 12,208 of 4,096.)
 constexpr size_t kAggSmemBudget2 = 110 * 1024;
 int pick_partition_width(size_t slot_bytes, int64_t m, int* wb_out) {
   for (const size_t budget : {kAggSmemBudget2, kAggSmemBudget}) {
@@ -906,7 +969,7 @@ int pick_partition_width(size_t slot_bytes, int64_t m, int* wb_out) {
     while (wb > 8 && ((size_t)1 << wb) * slot_bytes > budget) --wb;
     if (((size_t)1 << wb) * slot_bytes > budget) continue;
     const int64_t nb = (m + (1ll << wb) - 1) >> wb;
-    if (nb <= kMaxBuckets) {
+    if (nb <= (budget == kAggSmemBudget2 ? kMaxBuckets : kMaxWideBuckets)) {
       *wb_out = wb;
       return 0;
     }
@@ -927,8 +990,8 @@ struct PartLaunch {
   int64_t nfull;
   int32_t nc;         // coarse buckets (== nb when one level suffices)
   bool two_level;
+  int cshift;         // log2 of the fine buckets in a coarse one
   uint32_t* ccursor;  // coarse cursors [nc]
-  int64_t* coffs;     // [nc+1]
   uint32_t* cursor;   // fine cursors [nb]
   uint64_t* rec_a;    // pass-1 output (two-level)
   uint64_t* rec;      // fine-bucket records (aggregate input)
@@ -944,7 +1007,7 @@ static int launch_part(const PartLaunch& q, PartAggArgs& pa, cudaStream_t s, Sta
   const nfc_groupby_args* a = q.a;
   constexpr int NW = Rec<NC, PACK0>::NW;
   if (q.coalesced) {
-    const int shift = q.two_level ? q.wb + kCoarseShift : q.wb;
+    const int shift = q.two_level ? q.wb + q.cshift : q.wb;
     const uint32_t keep = q.two_level ? 0xFFFFFFFFu : (1u << q.wb) - 1u;
     uint32_t* cur1 = q.two_level ? q.ccursor : q.cursor;
     uint64_t* out1 = q.two_level ? q.rec_a : q.rec;
@@ -956,7 +1019,7 @@ static int launch_part(const PartLaunch& q, PartAggArgs& pa, cudaStream_t s, Sta
       const int64_t g = std::max<int64_t>(1, std::min<int64_t>(q.nfull, (int64_t)num_sms() * per_sm));
       k_part_pass1<NC, PACK0, SIG><<<(unsigned)g, kPartThreads, smem, s>>>(a->keys, q.vmask, q.cs, q.L, q.nfull,
                                                                           q.kmin, shift, q.nc, keep, cur1, out1,
-                                                                          q.d_err, q.wide);
+                                                                          q.d_err, q.wide, pa.n_merge + 2);
       NFC_CUDA(cudaGetLastError());
       tm->launched();
     }
@@ -972,7 +1035,8 @@ static int launch_part(const PartLaunch& q, PartAggArgs& pa, cudaStream_t s, Sta
       NFC_CUDA(cudaFuncSetAttribute(k_part_refine<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
       const int64_t nt2 = (q.nv + refine2_tile<NW>() - 1) / refine2_tile<NW>();
       const int64_t g2 = std::max<int64_t>(1, std::min<int64_t>(nt2, (int64_t)num_sms() * 2));
-      k_part_refine<NW><<<(unsigned)g2, kPartThreads, smem2, s>>>(q.rec_a, q.nv, q.wb, q.cursor, q.rec, q.d_err);
+      k_part_refine<NW><<<(unsigned)g2, kPartThreads, smem2, s>>>(q.rec_a, q.nv, q.wb, q.cursor, q.rec, q.d_err,
+                                                              pa.n_merge + 2);
       NFC_CUDA(cudaGetLastError());
       tm->launched();
     }
@@ -994,7 +1058,7 @@ static int launch_part(const PartLaunch& q, PartAggArgs& pa, cudaStream_t s, Sta
   if (q.max_slices > 0) {
     NFC_CUDA(cudaFuncSetAttribute(k_part_slices<NC, PACK0, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)q.agg_smem));
-    k_part_slices<NC, PACK0, SIG><<<(unsigned)std::min<int64_t>(q.max_slices, num_sms()), kPartThreads, q.agg_smem,
+    k_part_slices<NC, PACK0, SIG><<<(unsigned)std::min<int64_t>(q.max_slices, num_sms() * 2), kPartThreads, q.agg_smem,
                                      s>>>(pa);
     NFC_CUDA(cudaGetLastError());
     tm->launched();
@@ -1068,7 +1132,10 @@ int run_partition(const nfc_groupby_args* a, const ColSet& cs_in, const OutSet& 
   q.d_err = d_err;
   q.nv = p.n_valid;
   q.two_level = nb > 128;
-  q.nc = q.two_level ? (int32_t)((nb + (1 << kCoarseShift) - 1) >> kCoarseShift) : nb;
+  // 64 fine buckets per coarse one, 128 where that would make the first
+  // pass's fan-out too wide.
+  q.cshift = nb <= (kMaxPassBins << 6) ? 6 : 7;
+  q.nc = q.two_level ? (int32_t)((nb + (1 << q.cshift) - 1) >> q.cshift) : nb;
   // Coalesced scatter: 16-byte aligned inputs, coarse fan-out <= kMaxPassBins,
   // TMA stages + the tile's sort buffer fit in shared memory.
   if (q.al && (reinterpret_cast<uintptr_t>(vmask) & 15u) == 0 && q.nc <= kMaxPassBins) {
@@ -1105,19 +1172,17 @@ int run_partition(const nfc_groupby_args* a, const ColSet& cs_in, const OutSet& 
   unsigned char* small = nullptr;
   const size_t nbp = (size_t)nb + 1;
   const size_t ncp = (size_t)q.nc + 1;
-  const size_t small_bytes = nbp * (4 + 8 + 4 + 4 + 8) + ncp * (4 + 8 + 4) + 128;
+  const size_t small_bytes = nbp * (4 + 8 + 4 + 4 + 8) + ncp * 4 + 128;
   NFC_CUDA(sc.alloc(&small, small_bytes));
   NFC_CUDA(cudaMemsetAsync(small, 0, small_bytes, s));
   unsigned char* qq = small;
   w.offs = reinterpret_cast<int64_t*>(qq); qq += 8 * nbp;
   w.lb = reinterpret_cast<uint64_t*>(qq); qq += 8 * nbp;
-  q.coffs = reinterpret_cast<int64_t*>(qq); qq += 8 * ncp;
   w.ghist = reinterpret_cast<uint32_t*>(qq); qq += 4 * nbp;
   w.cursor = reinterpret_cast<uint32_t*>(qq); qq += 4 * nbp;
   w.merge_slot = reinterpret_cast<int32_t*>(qq); qq += 4 * nbp;
   q.ccursor = reinterpret_cast<uint32_t*>(qq); qq += 4 * ncp;
-  qq += 4 * ncp;
-  w.n_merge = reinterpret_cast<int32_t*>(qq); qq += 8;
+  w.n_merge = reinterpret_cast<int32_t*>(qq); qq += 12;
   w.ticket = reinterpret_cast<uint32_t*>(qq); qq += 8;
   q.wide = reinterpret_cast<uint32_t*>(qq); qq += 8;
   q.cursor = w.cursor;
@@ -1154,15 +1219,13 @@ int run_partition(const nfc_groupby_args* a, const ColSet& cs_in, const OutSet& 
   // of them.
   const int64_t max_slices = nv > kSlice ? 2 * (nv / kSlice) : 0;
   int2* slices = nullptr;
-  NFC_CUDA(sc.alloc(&slices, (size_t)std::max<int64_t>(max_slices, 1)));
-  PartPlan pl{w.offs, w.cursor, w.merge_slot, w.n_merge, slices};
-  k_part_plan<<<1, 1024, 0, s>>>(w.ghist, nb, kSlice, pl);
+  NFC_CUDA(sc.alloc(&slices, (size_t)std::max<int64_t>(2 * max_slices, 1)));
+  PartPlan pl{w.offs, w.cursor, w.merge_slot, w.n_merge, slices + max_slices, slices};
+  NFC_CUDA(cudaFuncSetAttribute(k_part_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(nb * 4)));
+  k_part_plan<<<1, 1024, (size_t)nb * 4, s>>>(w.ghist, nb, kSlice, q.cshift, q.two_level ? q.ccursor : nullptr, pl);
   NFC_CUDA(cudaGetLastError());
   tm->launched();
   if (q.coalesced && q.two_level) {
-    k_part_plan2<<<1, 1024, 0, s>>>(w.offs, nb, q.nc, q.ccursor, q.coffs);
-    NFC_CUDA(cudaGetLastError());
-    tm->launched();
     NFC_CUDA(sc.alloc(&q.rec_a, (size_t)std::max<int64_t>(nv, 1) * nw + 2));  // +2: 16-byte tail of the refine copies
   }
   tm->mark(s);
