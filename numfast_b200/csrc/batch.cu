@@ -44,6 +44,7 @@ constexpr int kBWarps = kBThreads / 32;
 constexpr int kBPer = 16;                    // rows per thread per sub-tile
 constexpr int kBSub = kBThreads * kBPer;     // 8192 rows per sub-tile
 constexpr int kBEmitRound = kBThreads * 4;   // slots per emit round
+constexpr int kSoloSlack = 16384;            // span a solo query may have above four slots per row
 
 enum : uint32_t { kItProbe = 0, kItSolo = 1, kItAgg = 2, kItEmit = 3 };
 
@@ -716,7 +717,7 @@ NFC_DEV void do_solo(const BatchParams& P, BSmem& S, uint32_t* s_cnt, int32_t* s
     int64_t ob = -1, off = 0;
     if (in_smem) {
       ob = reserve(&P.hdr->out_cursor, imin64(cnt, span), P.out_cap);
-    } else if (span <= 4 * qd.rows + P.smem_slots) {
+    } else if (span <= 4 * qd.rows + imax64(P.smem_slots, kSoloSlack)) {
       // Too wide for the shared table: packed global state in the arena,
       // still finished by this CTA alone.
       off = reserve(&P.hdr->arena_cursor, (span + 3) & ~3ll, P.arena_words);
@@ -912,17 +913,24 @@ void batch_free(nfc_batch* b) {
   delete b;
 }
 
+// Picked on mixed batches of 40 to 512 queries of 1K..4M rows.  The emit items
+// come last and a large query's eight slices of up to 512K slots left most of
+// the chip idle; slices of 16K slots halve the launch (512 queries, 253M rows:
+// 2.75 -> 1.58 ms; 40 queries: 0.76 -> 0.37).  Two CTAs per SM with the
+// shared-memory cache in front of the global state (warp_agg 3) take 3.1 ms of
+// the one-CTA, match_any form to 2.75.  Finer slices lose on large batches
+// (4K slots: 2.02 ms).
 void default_tuning(nfc_batch_tuning* t) {
   t->solo_rows = 32768;
   t->chunk_rows = 65536;
   t->probe_rows = 262144;
-  t->emit_slice = 65536;
-  t->emit_max_items = 8;
-  t->smem_slots = 16384;
+  t->emit_slice = 16384;
+  t->emit_max_items = 64;
+  t->smem_slots = 8192;
   t->smem_span_div = 2;
-  t->warp_agg = 1;
-  t->ctas_per_sm = 1;
-  t->schedule = 0;
+  t->warp_agg = 3;
+  t->ctas_per_sm = 2;
+  t->schedule = 2;
   t->agg_split = 0;
   t->arena_bytes = 0;
 }
@@ -1063,11 +1071,15 @@ extern "C" nfc_batch* nfc_batch_create(int64_t nq, const int64_t* row_offsets, c
   b->n_items = (int64_t)items.size();
   for (uint64_t it : items) b->counts_by_type[it >> 62]++;
   // Arena default: 2 bytes per row (at least 256 MiB), never more than every
-  // non-solo query's largest accepted span nor a quarter of free memory.  A
-  // query whose span does not fit in what is left is deferred.
+  // query's largest accepted span (a solo query's only where the shared table
+  // cannot hold it) nor a quarter of free memory.  A query whose span does not
+  // fit in what is left is deferred.
   int64_t want = 0;
-  for (const QDesc& d : b->hqd)
-    if (!d.solo) want += ((int64_t)d.n_emit * d.emit_slice + 3) & ~3ll;
+  for (const QDesc& d : b->hqd) {
+    const int64_t span = d.solo ? 4 * d.rows + std::max<int64_t>(t.smem_slots, kSoloSlack)
+                                : (int64_t)d.n_emit * d.emit_slice;
+    if (!d.solo || span > t.smem_slots) want += (span + 3) & ~3ll;
+  }
   size_t free_b = 0, total_b = 0;
   cudaMemGetInfo(&free_b, &total_b);
   int64_t words = t.arena_bytes ? t.arena_bytes / 8
