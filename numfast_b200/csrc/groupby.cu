@@ -30,6 +30,7 @@
 #include "agg_smem.cuh"
 #include "groupby_core.cuh"
 #include "groupby_host.h"
+#include "probe.cuh"
 
 namespace nfc {
 
@@ -43,25 +44,6 @@ namespace nfc {
 // bitmaps one 32-bit word per lane (lane l = rows [32l, 32l+32), which is
 // also the combined validity word it writes); each group takes its 4-bit
 // validity from the word's owner lane by a shuffle.
-
-struct BitmapSet {
-  int32_t nbm;
-  uint32_t word_aligned;  // bit b: bitmap b is 4-byte aligned
-  const uint8_t* bm[NFC_MAX_COLS + 2];  // key, columns, row filter
-};
-
-// Validity bits of rows [row0, row0+32) (row0 multiple of 32); only the
-// bitmap bytes that cover rows < n are read.
-NFC_DEV uint32_t bitmap_word(const uint8_t* bm, bool aligned4, int64_t row0, int64_t rem) {
-  const uint8_t* p = bm + (row0 >> 3);
-  if (rem >= 32) {
-    if (aligned4) return __ldg(reinterpret_cast<const uint32_t*>(p));
-    return (uint32_t)p[0] | ((uint32_t)p[1] << 8) | ((uint32_t)p[2] << 16) | ((uint32_t)p[3] << 24);
-  }
-  uint32_t w = 0;
-  for (int i = 0; i < (int)((rem + 7) >> 3); ++i) w |= (uint32_t)p[i] << (8 * i);
-  return w;
-}
 
 // In-order merge of two span records (row order a then b).
 NFC_DEV ProbeRec probe_rec_merge(const ProbeRec& a, const ProbeRec& b) {
@@ -223,47 +205,6 @@ __global__ void __launch_bounds__(256, 4) k_probe(const int32_t* __restrict__ ke
     }
     __syncthreads();
   }
-}
-
-struct ProbeAcc {
-  bool has, sorted;
-  int32_t first, last, kmin, kmax;
-  int64_t n;
-};
-
-NFC_DEV ProbeAcc probe_combine(const ProbeAcc& a, const ProbeAcc& b) {
-  ProbeAcc r;
-  r.has = a.has || b.has;
-  r.sorted = a.sorted && b.sorted && !(a.has && b.has && b.first < a.last);
-  r.first = a.has ? a.first : b.first;
-  r.last = b.has ? b.last : a.last;
-  r.kmin = min(a.kmin, b.kmin);
-  r.kmax = max(a.kmax, b.kmax);
-  r.n = a.n + b.n;
-  return r;
-}
-
-NFC_DEV ProbeAcc probe_shfl_down(const ProbeAcc& a, int off) {
-  ProbeAcc r;
-  r.has = __shfl_down_sync(0xffffffffu, (int)a.has, off) != 0;
-  r.sorted = __shfl_down_sync(0xffffffffu, (int)a.sorted, off) != 0;
-  r.first = __shfl_down_sync(0xffffffffu, a.first, off);
-  r.last = __shfl_down_sync(0xffffffffu, a.last, off);
-  r.kmin = __shfl_down_sync(0xffffffffu, a.kmin, off);
-  r.kmax = __shfl_down_sync(0xffffffffu, a.kmax, off);
-  r.n = __shfl_down_sync(0xffffffffu, a.n, off);
-  return r;
-}
-
-// In-order reduction of a warp's accumulators (lane order = row order).
-NFC_DEV ProbeAcc probe_warp_reduce(ProbeAcc acc) {
-  const int lane = lane_id();
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const ProbeAcc other = probe_shfl_down(acc, off);
-    if ((lane & (2 * off - 1)) == 0) acc = probe_combine(acc, other);
-  }
-  return acc;
 }
 
 // One block of 1024 threads reduces the span records in row order: warp w
@@ -487,15 +428,7 @@ bool inputs_aligned(const nfc_groupby_args* a) {
 int run_probe(const nfc_groupby_args* a, cudaStream_t s, Scratch& sc, uint32_t** vmask_out,
               nfc_probe* host_probe, StageTimer* tm, const ProbeRec** recs_out) {
   const int64_t n = a->n;
-  BitmapSet bms{};
-  bms.nbm = 0;
-  bms.word_aligned = 0;
-  if (a->key_validity) bms.bm[bms.nbm++] = a->key_validity;
-  for (int c = 0; c < a->ncols; ++c)
-    if (a->cols[c].validity) bms.bm[bms.nbm++] = a->cols[c].validity;
-  if (a->row_filter) bms.bm[bms.nbm++] = a->row_filter;
-  for (int b = 0; b < bms.nbm; ++b)
-    if ((reinterpret_cast<uintptr_t>(bms.bm[b]) & 3u) == 0) bms.word_aligned |= 1u << b;
+  const BitmapSet bms = bitmaps_of(a);
   uint32_t* vmask = nullptr;
   if (bms.nbm > 0) NFC_CUDA(sc.alloc(&vmask, (size_t)((n + 31) / 32 + 1)));
   const int64_t nspans = (n + kProbeSpan - 1) / kProbeSpan;
@@ -654,7 +587,15 @@ int64_t nfc::groupby_run(const nfc_groupby_args* a, int32_t strategy, PlanHook* 
   uint32_t* vmask = nullptr;
   nfc_probe p;
   const ProbeRec* recs = nullptr;
-  rc = run_probe(a, s, sc, &vmask, &p, &tm, &recs);
+  SmallResult small{};
+  // The library's own rule only: a forced strategy or a planner's pick runs as
+  // asked.
+  rc = NFC_ERR_UNSUPPORTED;
+  if (strategy == NFC_STRAT_AUTO && !hook && a->n > 0 && a->n <= kSmallRows) {
+    rc = run_small(a, cs, o, s, sc, &vmask, &recs, &small, &tm);
+    p = small.probe;
+  }
+  if (rc == NFC_ERR_UNSUPPORTED) rc = run_probe(a, s, sc, &vmask, &p, &tm, &recs);
   if (rc) return rc;
   int strat = strategy == NFC_STRAT_AUTO ? plan_strategy(cs, p) : strategy;
   int64_t hint = stats ? stats->distinct_hint : 0;
@@ -672,6 +613,13 @@ int64_t nfc::groupby_run(const nfc_groupby_args* a, int32_t strategy, PlanHook* 
     stats->nstages = 0;
   }
   if (p.n_valid == 0) return 0;
+  if (small.done) {
+    if (stats) {
+      stats->ng = small.ng;
+      stats->nstages = tm.finish(stats->stage_ms);
+    }
+    return small.ng;
+  }
   const int64_t m = p.kmax - p.kmin + 1;
   const int64_t ng_bound = std::min<int64_t>(m, p.n_valid);
   if (a->out_cap < ng_bound && a->out_cap < p.n_valid) {
@@ -831,15 +779,7 @@ extern "C" int64_t nfc_groupby_dense_noalloc(const nfc_groupby_args* a, void* st
   unsigned char* state = base + kNaState;
 
   // Probe: n_valid, kmin/kmax and the combined validity bitmap.
-  BitmapSet bms{};
-  bms.nbm = 0;
-  bms.word_aligned = 0;
-  if (a->key_validity) bms.bm[bms.nbm++] = a->key_validity;
-  for (int c = 0; c < a->ncols; ++c)
-    if (a->cols[c].validity) bms.bm[bms.nbm++] = a->cols[c].validity;
-  if (a->row_filter) bms.bm[bms.nbm++] = a->row_filter;
-  for (int b = 0; b < bms.nbm; ++b)
-    if ((reinterpret_cast<uintptr_t>(bms.bm[b]) & 3u) == 0) bms.word_aligned |= 1u << b;
+  const BitmapSet bms = bitmaps_of(a);
   uint32_t* vmask = bms.nbm > 0 ? vmask_buf : nullptr;
   NFC_CUDA(cudaMemsetAsync(base + kNaHdr, 0, 256, s));
   const int64_t nspans = (a->n + kProbeSpan - 1) / kProbeSpan;

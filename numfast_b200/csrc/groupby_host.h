@@ -63,6 +63,18 @@ int run_probe(const nfc_groupby_args* a, cudaStream_t s, Scratch& sc, uint32_t**
               nfc_probe* host_probe, StageTimer* tm, const ProbeRec** recs_out = nullptr);
 int plan_strategy(const ColSet& cs, const nfc_probe& p);
 
+// Small inputs (small.cu), n in [1, kSmallRows]: the probe and, if the key
+// span fits, the whole group-by in one launch.  done 0: only the probe, whose
+// bitmap and record the strategies then use.  NFC_ERR_UNSUPPORTED: nothing ran.
+constexpr int64_t kSmallRows = kProbeBlockRows;
+struct SmallResult {
+  nfc_probe probe;
+  int64_t ng;
+  int32_t done;
+};
+int run_small(const nfc_groupby_args* a, const ColSet& cs, const OutSet& o, cudaStream_t s, Scratch& sc,
+              uint32_t** vmask_out, const ProbeRec** recs_out, SmallResult* out, StageTimer* tm);
+
 // PARTITION strategy (partition.cu).
 int pick_partition_width(size_t slot_bytes, int64_t m, int* wb_out);
 int run_partition(const nfc_groupby_args* a, const ColSet& cs, const OutSet& o, const nfc_probe& p,
