@@ -231,6 +231,56 @@ NFC_DEV void agg_merge(const ColSet& cs, const StateRef& dst, int64_t d, const A
   }
 }
 
+// Entry e of an interleaved state (slot e >> lg of copy e & (2^lg - 1)): the
+// lanes of a group of 2^lg combine their copies and the first one folds the
+// slot into the global state.  Whole warp; lanes at or past `entries` add
+// nothing (entries is a multiple of the group).
+template <int NC, uint32_t SIG>
+NFC_DEV void agg_merge_copies(const ColSet& cs, const StateRef& dst, const AggState<NC>& st, int e, int entries,
+                              int lg) {
+  const bool in = e < entries;
+  uint32_t k = in ? st.cnt[e] : 0u;
+  for (int o = 1; o < (1 << lg); o <<= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
+  uint64_t sum[NC > 0 ? NC : 1], mn[NC > 0 ? NC : 1], mx[NC > 0 ? NC : 1];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int dt = col_dt<SIG>(cs, c), ag = col_ag<SIG>(cs, c);
+    uint64_t s = 0, lo = 0, hi = 0;
+    if (ag & NFC_AGG_SUM) {
+      s = in ? (uint64_t)agg_sum_bits<NC, SIG>(cs, st, c, e) : 0ull;
+      for (int o = 1; o < (1 << lg); o <<= 1) {
+        const uint64_t t = __shfl_xor_sync(0xffffffffu, s, o);
+        s = dt == NFC_F64 ? (uint64_t)__double_as_longlong(__longlong_as_double((long long)s) +
+                                                           __longlong_as_double((long long)t))
+                          : s + t;
+      }
+    }
+    // Minima and maxima as int64, float64 as the ordered encodings.
+    if (ag & NFC_AGG_MIN) {
+      lo = dt == NFC_F64 ? ~0ull : (uint64_t)LLONG_MAX;
+      if (in) lo = dt == NFC_I32 ? (uint64_t)(int64_t) static_cast<const int32_t*>(st.mn[c])[e]
+                                 : static_cast<const uint64_t*>(st.mn[c])[e];
+      for (int o = 1; o < (1 << lg); o <<= 1) {
+        const uint64_t t = __shfl_xor_sync(0xffffffffu, lo, o);
+        lo = dt == NFC_F64 ? min(lo, t) : (uint64_t)min((long long)lo, (long long)t);
+      }
+    }
+    if (ag & NFC_AGG_MAX) {
+      hi = dt == NFC_F64 ? 0ull : (uint64_t)LLONG_MIN;
+      if (in) hi = dt == NFC_I32 ? (uint64_t)(int64_t) static_cast<const int32_t*>(st.mx[c])[e]
+                                 : static_cast<const uint64_t*>(st.mx[c])[e];
+      for (int o = 1; o < (1 << lg); o <<= 1) {
+        const uint64_t t = __shfl_xor_sync(0xffffffffu, hi, o);
+        hi = dt == NFC_F64 ? max(hi, t) : (uint64_t)max((long long)hi, (long long)t);
+      }
+    }
+    sum[c] = s;
+    mn[c] = lo;
+    mx[c] = hi;
+  }
+  if (in && k && (lane_id() & ((1u << lg) - 1u)) == 0u) state_apply_group(cs, dst, e >> lg, k, sum, mn, mx);
+}
+
 template <int NC, uint32_t SIG>
 NFC_DEV void agg_emit(const ColSet& cs, const AggState<NC>& st, int g, const OutSet& o, int64_t pos, int64_t key) {
   o.ukeys[pos] = key;

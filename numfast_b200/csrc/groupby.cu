@@ -10,9 +10,9 @@
 //   * a key whose every row is invalid is absent (no NULL group).
 //
 // Strategies (all give the same integers; float sums within 1e-12 rel):
-//   DENSE_SMEM   span M fits one CTA's shared memory: each CTA folds a
-//                65,536-row chunk into the whole state on chip and merges it
-//                into a global table.
+//   DENSE_SMEM   span M fits one CTA's shared memory: each CTA folds a chunk of
+//                at most 65,536 rows into the whole state on chip and merges
+//                it into a global table.
 //   DENSE_GLOBAL span fits L2 and the input is small: rows update one global
 //                table with atomics.
 //   PARTITION    large span (or many rows): rows are scattered into
@@ -209,8 +209,26 @@ __global__ void __launch_bounds__(256, 4) k_probe(const int32_t* __restrict__ ke
 
 // One block of 1024 threads reduces the span records in row order: warp w
 // owns a contiguous range and walks it in coalesced windows of 32 records.
-__global__ void __launch_bounds__(1024) k_probe_finalize(const ProbeRec* recs, int64_t nspans, nfc_probe* out) {
+// With keys given it also samples 1,024 rows at even distances: out->pad is the
+// largest number of them in one slot of a 4,096-slot table, which is a few for
+// even key frequencies and the share of the hottest key (of 1,024) otherwise.
+__global__ void __launch_bounds__(1024) k_probe_finalize(const ProbeRec* recs, int64_t nspans, nfc_probe* out,
+                                                         const int32_t* __restrict__ keys,
+                                                         const uint32_t* __restrict__ vmask, int64_t n) {
   __shared__ ProbeAcc part[32];
+  __shared__ uint32_t s_slot[4096];
+  __shared__ uint32_t s_hot;
+  if (keys) {
+    for (int i = threadIdx.x; i < 4096; i += blockDim.x) s_slot[i] = 0u;
+    if (threadIdx.x == 0) s_hot = 0u;
+    const int64_t i = (int64_t)threadIdx.x * n / blockDim.x + (threadIdx.x * 2654435761u >> 8) % (uint32_t)(n / blockDim.x);
+    const int32_t k = __ldg(keys + i);
+    const bool ok = !vmask || ((vmask[i >> 5] >> (i & 31)) & 1u);
+    __syncthreads();
+    uint32_t c = ok ? atomicAdd(&s_slot[((uint32_t)k * 2654435761u) >> 20], 1u) + 1u : 0u;
+    c = __reduce_max_sync(0xffffffffu, c);
+    if (lane_id() == 0) atomicMax(&s_hot, c);
+  }
   const int lane = lane_id(), warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const ProbeAcc none{false, true, 0, 0, INT_MAX, INT_MIN, 0};
   const int64_t per_w = (nspans + nwarps - 1) / nwarps;
@@ -236,7 +254,7 @@ __global__ void __launch_bounds__(1024) k_probe_finalize(const ProbeRec* recs, i
       p.kmin = w.has ? w.kmin : 0;
       p.kmax = w.has ? w.kmax : 0;
       p.sorted = w.sorted ? 1 : 0;
-      p.pad = 0;
+      p.pad = keys ? (int32_t)s_hot : 0;  // complete since the barrier above
       *out = p;
     }
   }
@@ -287,32 +305,44 @@ __global__ void __launch_bounds__(256) k_dense_global(const int32_t* __restrict_
   });
 }
 
-// DENSE_SMEM, typed: one CTA per chunk of kDsChunk rows folds its rows into
-// a shared-memory state of the whole span with the split-sum / ordered
-// min-max state of the partition aggregate (native 32- and 64-bit shared
-// atomics only; a chunk of at most 65,536 rows keeps the 16-bit-half int32
-// sums exact), then merges its present slots into the global state.
+// DENSE_SMEM: one CTA per chunk of rows folds them into a shared-memory state
+// of the whole span with the split-sum / ordered min-max state of the partition
+// aggregate (native 32- and 64-bit shared atomics only; a chunk of at most
+// 65,536 rows keeps the 16-bit-half int32 sums exact), then merges its present
+// slots into the global state.
+//
+// What bounds it is the shared atomics: with few keys the lanes of a warp meet
+// on the same addresses, and a float64 sum is a compare-and-swap loop there.  So
+// the state has as many copies as fit (a power of two up to 32), interleaved:
+// slot g of copy r is entry g * R + r, lane l uses copy l mod R, and with 32
+// copies no two lanes of a warp share an address or a bank.  The chunk is
+// chosen so that the CTAs fill whole waves: fixed chunks of 65,536 rows left ten
+// CTAs of 20M rows for a second wave and most SMs idle below 10M rows.
 constexpr int64_t kDsChunk = 65536;
+constexpr size_t kDsState = 100 * 1024;  // two CTAs per SM
 
-template <int NC>
+template <int NC, uint32_t SIG>
 __global__ void __launch_bounds__(512, 2) k_dense_smem_t(const int32_t* __restrict__ keys,
                                                         const uint32_t* __restrict__ vmask, ColSet cs, int64_t n,
-                                                        bool aligned, int32_t kmin, int32_t m, StateRef gst) {
+                                                        bool aligned, int32_t kmin, int32_t m, int lg_copies,
+                                                        int64_t chunk, StateRef gst) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const AggState<NC> st = carve_agg<NC, 0>(cs, smem_raw, m);
-  for (int g = threadIdx.x; g < m; g += blockDim.x) agg_init<NC, 0>(cs, st, g);
+  const int entries = m << lg_copies;
+  const AggState<NC> st = carve_agg<NC, SIG>(cs, smem_raw, entries);
+  for (int g = threadIdx.x; g < entries; g += blockDim.x) agg_init<NC, SIG>(cs, st, g);
   __syncthreads();
-  const int64_t r0 = blockIdx.x * kDsChunk;
-  const int64_t r1 = min(n, r0 + kDsChunk);
+  const int64_t r0 = blockIdx.x * chunk;
+  const int64_t r1 = min(n, r0 + chunk);
   const int lane = lane_id(), warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  constexpr int U = NC >= 2 ? 1 : 2;  // 128-row tiles in flight per warp (registers)
+  const uint32_t copy = (uint32_t)lane & ((1u << lg_copies) - 1u);
+  constexpr int U = NC >= (SIG ? 3 : 2) ? 1 : 2;  // 128-row tiles in flight per warp (registers)
   for (int64_t t0 = r0 + (int64_t)warp * 128 * U; t0 < r1; t0 += (int64_t)nwarps * 128 * U) {
     TileT<NC> t[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t row0 = t0 + u * 128 + 4 * lane;
-      if (aligned && row0 + 4 <= r1) load_tile4_full<true, NC, 0>(keys, vmask, cs, row0, t[u]);
-      else load_tile4_tail<true, NC, 0>(keys, vmask, cs, row0, r1, t[u]);
+      if (aligned && row0 + 4 <= r1) load_tile4_full<true, NC, SIG>(keys, vmask, cs, row0, t[u]);
+      else load_tile4_tail<true, NC, SIG>(keys, vmask, cs, row0, r1, t[u]);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u)
@@ -322,20 +352,34 @@ __global__ void __launch_bounds__(512, 2) k_dense_smem_t(const int32_t* __restri
           uint64_t raw[NC > 0 ? NC : 1];
 #pragma unroll
           for (int c = 0; c < NC; ++c) raw[c] = t[u].raw[c][r];
-          agg_apply<NC, 0>(cs, st, (uint32_t)(t[u].key[r] - kmin), raw);
+          agg_apply<NC, SIG>(cs, st, ((uint32_t)(t[u].key[r] - kmin) << lg_copies) + copy, raw);
         }
   }
   __syncthreads();
-  for (int g = threadIdx.x; g < m; g += blockDim.x) agg_merge<NC, 0>(cs, gst, g, st, g);
+  if (lg_copies == 0) {
+    for (int g = threadIdx.x; g < m; g += blockDim.x) agg_merge<NC, SIG>(cs, gst, g, st, g);
+    return;
+  }
+  // Groups of 2^lg_copies lanes combine the copies of one slot each.
+  for (int e0 = threadIdx.x & ~31; e0 < entries; e0 += blockDim.x)
+    agg_merge_copies<NC, SIG>(cs, gst, st, e0 + lane, entries, lg_copies);
 }
 
-template <int NC>
+template <int NC, uint32_t SIG>
 static int launch_dense_smem_t(const int32_t* keys, const uint32_t* vmask, const ColSet& cs, int64_t n, bool al,
                                int32_t kmin, int32_t m, const StateRef& gst, cudaStream_t s) {
-  const size_t smem = (size_t)m * state_bytes_per_slot(cs) + 64;
-  NFC_CUDA(cudaFuncSetAttribute(k_dense_smem_t<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int64_t grid = std::max<int64_t>(1, (n + kDsChunk - 1) / kDsChunk);
-  k_dense_smem_t<NC><<<(unsigned)grid, 512, smem, s>>>(keys, vmask, cs, n, al, kmin, m, gst);
+  const size_t slot = state_bytes_per_slot(cs);
+  int lg = 0;
+  while (lg < 5 && ((size_t)m << (lg + 1)) * slot + 64 <= kDsState) ++lg;
+  const size_t smem = ((size_t)m << lg) * slot + 64;
+  const int per_sm = 2 * (smem + 2048) <= 227 * 1024 ? 2 : 1;
+  NFC_CUDA(cudaFuncSetAttribute(k_dense_smem_t<NC, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // Whole waves of equal chunks (a multiple of a CTA's 2,048-row step).
+  const int64_t slots = (int64_t)num_sms() * per_sm;
+  const int64_t waves = std::max<int64_t>(1, (n + slots * kDsChunk - 1) / (slots * kDsChunk));
+  const int64_t chunk = std::min<int64_t>(kDsChunk, ((n + slots * waves - 1) / (slots * waves) + 2047) / 2048 * 2048);
+  const int64_t grid = std::max<int64_t>(1, (n + chunk - 1) / chunk);
+  k_dense_smem_t<NC, SIG><<<(unsigned)grid, 512, smem, s>>>(keys, vmask, cs, n, al, kmin, m, lg, chunk, gst);
   NFC_CUDA(cudaGetLastError());
   return NFC_OK;
 }
@@ -425,6 +469,14 @@ bool inputs_aligned(const nfc_groupby_args* a) {
   return true;
 }
 
+// Rows from which the probe samples for hot keys, and the sampled count (of
+// 1,024) from which a key counts as hot.  Global atomics on a hot key run one
+// after the other: 1M rows of Zipf(1.1) keys take 208 us with DENSE_GLOBAL and
+// 146 with PARTITION for one int32 sum, 389 and 175 for six aggregates; even
+// keys 106 and 146, 142 and 167.
+constexpr int64_t kSkewMinRows = 1 << 20;
+constexpr int32_t kSkewHot = 16;
+
 int run_probe(const nfc_groupby_args* a, cudaStream_t s, Scratch& sc, uint32_t** vmask_out,
               nfc_probe* host_probe, StageTimer* tm, const ProbeRec** recs_out) {
   const int64_t n = a->n;
@@ -443,7 +495,7 @@ int run_probe(const nfc_groupby_args* a, cudaStream_t s, Scratch& sc, uint32_t**
     NFC_CUDA(cudaGetLastError());
     tm->launched();
   }
-  k_probe_finalize<<<1, 1024, 0, s>>>(recs, (nspans + 7) / 8, dprobe);
+  k_probe_finalize<<<1, 1024, 0, s>>>(recs, (nspans + 7) / 8, dprobe, n >= kSkewMinRows ? a->keys : nullptr, vmask, n);
   NFC_CUDA(cudaGetLastError());
   tm->launched();
   tm->mark(s);
@@ -472,8 +524,9 @@ int plan_strategy(const ColSet& cs, const nfc_probe& p) {
   // update.  From a few million rows the partition path (two coalesced
   // scatter passes, shared-memory aggregation) is faster on B200 (100M rows
   // over 50K..200K keys: 1.7 against 3.3 ms; 10M rows: 0.41 against 0.47 ms).
+  const bool hot = p.pad >= kSkewHot;
   if ((size_t)m * slot <= (size_t)24 << 20 && m <= 4 * p.n_valid + 4096 &&
-      (!part || p.n_valid < kDenseGlobalMaxRows))
+      (!part || (p.n_valid < kDenseGlobalMaxRows && !hot)))
     return NFC_STRAT_DENSE_GLOBAL;
   if (part) return NFC_STRAT_PARTITION;
   return NFC_STRAT_HASH;
@@ -529,12 +582,18 @@ int run_dense(const nfc_groupby_args* a, const ColSet& cs, const OutSet& o, cons
   const int64_t ntiles128 = (a->n + 127) / 128;
   if (smem_variant) {
     int rc;
-    switch (cs.ncols) {
-      case 0: rc = launch_dense_smem_t<0>(a->keys, vmask, cs, a->n, al, (int32_t)p.kmin, (int32_t)m, gst, s); break;
-      case 1: rc = launch_dense_smem_t<1>(a->keys, vmask, cs, a->n, al, (int32_t)p.kmin, (int32_t)m, gst, s); break;
-      case 2: rc = launch_dense_smem_t<2>(a->keys, vmask, cs, a->n, al, (int32_t)p.kmin, (int32_t)m, gst, s); break;
-      case 3: rc = launch_dense_smem_t<3>(a->keys, vmask, cs, a->n, al, (int32_t)p.kmin, (int32_t)m, gst, s); break;
-      default: rc = launch_dense_smem_t<4>(a->keys, vmask, cs, a->n, al, (int32_t)p.kmin, (int32_t)m, gst, s); break;
+    const uint32_t sig = sig_of(cs);
+    if (cs.ncols == 2 && sig == kSigI32SumMinMax_F64SumMinMax)
+      rc = launch_dense_smem_t<2, kSigI32SumMinMax_F64SumMinMax>(a->keys, vmask, cs, a->n, al, (int32_t)p.kmin,
+                                                                 (int32_t)m, gst, s);
+    else if (cs.ncols == 1 && sig == kSigI32Sum)
+      rc = launch_dense_smem_t<1, kSigI32Sum>(a->keys, vmask, cs, a->n, al, (int32_t)p.kmin, (int32_t)m, gst, s);
+    else switch (cs.ncols) {
+      case 0: rc = launch_dense_smem_t<0, 0>(a->keys, vmask, cs, a->n, al, (int32_t)p.kmin, (int32_t)m, gst, s); break;
+      case 1: rc = launch_dense_smem_t<1, 0>(a->keys, vmask, cs, a->n, al, (int32_t)p.kmin, (int32_t)m, gst, s); break;
+      case 2: rc = launch_dense_smem_t<2, 0>(a->keys, vmask, cs, a->n, al, (int32_t)p.kmin, (int32_t)m, gst, s); break;
+      case 3: rc = launch_dense_smem_t<3, 0>(a->keys, vmask, cs, a->n, al, (int32_t)p.kmin, (int32_t)m, gst, s); break;
+      default: rc = launch_dense_smem_t<4, 0>(a->keys, vmask, cs, a->n, al, (int32_t)p.kmin, (int32_t)m, gst, s); break;
     }
     if (rc) return rc;
   } else {
@@ -789,7 +848,7 @@ extern "C" int64_t nfc_groupby_dense_noalloc(const nfc_groupby_args* a, void* st
                                  (reinterpret_cast<uintptr_t>(a->keys) & 15u) == 0);
     NFC_CUDA(cudaGetLastError());
   }
-  k_probe_finalize<<<1, 1024, 0, s>>>(recs, (nspans + 7) / 8, d_probe);
+  k_probe_finalize<<<1, 1024, 0, s>>>(recs, (nspans + 7) / 8, d_probe, nullptr, nullptr, a->n);
   NFC_CUDA(cudaGetLastError());
   nfc_probe p;
   NFC_CUDA(cudaMemcpyAsync(&p, d_probe, sizeof(p), cudaMemcpyDeviceToHost, s));

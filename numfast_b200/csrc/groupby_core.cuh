@@ -34,6 +34,10 @@ NFC_DEV int col_ag(const ColSet& cs, int c) {
   if constexpr (SIG != 0) return (int)((SIG >> (5 * c + 2)) & 7u);
   else return cs.aggs[c];
 }
+// Column signatures with a dedicated instantiation .
+constexpr uint32_t kSigI32SumMinMax_F64SumMinMax =
+    sig_col(0, NFC_I32, NFC_AGG_SUM | NFC_AGG_MIN | NFC_AGG_MAX) | sig_col(1, NFC_F64, NFC_AGG_SUM | NFC_AGG_MIN | NFC_AGG_MAX);
+constexpr uint32_t kSigI32Sum = sig_col(0, NFC_I32, NFC_AGG_SUM);
 static inline uint32_t sig_of(const ColSet& cs) {
   uint32_t s = 0;
   for (int c = 0; c < cs.ncols; ++c) s |= sig_col(c, cs.dtype[c], cs.aggs[c]);

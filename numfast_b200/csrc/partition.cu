@@ -3,8 +3,8 @@
 //   1. histogram   rows -> key-range buckets of W = 2^wb keys (bulk-copy
 //                  tiles when the keys and the combined bitmap are 16-byte
 //                  aligned)
-//   2. plan        bucket offsets, slices of the buckets larger than kSlice
-//                  records, merge slots
+//   2. plan        bucket offsets, slices of the buckets larger than a
+//                  slice (at most kSlice records), merge slots
 //   3. scatter     rows -> packed records in bucket order.  Aligned inputs:
 //                  pass 1 sends TMA-staged row tiles to coarse buckets of 64
 //                  or 128 fine ones, the refine pass splits the coarse buckets into
@@ -12,13 +12,14 @@
 //                  and written as contiguous runs, one global reservation per
 //                  bucket and tile.  Otherwise one plain scatter pass (two
 //                  sweeps per tile: count, reserve, place).
-//   4. slices      one CTA per slice of a large bucket folds its records into
-//                  a shared-memory state of W groups, the bucket's hottest
-//                  keys into registers, and merges it into a global state
-//   5. aggregate   one CTA per bucket folds its records into a shared-memory
-//                  state of W groups (or takes the merged state of a large
-//                  bucket) and writes the present groups straight to their
-//                  final, ascending position (decoupled look-back over buckets)
+//   4. hot keys    of the large buckets, from a sample; a bucket that has some
+//                  is folded slice by slice (shared-memory state of W groups,
+//                  hot keys in registers) and merged into a global state
+//   5. aggregate   one CTA per slice of the other large buckets (merged the same
+//                  way) and per bucket: it folds the bucket's records into a
+//                  shared-memory state of W groups, or takes the merged state
+//                  of a large one, and writes the present groups straight to
+//                  their final, ascending position (decoupled look-back)
 //
 // Record = u64 words.  Columns are ordered so that 4-byte columns come
 // first; word 0 = klow | (first column << 32) when that column is 4 bytes
@@ -154,7 +155,7 @@ struct PartPlan {
   int64_t* offs;        // [nb+1] record offsets
   uint32_t* cursor;     // [nb]   scatter cursors
   int32_t* merge_slot;  // [nb]   merge-state slot of a bucket of several slices, else -1
-  int32_t* n_merge;     // [3]    merge slots, slices, skew (1: slices hold over a quarter of the records)
+  int32_t* n_merge;     // [3]    merge slots, slices, skew (1: one bucket holds over half of the records)
   int2* multi;          // [max slices] per merge slot: its bucket, its first slice
   int2* slices;         // [max slices] (bucket, slice number)
 };
@@ -169,6 +170,7 @@ __global__ void __launch_bounds__(1024) k_part_plan(const uint32_t* __restrict__
                                                     int cshift, uint32_t* __restrict__ ccursor, PartPlan pl) {
   extern __shared__ uint32_t s_off[];  // counts, then offsets
   __shared__ uint32_t s_scan[33];
+  __shared__ uint32_t s_most;
   const int32_t per = ((nb + (int32_t)blockDim.x - 1) / (int32_t)blockDim.x) | 1;  // odd: no bank conflicts
   const int32_t b0 = min(nb, (int32_t)threadIdx.x * per), b1 = min(nb, b0 + per);
   auto slices_of = [&](uint32_t h) { return h > slice ? (uint32_t)((h + slice - 1) / slice) : 0u; };
@@ -178,19 +180,19 @@ __global__ void __launch_bounds__(1024) k_part_plan(const uint32_t* __restrict__
     pl.merge_slot[b] = -1;
   }
   __syncthreads();
-  uint32_t rows = 0, packed = 0, sliced = 0;
+  uint32_t rows = 0, packed = 0, most = 0;
   for (int32_t b = b0; b < b1; ++b) {
     const uint32_t h = s_off[b], k = slices_of(h);
     rows += h;
-    if (k) {
-      packed += k << 15 | 1u;
-      sliced += h;
-    }
+    most = max(most, h);
+    if (k) packed += k << 15 | 1u;
   }
-  uint32_t t_rows, t_packed, t_sliced;
+  if (threadIdx.x == 0) s_most = 0u;
+  uint32_t t_rows, t_packed;
   uint32_t off = block_excl_scan(rows, s_scan, &t_rows);
   uint32_t x = block_excl_scan(packed, s_scan, &t_packed);
-  block_excl_scan(sliced, s_scan, &t_sliced);
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (lane_id() == 0) atomicMax(&s_most, most);
   for (int32_t b = b0; b < b1; ++b) {
     const uint32_t h = s_off[b], k = slices_of(h);
     s_off[b] = off;
@@ -214,7 +216,7 @@ __global__ void __launch_bounds__(1024) k_part_plan(const uint32_t* __restrict__
     pl.offs[nb] = t_rows;
     pl.n_merge[0] = n_multi;
     pl.n_merge[1] = n_slices;
-    pl.n_merge[2] = t_sliced > t_rows / 4 ? 1 : 0;
+    pl.n_merge[2] = s_most > t_rows / 2 ? 1 : 0;
   }
   // The slices of each large bucket, a warp per bucket.
   for (int32_t i = threadIdx.x >> 5; i < n_multi; i += blockDim.x >> 5) {
@@ -771,6 +773,9 @@ struct PartAggArgs {
   const int32_t* merge_slot;
   const int32_t* n_merge;
   const int2* slices;
+  const int2* multi;
+  const uint2* hot;  // per merge slot: its hot keys, 0xFFFFFFFF none
+  uint32_t* slice_done;  // per merge slot
   StateRef gm;  // merge state, n_merge * W slots
   uint64_t* lb;
   uint32_t* ticket;
@@ -854,16 +859,52 @@ NFC_DEV void for_records(const uint64_t* __restrict__ rp, int64_t i_lo, int64_t 
   }
 }
 
-// One slice of a bucket with more than kSlice records.  Such a bucket exists
-// because few of its keys own most rows; on 100M rows of Zipf(1.1) keys over a
-// 50M domain the shared atomics on those keys made the aggregate 2.51 ms,
-// against 0.80 ms for the same rows of uniform keys.  The first records are
-// counted into the state, the keys with the largest counts then collect in
-// registers.
-template <int NC, bool PACK0, uint32_t SIG>
-__global__ void __launch_bounds__(kPartThreads, 2) k_part_slices(PartAggArgs a) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
+// Buckets of several slices: merge state set to the identities, and up to two
+// hot keys found from the bucket's first records (a key with 1/16 of them: two
+// lanes of a warp on average).
+// Such a bucket exists because a few keys own most rows or because there are few
+// buckets; on 100M rows of Zipf(1.1) keys over a 50M domain the shared atomics
+// on hot keys made the aggregate 2.51 ms, against 0.80 ms for uniform keys.
+constexpr int kHotSample = 2048;
+
+__global__ void __launch_bounds__(kPartThreads) k_part_multi(ColSet cs, StateRef gm, const uint64_t* __restrict__ rec,
+                                                            int nw, const int64_t* __restrict__ offs, int wb,
+                                                            const int32_t* __restrict__ n_merge,
+                                                            const int2* __restrict__ multi, bool sample,
+                                                            uint2* __restrict__ hot,
+                                                            uint32_t* __restrict__ slice_done) {
+  extern __shared__ uint32_t s_cnt[];  // 2^wb counters (sample)
   __shared__ uint32_t s_red[33];
+  const int32_t W = 1 << wb, n = n_merge[0];
+  for (int32_t i = blockIdx.x; i < n; i += gridDim.x) {
+    for (int32_t g = threadIdx.x; g < W; g += blockDim.x) {
+      state_init_slot(cs, gm, (int64_t)i * W + g);
+      if (sample) s_cnt[g] = 0u;
+    }
+    uint32_t h[2] = {0xFFFFFFFFu, 0xFFFFFFFFu};
+    if (sample) {
+      const int32_t b = multi[i].x;
+      const int64_t r0 = offs[b];
+      const int m = (int)min((int64_t)kHotSample, offs[b + 1] - r0);
+      __syncthreads();
+#pragma unroll 4
+      for (int r = threadIdx.x; r < m; r += blockDim.x) atomicAdd(&s_cnt[(uint32_t)__ldg(rec + (size_t)(r0 + r) * nw)], 1u);
+      __syncthreads();
+      pick_hot<2>(s_cnt, W, (uint32_t)(m >> 4), s_red, h);
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+      hot[i] = make_uint2(h[0], h[1]);
+      slice_done[i] = 0u;
+    }
+  }
+}
+
+// The slices of buckets with hot keys, which collect in registers; a kernel of
+// its own, because the registers of this loop slow the plain one.
+template <int NC, bool PACK0, uint32_t SIG>
+__global__ void __launch_bounds__(kPartThreads, SIG == 0 && NC >= 2 ? 1 : 2) k_part_hot(PartAggArgs a) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
   const int32_t W = 1 << a.wb;
   const int32_t nslices = a.n_merge[1];
   const AggState<NC> st = carve_agg<NC, SIG>(a.cs, smem_raw, W, ~__ldg(a.wide));
@@ -873,23 +914,19 @@ __global__ void __launch_bounds__(kPartThreads, 2) k_part_slices(PartAggArgs a) 
   for (int32_t it = blockIdx.x; it < nslices; it += gridDim.x) {
     const int2 sl = a.slices[it];
     const int32_t b = sl.x;
+    const int32_t ms = a.merge_slot[b];
+    const uint2 hk = a.hot[ms];
+    if (hk.x == 0xFFFFFFFFu) continue;
+    const uint32_t hot[2] = {hk.x, hk.y};
     const int32_t wbk = (int32_t)min((int64_t)W, a.m - ((int64_t)b << a.wb));
     const int64_t r_lo = a.offs[b] + (int64_t)sl.y * a.slice;
     const int64_t r_hi = min(a.offs[b + 1], r_lo + a.slice);
     agg_init_all<NC, SIG>(a.cs, st, W);
-    __syncthreads();
-    const uint64_t* rp = a.rec + (size_t)r_lo * NW;
-    const int64_t nrec = r_hi - r_lo;
-    const int64_t head = min(nrec, (int64_t)U * kPartThreads);
-    for_records<NC, PACK0, U>(rp, 0, head,
-                              [&](uint32_t g, const uint64_t* raw) { agg_apply<NC, SIG>(a.cs, st, g, raw); });
-    __syncthreads();
-    uint32_t hot[H];
-    pick_hot<H>(st.cnt, wbk, (uint32_t)(head >> 6), s_red, hot);
     HotAcc<NC> acc[H];
 #pragma unroll
     for (int h = 0; h < H; ++h) hot_init<NC, SIG>(a.cs, acc[h]);
-    for_records<NC, PACK0, U>(rp, head, nrec, [&](uint32_t g, const uint64_t* raw) {
+    __syncthreads();
+    for_records<NC, PACK0, U>(a.rec + (size_t)r_lo * NW, 0, r_hi - r_lo, [&](uint32_t g, const uint64_t* raw) {
       bool in_reg = false;
 #pragma unroll
       for (int h = 0; h < H; ++h)
@@ -897,64 +934,92 @@ __global__ void __launch_bounds__(kPartThreads, 2) k_part_slices(PartAggArgs a) 
           hot_add<NC, SIG>(a.cs, acc[h], raw);
           in_reg = true;
         }
-      if (!in_reg) agg_apply<NC, SIG>(a.cs, st, g, raw);
+      if (!in_reg) agg_apply<NC, SIG, false>(a.cs, st, g, raw);
     });
 #pragma unroll
     for (int h = 0; h < H; ++h)
       if (hot[h] != 0xFFFFFFFFu) hot_flush<NC, SIG>(a.cs, st, hot[h], acc[h]);
     __syncthreads();
-    const int64_t m0 = (int64_t)a.merge_slot[b] * W;
+    const int64_t m0 = (int64_t)ms * W;
     for (int g = threadIdx.x; g < wbk; g += blockDim.x) agg_merge<NC, SIG>(a.cs, a.gm, m0 + g, st, g);
     __syncthreads();  // the state is reused
   }
 }
 
-// One CTA per bucket, claimed in order.  A persistent form that fetched its next
-// ticket and bounds ahead was slower on skewed keys (1.0-1.2 against 0.81 ms):
-// a CTA that holds a ticket while it works on a large bucket delays the
-// look-back of every bucket after it.
+// Work items, one CTA each, claimed in order: first the slices of the large
+// buckets without hot keys (folded and merged into the global state), then the
+// buckets, each folded and emitted, or emitted from the merged state once its
+// slices are done.  A bucket waits only for items claimed before it (its slices;
+// the look-back), so every wait ends.  One kernel for both, so that long slices
+// and buckets overlap.  A persistent form that fetched its next ticket ahead was
+// slower on skewed keys (1.0-1.2 against 0.81 ms): a CTA that holds a ticket
+// while it works on a large bucket delays every bucket after it.
 template <int NC, bool PACK0, uint32_t SIG>
 __global__ void __launch_bounds__(kPartThreads, 2) k_part_agg(PartAggArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ uint32_t s_warp[kPartThreads / 32];
   __shared__ int64_t s_base;
-  __shared__ int32_t s_bucket;
-  if (threadIdx.x == 0) s_bucket = (int32_t)atomicAdd(a.ticket, 1u);
+  __shared__ int32_t s_item;
+  if (threadIdx.x == 0) s_item = (int32_t)atomicAdd(a.ticket, 1u);
   __syncthreads();
-  const int32_t b = s_bucket;
+  const int32_t nslices = a.n_merge[1];
+  const int32_t it = s_item;
+  if (it >= nslices + a.nb) return;
+  const bool slice = it < nslices;
+  const int2 sl = slice ? a.slices[it] : make_int2(it - nslices, 0);
+  const int32_t b = sl.x;
   const int32_t W = 1 << a.wb;
   const int64_t key0 = a.kmin + ((int64_t)b << a.wb);
   const int32_t wbk = (int32_t)min((int64_t)W, a.m - ((int64_t)b << a.wb));
   constexpr int NW = Rec<NC, PACK0>::NW;
   constexpr int U = 4;  // records in flight per thread
   const int32_t ms = a.merge_slot[b];
-  if (ms >= 0) {  // its slices are merged in the global state
-    const int64_t m0 = (int64_t)ms * W;
-    part_emit(a, b, wbk, [&](int g) { return a.gm.cnt[m0 + g]; },
+  const int64_t m0 = (int64_t)ms * W;
+  const bool hot = ms >= 0 && a.hot[ms].x != 0xFFFFFFFFu;
+  if (slice && hot) return;
+  if (!slice && ms >= 0) {
+    if (!hot) {  // wait for its slices
+      if (threadIdx.x == 0) {
+        const int32_t end = ms + 1 < a.n_merge[0] ? a.multi[ms + 1].y : nslices;
+        const uint32_t want = (uint32_t)(end - a.multi[ms].y);
+        uint32_t spins = 0;
+        while (ld_volatile_u32(a.slice_done + ms) < want)
+          if (++spins > kSpinLimit) {
+            atomicExch(a.err, NFC_ERR_TIMEOUT);
+            break;
+          }
+        __threadfence();
+      }
+      __syncthreads();
+    }
+    part_emit(a, b, wbk, [&](int g) { return __ldcg(&a.gm.cnt[m0 + g]); },
               [&](int g, int64_t pos) { state_emit(a.cs, a.gm, m0 + g, a.o, pos, key0 + g); }, s_warp, &s_base);
     return;
   }
-  const int64_t r_lo = a.offs[b];
+  const int64_t r_lo = a.offs[b] + (int64_t)sl.y * a.slice;
+  const int64_t r_hi = slice ? min(a.offs[b + 1], r_lo + a.slice) : a.offs[b + 1];
   const AggState<NC> st = carve_agg<NC, SIG>(a.cs, smem_raw, W, ~__ldg(a.wide));
   agg_init_all<NC, SIG>(a.cs, st, W);
   __syncthreads();
-  for_records<NC, PACK0, U>(a.rec + (size_t)r_lo * NW, 0, a.offs[b + 1] - r_lo,
+  for_records<NC, PACK0, U>(a.rec + (size_t)r_lo * NW, 0, r_hi - r_lo,
                             [&](uint32_t g, const uint64_t* raw) { agg_apply<NC, SIG, false>(a.cs, st, g, raw); });
   __syncthreads();
+  if (slice) {
+    for (int g = threadIdx.x; g < wbk; g += blockDim.x) agg_merge<NC, SIG>(a.cs, a.gm, m0 + g, st, g);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(a.slice_done + ms, 1u);
+    return;
+  }
   part_emit(a, b, wbk, [&](int g) { return st.cnt[g]; },
             [&](int g, int64_t pos) { agg_emit<NC, SIG>(a.cs, st, g, a.o, pos, key0 + g); }, s_warp, &s_base);
-}
-
-__global__ void k_merge_init(ColSet cs, StateRef gm, const int32_t* n_merge, int64_t w) {
-  const int64_t slots = (int64_t)(*n_merge) * w;
-  for (int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; d < slots; d += (int64_t)gridDim.x * blockDim.x)
-    state_init_slot(cs, gm, d);
 }
 
 // ---------------------------------------------------------------- host
 constexpr int64_t kMaxBuckets = 28672;  // two shared 32-bit tables of them in the plain scatter
 constexpr int64_t kMaxWideBuckets = 16384;
 constexpr int64_t kSlice = 65536;  // <= 65536 keeps the 16-bit-split int32 sums exact
+constexpr int64_t kMinSlice = 8192;
 constexpr size_t kAggSmemBudget = 200 * 1024;
 
 // Bucket width: the widest whose shared-memory state leaves room for two
@@ -997,6 +1062,8 @@ struct PartLaunch {
   uint64_t* rec;      // fine-bucket records (aggregate input)
   size_t agg_smem;
   int64_t max_slices;
+  const int2* multi;
+  uint2* hot;
   int64_t nv;         // valid rows (records)
   uint32_t* wide;     // wide-int32-column bits (zeroed, set by the scatter)
   int32_t* d_err;
@@ -1056,23 +1123,30 @@ static int launch_part(const PartLaunch& q, PartAggArgs& pa, cudaStream_t s, Sta
   NFC_CUDA(cudaFuncSetAttribute(k_part_agg<NC, PACK0, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)q.agg_smem));
   if (q.max_slices > 0) {
-    NFC_CUDA(cudaFuncSetAttribute(k_part_slices<NC, PACK0, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)q.agg_smem));
-    k_part_slices<NC, PACK0, SIG><<<(unsigned)std::min<int64_t>(q.max_slices, num_sms() * 2), kPartThreads, q.agg_smem,
-                                     s>>>(pa);
+    const unsigned g = (unsigned)std::min<int64_t>(q.max_slices, 2 * (int64_t)num_sms());
+    // 128 KB of counters at most; 32-bit aggregates alone keep up on hot keys.
+    bool wide64 = false;
+    for (int c = 0; c < NC; ++c) wide64 |= q.cs.dtype[c] != NFC_I32 && q.cs.aggs[c] != 0;
+    const bool sample = wide64 && q.wb <= 15;
+    const size_t cnt = sample ? (size_t)4 << q.wb : 0;
+    NFC_CUDA(cudaFuncSetAttribute(k_part_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cnt));
+    k_part_multi<<<g, kPartThreads, cnt, s>>>(q.cs, pa.gm, pa.rec, NW, pa.offs, q.wb, pa.n_merge, q.multi, sample,
+                                              q.hot, pa.slice_done);
     NFC_CUDA(cudaGetLastError());
     tm->launched();
+    if (sample) {
+      NFC_CUDA(cudaFuncSetAttribute(k_part_hot<NC, PACK0, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)q.agg_smem));
+      k_part_hot<NC, PACK0, SIG><<<g, kPartThreads, q.agg_smem, s>>>(pa);
+      NFC_CUDA(cudaGetLastError());
+      tm->launched();
+    }
   }
-  k_part_agg<NC, PACK0, SIG><<<(unsigned)q.nb, kPartThreads, q.agg_smem, s>>>(pa);
+  k_part_agg<NC, PACK0, SIG><<<(unsigned)(q.nb + q.max_slices), kPartThreads, q.agg_smem, s>>>(pa);
   NFC_CUDA(cudaGetLastError());
   tm->launched();
   return NFC_OK;
 }
-
-// Column signatures with a dedicated instantiation (after 4-byte-first ordering).
-constexpr uint32_t kSigI32SumMinMax_F64SumMinMax =
-    sig_col(0, NFC_I32, NFC_AGG_SUM | NFC_AGG_MIN | NFC_AGG_MAX) | sig_col(1, NFC_F64, NFC_AGG_SUM | NFC_AGG_MIN | NFC_AGG_MAX);
-constexpr uint32_t kSigI32Sum = sig_col(0, NFC_I32, NFC_AGG_SUM);
 
 template <int NC>
 static int launch_part_nc(bool pack0, const PartLaunch& q, PartAggArgs& pa, cudaStream_t s, StageTimer* tm) {
@@ -1215,14 +1289,19 @@ int run_partition(const nfc_groupby_args* a, const ColSet& cs_in, const OutSet& 
       tm->launched();
     }
   }
-  // A bucket of more than kSlice records has fewer than two slices per kSlice
-  // of them.
-  const int64_t max_slices = nv > kSlice ? 2 * (nv / kSlice) : 0;
+  // Slices of an equal share of the chip, within [kMinSlice, kSlice]: at 2M rows
+  // slices of 65,536 leave 30 CTAs with 130 us of work each.  A bucket of more
+  // than one slice has fewer than two slices per `slice` of its records.
+  const int64_t slice = std::min<int64_t>(kSlice, std::max<int64_t>(kMinSlice, nv / (2 * num_sms())));
+  const int64_t max_slices = nv > slice ? 2 * (nv / slice) : 0;
   int2* slices = nullptr;
-  NFC_CUDA(sc.alloc(&slices, (size_t)std::max<int64_t>(2 * max_slices, 1)));
+  NFC_CUDA(sc.alloc(&slices, (size_t)std::max<int64_t>(4 * max_slices, 1)));
   PartPlan pl{w.offs, w.cursor, w.merge_slot, w.n_merge, slices + max_slices, slices};
+  q.multi = pl.multi;
+  q.hot = reinterpret_cast<uint2*>(slices + 2 * max_slices);
+  uint32_t* slice_done = reinterpret_cast<uint32_t*>(slices + 3 * max_slices);
   NFC_CUDA(cudaFuncSetAttribute(k_part_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(nb * 4)));
-  k_part_plan<<<1, 1024, (size_t)nb * 4, s>>>(w.ghist, nb, kSlice, q.cshift, q.two_level ? q.ccursor : nullptr, pl);
+  k_part_plan<<<1, 1024, (size_t)nb * 4, s>>>(w.ghist, nb, slice, q.cshift, q.two_level ? q.ccursor : nullptr, pl);
   NFC_CUDA(cudaGetLastError());
   tm->launched();
   if (q.coalesced && q.two_level) {
@@ -1232,7 +1311,7 @@ int run_partition(const nfc_groupby_args* a, const ColSet& cs_in, const OutSet& 
 
   NFC_CUDA(sc.alloc(&q.rec, (size_t)std::max<int64_t>(nv, 1) * nw));
   const int64_t W = 1ll << wb;
-  const int64_t max_merge = nv / (kSlice + 1) + 1;
+  const int64_t max_merge = nv / (slice + 1) + 1;
   unsigned char* gmb = nullptr;
   NFC_CUDA(sc.alloc(&gmb, (size_t)max_merge * W * slot + 64));
   const StateRef gm = carve_state(cs, gmb, max_merge * W);
@@ -1244,13 +1323,16 @@ int run_partition(const nfc_groupby_args* a, const ColSet& cs_in, const OutSet& 
   pa.merge_slot = w.merge_slot;
   pa.n_merge = w.n_merge;
   pa.slices = slices;
+  pa.multi = pl.multi;
+  pa.hot = q.hot;
+  pa.slice_done = slice_done;
   pa.gm = gm;
   pa.lb = w.lb;
   pa.ticket = w.ticket;
   pa.o = o;
   pa.kmin = p.kmin;
   pa.m = m;
-  pa.slice = kSlice;
+  pa.slice = slice;
   pa.nb = nb;
   pa.wb = wb;
   pa.ng_out = d_ng;
@@ -1258,10 +1340,6 @@ int run_partition(const nfc_groupby_args* a, const ColSet& cs_in, const OutSet& 
   pa.wide = q.wide;
   q.agg_smem = (size_t)W * slot + 64;
   q.max_slices = max_slices;
-  k_merge_init<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((max_merge * W + 255) / 256, (int64_t)num_sms() * 4)),
-                 256, 0, s>>>(cs, gm, w.n_merge, W);
-  NFC_CUDA(cudaGetLastError());
-  tm->launched();
   int rc;
   switch (cs.ncols) {
     case 0: rc = launch_part_nc<0>(pack0, q, pa, s, tm); break;

@@ -125,7 +125,6 @@ __global__ void __launch_bounds__(kShThreads, 2)
   }
 }
 
-constexpr uint32_t kSigI32Sum = sig_col(0, NFC_I32, NFC_AGG_SUM);
 
 struct ShLaunch {
   const int32_t* keys;

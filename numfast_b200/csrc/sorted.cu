@@ -809,9 +809,6 @@ int launch_sorted(const nfc_groupby_args* a, const ColSet& cs, const OutSet& o, 
   return NFC_OK;
 }
 
-constexpr uint32_t kSigI32SumMinMax_F64SumMinMax =
-    sig_col(0, NFC_I32, NFC_AGG_SUM | NFC_AGG_MIN | NFC_AGG_MAX) | sig_col(1, NFC_F64, NFC_AGG_SUM | NFC_AGG_MIN | NFC_AGG_MAX);
-constexpr uint32_t kSigI32Sum = sig_col(0, NFC_I32, NFC_AGG_SUM);
 
 Pieces carve_pieces(uint64_t*& q, int64_t np) {
   Pieces P{};

@@ -111,7 +111,6 @@ __global__ void k_sort_emit(ColSet cs, StateRef st, const int64_t* ng_ptr, OutSe
     state_emit(cs, st, r, o, r, o.ukeys[r]);
 }
 
-constexpr uint32_t kSigI32Sum = sig_col(0, NFC_I32, NFC_AGG_SUM);
 
 template <int NC, uint32_t SIG>
 int launch_runs(const int32_t* keys, const uint32_t* perm, int64_t nv, const ColSet& cs, const StateRef& gst,
