@@ -24,14 +24,17 @@ NFC_HD int dtype_bytes(int dt) { return dt == NFC_I32 ? 4 : 8; }
 // dtype and [5c+2, 5c+5) for its NFC_AGG_* mask.  SIG == 0 means "read the
 // dtype/aggs from the ColSet at run time" (generic instantiation).
 constexpr uint32_t sig_col(int c, int dtype, int aggs) { return (uint32_t)(dtype | (aggs << 2)) << (5 * c); }
+// kSigSums: dtypes at run time, no aggregate but sums (and counts) requested.
+constexpr uint32_t kSigSums = 0x80000000u;
 template <uint32_t SIG>
 NFC_DEV int col_dt(const ColSet& cs, int c) {
-  if constexpr (SIG != 0) return (int)((SIG >> (5 * c)) & 3u);
+  if constexpr (SIG != 0 && SIG != kSigSums) return (int)((SIG >> (5 * c)) & 3u);
   else return cs.dtype[c];
 }
 template <uint32_t SIG>
 NFC_DEV int col_ag(const ColSet& cs, int c) {
-  if constexpr (SIG != 0) return (int)((SIG >> (5 * c + 2)) & 7u);
+  if constexpr (SIG == kSigSums) return cs.aggs[c] & NFC_AGG_SUM;
+  else if constexpr (SIG != 0) return (int)((SIG >> (5 * c + 2)) & 7u);
   else return cs.aggs[c];
 }
 // Column signatures with a dedicated instantiation .
@@ -42,6 +45,12 @@ static inline uint32_t sig_of(const ColSet& cs) {
   uint32_t s = 0;
   for (int c = 0; c < cs.ncols; ++c) s |= sig_col(c, cs.dtype[c], cs.aggs[c]);
   return s;
+}
+
+static inline bool sums_only(const ColSet& cs) {
+  for (int c = 0; c < cs.ncols; ++c)
+    if (cs.aggs[c] & ~NFC_AGG_SUM) return false;
+  return true;
 }
 
 // ---------------------------------------------------------------------

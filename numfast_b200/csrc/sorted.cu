@@ -12,24 +12,18 @@
 //   1. k_sorted_prev    one CTA turns the probe records into the last valid
 //                       key before every tile (an exclusive "last non-empty"
 //                       scan over the 16,384-row blocks the probe summarised);
-//   2. k_sorted_agg     one CTA per tile of 16,384 rows, claimed in order.
-//                       The tile's keys and combined validity come into
-//                       shared memory with one bulk (TMA) copy.  Pass 1: each
-//                       warp marks the run heads of its 2,048-row chunk (a
-//                       valid row whose key differs from the previous valid
-//                       row's) and counts them; a decoupled look-back gives
-//                       the tile its first run number.  Pass 2: each warp
-//                       streams its chunk's values in steps of 128 rows (4
-//                       per lane, 128-bit loads, the next step in flight) and
-//                       reduces the runs with a segmented scan in registers
-//                       (lane, then warp shuffles that stop once every lane
-//                       has met a head).  Runs that end inside a step go to a
-//                       per-warp shared-memory buffer (where the keys were)
-//                       and leave in one coalesced pass per step.  The warps'
-//                       edge runs are merged by one warp; the tile's first run
-//                       (continued from earlier tiles) and last run (possibly
-//                       continued by later ones) leave as two partial
-//                       "pieces";
+//   2. k_sorted_agg     one CTA per tile of 2,048 or 4,096 rows, claimed in
+//                       order, a thread per 8 or 16 consecutive rows.  A thread finds its
+//                       run heads (valid rows whose key differs from the
+//                       previous valid row's), sums the rows before its first
+//                       head and after its last one into shared memory, and a
+//                       decoupled look-back gives the tile its first run
+//                       number.  The thread that holds a run's head then adds
+//                       what the threads after it have of that run (a whole
+//                       warp without heads is one step) and writes the run.
+//                       The tile's first run (continued from earlier tiles) and
+//                       last run (possibly continued by later ones) leave as
+//                       two partial "pieces";
 //   3. k_sorted_fix     the pieces are merged in order (segmented scan by run
 //                       number): chunks of 1,024 in parallel CTAs, then the
 //                       chunks' own edge runs in one CTA.
@@ -37,22 +31,20 @@
 // are reduced as a tree (order differs from the reference's row loop; within
 // 1e-12 relative); everything else is exact.
 #include <algorithm>
+#include <type_traits>
 
-#include "bulk.cuh"
 #include "groupby_host.h"
 
 namespace nfc {
 namespace {
 
-constexpr int kSoThreads = 256;
+constexpr int kSoThreads = 256;                    // threads with rows; one more warp looks back
 constexpr int kSoWarps = kSoThreads / 32;
-constexpr int kSoWarpRows = 2048;                 // rows of one warp chunk
-constexpr int kSoTile = kSoWarps * kSoWarpRows;   // rows per CTA tile (16,384)
-static_assert(kSoTile == kProbeBlockRows, "one probe record per tile");
-constexpr int kSoLaneRows = 4;                    // pass 2: rows per lane and step
-constexpr int kSoStepRows = 32 * kSoLaneRows;
-constexpr int kSoSteps = kSoWarpRows / kSoStepRows;
-constexpr int kRunBuf = kSoStepRows;              // runs ending inside one step
+// Consecutive rows per thread and rows per tile: more where a row is little work.
+constexpr int so_rows(int nc) { return nc <= 1 ? 16 : 8; }
+constexpr int so_tile(int nc) { return kSoThreads * so_rows(nc); }
+static_assert(kProbeBlockRows % so_tile(0) == 0 && kProbeBlockRows % so_tile(4) == 0,
+              "tiles do not straddle probe records");
 constexpr int kFixThreads = 1024;
 
 // ---------------------------------------------------------------- run aggregate
@@ -165,6 +157,44 @@ NFC_DEV void seg_shfl(const ColSet& cs, const Seg<NC>& a, Seg<NC>& out, int arg)
       if (ag & NFC_AGG_MIN) out.mn[c] = sh64(a.mn[c]);
       if (ag & NFC_AGG_MAX) out.mx[c] = sh64(a.mx[c]);
     }
+  }
+}
+
+// All lanes' run aggregates combined: 32-bit fields by warp reductions, 64-bit
+// ones by shuffles.
+template <int NC, uint32_t SIG>
+NFC_DEV void seg_warp_reduce(const ColSet& cs, const Seg<NC>& a, Seg<NC>& out) {
+  out.cnt = __reduce_add_sync(0xffffffffu, a.cnt);
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int dt = col_dt<SIG>(cs, c), ag = col_ag<SIG>(cs, c);
+    uint64_t s = a.sum[c], lo = a.mn[c], hi = a.mx[c];
+    if (ag & NFC_AGG_SUM) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const uint64_t t = __shfl_xor_sync(0xffffffffu, s, o);
+        s = dt == NFC_F64 ? f64_add_bits(s, t) : s + t;
+      }
+    }
+    if (dt == NFC_I32) {
+      if (ag & NFC_AGG_MIN) lo = (uint64_t)(int64_t)__reduce_min_sync(0xffffffffu, (int32_t)lo);
+      if (ag & NFC_AGG_MAX) hi = (uint64_t)(int64_t)__reduce_max_sync(0xffffffffu, (int32_t)hi);
+    } else {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        if (ag & NFC_AGG_MIN) {
+          const uint64_t t = __shfl_xor_sync(0xffffffffu, lo, o);
+          lo = dt == NFC_F64 ? min(lo, t) : (uint64_t)min((long long)lo, (long long)t);
+        }
+        if (ag & NFC_AGG_MAX) {
+          const uint64_t t = __shfl_xor_sync(0xffffffffu, hi, o);
+          hi = dt == NFC_F64 ? max(hi, t) : (uint64_t)max((long long)hi, (long long)t);
+        }
+      }
+    }
+    out.sum[c] = s;
+    out.mn[c] = lo;
+    out.mx[c] = hi;
   }
 }
 
@@ -319,10 +349,12 @@ NFC_DEV void block_seg_scan(const ColSet& cs, uint32_t f, const Seg<NC>& a, uint
   __syncthreads();
 }
 
-// Last valid key before each tile: prev[t] = (1 << 32 | key) or 0 when no
-// valid row precedes tile t.  One CTA walks the probe records (one per tile)
-// in order.
-__global__ void __launch_bounds__(1024) k_sorted_prev(const ProbeRec* recs, int64_t nrec, uint64_t* prev) {
+// Last valid key before each probe block of kProbeBlockRows rows: prev[i] =
+// (1 << 32 | key) or 0 when no valid row precedes it.  One CTA walks the probe
+// records in order; it also empties the nq second-level pieces.
+__global__ void __launch_bounds__(1024) k_sorted_prev(const ProbeRec* recs, int64_t nrec, uint64_t* prev,
+                                                      int64_t* q_idx, int64_t nq) {
+  for (int64_t i = threadIdx.x; i < nq; i += blockDim.x) q_idx[i] = -1;
   __shared__ uint64_t s_w[32];
   __shared__ uint64_t s_carry;
   const int lane = lane_id(), warp = threadIdx.x >> 5;
@@ -356,365 +388,433 @@ __global__ void __launch_bounds__(1024) k_sorted_prev(const ProbeRec* recs, int6
   }
 }
 
-// Values of one pass-2 step for one lane (kSoLaneRows consecutive rows):
-// 32-bit words, the high words only for 8-byte columns.
-template <int NC>
-struct StepVals {
-  uint32_t lo[NC > 0 ? NC : 1][kSoLaneRows];
-  uint32_t hi[NC > 0 ? NC : 1][kSoLaneRows];
-};
-
+// Four rows' values of every column, from row (a multiple of 4) on: 32-bit
+// words as they are, 8-byte values as bits; rows at or past n are not read.
 template <int NC, uint32_t SIG>
-NFC_DEV void load_step(const ColSet& cs, int64_t n, bool aligned, int64_t row, StepVals<NC>& b) {
-  if (row >= n) return;
-  if (aligned && row + kSoLaneRows <= n) {
+NFC_DEV void load_rows4(const ColSet& cs, int64_t n, bool aligned, int64_t row, uint64_t (&v)[4][NC > 0 ? NC : 1]) {
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
+  for (int c = 0; c < NC; ++c) {
+    if (aligned && row + 4 <= n) {
       if (col_dt<SIG>(cs, c) == NFC_I32) {
-        const int4 x = __ldcs(reinterpret_cast<const int4*>(static_cast<const int32_t*>(cs.data[c]) + row));
-        b.lo[c][0] = x.x; b.lo[c][1] = x.y; b.lo[c][2] = x.z; b.lo[c][3] = x.w;
+        const int4 x = __ldg(reinterpret_cast<const int4*>(static_cast<const int32_t*>(cs.data[c]) + row));
+        v[0][c] = (uint32_t)x.x; v[1][c] = (uint32_t)x.y; v[2][c] = (uint32_t)x.z; v[3][c] = (uint32_t)x.w;
       } else {
-        const int4* q = reinterpret_cast<const int4*>(static_cast<const uint64_t*>(cs.data[c]) + row);
-        const int4 x = __ldcs(q), y = __ldcs(q + 1);
-        b.lo[c][0] = x.x; b.hi[c][0] = x.y; b.lo[c][1] = x.z; b.hi[c][1] = x.w;
-        b.lo[c][2] = y.x; b.hi[c][2] = y.y; b.lo[c][3] = y.z; b.hi[c][3] = y.w;
+        const ulonglong2* q = reinterpret_cast<const ulonglong2*>(static_cast<const uint64_t*>(cs.data[c]) + row);
+        const ulonglong2 x = __ldg(q), y = __ldg(q + 1);
+        v[0][c] = x.x; v[1][c] = x.y; v[2][c] = y.x; v[3][c] = y.y;
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        v[r][c] = row + r >= n                       ? 0ull
+                  : col_dt<SIG>(cs, c) == NFC_I32 ? (uint64_t)(uint32_t) static_cast<const int32_t*>(cs.data[c])[row + r]
+                                                  : static_cast<const uint64_t*>(cs.data[c])[row + r];
+    }
+  }
+}
+
+// A thread's rows of column c (load_rows4's conventions).
+template <int kSoRows, uint32_t SIG>
+NFC_DEV void load_rows(const ColSet& cs, int c, int64_t n, bool aligned, int64_t row, uint64_t (&v)[kSoRows]) {
+  if (aligned && row + kSoRows <= n) {
+    if (col_dt<SIG>(cs, c) == NFC_I32) {
+      const int4* q = reinterpret_cast<const int4*>(static_cast<const int32_t*>(cs.data[c]) + row);
+#pragma unroll
+      for (int e = 0; e < kSoRows / 4; ++e) {
+        const int4 x = __ldg(q + e);
+        v[4 * e] = (uint32_t)x.x; v[4 * e + 1] = (uint32_t)x.y; v[4 * e + 2] = (uint32_t)x.z; v[4 * e + 3] = (uint32_t)x.w;
+      }
+    } else {
+      const ulonglong2* q = reinterpret_cast<const ulonglong2*>(static_cast<const uint64_t*>(cs.data[c]) + row);
+#pragma unroll
+      for (int e = 0; e < kSoRows / 2; ++e) {
+        const ulonglong2 x = __ldg(q + e);
+        v[2 * e] = x.x;
+        v[2 * e + 1] = x.y;
       }
     }
   } else {
 #pragma unroll
-    for (int r = 0; r < kSoLaneRows; ++r)
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        if (row + r >= n) continue;
-        if (col_dt<SIG>(cs, c) == NFC_I32) {
-          b.lo[c][r] = (uint32_t) static_cast<const int32_t*>(cs.data[c])[row + r];
-        } else {
-          const uint64_t v = static_cast<const uint64_t*>(cs.data[c])[row + r];
-          b.lo[c][r] = (uint32_t)v;
-          b.hi[c][r] = (uint32_t)(v >> 32);
-        }
-      }
+    for (int r = 0; r < kSoRows; ++r)
+      v[r] = row + r >= n                       ? 0ull
+             : col_dt<SIG>(cs, c) == NFC_I32 ? (uint64_t)(uint32_t) static_cast<const int32_t*>(cs.data[c])[row + r]
+                                             : static_cast<const uint64_t*>(cs.data[c])[row + r];
   }
 }
 
-// Runs that end inside one pass-2 step, buffered per warp: entry j = run
-// (first run of the step - 1 + j).
+// Partial runs of the tile's threads, one array per field so that neighbouring
+// threads touch neighbouring words.
 template <int NC>
-struct RunBuf {
-  uint64_t sum[NC > 0 ? NC : 1][kRunBuf];
-  uint64_t mn[NC > 0 ? NC : 1][kRunBuf];
-  uint64_t mx[NC > 0 ? NC : 1][kRunBuf];
-  uint32_t cnt[kRunBuf];
+struct Partials {
+  uint64_t sum[NC > 0 ? NC : 1][kSoThreads];
+  uint64_t mn[NC > 0 ? NC : 1][kSoThreads];
+  uint64_t mx[NC > 0 ? NC : 1][kSoThreads];
+  uint32_t cnt[kSoThreads];
 };
 
 template <int NC, uint32_t SIG>
-NFC_DEV void rb_store(const ColSet& cs, RunBuf<NC>& rb, int j, const Seg<NC>& a) {
-  rb.cnt[j] = a.cnt;
+NFC_DEV void part_store(const ColSet& cs, Partials<NC>& p, int t, const Seg<NC>& a) {
+  p.cnt[t] = a.cnt;
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     const int ag = col_ag<SIG>(cs, c);
-    if (ag & NFC_AGG_SUM) rb.sum[c][j] = a.sum[c];
-    if (ag & NFC_AGG_MIN) rb.mn[c][j] = a.mn[c];
-    if (ag & NFC_AGG_MAX) rb.mx[c][j] = a.mx[c];
+    if (ag & NFC_AGG_SUM) p.sum[c][t] = a.sum[c];
+    if (ag & NFC_AGG_MIN) p.mn[c][t] = a.mn[c];
+    if (ag & NFC_AGG_MAX) p.mx[c][t] = a.mx[c];
   }
 }
 
 template <int NC, uint32_t SIG>
-NFC_DEV void rb_load(const ColSet& cs, const RunBuf<NC>& rb, int j, Seg<NC>& a) {
-  a.cnt = rb.cnt[j];
+NFC_DEV void part_add(const ColSet& cs, Seg<NC>& a, const Partials<NC>& p, int t) {
+  Seg<NC> b;
+  b.cnt = p.cnt[t];
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     const int ag = col_ag<SIG>(cs, c);
-    if (ag & NFC_AGG_SUM) a.sum[c] = rb.sum[c][j];
-    if (ag & NFC_AGG_MIN) a.mn[c] = rb.mn[c][j];
-    if (ag & NFC_AGG_MAX) a.mx[c] = rb.mx[c][j];
+    b.sum[c] = ag & NFC_AGG_SUM ? p.sum[c][t] : 0ull;
+    b.mn[c] = ag & NFC_AGG_MIN ? p.mn[c][t] : 0ull;
+    b.mx[c] = ag & NFC_AGG_MAX ? p.mx[c][t] : 0ull;
   }
+  seg_combine<NC, SIG>(cs, a, b);
 }
+
+// CTAs per SM that the registers of the run aggregates leave room for.
+template <int NC, uint32_t SIG>
+constexpr int so_ctas() { return NC == 0 ? 4 : NC <= 2 ? 3 : 2; }
 
 template <int NC, uint32_t SIG>
 struct SortedSmem {
   union {
-    int32_t keys[kSoTile];       // pass 1: the tile's keys
-    RunBuf<NC> rb[kSoWarps];     // pass 2: per-warp run buffers
-  } u;
-  alignas(16) uint32_t vbits[kSoTile / 32];
-  uint32_t hbits[kSoTile / 32];
-  uint64_t bar;
+    Partials<NC> lead;             // rows before the thread's first head; all its rows when it has none
+    uint64_t stage[so_tile(NC)];  // short runs: one output column of the tile's runs
+  };
+  Seg<NC> wsum[kSoWarps];  // all rows of a warp without heads
+  uint64_t wlast[kSoWarps];  // last valid key of the warp (1 << 32 | key), 0 none
   uint32_t wheads[kSoWarps];
-  int64_t wbase[kSoWarps];
-  int64_t pidx[2 * kSoWarps];  // warp pieces: 2w = run continued into chunk w, 2w+1 = its last run
-  Seg<NC> pseg[2 * kSoWarps];
-  int64_t excl;
-  int64_t tile;
-  int32_t abort;
+  uint32_t wany[kSoWarps];  // bit l: lane l has a head
+  uint64_t carry;
+  int64_t tile, excl;
 };
 
+// What bounds it: 40M rows of one int64 and one float64 sum in runs of 16 are
+// 0.88 GB (135 us); the form with a segmented warp scan per 128 rows, four rows
+// per lane, was issue bound at 1,145 us (and 16,384-row tiles left most SMs
+// without work below 2M rows).
 template <int NC, uint32_t SIG>
-__global__ void __launch_bounds__(kSoThreads, 2) k_sorted_agg(const int32_t* __restrict__ keys,
-                                                              const uint32_t* __restrict__ vmask, ColSet cs,
-                                                              int64_t n, bool aligned, bool bulk_ok,
-                                                              const uint64_t* __restrict__ prev, OutSet o,
-                                                              int64_t cap, Pieces P, uint64_t* lb, uint32_t* ticket,
-                                                              int64_t* ng_out, int32_t* err) {
+__global__ void __launch_bounds__(kSoThreads + 32, so_ctas<NC, SIG>())
+    k_sorted_agg(const int32_t* __restrict__ keys, const uint32_t* __restrict__ vmask, ColSet cs, int64_t n,
+                 bool aligned, const uint64_t* __restrict__ prev, OutSet o, int64_t cap, Pieces P, uint64_t* lb,
+                 uint32_t* ticket, int64_t* ng_out, int32_t* err) {
   extern __shared__ __align__(128) unsigned char sm_raw[];
   SortedSmem<NC, SIG>& sm = *reinterpret_cast<SortedSmem<NC, SIG>*>(sm_raw);
+  constexpr int kSoRows = so_rows(NC), kSoTile = so_tile(NC);
   const int tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
-  if (tid == 0) {
-    sm.tile = atomicAdd(ticket, 1u);
-    sm.abort = 0;
-    mbar_init(&sm.bar, 1);
-    mbar_fence_init();
-  }
-  if (tid < 2 * kSoWarps) sm.pidx[tid] = -1;
+  if (tid == 0) sm.tile = atomicAdd(ticket, 1u);
   __syncthreads();
   const int64_t tile = sm.tile;
   const int64_t ntiles = (n + kSoTile - 1) / kSoTile;
   if (tile >= ntiles) return;
   const int64_t tbase = tile * kSoTile;
-  const int c0 = warp * kSoWarpRows;  // chunk start (tile row)
-
-  // The values do not depend on the keys: the first step's loads go out now
-  // and land while the keys are staged, the heads counted and the tile's run
-  // number looked up.
-  StepVals<NC> va, vb2;
-  load_step<NC, SIG>(cs, n, aligned, tbase + c0 + kSoLaneRows * lane, va);
-
-  // ---- keys and validity of the tile -> shared memory.
-  const bool full = tbase + kSoTile <= n;
-  if (full && bulk_ok) {
-    if (tid == 0) {
-      fence_proxy_async_smem();
-      mbar_arrive_expect_tx(&sm.bar, (uint32_t)(kSoTile * 4 + (vmask ? kSoTile / 8 : 0)));
-      bulk_g2s(sm.u.keys, keys + tbase, (uint32_t)(kSoTile * 4), &sm.bar);
-      if (vmask) bulk_g2s(sm.vbits, vmask + tbase / 32, (uint32_t)(kSoTile / 8), &sm.bar);
+  if (warp == kSoWarps) {
+    // The extra warp: last valid key before the tile (usually one of the 32
+    // rows before it; else the rows back to the probe block's start, 1,024 at a
+    // time, then the probe's own record), then the look-back, while the other
+    // warps load and sum.
+    const int64_t block = tbase / kProbeBlockRows;
+    const int64_t w_lo = block * (kProbeBlockRows / 32);
+    uint64_t carry = prev[block];
+    int64_t w0 = tbase / 32 - 1;
+    if (w0 >= w_lo) {
+      const uint32_t bits = vmask ? __ldg(vmask + w0) : 0xFFFFFFFFu;
+      const int32_t key = keys[tbase - 32 + lane];
+      const int32_t got = __shfl_sync(0xffffffffu, key, bits ? 31 - __clz(bits) : 0);
+      if (bits) carry = (1ull << 32) | (uint32_t)got;
+      w0 = bits ? w_lo - 1 : w0 - 1;
     }
-    if (!vmask)
-      for (int w = tid; w < kSoTile / 32; w += kSoThreads) sm.vbits[w] = 0xFFFFFFFFu;
-    if (!mbar_wait(&sm.bar, 0)) sm.abort = 1;
-  } else {
-    for (int i = tid; i < kSoTile; i += kSoThreads) sm.u.keys[i] = tbase + i < n ? __ldg(keys + tbase + i) : 0;
-    for (int w = tid; w < kSoTile / 32; w += kSoThreads) {
-      const int64_t r0 = tbase + 32 * (int64_t)w;
-      uint32_t b = 0;
-      if (r0 < n) {
-        b = vmask ? __ldg(vmask + (r0 >> 5)) : 0xFFFFFFFFu;
-        if (n - r0 < 32) b &= (1u << (n - r0)) - 1u;
-      }
-      sm.vbits[w] = b;
-    }
-  }
-  __syncthreads();
-  if (sm.abort) {
-    // Let the copy land before the shared memory goes away.
-    if (tid == 0) {
-      atomicExch(err, NFC_ERR_TIMEOUT);
-      mbar_wait(&sm.bar, 0);
-    }
-    __syncthreads();
-    return;
-  }
-
-  // ---- pass 1: run heads of every warp chunk, 8 rows per lane and step.
-  uint64_t carry = prev[tile];  // (1 << 32 | key) of the last valid row before the chunk
-  if (warp > 0) {
-    // Last valid row before the chunk inside the tile, if any: the warp reads
-    // 32 validity words per round, nearest first.
-    for (int w0 = c0 / 32 - 1; w0 >= 0; w0 -= 32) {
-      const int wi = w0 - lane;
-      const uint32_t b = wi >= 0 ? sm.vbits[wi] : 0u;
-      const unsigned nz = __ballot_sync(0xffffffffu, b != 0u);
+    for (; w0 >= w_lo; w0 -= 32) {
+      const int64_t w = w0 - lane;
+      const uint32_t bits = w < w_lo ? 0u : __ldg(vmask + w);  // a bitmap: without one every row is valid
+      const unsigned nz = __ballot_sync(0xffffffffu, bits != 0u);
       if (nz) {
         const int l = __ffs(nz) - 1;
-        const uint32_t bs = __shfl_sync(0xffffffffu, b, l);
-        const int row = (w0 - l) * 32 + (31 - __clz(bs));
-        carry = (1ull << 32) | (uint32_t)sm.u.keys[row];
+        const uint32_t b = __shfl_sync(0xffffffffu, bits, l);
+        carry = (1ull << 32) | (uint32_t)keys[(w0 - l) * 32 + (31 - __clz(b))];
         break;
       }
     }
-  }
-  uint32_t heads = 0;
-  for (int st = 0; st < kSoWarpRows / 256; ++st) {
-    const int r0 = c0 + st * 256 + 8 * lane;
-    const int4 ka = *reinterpret_cast<const int4*>(&sm.u.keys[r0]);
-    const int4 kb = *reinterpret_cast<const int4*>(&sm.u.keys[r0 + 4]);
-    const int32_t k[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
-    const uint32_t vb = (sm.vbits[r0 >> 5] >> (r0 & 31)) & 0xFFu;
-    uint64_t mine = 0;
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-      if (vb & (1u << r)) mine = (1ull << 32) | (uint32_t)k[r];
-    uint64_t inc = mine;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      if (__all_sync(0xffffffffu, inc >> 32)) break;
-      const uint64_t y = __shfl_up_sync(0xffffffffu, inc, off);
-      if (lane >= off && !(inc >> 32)) inc = y;
-    }
-    uint64_t p = __shfl_up_sync(0xffffffffu, inc, 1);
-    if (lane == 0 || !(p >> 32)) p = carry;
-    uint32_t hb = 0;
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-      if (vb & (1u << r)) {
-        if (!(p >> 32) || (int32_t)(uint32_t)p != k[r]) hb |= 1u << r;
-        p = (1ull << 32) | (uint32_t)k[r];
-      }
-    reinterpret_cast<uint8_t*>(sm.hbits)[r0 >> 3] = (uint8_t)hb;
-    heads += __popc(hb);
-    const uint64_t l31 = __shfl_sync(0xffffffffu, inc, 31);
-    if (l31 >> 32) carry = l31;
-  }
-  heads = warp_sum(heads);
-  if (lane == 0) sm.wheads[warp] = heads;
-  __syncthreads();  // also: every warp is done with the staged keys
-  if (warp == 0) {
-    const uint32_t h = lane < kSoWarps ? sm.wheads[lane] : 0u;
-    uint32_t hi = h;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, hi, off);
-      if (lane >= off) hi += y;
-    }
-    const uint32_t total = __shfl_sync(0xffffffffu, hi, 31);
+    if (lane == 0) sm.carry = carry;
+    __syncthreads();  // carry and the warps' last keys
+    __syncthreads();  // head counts
+    const uint32_t total = __reduce_add_sync(0xffffffffu, lane < kSoWarps ? sm.wheads[lane] : 0u);
     const int64_t ex = lookback_exclusive(lb, tile, total, err);  // whole warp
-    if (lane < kSoWarps) sm.wbase[lane] = ex + hi - h;
     if (lane == 0) {
       sm.excl = ex;
       if (tile == ntiles - 1) *ng_out = ex + total;
     }
+    __syncthreads();  // run numbers and partial sums
+    return;
   }
-  __syncthreads();
-  const int64_t excl_tile = sm.excl;
-  const int64_t wbase = sm.wbase[warp];
-  RunBuf<NC>& rb = sm.u.rb[warp];
+  const int64_t row0 = tbase + tid * kSoRows;
 
-  // ---- pass 2: values; runs reduced by a segmented scan per warp step.
-  uint32_t cf = 0;
-  Seg<NC> ca;
-  seg_identity<NC, SIG>(cs, ca);
-  int64_t hrun = wbase;  // run number of the next head in the chunk
-  auto step = [&](int st, const StepVals<NC>& vals) {
-    const int r0 = c0 + st * kSoStepRows + kSoLaneRows * lane;  // tile row
-    const uint32_t vb = (sm.vbits[r0 >> 5] >> (r0 & 31)) & 0xFu;
-    const uint32_t hb = (sm.hbits[r0 >> 5] >> (r0 & 31)) & 0xFu;
-    const uint32_t hc = __popc(hb);
-    uint32_t hi = hc;
+  // ---- keys and validity of the thread's rows.
+  int32_t k[kSoRows];
+  constexpr uint32_t kAll = (1u << kSoRows) - 1u;
+  uint32_t vb = row0 + kSoRows <= n ? kAll : row0 < n ? (1u << (uint32_t)(n - row0)) - 1u : 0u;
+  if (vmask && vb) vb &= (__ldg(vmask + (row0 >> 5)) >> (row0 & 31)) & kAll;
+  if (aligned && row0 + kSoRows <= n) {
 #pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, hi, off);
-      if (lane >= off) hi += y;
+    for (int e = 0; e < kSoRows / 4; ++e) {
+      const int4 x = __ldg(reinterpret_cast<const int4*>(keys + row0) + e);
+      k[4 * e] = x.x; k[4 * e + 1] = x.y; k[4 * e + 2] = x.z; k[4 * e + 3] = x.w;
     }
-    const uint32_t H = __shfl_sync(0xffffffffu, hi, 31);
-    // Head j of the step starts run hrun + j and ends run hrun + j - 1, which
-    // is buffer entry j.
-    const int j0 = (int)(hi - hc);  // this lane's first head
-    Seg<NC> lead, cur;
-    seg_identity<NC, SIG>(cs, lead);
-    seg_identity<NC, SIG>(cs, cur);
-    bool seen = false;
-    int j = j0;
+  } else {
 #pragma unroll
-    for (int r = 0; r < kSoLaneRows; ++r) {
-      if (!(vb & (1u << r))) continue;
-      if (hb & (1u << r)) {
-        if (!seen) {
-          lead = cur;
-          seen = true;
-        } else {
-          rb_store<NC, SIG>(cs, rb, j, cur);  // a run that began and ended in this lane
-        }
-        // Runs never outnumber min(span, valid rows) <= cap for sorted keys;
-        // the check only keeps a broken sortedness flag from writing past it.
-        const int64_t g = hrun + j;
-        if (g < cap) o.ukeys[g] = (int64_t)__ldg(keys + tbase + r0 + r);
-        else atomicExch(err, NFC_ERR_RANGE);
-        ++j;
+    for (int r = 0; r < kSoRows; ++r) k[r] = row0 + r < n ? keys[row0 + r] : 0;
+  }
+  uint64_t last = 0;
+#pragma unroll
+  for (int r = 0; r < kSoRows; ++r)
+    if (vb & (1u << r)) last = (1ull << 32) | (uint32_t)k[r];
+  const unsigned has = __ballot_sync(0xffffffffu, vb != 0u);
+  const unsigned below = has & lanemask_lt();
+  const uint64_t before = __shfl_sync(0xffffffffu, last, below ? 31 - __clz(below) : 0);
+  const uint64_t wl = __shfl_sync(0xffffffffu, last, has ? 31 - __clz(has) : 0);
+  if (lane == 0) sm.wlast[warp] = has ? wl : 0ull;
+  __syncthreads();
+
+  // ---- run heads.
+  uint64_t p = before;
+  if (!below) {
+    p = sm.carry;
+    for (int w = 0; w < warp; ++w)
+      if (sm.wlast[w]) p = sm.wlast[w];
+  }
+  uint32_t hb = 0;
+#pragma unroll
+  for (int r = 0; r < kSoRows; ++r)
+    if (vb & (1u << r)) {
+      if (p != ((1ull << 32) | (uint32_t)k[r])) hb |= 1u << r;
+      p = (1ull << 32) | (uint32_t)k[r];
+    }
+  const uint32_t hc = (uint32_t)__popc(hb);
+  uint32_t hi = hc;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, hi, off);
+    if (lane >= off) hi += y;
+  }
+  const unsigned any = __ballot_sync(0xffffffffu, hb != 0u);
+  if (lane == 31) sm.wheads[warp] = hi;
+  if (lane == 0) sm.wany[warp] = any;
+  __syncthreads();
+
+  // ---- partial sums before the first and from the last head.
+  Seg<NC> cur, lead;
+  seg_identity<NC, SIG>(cs, cur);
+  seg_identity<NC, SIG>(cs, lead);
+#pragma unroll
+  for (int q = 0; q < kSoRows / 4; ++q) {
+    if (((vb >> (4 * q)) & 0xFu) == 0u) continue;
+    uint64_t v[4][NC > 0 ? NC : 1];
+    load_rows4<NC, SIG>(cs, n, aligned, row0 + 4 * q, v);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const uint32_t bit = 1u << (4 * q + r);
+      if (hb & bit) {
+        if ((hb & (bit - 1u)) == 0u) lead = cur;
         seg_identity<NC, SIG>(cs, cur);
       }
-      uint64_t rv[NC > 0 ? NC : 1];
-#pragma unroll
-      for (int c = 0; c < NC; ++c)
-        rv[c] = col_dt<SIG>(cs, c) == NFC_I32 ? (uint64_t)vals.lo[c][r]
-                                              : ((uint64_t)vals.hi[c][r] << 32) | vals.lo[c][r];
-      seg_add_row<NC, SIG>(cs, cur, rv);
+      if (vb & bit) seg_add_row<NC, SIG>(cs, cur, v[r]);
     }
-    if (!seen) lead = cur;
-    Seg<NC> ex;
-    warp_seg_scan<NC, SIG>(cs, seen ? 1u : 0u, seen ? cur : lead, cf, ca, ex);
-    if (seen) {
-      // The run that ends just before this lane's first head (run hrun+j0-1).
-      seg_combine<NC, SIG>(cs, ex, lead);
-      if (hrun + j0 - 1 < wbase) {
-        // It began before the chunk: the warp's front piece.
-        if (ex.cnt > 0) {
-          sm.pidx[2 * warp] = hrun + j0 - 1;
-          sm.pseg[2 * warp] = ex;
-        }
-      } else {
-        rb_store<NC, SIG>(cs, rb, j0, ex);
-      }
-    }
-    __syncwarp();
-    // Runs hrun - 1 + j (j < H) ended in this step: out in one coalesced pass.
-    for (int jj = lane; jj < (int)H; jj += 32) {
-      const int64_t g = hrun - 1 + jj;
-      if (g < wbase || g >= cap) continue;
-      Seg<NC> a;
-      rb_load<NC, SIG>(cs, rb, jj, a);
-      seg_emit<NC, SIG>(cs, o, g, a);
-    }
-    __syncwarp();
-    hrun += H;
-  };
-  for (int st = 0; st < kSoSteps; st += 2) {
-    load_step<NC, SIG>(cs, n, aligned, tbase + c0 + (st + 1) * kSoStepRows + kSoLaneRows * lane, vb2);
-    step(st, va);
-    if (st + 2 < kSoSteps)
-      load_step<NC, SIG>(cs, n, aligned, tbase + c0 + (st + 2) * kSoStepRows + kSoLaneRows * lane, va);
-    step(st + 1, vb2);
   }
-  if (lane == 0) {
-    if (hrun > wbase) {
-      sm.pidx[2 * warp + 1] = hrun - 1;
-      sm.pseg[2 * warp + 1] = ca;
-    } else if (ca.cnt > 0) {
-      sm.pidx[2 * warp] = wbase - 1;  // no head in the chunk: it continues one run
-      sm.pseg[2 * warp] = ca;
-    }
+  part_store<NC, SIG>(cs, sm.lead, tid, hb ? lead : cur);
+  if (any == 0u) {
+    Seg<NC> w;
+    seg_warp_reduce<NC, SIG>(cs, cur, w);
+    if (lane == 0) sm.wsum[warp] = w;
   }
   __syncthreads();
-
-  // ---- warp pieces -> runs of the tile (one warp, one piece per lane).
-  if (warp == 0) {
-    const int64_t idx = lane < 2 * kSoWarps ? sm.pidx[lane] : -1;
-    Seg<NC> a;
-    if (idx >= 0) a = sm.pseg[lane];
-    else seg_identity<NC, SIG>(cs, a);
-    int64_t mx = idx;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int64_t y = __shfl_up_sync(0xffffffffu, mx, off);
-      if (lane >= off) mx = max(mx, y);
-    }
-    int64_t before = __shfl_up_sync(0xffffffffu, mx, 1);
-    if (lane == 0) before = -1;
-    const bool head = idx >= 0 && idx > before;
-    uint32_t tcf = 0;
-    Seg<NC> tca, ex;
-    seg_identity<NC, SIG>(cs, tca);
-    warp_seg_scan<NC, SIG>(cs, head ? 1u : 0u, a, tcf, tca, ex);
-    if (head && before >= 0) {
-      if (before < excl_tile) piece_store<NC>(P, 2 * tile, before, ex);
-      else if (before < cap) seg_emit<NC, SIG>(cs, o, before, ex);
-    }
-    const int64_t last = __shfl_sync(0xffffffffu, mx, 31);
-    if (lane == 0 && last >= 0) piece_store<NC>(P, last < excl_tile ? 2 * tile : 2 * tile + 1, last, tca);
+  uint32_t total = 0, mine = 0;
+  for (int w = 0; w < kSoWarps; ++w) {
+    if (w < warp) mine += sm.wheads[w];
+    total += sm.wheads[w];
   }
-}
+  const int64_t excl = sm.excl;
 
-__global__ void k_pieces_clear(int64_t* idx, int64_t m) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x)
-    idx[i] = -1;
+  // Adds to `a` what the threads from t on hold of an open run; true when the
+  // run ends inside the tile.
+  auto follow = [&](Seg<NC>& a, int t) {
+    while (t < kSoThreads) {
+      const uint32_t rest = sm.wany[t >> 5] >> (t & 31);
+      if (rest == 0u && (t & 31) == 0) {
+        seg_combine<NC, SIG>(cs, a, sm.wsum[t >> 5]);
+        t += 32;
+        continue;
+      }
+      part_add<NC, SIG>(cs, a, sm.lead, t);
+      if (rest & 1u) return true;
+      ++t;
+    }
+    return false;
+  };
+  // The run that the tile continues (its rows before the first head).
+  if (tid == 0) {
+    Seg<NC> run = hb ? lead : any ? cur : sm.wsum[0];
+    if (!hb) follow(run, any ? 1 : 32);
+    if (run.cnt > 0) piece_store<NC>(P, 2 * tile, excl - 1, run);
+    else P.idx[2 * tile] = -1;
+    if (total == 0) P.idx[2 * tile + 1] = -1;
+  }
+  // The run of the thread's last head; the tile's last run stays open.
+  const int64_t g = excl + mine + hi - hc;
+  Seg<NC> run = cur;
+  bool ended = false;
+  if (hb) {
+    ended = follow(run, tid + 1);
+    if (!ended) piece_store<NC>(P, 2 * tile + 1, g + hc - 1, run);
+  }
+  // Runs never outnumber min(span, valid rows) <= cap for sorted keys; the
+  // checks only keep a broken sortedness flag in bounds.
+  if (excl + total > cap) {
+    if (tid == 0) atomicExch(err, NFC_ERR_RANGE);
+    return;
+  }
+  const uint32_t last_head = hb ? 31u - (uint32_t)__clz(hb) : 0u;
+  if (total < kSoTile / 4) {
+    // Few runs: every thread writes its own.
+    if (hb == 0u) return;
+    if (ended) seg_emit<NC, SIG>(cs, o, g + hc - 1, run);
+    int64_t gi = g;
+#pragma unroll
+    for (int r = 0; r < kSoRows; ++r)
+      if (hb & (1u << r)) o.ukeys[gi++] = (int64_t)k[r];
+    if ((hb & (hb - 1u)) == 0u) return;
+    // Runs inside the thread: from each head to the next.
+    seg_identity<NC, SIG>(cs, run);
+    gi = g - 1;
+#pragma unroll
+    for (int q = 0; q < kSoRows / 4; ++q) {
+      if (4u * q > last_head) continue;
+      uint64_t v[4][NC > 0 ? NC : 1];
+      load_rows4<NC, SIG>(cs, n, aligned, row0 + 4 * q, v);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const uint32_t bit = 1u << (4 * q + r);
+        if (hb & bit) {
+          if (gi >= g) seg_emit<NC, SIG>(cs, o, gi, run);
+          ++gi;
+          seg_identity<NC, SIG>(cs, run);
+        }
+        if (vb & bit) seg_add_row<NC, SIG>(cs, run, v[r]);
+      }
+    }
+    return;
+  }
+  // Many short runs: threads writing several runs each would scatter 8-byte
+  // stores (20M rows in runs of 1.6, six aggregates: 763 us), so the outputs
+  // leave column by column through shared memory.
+  const uint32_t l0 = mine + hi - hc;
+  uint32_t last_key = 0u;  // of the thread's last head
+#pragma unroll
+  for (int r = 0; r < kSoRows; ++r)
+    if (hb & (1u << r)) last_key = (uint32_t)k[r];
+  // fill() sets the thread's entries of the stage, store(i, x) writes entry i.
+  auto put = [&](auto fill, auto store) {
+    __syncthreads();  // the stage is free
+    fill();
+    __syncthreads();
+    for (uint32_t i = tid; i < total; i += kSoThreads) store(i, sm.stage[i]);
+  };
+  // One aggregate of every run: `first` starts a run's value, `add` folds a
+  // row's, `dec` gives what is staged of it, `fin` is that of the thread's last
+  // run.  The tile's last run is open; its entry is not written out.
+  auto runs_of = [&](uint64_t first, uint64_t fin, auto add, auto dec) {
+    uint32_t l = l0;
+    uint64_t x = first;
+    bool open = false;
+#pragma unroll
+    for (int r = 0; r < kSoRows; ++r) {
+      if (hb & (1u << r)) {
+        if (open) sm.stage[l++] = dec(x);
+        open = true;
+        x = first;
+      }
+      if (vb & (1u << r)) x = add(x, r);
+    }
+    if (hb) sm.stage[l] = fin;
+  };
+  auto same = [](uint64_t x) { return x; };
+  // Keys and counts in one go: a run's key is any of its rows' keys.
+  put([&] {
+        runs_of(0, (uint64_t)run.cnt << 32 | last_key,
+                [&](uint64_t x, int r) { return ((x >> 32) + 1) << 32 | (uint32_t)k[r]; }, same);
+      },
+      [&](uint32_t i, uint64_t x) {
+        o.ukeys[excl + i] = (int64_t)(int32_t)(uint32_t)x;
+        if (i + 1 < total) o.counts[excl + i] = (int64_t)(x >> 32);
+      });
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int dt = col_dt<SIG>(cs, c), ag = col_ag<SIG>(cs, c);
+    if (ag == 0) continue;
+    uint64_t v[kSoRows];
+    load_rows<kSoRows, SIG>(cs, c, n, aligned, row0, v);
+    auto to64 = [&](void* dst) {
+      uint64_t* d = static_cast<uint64_t*>(dst) + excl;
+      return [d, total](uint32_t i, uint64_t x) {
+        if (i + 1 < total) d[i] = x;
+      };
+    };
+    if (ag & NFC_AGG_SUM)
+      put([&] {
+            runs_of(0, run.sum[c],
+                    [&](uint64_t x, int r) {
+                      return dt == NFC_F64 ? f64_add_bits(x, v[r])
+                                           : x + (dt == NFC_I32 ? (uint64_t)(int64_t)(int32_t)v[r] : v[r]);
+                    },
+                    same);
+          },
+          to64(o.sum[c]));
+    if (dt == NFC_I32) {
+      if (ag & (NFC_AGG_MIN | NFC_AGG_MAX))  // both in one word: maximum above minimum
+        put([&] {
+              runs_of((uint64_t)0x80000000u << 32 | 0x7FFFFFFFu,
+                      (uint64_t)(uint32_t)run.mx[c] << 32 | (uint32_t)run.mn[c],
+                      [&](uint64_t x, int r) {
+                        const int32_t y = (int32_t)v[r];
+                        const int32_t lo = min((int32_t)(uint32_t)x, y), hi = max((int32_t)(x >> 32), y);
+                        return (uint64_t)(uint32_t)hi << 32 | (uint32_t)lo;
+                      },
+                      same);
+            },
+            [&](uint32_t i, uint64_t x) {
+              if (i + 1 >= total) return;
+              if (ag & NFC_AGG_MIN) static_cast<int32_t*>(o.mn[c])[excl + i] = (int32_t)(uint32_t)x;
+              if (ag & NFC_AGG_MAX) static_cast<int32_t*>(o.mx[c])[excl + i] = (int32_t)(x >> 32);
+            });
+      continue;
+    }
+    if (ag & NFC_AGG_MIN)
+      put([&] {
+            if (dt == NFC_F64)
+              runs_of(~0ull, f64_min_dec(run.mn[c]), [&](uint64_t x, int r) { return min(x, f64_min_enc(v[r])); },
+                      [](uint64_t x) { return f64_min_dec(x); });
+            else
+              runs_of((uint64_t)LLONG_MAX, run.mn[c],
+                      [&](uint64_t x, int r) { return (uint64_t)min((long long)x, (long long)v[r]); }, same);
+          },
+          to64(o.mn[c]));
+    if (ag & NFC_AGG_MAX)
+      put([&] {
+            if (dt == NFC_F64)
+              runs_of(0ull, f64_max_dec(run.mx[c]), [&](uint64_t x, int r) { return max(x, f64_max_enc(v[r])); },
+                      [](uint64_t x) { return f64_max_dec(x); });
+            else
+              runs_of((uint64_t)LLONG_MIN, run.mx[c],
+                      [&](uint64_t x, int r) { return (uint64_t)max((long long)x, (long long)v[r]); }, same);
+          },
+          to64(o.mx[c]));
+  }
 }
 
 // Merge pieces (nondecreasing run numbers; -1 = none) by run number.
@@ -785,12 +885,8 @@ int launch_sorted(const nfc_groupby_args* a, const ColSet& cs, const OutSet& o, 
                   uint64_t* lb, uint32_t* ticket, int64_t* d_ng, int32_t* d_err, cudaStream_t s, StageTimer* tm) {
   const size_t smem = sizeof(SortedSmem<NC, SIG>);
   NFC_CUDA(cudaFuncSetAttribute(k_sorted_agg<NC, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  // Bulk copies need 16-byte aligned sources (the combined bitmap is ours).
-  const bool bulk_ok = (reinterpret_cast<uintptr_t>(a->keys) & 15u) == 0 &&
-                       (reinterpret_cast<uintptr_t>(vmask) & 15u) == 0;
-  k_sorted_agg<NC, SIG><<<(unsigned)ntiles, kSoThreads, smem, s>>>(a->keys, vmask, cs, a->n, inputs_aligned(a),
-                                                                   bulk_ok, prev, o, a->out_cap, P, lb, ticket,
-                                                                   d_ng, d_err);
+  k_sorted_agg<NC, SIG><<<(unsigned)ntiles, kSoThreads + 32, smem, s>>>(a->keys, vmask, cs, a->n, inputs_aligned(a), prev, o,
+                                                                   a->out_cap, P, lb, ticket, d_ng, d_err);
   NFC_CUDA(cudaGetLastError());
   tm->launched();
   tm->mark(s);
@@ -828,8 +924,8 @@ int run_sorted(const nfc_groupby_args* a, const ColSet& cs, const OutSet& o, con
                const uint32_t* vmask, const ProbeRec* recs, cudaStream_t s, Scratch& sc, int64_t* d_ng,
                int32_t* d_err, StageTimer* tm) {
   const int64_t n = a->n;
-  const int64_t ntiles = (n + kSoTile - 1) / kSoTile;
-  const int64_t nrec = (n + kProbeBlockRows - 1) / kProbeBlockRows;  // == ntiles
+  const int64_t ntiles = (n + so_tile(a->ncols) - 1) / so_tile(a->ncols);
+  const int64_t nrec = (n + kProbeBlockRows - 1) / kProbeBlockRows;  // <= ntiles
   const int64_t np = 2 * ntiles;
   const int64_t nchunks = (np + kFixThreads - 1) / kFixThreads;
   const int64_t nq = 2 * nchunks;
@@ -845,28 +941,30 @@ int run_sorted(const nfc_groupby_args* a, const ColSet& cs, const OutSet& o, con
   const Pieces P = carve_pieces(q, np);
   const Pieces Q = carve_pieces(q, nq);
   NFC_CUDA(cudaMemsetAsync(lb, 0, sizeof(uint64_t) * ((size_t)ntiles + 2), s));
-  k_pieces_clear<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((np + 255) / 256, (int64_t)num_sms() * 4)), 256,
-                   0, s>>>(P.idx, np);
+  k_sorted_prev<<<1, 1024, 0, s>>>(recs, nrec, prev, Q.idx, nq);
   NFC_CUDA(cudaGetLastError());
-  k_pieces_clear<<<1, 256, 0, s>>>(Q.idx, nq);
-  NFC_CUDA(cudaGetLastError());
-  k_sorted_prev<<<1, 1024, 0, s>>>(recs, nrec, prev);
-  NFC_CUDA(cudaGetLastError());
-  tm->launched(3);
+  tm->launched();
   tm->mark(s);
   const uint32_t sig = sig_of(cs);
+  const bool sums = sums_only(cs);
 #define NFC_SORTED_LAUNCH(NCV, SIGV) \
   launch_sorted<NCV, SIGV>(a, cs, o, vmask, prev, P, Q, ntiles, nchunks, lb, ticket, d_ng, d_err, s, tm)
   switch (cs.ncols) {
     case 0: return NFC_SORTED_LAUNCH(0, 0);
     case 1:
       if (sig == kSigI32Sum) return NFC_SORTED_LAUNCH(1, kSigI32Sum);
+      if (sums) return NFC_SORTED_LAUNCH(1, kSigSums);
       return NFC_SORTED_LAUNCH(1, 0);
     case 2:
       if (sig == kSigI32SumMinMax_F64SumMinMax) return NFC_SORTED_LAUNCH(2, kSigI32SumMinMax_F64SumMinMax);
+      if (sums) return NFC_SORTED_LAUNCH(2, kSigSums);
       return NFC_SORTED_LAUNCH(2, 0);
-    case 3: return NFC_SORTED_LAUNCH(3, 0);
-    default: return NFC_SORTED_LAUNCH(4, 0);
+    case 3:
+      if (sums) return NFC_SORTED_LAUNCH(3, kSigSums);
+      return NFC_SORTED_LAUNCH(3, 0);
+    default:
+      if (sums) return NFC_SORTED_LAUNCH(4, kSigSums);
+      return NFC_SORTED_LAUNCH(4, 0);
   }
 #undef NFC_SORTED_LAUNCH
 }
