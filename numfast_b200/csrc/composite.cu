@@ -15,7 +15,7 @@
 //   2. range of the flipped halves, then word = (ta - ta_min) << wb |
 //      (tb - tb_min) with ta = a ^ a_flip, tb = b ^ b_flip and wb the bit
 //      width of tb's range: the pair's order in just the bits it needs;
-//   3. onesweep radix sort of (word, position index) over those bits;
+//   3. radix sort of (word, position index) over those bits;
 //   4. k_cc_runs: run heads of equal words, run ids by a block scan and a
 //      decoupled look-back; codes[row] = run id, and each head writes its
 //      pair (ua, ub) at the run id.  Rows not valid keep code -1.

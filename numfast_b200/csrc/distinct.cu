@@ -6,7 +6,8 @@
 // group bounds and value transitions (_count_distinct_sorted_dedup,
 // cpu.py:2647-2700); output ukeys ascending and nunique, both int64.
 //
-// Here:
+// Large inputs whose keys spread over many buckets are counted bucket by bucket
+// (distinct_part.cu).  The others here:
 //   1. k_cd_range: count of valid rows and the range of tk = key ^ 2^31 and
 //      tv = value ^ 2^31 over them; k_cd_pack: pair = (tk - tk_min) << wv |
 //      (tv - tv_min), wv the bit width of tv's range, an unsigned order equal
@@ -15,8 +16,7 @@
 //      exactly the valid pairs (an all-ones valid pair is identical to the
 //      filler and indistinguishable from it, so dropping n - n_valid of them
 //      keeps the right multiset);
-//   2. onesweep radix sort of the pairs over wk + wv bits (radix.cu; passes
-//      whose digit is the same for every pair are skipped);
+//   2. radix sort of the pairs over wk + wv bits (radix_sort.cu);
 //   3. k_cd_runs: 4096 sorted pairs per tile; a key head is a change of the
 //      high half, a pair head any change; one decoupled look-back carries
 //      both counts (key heads << 31 | pair heads), so key run r learns its
@@ -219,6 +219,11 @@ extern "C" int64_t nfc_group_count_distinct(const int32_t* keys, const uint8_t* 
     return NFC_ERR_UNSUPPORTED;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  {
+    const int64_t ng = count_distinct_by_partition(keys, key_validity, values, value_validity, n, out_cap, ukeys_out,
+                                                   nunique_out, s);
+    if (ng != NFC_ERR_UNSUPPORTED) return ng;
+  }
   Scratch sc(s);
   uint64_t *p0 = nullptr, *p1 = nullptr;
   int64_t* small = nullptr;  // nvalid | ng | pairs | err

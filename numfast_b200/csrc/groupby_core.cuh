@@ -18,6 +18,9 @@ struct ColSet {
   const void* data[NFC_MAX_COLS];
 };
 
+// Internal column type of the partition records: the row number itself.
+constexpr int kRowId = 3;
+
 NFC_HD int dtype_bytes(int dt) { return dt == NFC_I32 ? 4 : 8; }
 
 // Compile-time column signature: column c uses bits [5c, 5c+2) for its

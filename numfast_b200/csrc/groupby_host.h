@@ -81,6 +81,29 @@ int run_partition(const nfc_groupby_args* a, const ColSet& cs, const OutSet& o, 
                   const uint32_t* vmask, cudaStream_t s, Scratch& sc, int64_t* d_ng, int32_t* d_err,
                   int64_t* buckets_out, StageTimer* tm);
 
+// Rows of int32 keys as 8-byte records in buckets of 2^wb consecutive keys:
+// (key - kmin) mod 2^wb in the low half, the int32 value -- or with dtype kRowId
+// the row number -- in the high half; order within a bucket is free.
+// NFC_ERR_UNSUPPORTED (nothing scattered) for unaligned columns, too many
+// buckets, or a bucket of more than max_rows rows.
+struct PartRecords {
+  const uint64_t* rec;
+  const int64_t* offs;  // [nb + 1]
+  int32_t nb;
+  int64_t most;  // rows of the largest bucket
+};
+int partition_records(const nfc_groupby_args* a, int32_t dtype, const void* values, const nfc_probe& p,
+                      const uint32_t* vmask, int wb, int64_t max_rows, cudaStream_t s, Scratch& sc, int32_t* d_err,
+                      PartRecords* out);
+
+// unique / count distinct by partition (distinct_part.cu): the number of groups,
+// or NFC_ERR_UNSUPPORTED where the sorted forms are to be used.
+int64_t unique_by_partition(const int32_t* keys, int64_t n, int32_t* uniq_out, int32_t* first_out,
+                            int64_t* counts_out, int32_t* inv_out, cudaStream_t s);
+int64_t count_distinct_by_partition(const int32_t* keys, const uint8_t* key_validity, const int32_t* values,
+                                    const uint8_t* value_validity, int64_t n, int64_t out_cap, int64_t* ukeys_out,
+                                    int64_t* nunique_out, cudaStream_t s);
+
 // HASH strategy (hash.cu): global open-addressing table keyed by the raw
 // int32 key, then a radix sort of the occupied slots by key.
 int run_hash(const nfc_groupby_args* a, const ColSet& cs, const OutSet& o, const nfc_probe& p,

@@ -155,7 +155,8 @@ struct PartPlan {
   int64_t* offs;        // [nb+1] record offsets
   uint32_t* cursor;     // [nb]   scatter cursors
   int32_t* merge_slot;  // [nb]   merge-state slot of a bucket of several slices, else -1
-  int32_t* n_merge;     // [3]    merge slots, slices, skew (1: one bucket holds over half of the records)
+  int32_t* n_merge;     // [4]    merge slots, slices, skew (1: one bucket holds over half of the records),
+                        //        records of the largest bucket
   int2* multi;          // [max slices] per merge slot: its bucket, its first slice
   int2* slices;         // [max slices] (bucket, slice number)
 };
@@ -217,6 +218,7 @@ __global__ void __launch_bounds__(1024) k_part_plan(const uint32_t* __restrict__
     pl.n_merge[0] = n_multi;
     pl.n_merge[1] = n_slices;
     pl.n_merge[2] = s_most > t_rows / 2 ? 1 : 0;
+    pl.n_merge[3] = (int32_t)s_most;
   }
   // The slices of each large bucket, a warp per bucket.
   for (int32_t i = threadIdx.x >> 5; i < n_multi; i += blockDim.x >> 5) {
@@ -494,7 +496,7 @@ __global__ void __launch_bounds__(kPartThreads, 2) k_part_pass1(const int32_t* _
     if (vmask) bulk_g2s_hint(dst + L.off_vmask, vmask + (row0 >> 5), L.bytes_vmask, &bars[st], pol_in);
 #pragma unroll
     for (int c = 0; c < NC; ++c)
-      bulk_g2s_hint(dst + L.off_col[c],
+      if (col_dt<SIG>(cs, c) != kRowId) bulk_g2s_hint(dst + L.off_col[c],
                     static_cast<const unsigned char*>(cs.data[c]) + (size_t)row0 * (L.bytes_col[c] / kBulkTile),
                     L.bytes_col[c], &bars[st], pol_in);
   };
@@ -548,7 +550,9 @@ __global__ void __launch_bounds__(kPartThreads, 2) k_part_pass1(const int32_t* _
       uint64_t rv[NC > 0 ? NC : 1];
 #pragma unroll
       for (int c = 0; c < NC; ++c)
-        rv[c] = col_dt<SIG>(cs, c) == NFC_I32
+        rv[c] = col_dt<SIG>(cs, c) == kRowId
+                    ? (uint64_t)((blockIdx.x + k * (int64_t)gridDim.x) * kBulkTile + i)
+                : col_dt<SIG>(cs, c) == NFC_I32
                     ? (uint64_t)(int64_t) reinterpret_cast<const int32_t*>(sp + L.off_col[c])[i]
                     : reinterpret_cast<const uint64_t*>(sp + L.off_col[c])[i];
       wide |= wide_bits<NC, SIG>(cs, rv);
@@ -586,8 +590,9 @@ __global__ void __launch_bounds__(kPartThreads) k_part_pass1_tail(const int32_t*
     uint64_t rv[NC > 0 ? NC : 1];
 #pragma unroll
     for (int c = 0; c < NC; ++c)
-      rv[c] = col_dt<SIG>(cs, c) == NFC_I32 ? (uint64_t)(int64_t) static_cast<const int32_t*>(cs.data[c])[i]
-                                            : static_cast<const uint64_t*>(cs.data[c])[i];
+      rv[c] = col_dt<SIG>(cs, c) == kRowId    ? (uint64_t)i
+              : col_dt<SIG>(cs, c) == NFC_I32 ? (uint64_t)(int64_t) static_cast<const int32_t*>(cs.data[c])[i]
+                                              : static_cast<const uint64_t*>(cs.data[c])[i];
     wide |= wide_bits<NC, SIG>(cs, rv);
     rec_store<NC, PACK0>(out + (size_t)pos * NW, d & keep_mask, rv);
   }
@@ -1018,6 +1023,7 @@ __global__ void __launch_bounds__(kPartThreads, 2) k_part_agg(PartAggArgs a) {
 // ---------------------------------------------------------------- host
 constexpr int64_t kMaxBuckets = 28672;  // two shared 32-bit tables of them in the plain scatter
 constexpr int64_t kMaxWideBuckets = 16384;
+constexpr int64_t kMaxRecordBuckets = 32768;  // 256 coarse buckets of 128
 constexpr int64_t kSlice = 65536;  // <= 65536 keeps the 16-bit-split int32 sums exact
 constexpr int64_t kMinSlice = 8192;
 constexpr size_t kAggSmemBudget = 200 * 1024;
@@ -1069,8 +1075,72 @@ struct PartLaunch {
   int32_t* d_err;
 };
 
+// The coalesced two-level scatter, where it applies.
+static void set_layout(PartLaunch& q) {
+  // Coalesced scatter: 16-byte aligned inputs, coarse fan-out <= kMaxPassBins,
+  // TMA stages + the tile's sort buffer fit in shared memory.
+  if (q.al && (reinterpret_cast<uintptr_t>(q.vmask) & 15u) == 0 && q.nc <= kMaxPassBins) {
+    BulkLayout& L = q.L;
+    uint32_t off = kBulkTile * 4;
+    L.bytes_keys = kBulkTile * 4;
+    L.off_vmask = off;
+    L.bytes_vmask = kBulkTile / 8;
+    if (q.vmask) off += L.bytes_vmask;
+    for (int c = 0; c < q.cs.ncols; ++c) {
+      off = (off + 15u) & ~15u;
+      L.off_col[c] = off;
+      L.bytes_col[c] = q.cs.dtype[c] == kRowId ? 0u : kBulkTile * (uint32_t)dtype_bytes(q.cs.dtype[c]);
+      off += L.bytes_col[c];
+    }
+    L.stage_bytes = (off + 127u) & ~127u;
+    // Three stages within half an SM's shared memory (two CTAs per SM), else
+    // as many as one CTA can hold.
+    for (const size_t budget : {kPass1SmemPerSm / 2, kPass1SmemPerCta}) {
+      L.stages = 3;
+      while (L.stages >= 2 && pass1_smem(L) > budget) --L.stages;
+      if (L.stages >= 2) break;
+    }
+    if (L.stages >= 2) {
+      q.coalesced = true;
+      q.nfull = q.a->n / kBulkTile;
+    }
+  }
+}
+
+static int launch_hist(const PartLaunch& q, uint32_t* ghist, cudaStream_t s, StageTimer* tm) {
+  {
+    // Full tiles through the bulk-copy histogram when the keys and the
+    // combined bitmap are 16-byte aligned; the remaining rows (or all of
+    // them) through k_part_hist.
+    int64_t hfull = 0;
+    if ((reinterpret_cast<uintptr_t>(q.a->keys) & 15u) == 0 && (reinterpret_cast<uintptr_t>(q.vmask) & 15u) == 0)
+      hfull = q.a->n / kHistTile;
+    if (hfull > 0) {
+      const size_t smem = 128 + (size_t)kHistStages * kHistStageBytes + (size_t)q.nb * 4;
+      NFC_CUDA(cudaFuncSetAttribute(k_part_hist_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      const int per_sm = 2 * (smem + 1024) <= 228 * 1024 ? 2 : 1;
+      const int64_t g = std::max<int64_t>(1, std::min<int64_t>(hfull, (int64_t)num_sms() * per_sm));
+      k_part_hist_bulk<<<(unsigned)g, 512, smem, s>>>(q.a->keys, q.vmask, hfull, q.kmin, q.wb, q.nb, ghist, q.d_err);
+      NFC_CUDA(cudaGetLastError());
+      tm->launched();
+    }
+    const int64_t r0 = hfull * kHistTile;
+    if (q.a->n > r0) {
+      const int64_t ntiles128 = (q.a->n - r0 + 127) / 128;
+      const size_t smem = (size_t)q.nb * 4;
+      NFC_CUDA(cudaFuncSetAttribute(k_part_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      const int64_t g = std::max<int64_t>(1, std::min<int64_t>((ntiles128 + 15) / 16, (int64_t)num_sms() * 4));
+      k_part_hist<<<(unsigned)g, 256, smem, s>>>(q.a->keys + r0, q.vmask ? q.vmask + (r0 >> 5) : nullptr, q.a->n - r0,
+                                                  q.al, q.kmin, q.wb, q.nb, ghist);
+      NFC_CUDA(cudaGetLastError());
+      tm->launched();
+    }
+  }
+  return NFC_OK;
+}
+
 template <int NC, bool PACK0, uint32_t SIG>
-static int launch_part(const PartLaunch& q, PartAggArgs& pa, cudaStream_t s, StageTimer* tm) {
+static int launch_records(const PartLaunch& q, const int32_t* skew, cudaStream_t s, StageTimer* tm) {
   const nfc_groupby_args* a = q.a;
   constexpr int NW = Rec<NC, PACK0>::NW;
   if (q.coalesced) {
@@ -1086,7 +1156,7 @@ static int launch_part(const PartLaunch& q, PartAggArgs& pa, cudaStream_t s, Sta
       const int64_t g = std::max<int64_t>(1, std::min<int64_t>(q.nfull, (int64_t)num_sms() * per_sm));
       k_part_pass1<NC, PACK0, SIG><<<(unsigned)g, kPartThreads, smem, s>>>(a->keys, q.vmask, q.cs, q.L, q.nfull,
                                                                           q.kmin, shift, q.nc, keep, cur1, out1,
-                                                                          q.d_err, q.wide, pa.n_merge + 2);
+                                                                          q.d_err, q.wide, skew);
       NFC_CUDA(cudaGetLastError());
       tm->launched();
     }
@@ -1103,7 +1173,7 @@ static int launch_part(const PartLaunch& q, PartAggArgs& pa, cudaStream_t s, Sta
       const int64_t nt2 = (q.nv + refine2_tile<NW>() - 1) / refine2_tile<NW>();
       const int64_t g2 = std::max<int64_t>(1, std::min<int64_t>(nt2, (int64_t)num_sms() * 2));
       k_part_refine<NW><<<(unsigned)g2, kPartThreads, smem2, s>>>(q.rec_a, q.nv, q.wb, q.cursor, q.rec, q.d_err,
-                                                              pa.n_merge + 2);
+                                                              skew);
       NFC_CUDA(cudaGetLastError());
       tm->launched();
     }
@@ -1119,6 +1189,14 @@ static int launch_part(const PartLaunch& q, PartAggArgs& pa, cudaStream_t s, Sta
     NFC_CUDA(cudaGetLastError());
     tm->launched();
   }
+  return NFC_OK;
+}
+
+template <int NC, bool PACK0, uint32_t SIG>
+static int launch_part(const PartLaunch& q, PartAggArgs& pa, cudaStream_t s, StageTimer* tm) {
+  constexpr int NW = Rec<NC, PACK0>::NW;
+  const int rc = launch_records<NC, PACK0, SIG>(q, pa.n_merge + 2, s, tm);
+  if (rc) return rc;
   tm->mark(s);
   NFC_CUDA(cudaFuncSetAttribute(k_part_agg<NC, PACK0, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)q.agg_smem));
@@ -1210,34 +1288,7 @@ int run_partition(const nfc_groupby_args* a, const ColSet& cs_in, const OutSet& 
   // pass's fan-out too wide.
   q.cshift = nb <= (kMaxPassBins << 6) ? 6 : 7;
   q.nc = q.two_level ? (int32_t)((nb + (1 << q.cshift) - 1) >> q.cshift) : nb;
-  // Coalesced scatter: 16-byte aligned inputs, coarse fan-out <= kMaxPassBins,
-  // TMA stages + the tile's sort buffer fit in shared memory.
-  if (q.al && (reinterpret_cast<uintptr_t>(vmask) & 15u) == 0 && q.nc <= kMaxPassBins) {
-    BulkLayout& L = q.L;
-    uint32_t off = kBulkTile * 4;
-    L.bytes_keys = kBulkTile * 4;
-    L.off_vmask = off;
-    L.bytes_vmask = kBulkTile / 8;
-    if (vmask) off += L.bytes_vmask;
-    for (int c = 0; c < cs.ncols; ++c) {
-      off = (off + 15u) & ~15u;
-      L.off_col[c] = off;
-      L.bytes_col[c] = kBulkTile * (uint32_t)dtype_bytes(cs.dtype[c]);
-      off += L.bytes_col[c];
-    }
-    L.stage_bytes = (off + 127u) & ~127u;
-    // Three stages within half an SM's shared memory (two CTAs per SM), else
-    // as many as one CTA can hold.
-    for (const size_t budget : {kPass1SmemPerSm / 2, kPass1SmemPerCta}) {
-      L.stages = 3;
-      while (L.stages >= 2 && pass1_smem(L) > budget) --L.stages;
-      if (L.stages >= 2) break;
-    }
-    if (L.stages >= 2) {
-      q.coalesced = true;
-      q.nfull = a->n / kBulkTile;
-    }
-  }
+  set_layout(q);
 
   struct {
     uint32_t* ghist; int64_t* offs; uint32_t* cursor; int32_t* merge_slot;
@@ -1256,38 +1307,14 @@ int run_partition(const nfc_groupby_args* a, const ColSet& cs_in, const OutSet& 
   w.cursor = reinterpret_cast<uint32_t*>(qq); qq += 4 * nbp;
   w.merge_slot = reinterpret_cast<int32_t*>(qq); qq += 4 * nbp;
   q.ccursor = reinterpret_cast<uint32_t*>(qq); qq += 4 * ncp;
-  w.n_merge = reinterpret_cast<int32_t*>(qq); qq += 12;
+  w.n_merge = reinterpret_cast<int32_t*>(qq); qq += 16;
   w.ticket = reinterpret_cast<uint32_t*>(qq); qq += 8;
   q.wide = reinterpret_cast<uint32_t*>(qq); qq += 8;
   q.cursor = w.cursor;
 
   {
-    // Full tiles through the bulk-copy histogram when the keys and the
-    // combined bitmap are 16-byte aligned; the remaining rows (or all of
-    // them) through k_part_hist.
-    int64_t hfull = 0;
-    if ((reinterpret_cast<uintptr_t>(a->keys) & 15u) == 0 && (reinterpret_cast<uintptr_t>(vmask) & 15u) == 0)
-      hfull = a->n / kHistTile;
-    if (hfull > 0) {
-      const size_t smem = 128 + (size_t)kHistStages * kHistStageBytes + (size_t)nb * 4;
-      NFC_CUDA(cudaFuncSetAttribute(k_part_hist_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      const int per_sm = 2 * (smem + 1024) <= 228 * 1024 ? 2 : 1;
-      const int64_t g = std::max<int64_t>(1, std::min<int64_t>(hfull, (int64_t)num_sms() * per_sm));
-      k_part_hist_bulk<<<(unsigned)g, 512, smem, s>>>(a->keys, vmask, hfull, q.kmin, wb, nb, w.ghist, d_err);
-      NFC_CUDA(cudaGetLastError());
-      tm->launched();
-    }
-    const int64_t r0 = hfull * kHistTile;
-    if (a->n > r0) {
-      const int64_t ntiles128 = (a->n - r0 + 127) / 128;
-      const size_t smem = (size_t)nb * 4;
-      NFC_CUDA(cudaFuncSetAttribute(k_part_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      const int64_t g = std::max<int64_t>(1, std::min<int64_t>((ntiles128 + 15) / 16, (int64_t)num_sms() * 4));
-      k_part_hist<<<(unsigned)g, 256, smem, s>>>(a->keys + r0, vmask ? vmask + (r0 >> 5) : nullptr, a->n - r0,
-                                                  q.al, q.kmin, wb, nb, w.ghist);
-      NFC_CUDA(cudaGetLastError());
-      tm->launched();
-    }
+    const int rc = launch_hist(q, w.ghist, s, tm);
+    if (rc) return rc;
   }
   // Slices of an equal share of the chip, within [kMinSlice, kSlice]: at 2M rows
   // slices of 65,536 leave 30 CTAs with 130 us of work each.  A bucket of more
@@ -1350,6 +1377,67 @@ int run_partition(const nfc_groupby_args* a, const ColSet& cs_in, const OutSet& 
   }
   if (rc) return rc;
   tm->mark(s);
+  return NFC_OK;
+}
+
+int partition_records(const nfc_groupby_args* a, int32_t dtype, const void* values, const nfc_probe& p,
+                      const uint32_t* vmask, int wb, int64_t max_rows, cudaStream_t s, Scratch& sc, int32_t* d_err,
+                      PartRecords* out) {
+  const int64_t m = p.kmax - p.kmin + 1;
+  const int64_t nb = (m + (1ll << wb) - 1) >> wb;
+  if (nb > kMaxRecordBuckets || p.n_valid == 0) return NFC_ERR_UNSUPPORTED;
+  PartLaunch q{};
+  q.a = a;
+  q.cs.ncols = 1;
+  q.cs.dtype[0] = dtype;
+  q.cs.aggs[0] = NFC_AGG_SUM;
+  q.cs.data[0] = values;
+  q.vmask = vmask;
+  q.al = (reinterpret_cast<uintptr_t>(a->keys) & 15u) == 0 && (reinterpret_cast<uintptr_t>(values) & 15u) == 0;
+  q.kmin = (int32_t)p.kmin;
+  q.wb = wb;
+  q.nb = (int32_t)nb;
+  q.d_err = d_err;
+  q.nv = p.n_valid;
+  q.two_level = nb > 128;
+  q.cshift = nb <= (kMaxPassBins << 6) ? 6 : 7;
+  q.nc = q.two_level ? (int32_t)((nb + (1 << q.cshift) - 1) >> q.cshift) : (int32_t)nb;
+  set_layout(q);
+  if (!q.coalesced) return NFC_ERR_UNSUPPORTED;
+  // offs i64 | ghist, cursor, merge_slot, ccursor u32 | n_merge[4], wide
+  const size_t nbp = (size_t)nb + 1, ncp = (size_t)q.nc + 1;
+  unsigned char* small = nullptr;
+  const size_t small_bytes = nbp * (8 + 4 + 4 + 4) + ncp * 4 + 64;
+  NFC_CUDA(sc.alloc(&small, small_bytes));
+  NFC_CUDA(cudaMemsetAsync(small, 0, small_bytes, s));
+  PartPlan pl{};
+  pl.offs = reinterpret_cast<int64_t*>(small);
+  uint32_t* ghist = reinterpret_cast<uint32_t*>(pl.offs + nbp);
+  pl.cursor = ghist + nbp;
+  pl.merge_slot = reinterpret_cast<int32_t*>(pl.cursor + nbp);
+  q.ccursor = reinterpret_cast<uint32_t*>(pl.merge_slot + nbp);
+  pl.n_merge = reinterpret_cast<int32_t*>(q.ccursor + ncp);
+  q.wide = reinterpret_cast<uint32_t*>(pl.n_merge + 4);
+  q.cursor = pl.cursor;
+  StageTimer tm;
+  int rc = launch_hist(q, ghist, s, &tm);
+  if (rc) return rc;
+  NFC_CUDA(cudaFuncSetAttribute(k_part_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(nb * 4)));
+  // A slice longer than any bucket: nothing is split.
+  k_part_plan<<<1, 1024, (size_t)nb * 4, s>>>(ghist, q.nb, INT32_MAX, q.cshift, q.two_level ? q.ccursor : nullptr, pl);
+  NFC_CUDA(cudaGetLastError());
+  int32_t most = 0;
+  NFC_CUDA(readback(&most, pl.n_merge + 3, sizeof(most), s));
+  if (most > max_rows) return NFC_ERR_UNSUPPORTED;
+  if (q.two_level) NFC_CUDA(sc.alloc(&q.rec_a, (size_t)p.n_valid + 2));  // +2: 16-byte tail of the refine copies
+  NFC_CUDA(sc.alloc(&q.rec, (size_t)p.n_valid));
+  rc = dtype == kRowId ? launch_records<1, true, sig_col(0, kRowId, 0)>(q, pl.n_merge + 2, s, &tm)
+                       : launch_records<1, true, kSigI32Sum>(q, pl.n_merge + 2, s, &tm);
+  if (rc) return rc;
+  out->rec = q.rec;
+  out->offs = pl.offs;
+  out->nb = q.nb;
+  out->most = most;
   return NFC_OK;
 }
 

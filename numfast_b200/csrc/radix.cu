@@ -668,6 +668,10 @@ extern "C" int64_t nfc_unique(const int32_t* keys, int64_t n, int32_t* uniq_out,
       return ng;
     }
   }
+  {
+    const int64_t ng = unique_by_partition(keys, n, uniq_out, first_out, counts_out, inv_out, s);
+    if (ng != NFC_ERR_UNSUPPORTED) return ng;
+  }
   uint32_t *k0 = nullptr, *k1 = nullptr, *v0 = nullptr, *v1 = nullptr, *kres = nullptr, *vres = nullptr;
   NFC_CUDA(sc.alloc(&k0, (size_t)n));
   NFC_CUDA(sc.alloc(&k1, (size_t)n));

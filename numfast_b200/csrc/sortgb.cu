@@ -4,7 +4,7 @@
 // for a dense index: a sorted unique with inverse codes, then per-group
 // bincounts (src/Drivers/CPU/_lib/groupindex.py:178-211; planner.py:254-262).
 // Here:
-//   1. positions of the valid rows, sorted stably by key (onesweep radix
+//   1. positions of the valid rows, sorted stably by key (radix
 //      sort of (key, row) pairs, radix.cu)
 //   2. k_sort_runs: tiles of 1024 sorted positions; run heads by comparing
 //      neighbouring keys, run ids by a block scan plus a decoupled look-back
