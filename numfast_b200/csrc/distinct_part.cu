@@ -11,8 +11,8 @@
 //                   per key
 // Against the sorted forms (radix_sort.cu) that is two passes of 8-byte records
 // instead of four of pairs (or of one per eight bits of the pair), and no run
-// pass: 200M keys over the full int32 range 5.85 -> 3.93 ms, COUNT DISTINCT of
-// 50M rows over 1M keys 2.10 -> 1.58 ms.  Rows that do not spread over the
+// pass: 200M keys over the full int32 range 5.85 -> 3.89 ms, COUNT DISTINCT of
+// 50M rows over 1M keys 2.10 -> 1.28 ms.  Rows that do not spread over the
 // buckets (few keys, skew) and small inputs stay with the sort: a bucket has to
 // fit one CTA.
 #include <algorithm>
@@ -39,17 +39,72 @@ struct DpArgs {
   int32_t* err;
 };
 
-// The bucket's place among the outputs: warp 0 looks back, everyone gets it.
-NFC_DEV int64_t dp_base(const DpArgs& a, int32_t b, uint32_t total, int64_t* s_base) {
-  if (threadIdx.x < 32) {
-    const int64_t ex = lookback_exclusive(a.lb, b, total, a.err);  // whole warp
-    if (threadIdx.x == 0) {
-      *s_base = ex;
-      if (b == a.nb - 1) *a.ng_out = ex + total;
+// The bucket's place among the outputs.  The whole CTA looks back, 512 buckets
+// at a time: the CTAs of a wave reach this point together, and a warp's walk
+// over the 444 of them, 32 at a time, is 14 loads one after the other (unique of
+// 200M rows 1,470 -> 1,425 us, with the totals published before the counts).
+// dp_publish makes the bucket's total known; dp_base returns the place to every
+// thread.
+NFC_DEV void dp_publish(const DpArgs& a, int32_t b, uint32_t total) {
+  if (threadIdx.x == 0) lb_store(a.lb + b, (b == 0 ? kLbInc : kLbAgg) | (uint64_t)total);
+}
+
+struct DpWalk {
+  uint64_t sum[kDpWarps];
+  int32_t state[kDpWarps];  // 0 totals only, 1 ends at an inclusive one, 2 one is not published yet
+};
+
+NFC_DEV int64_t dp_base(const DpArgs& a, int32_t b, uint32_t total, DpWalk* sw) {
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  uint64_t excl = 0;
+  if (b > 0) {  // the same for every thread, as is every branch below
+    int32_t j = b - 1;
+    uint32_t spins = 0;
+    while (true) {
+      const int32_t t = j - (int32_t)threadIdx.x;
+      const uint64_t w = t >= 0 ? ld_volatile_u64(a.lb + t) : kLbInc;
+      const uint64_t flag = w & ~kLbVal;
+      const unsigned inc = __ballot_sync(0xffffffffu, flag == kLbInc);
+      const unsigned pending = __ballot_sync(0xffffffffu, flag == 0);
+      const unsigned upto = inc ? (((inc & (0u - inc)) << 1) - 1u) : 0xffffffffu;  // lanes 0 .. first inclusive
+      const uint64_t v = warp_sum((upto >> lane) & 1u ? (w & kLbVal) : 0ull);
+      if (lane == 0) {
+        sw->sum[warp] = v;
+        sw->state[warp] = (pending & upto) ? 2 : inc ? 1 : 0;
+      }
+      __syncthreads();
+      const int32_t st = lane < kDpWarps ? sw->state[lane] : 0;
+      const unsigned done = __ballot_sync(0xffffffffu, st == 1), wait = __ballot_sync(0xffffffffu, st == 2);
+      const unsigned stop = done | wait;
+      const unsigned use = stop ? (((stop & (0u - stop)) << 1) - 1u) : 0xffffffffu;  // warps 0 .. first that stops
+      const uint64_t part = warp_sum(lane < kDpWarps && ((use >> lane) & 1u) ? sw->sum[lane] : 0ull);
+      __syncthreads();
+      if (wait & use) {  // read these again
+        if (++spins > kSpinLimit) {
+          if (threadIdx.x == 0) atomicExch(a.err, NFC_ERR_TIMEOUT);
+          break;
+        }
+        continue;
+      }
+      excl += part;
+      if (done & use) break;
+      j -= kDpThreads;
     }
   }
+  if (threadIdx.x == 0) {
+    if (b > 0) {
+      __threadfence();
+      lb_store(a.lb + b, kLbInc | (excl + total));
+    }
+    if (b == a.nb - 1) *a.ng_out = (int64_t)(excl + total);
+  }
+  return (int64_t)excl;
+}
+
+NFC_DEV int32_t dp_claim(const DpArgs& a, int32_t* s_bucket) {
+  if (threadIdx.x == 0) *s_bucket = (int32_t)atomicAdd(a.ticket, 1u);
   __syncthreads();
-  return *s_base;
+  return *s_bucket;
 }
 
 // How the rows are cut up.  wb: the widest bucket (2^wb keys, lo <= wb <= hi) of
@@ -139,14 +194,8 @@ __global__ void __launch_bounds__(kDpSampleThreads) k_dp_sample(const int32_t* _
   if (tid == 0) *ok = s_max <= 12 + share + share / 2 ? 1 : 0;
 }
 
-NFC_DEV int32_t dp_claim(const DpArgs& a, int32_t* s_bucket) {
-  if (threadIdx.x == 0) *s_bucket = (int32_t)atomicAdd(a.ticket, 1u);
-  __syncthreads();
-  return *s_bucket;
-}
-
 // ---------------------------------------------------------------- unique
-// 200M rows in 32,768 buckets of 2^17 keys: 1,470 us, 3.3 TB/s; latency of the
+// 200M rows in 32,768 buckets of 2^17 keys: 1,425 us, 3.4 TB/s; issue (62%) and the latency of the
 // record loads and shared atomics, with three CTAs per SM (two, with 32-bit
 // counts and ranks: 2,017 us).
 // Shared memory: bits[words] | first[most] | count[most] u16 | prefix[words]
@@ -157,7 +206,7 @@ __global__ void __launch_bounds__(kDpThreads, 3) k_dp_unique(DpArgs a, int32_t m
                                                             int64_t* __restrict__ counts, int32_t* __restrict__ inv) {
   extern __shared__ __align__(16) uint32_t dp_smem[];
   __shared__ uint32_t s_scan[33];
-  __shared__ int64_t s_base;
+  __shared__ DpWalk s_walk;
   __shared__ int32_t s_bucket;
   const int32_t b = dp_claim(a, &s_bucket);
   const int32_t words = (1 << a.wb) >> 5;
@@ -193,6 +242,7 @@ __global__ void __launch_bounds__(kDpThreads, 3) k_dp_unique(DpArgs a, int32_t m
     total += t;
     __syncthreads();
   }
+  dp_publish(a, b, total);
   auto rank_of = [&](uint32_t k) {
     return (uint32_t)prefix[k >> 5] + (uint32_t)__popc(bits[k >> 5] & ((1u << (k & 31)) - 1u));
   };
@@ -203,7 +253,8 @@ __global__ void __launch_bounds__(kDpThreads, 3) k_dp_unique(DpArgs a, int32_t m
     atomicMin(&first[q], (uint32_t)(r >> 32));
     atomicAdd(&cnt[q >> 1], 1u << (16 * (q & 1)));
   }
-  const int64_t base = dp_base(a, b, total, &s_base);
+  __syncthreads();
+  const int64_t base = dp_base(a, b, total, &s_walk);
   for (uint32_t i = threadIdx.x; i < total; i += kDpThreads) {
     first_out[base + i] = (int32_t)first[i];
     counts[base + i] = (int64_t)reinterpret_cast<const uint16_t*>(cnt)[i];
@@ -221,8 +272,9 @@ __global__ void __launch_bounds__(kDpThreads, 3) k_dp_unique(DpArgs a, int32_t m
 }
 
 // ---------------------------------------------------------------- count distinct
-// 47.5M records in 15,625 buckets: 710 us, bound by the walks' shared-memory
-// round trips and the 64-bit compare-and-swap of each new pair.
+// 47.5M records in 7,813 buckets: 551 us, bound by the walks' shared-memory
+// round trips and the 64-bit compare-and-swap of each new pair (with linear
+// probing and a loop per record 1,538; at half that load 710).
 // Shared memory: set[slots] u64 | distinct[keys of a bucket] u32.  A record is
 // its own hash key (the key part is below 2^wb, so all ones is free).
 constexpr uint64_t kDpEmpty = ~0ull;
@@ -231,7 +283,7 @@ __global__ void __launch_bounds__(kDpThreads, 3) k_dp_count(DpArgs a, int lg_slo
                                                            int64_t* __restrict__ nunique) {
   extern __shared__ __align__(16) uint64_t dp_set[];
   __shared__ uint32_t s_warp[kDpWarps];
-  __shared__ int64_t s_base;
+  __shared__ DpWalk s_walk;
   __shared__ int32_t s_bucket;
   const int32_t b = dp_claim(a, &s_bucket);
   const int32_t slots = 1 << lg_slots, W = 1 << a.wb;
@@ -243,23 +295,34 @@ __global__ void __launch_bounds__(kDpThreads, 3) k_dp_count(DpArgs a, int lg_slo
     reinterpret_cast<ulonglong2*>(dp_set)[i] = make_ulonglong2(kDpEmpty, kDpEmpty);
   for (int i = threadIdx.x; i < W; i += kDpThreads) distinct[i] = 0u;
   __syncthreads();
-#pragma unroll 4
-  for (int i = threadIdx.x; i < n; i += kDpThreads) {
-    const uint64_t r = __ldg(rec + i);
-    const uint32_t k = (uint32_t)r;
-    uint32_t h = (((uint32_t)(r >> 32) * 0x9E3779B1u) ^ (k * 0x85EBCA77u)) * 0xC2B2AE3Du >> (32 - lg_slots);
-    // At most 3/4 of the slots are taken, so a free one ends the walk.
-    for (int probe = 0; probe < slots; ++probe) {
-      uint64_t cur = *reinterpret_cast<volatile uint64_t*>(&dp_set[h]);
-      if (cur == kDpEmpty)
-        cur = atomicCAS(reinterpret_cast<unsigned long long*>(&dp_set[h]), (unsigned long long)kDpEmpty,
-                        (unsigned long long)r);
+  // Each lane walks through its own records, one slot an iteration, the next
+  // record loaded ahead: lanes with short walks go on while others still probe
+  // (a loop per record lasts as long as the longest of 32 walks).
+  const uint32_t mask = (uint32_t)slots - 1u;
+  auto hash = [](uint64_t r) {
+    return (((uint32_t)(r >> 32) * 0x9E3779B1u) ^ ((uint32_t)r * 0x85EBCA77u)) * 0xC2B2AE3Du;
+  };
+  int i = threadIdx.x;
+  uint64_t r = i < n ? __ldg(rec + i) : 0ull, next = i + kDpThreads < n ? __ldg(rec + i + kDpThreads) : 0ull;
+  uint32_t f = hash(r), h = f >> (32 - lg_slots);
+  while (i < n) {
+    uint64_t cur = *reinterpret_cast<volatile uint64_t*>(&dp_set[h]);
+    if (cur == kDpEmpty) {
+      cur = atomicCAS(reinterpret_cast<unsigned long long*>(&dp_set[h]), (unsigned long long)kDpEmpty,
+                      (unsigned long long)r);
       if (cur == kDpEmpty) {
-        atomicAdd(&distinct[k], 1u);
-        break;
+        atomicAdd(&distinct[(uint32_t)r], 1u);
+        cur = r;
       }
-      if (cur == r) break;
-      h = (h + 1) & (uint32_t)(slots - 1);
+    }
+    // An odd step reaches every slot, and more slots than records stay free.
+    h = (h + (f << 1 | 1u)) & mask;
+    if (cur == r) {
+      i += kDpThreads;
+      r = next;
+      next = i + kDpThreads < n ? __ldg(rec + i + kDpThreads) : 0ull;
+      f = hash(r);
+      h = f >> (32 - lg_slots);
     }
   }
   __syncthreads();
@@ -277,7 +340,8 @@ __global__ void __launch_bounds__(kDpThreads, 3) k_dp_count(DpArgs a, int lg_slo
     if (w < warp) mine += s_warp[w];
     total += s_warp[w];
   }
-  int64_t pos = dp_base(a, b, total, &s_base) + mine;
+  dp_publish(a, b, total);
+  int64_t pos = dp_base(a, b, total, &s_walk) + mine;
   const int64_t key0 = a.kmin + ((int64_t)b << a.wb);
   const unsigned lt = lanemask_lt();
   for (int g = g0; g < g1; g += 32) {
@@ -380,10 +444,9 @@ int64_t unique_by_partition(const int32_t* keys, int64_t n, int32_t* uniq_out, i
   return dp_finish(a, s);
 }
 
-// Rows per bucket: up to 5,400, so that the set of the largest bucket has 8,192
-// slots (64 KB, three CTAs per SM) and is at most 3/4 full; with 16,384 slots
-// there is one CTA per SM, which takes more than twice as long (50M rows:
-// 1,538 us), so that is left to inputs of more than 32,768 such buckets.
+// Rows per bucket: up to 6,200, so that the set of the largest bucket has 8,192
+// slots (64 KB, three CTAs per SM) and is at most 4/5 full.  16,384 slots leave
+// one CTA per SM; that is for inputs of more than 32,768 such buckets.
 int64_t count_distinct_by_partition(const int32_t* keys, const uint8_t* key_validity, const int32_t* values,
                                     const uint8_t* value_validity, int64_t n, int64_t out_cap, int64_t* ukeys_out,
                                     int64_t* nunique_out, cudaStream_t s) {
@@ -401,11 +464,11 @@ int64_t count_distinct_by_partition(const int32_t* keys, const uint8_t* key_vali
   g.cols = &col;
   DpArgs a{};
   int64_t most = 0, nv = 0;
-  const int rc = dp_prepare(&g, NFC_I32, values, DpRule{5400, 512, 12288, 0, 13}, s, sc, &a, &most, &nv);
+  const int rc = dp_prepare(&g, NFC_I32, values, DpRule{6200, 512, 13000, 0, 13}, s, sc, &a, &most, &nv);
   if (rc) return rc;
   if (out_cap < std::min<int64_t>(a.m, nv)) return NFC_ERR_UNSUPPORTED;
   int lg = 10;
-  while ((3ll << lg) / 4 < most) ++lg;
+  while ((4ll << lg) / 5 < most) ++lg;
   const size_t smem = ((size_t)8 << lg) + ((size_t)4 << a.wb);
   NFC_CUDA(cudaFuncSetAttribute(k_dp_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k_dp_count<<<(unsigned)a.nb, kDpThreads, smem, s>>>(a, lg, ukeys_out, nunique_out);
