@@ -139,6 +139,19 @@ NFC_DEV uint64_t ld_volatile_u64(const uint64_t* p) {
   return v;
 }
 
+// s += x; returns the rounding error of the addition, exactly (Knuth's two-sum:
+// s + error == old s + x; NaN once an infinity or NaN is involved).
+NFC_DEV double f64_two_sum(double& s, double x) {
+  const double old = s;
+  s = old + x;
+  const double got = s - old;
+  return (old - (s - got)) + (x - got);
+}
+
+// A sum and the errors of its additions as one number.  The errors are NaN when
+// the sum is infinite or NaN (or passed through an infinity); it then stands.
+NFC_DEV double f64_close(double s, double err) { return isfinite(err) ? s + err : s; }
+
 // Bit i of an LSB-first validity bitmap (Arrow layout).
 NFC_DEV bool bit_at(const uint8_t* bm, int64_t i) {
   return (bm[i >> 3] >> (i & 7)) & 1u;
