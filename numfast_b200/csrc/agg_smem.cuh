@@ -8,7 +8,8 @@
 // (bit c of `narrow`), as one signed 32-bit sum in the low array (exact for
 // the same 65,536 rows); float64
 // min/max use native 64-bit min/max on an order-preserving encoding;
-// float64 sums use the 64-bit float add.  agg_merge folds a slot into the
+// float64 sums use the 64-bit float add, with ERR also a second array for the
+// rounding errors of the additions.  agg_merge folds a slot into the
 // global state layout (StateRef) with global atomics.
 #pragma once
 
@@ -22,12 +23,13 @@ struct AggState {
   uint32_t* slo[NC > 0 ? NC : 1];   // int32 columns: sum of low 16-bit halves
   int32_t* shi[NC > 0 ? NC : 1];    // int32 columns: sum of high 16-bit halves
   uint64_t* s64[NC > 0 ? NC : 1];   // int64 / float64 columns: sum
+  double* err[NC > 0 ? NC : 1];     // float64 columns, ERR: rounding errors of the sum
   void* mn[NC > 0 ? NC : 1];
   void* mx[NC > 0 ? NC : 1];
   uint32_t narrow;  // bit c: int32 column c summed with one signed 32-bit atomic
 };
 
-template <int NC, uint32_t SIG>
+template <int NC, uint32_t SIG, bool ERR = false>
 NFC_DEV AggState<NC> carve_agg(const ColSet& cs, unsigned char* base, int w, uint32_t narrow = 0u) {
   AggState<NC> st;
   st.narrow = narrow;
@@ -35,9 +37,11 @@ NFC_DEV AggState<NC> carve_agg(const ColSet& cs, unsigned char* base, int w, uin
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     st.slo[c] = nullptr; st.shi[c] = nullptr; st.s64[c] = nullptr; st.mn[c] = nullptr; st.mx[c] = nullptr;
+    st.err[c] = nullptr;
     const bool wide = col_dt<SIG>(cs, c) != NFC_I32;
     const int ag = col_ag<SIG>(cs, c);
     if (wide && (ag & NFC_AGG_SUM)) { st.s64[c] = reinterpret_cast<uint64_t*>(p); p += 8 * w; }
+    if (ERR && col_dt<SIG>(cs, c) == NFC_F64 && (ag & NFC_AGG_SUM)) { st.err[c] = reinterpret_cast<double*>(p); p += 8 * w; }
     if (wide && (ag & NFC_AGG_MIN)) { st.mn[c] = p; p += 8 * w; }
     if (wide && (ag & NFC_AGG_MAX)) { st.mx[c] = p; p += 8 * w; }
   }
@@ -56,7 +60,7 @@ NFC_DEV AggState<NC> carve_agg(const ColSet& cs, unsigned char* base, int w, uin
   return st;
 }
 
-template <int NC, uint32_t SIG>
+template <int NC, uint32_t SIG, bool ERR = false>
 NFC_DEV void agg_init(const ColSet& cs, const AggState<NC>& st, int g) {
   st.cnt[g] = 0u;
 #pragma unroll
@@ -68,6 +72,7 @@ NFC_DEV void agg_init(const ColSet& cs, const AggState<NC>& st, int g) {
       if (ag & NFC_AGG_MAX) static_cast<int32_t*>(st.mx[c])[g] = INT_MIN;
     } else {
       if (ag & NFC_AGG_SUM) st.s64[c][g] = 0ull;
+      if (ERR && dt == NFC_F64 && (ag & NFC_AGG_SUM)) st.err[c][g] = 0.0;
       if (dt == NFC_I64) {
         if (ag & NFC_AGG_MIN) static_cast<int64_t*>(st.mn[c])[g] = LLONG_MAX;
         if (ag & NFC_AGG_MAX) static_cast<int64_t*>(st.mx[c])[g] = LLONG_MIN;
@@ -163,7 +168,7 @@ NFC_DEV void agg_apply(const ColSet& cs, const AggState<NC>& st, uint32_t g, con
 // minima / maxima as int64 / ordered float64 lanes) into slot g.  An int32
 // sum goes into the split halves as its own low 16 bits and the rest, which
 // keeps value = high * 65536 + low and the same bounds as k single rows.
-template <int NC, uint32_t SIG>
+template <int NC, uint32_t SIG, bool ERR = false>
 NFC_DEV void agg_apply_group(const ColSet& cs, const AggState<NC>& st, uint32_t g, uint32_t k, const uint64_t* sum,
                              const uint64_t* mn, const uint64_t* mx) {
   atomicAdd(&st.cnt[g], k);
@@ -187,7 +192,11 @@ NFC_DEV void agg_apply_group(const ColSet& cs, const AggState<NC>& st, uint32_t 
       if (ag & NFC_AGG_MIN) atomicMin(static_cast<long long*>(st.mn[c]) + g, (long long)mn[c]);
       if (ag & NFC_AGG_MAX) atomicMax(static_cast<long long*>(st.mx[c]) + g, (long long)mx[c]);
     } else {
-      if (ag & NFC_AGG_SUM) atomicAdd(reinterpret_cast<double*>(st.s64[c]) + g, __longlong_as_double((long long)sum[c]));
+      if (ag & NFC_AGG_SUM) {
+        double* dst = reinterpret_cast<double*>(st.s64[c]) + g;
+        if (ERR) f64_atomic_add_err(dst, st.err[c] + g, __longlong_as_double((long long)sum[c]));
+        else atomicAdd(dst, __longlong_as_double((long long)sum[c]));
+      }
       if (ag & NFC_AGG_MIN) atomicMin(static_cast<unsigned long long*>(st.mn[c]) + g, (unsigned long long)mn[c]);
       if (ag & NFC_AGG_MAX) atomicMax(static_cast<unsigned long long*>(st.mx[c]) + g, (unsigned long long)mx[c]);
     }
@@ -281,14 +290,17 @@ NFC_DEV void agg_merge_copies(const ColSet& cs, const StateRef& dst, const AggSt
   if (in && k && (lane_id() & ((1u << lg) - 1u)) == 0u) state_apply_group(cs, dst, e >> lg, k, sum, mn, mx);
 }
 
-template <int NC, uint32_t SIG>
+template <int NC, uint32_t SIG, bool ERR = false>
 NFC_DEV void agg_emit(const ColSet& cs, const AggState<NC>& st, int g, const OutSet& o, int64_t pos, int64_t key) {
   o.ukeys[pos] = key;
   o.counts[pos] = (int64_t)st.cnt[g];
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     const int dt = col_dt<SIG>(cs, c), ag = col_ag<SIG>(cs, c);
-    if (ag & NFC_AGG_SUM) static_cast<int64_t*>(o.sum[c])[pos] = agg_sum_bits<NC, SIG>(cs, st, c, g);
+    if (ERR && dt == NFC_F64 && (ag & NFC_AGG_SUM))
+      static_cast<double*>(o.sum[c])[pos] = f64_close(reinterpret_cast<const double*>(st.s64[c])[g], st.err[c][g]);
+    else if (ag & NFC_AGG_SUM)
+      static_cast<int64_t*>(o.sum[c])[pos] = agg_sum_bits<NC, SIG>(cs, st, c, g);
     if (dt == NFC_I32) {
       if (ag & NFC_AGG_MIN) static_cast<int32_t*>(o.mn[c])[pos] = static_cast<const int32_t*>(st.mn[c])[g];
       if (ag & NFC_AGG_MAX) static_cast<int32_t*>(o.mx[c])[pos] = static_cast<const int32_t*>(st.mx[c])[g];
@@ -362,8 +374,21 @@ NFC_DEV void hot_add(const ColSet& cs, HotAcc<NC>& a, const uint64_t* raw) {
   }
 }
 
+// One thread's accumulators into slot g.
+template <int NC, uint32_t SIG, bool ERR = false>
+NFC_DEV void hot_apply(const ColSet& cs, const AggState<NC>& st, uint32_t g, const HotAcc<NC>& a) {
+  uint64_t mn[NC > 0 ? NC : 1], mx[NC > 0 ? NC : 1];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const bool narrow = col_dt<SIG>(cs, c) == NFC_I32;
+    mn[c] = narrow ? (uint64_t)(int64_t)a.mn32[c] : a.mn64[c];
+    mx[c] = narrow ? (uint64_t)(int64_t)a.mx32[c] : a.mx64[c];
+  }
+  agg_apply_group<NC, SIG, ERR>(cs, st, g, a.cnt, a.sum, mn, mx);
+}
+
 // Reduce one hot key over the warp and fold it into slot g (whole warp).
-template <int NC, uint32_t SIG>
+template <int NC, uint32_t SIG, bool ERR = false>
 NFC_DEV void hot_flush(const ColSet& cs, const AggState<NC>& st, uint32_t g, const HotAcc<NC>& a) {
   const uint32_t k = __reduce_add_sync(0xffffffffu, a.cnt);
   if (k == 0u) return;
@@ -404,7 +429,7 @@ NFC_DEV void hot_flush(const ColSet& cs, const AggState<NC>& st, uint32_t g, con
       mx[c] = hi;
     }
   }
-  if (lane_id() == 0) agg_apply_group<NC, SIG>(cs, st, g, k, sum, mn, mx);
+  if (lane_id() == 0) agg_apply_group<NC, SIG, ERR>(cs, st, g, k, sum, mn, mx);
 }
 
 // The up to H slots of [0, w) with the most rows counted so far, at least

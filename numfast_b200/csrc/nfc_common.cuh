@@ -152,6 +152,14 @@ NFC_DEV double f64_two_sum(double& s, double x) {
 // the sum is infinite or NaN (or passed through an infinity); it then stands.
 NFC_DEV double f64_close(double s, double err) { return isfinite(err) ? s + err : s; }
 
+// *sum += x with the rounding error of that addition in *err, for any number of
+// threads: the old value the atomic returns gives the error exactly.
+NFC_DEV void f64_atomic_add_err(double* sum, double* err, double x) {
+  double s = atomicAdd(sum, x);
+  const double e = f64_two_sum(s, x);
+  if (!(e == 0.0)) atomicAdd(err, e);
+}
+
 // Bit i of an LSB-first validity bitmap (Arrow layout).
 NFC_DEV bool bit_at(const uint8_t* bm, int64_t i) {
   return (bm[i >> 3] >> (i & 7)) & 1u;

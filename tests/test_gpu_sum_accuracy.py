@@ -73,3 +73,26 @@ def test_sorted_sums_of_infinities_and_nan(cuda):
     with np.errstate(over="ignore", invalid="ignore"):
         want = v.reshape(-1, 20).sum(axis=1)
     np.testing.assert_array_equal(r.sums["f"].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("two_columns", [False, True])
+@pytest.mark.parametrize("order", ["sorted", None])
+@pytest.mark.parametrize("n,card", [(10_007, 10), (16_384, 40), (9_000, 250), (16_000, 1500)])
+def test_small_sums(cuda, n, card, order, two_columns):
+    keys = np.random.default_rng(card).integers(0, card, n, dtype=np.int32)
+    assert _mean_error(keys, card, "auto", two_columns, order) <= MEAN_BOUND
+
+
+def test_small_sums_of_infinities_and_nan(cuda):
+    k = np.arange(6000, dtype=np.int32) % 300
+    v = np.ones(6000)
+    v[5], v[905] = np.inf, np.inf
+    v[6], v[906] = np.inf, -np.inf
+    v[7] = np.nan
+    v[8], v[308] = 1.7e308, 1.7e308
+    v[9] = -np.inf
+    dev = torch.device("cuda")
+    r = D.groupby(torch.from_numpy(k).to(dev), [D.DeviceColumn("f", torch.from_numpy(v).to(dev), ("sum",))])
+    with np.errstate(over="ignore", invalid="ignore"):
+        want = v.reshape(-1, 300).sum(axis=0)
+    np.testing.assert_array_equal(r.sums["f"].cpu().numpy(), want)
