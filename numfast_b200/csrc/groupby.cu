@@ -357,12 +357,17 @@ __global__ void __launch_bounds__(512, 2) k_dense_smem_t(const int32_t* __restri
   }
   __syncthreads();
   if (lg_copies == 0) {
-    for (int g = threadIdx.x; g < m; g += blockDim.x) agg_merge<NC, SIG>(cs, gst, g, st, g);
+    for (int g = threadIdx.x; g < m; g += blockDim.x) agg_merge<NC, SIG, true>(cs, gst, g, st, g);
     return;
   }
-  // Groups of 2^lg_copies lanes combine the copies of one slot each.
-  for (int e0 = threadIdx.x & ~31; e0 < entries; e0 += blockDim.x)
+  // Groups of 2^lg_copies lanes combine the copies of one slot each.  Every CTA
+  // starts somewhere else: the CTAs of a wave get here together and would add to
+  // the same slots at the same time.
+  const int steps = (entries + 31) / 32, turn = (int)((blockIdx.x * 7u) % (uint32_t)steps);
+  for (int i = warp; i < steps; i += nwarps) {
+    const int e0 = (i + turn < steps ? i + turn : i + turn - steps) * 32;
     agg_merge_copies<NC, SIG>(cs, gst, st, e0 + lane, entries, lg_copies);
+  }
 }
 
 template <int NC, uint32_t SIG>
@@ -571,9 +576,10 @@ int run_dense(const nfc_groupby_args* a, const ColSet& cs, const OutSet& o, cons
   const size_t slot = state_bytes_per_slot(cs);
   void* gbase = nullptr;
   unsigned char* gb = nullptr;
-  NFC_CUDA(sc.alloc(&gb, (size_t)m * slot + 64));
+  // The CTAs of the shared-memory form each add a partial sum to every slot.
+  NFC_CUDA(sc.alloc(&gb, (size_t)m * (slot + (smem_variant ? state_err_bytes_per_slot(cs) : 0)) + 64));
   gbase = gb;
-  const StateRef gst = carve_state(cs, gbase, m);
+  const StateRef gst = carve_state(cs, gbase, m, smem_variant);
   k_state_init<<<grid_stream((m + 255) / 256, 8), 256, 0, s>>>(cs, gst, m);
   NFC_CUDA(cudaGetLastError());
   tm->launched();

@@ -62,6 +62,7 @@ static inline bool sums_only(const ColSet& cs) {
 //   sum[c]    i64 (integer columns) / f64
 //   mn[c]     i32 / i64 / ordered-u64 (f64 MIN lane encoding)
 //   mx[c]     i32 / i64 / ordered-u64 (f64 MAX lane encoding)
+//   err[c]    f64: rounding errors of the sum's additions, only where asked for
 // The same layout is used in shared memory and in global memory.
 // ---------------------------------------------------------------------
 struct StateRef {
@@ -69,9 +70,15 @@ struct StateRef {
   void* sum[NFC_MAX_COLS];
   void* mn[NFC_MAX_COLS];
   void* mx[NFC_MAX_COLS];
+  double* err[NFC_MAX_COLS];
 };
 
-// Bytes of state per slot for a column set.
+// Bytes of state per slot for a column set, of the errors on top of it.
+static inline size_t state_err_bytes_per_slot(const ColSet& cs) {
+  size_t b = 0;
+  for (int c = 0; c < cs.ncols; ++c) b += cs.dtype[c] == NFC_F64 && (cs.aggs[c] & NFC_AGG_SUM) ? 8 : 0;
+  return b;
+}
 static inline size_t state_bytes_per_slot(const ColSet& cs) {
   size_t b = 4;
   for (int c = 0; c < cs.ncols; ++c) {
@@ -84,14 +91,19 @@ static inline size_t state_bytes_per_slot(const ColSet& cs) {
 }
 
 // Carve a StateRef for `slots` entries out of base (8-byte arrays first).
-NFC_HD StateRef carve_state(const ColSet& cs, void* base, int64_t slots) {
+NFC_HD StateRef carve_state(const ColSet& cs, void* base, int64_t slots, bool errors = false) {
   StateRef st;
   char* p = static_cast<char*>(base);
   for (int c = 0; c < NFC_MAX_COLS; ++c) {
     st.sum[c] = st.mn[c] = st.mx[c] = nullptr;
+    st.err[c] = nullptr;
   }
   for (int c = 0; c < cs.ncols; ++c) {
     if (cs.aggs[c] & NFC_AGG_SUM) { st.sum[c] = p; p += 8 * slots; }
+    if (errors && cs.dtype[c] == NFC_F64 && (cs.aggs[c] & NFC_AGG_SUM)) {
+      st.err[c] = reinterpret_cast<double*>(p);
+      p += 8 * slots;
+    }
     if (dtype_bytes(cs.dtype[c]) == 8) {
       if (cs.aggs[c] & NFC_AGG_MIN) { st.mn[c] = p; p += 8 * slots; }
       if (cs.aggs[c] & NFC_AGG_MAX) { st.mx[c] = p; p += 8 * slots; }
@@ -114,6 +126,7 @@ NFC_DEV void state_init_slot(const ColSet& cs, const StateRef& st, int64_t d) {
     if (c >= cs.ncols) break;
     const int dt = cs.dtype[c], ag = cs.aggs[c];
     if (ag & NFC_AGG_SUM) static_cast<uint64_t*>(st.sum[c])[d] = 0ull;
+    if (st.err[c]) st.err[c][d] = 0.0;
     if (dt == NFC_I32) {
       if (ag & NFC_AGG_MIN) static_cast<int32_t*>(st.mn[c])[d] = INT_MAX;
       if (ag & NFC_AGG_MAX) static_cast<int32_t*>(st.mx[c])[d] = INT_MIN;
@@ -157,7 +170,8 @@ NFC_DEV void state_apply(const ColSet& cs, const StateRef& st, int64_t d, const 
 
 // Fold a combined row group -- k rows with the given per-column sums (int64
 // bits / float64 bits), minima and maxima (int64 / ordered float64 lanes) --
-// into slot d with one set of atomics.
+// into slot d with one set of atomics.  ERR: the state keeps rounding errors.
+template <bool ERR = false>
 NFC_DEV void state_apply_group(const ColSet& cs, const StateRef& st, int64_t d, uint32_t k, const uint64_t* sum,
                                const uint64_t* mn, const uint64_t* mx) {
   atomicAdd(&st.cnt[d], k);
@@ -166,7 +180,11 @@ NFC_DEV void state_apply_group(const ColSet& cs, const StateRef& st, int64_t d, 
     if (c >= cs.ncols) break;
     const int dt = cs.dtype[c], ag = cs.aggs[c];
     if (dt == NFC_F64) {
-      if (ag & NFC_AGG_SUM) atomicAdd(static_cast<double*>(st.sum[c]) + d, __longlong_as_double((long long)sum[c]));
+      if (ag & NFC_AGG_SUM) {
+        const double x = __longlong_as_double((long long)sum[c]);
+        if (ERR) f64_atomic_add_err(static_cast<double*>(st.sum[c]) + d, st.err[c] + d, x);
+        else atomicAdd(static_cast<double*>(st.sum[c]) + d, x);
+      }
       if (ag & NFC_AGG_MIN) atomicMin(static_cast<unsigned long long*>(st.mn[c]) + d, (unsigned long long)mn[c]);
       if (ag & NFC_AGG_MAX) atomicMax(static_cast<unsigned long long*>(st.mx[c]) + d, (unsigned long long)mx[c]);
     } else {
@@ -325,7 +343,10 @@ NFC_DEV void state_emit(const ColSet& cs, const StateRef& st, int64_t s, const O
   for (int c = 0; c < NFC_MAX_COLS; ++c) {
     if (c >= cs.ncols) break;
     const int dt = cs.dtype[c], ag = cs.aggs[c];
-    if (ag & NFC_AGG_SUM) static_cast<uint64_t*>(o.sum[c])[pos] = static_cast<const uint64_t*>(st.sum[c])[s];
+    if (st.err[c])
+      static_cast<double*>(o.sum[c])[pos] = f64_close(static_cast<const double*>(st.sum[c])[s], st.err[c][s]);
+    else if (ag & NFC_AGG_SUM)
+      static_cast<uint64_t*>(o.sum[c])[pos] = static_cast<const uint64_t*>(st.sum[c])[s];
     if (dt == NFC_I32) {
       if (ag & NFC_AGG_MIN) static_cast<int32_t*>(o.mn[c])[pos] = static_cast<const int32_t*>(st.mn[c])[s];
       if (ag & NFC_AGG_MAX) static_cast<int32_t*>(o.mx[c])[pos] = static_cast<const int32_t*>(st.mx[c])[s];

@@ -305,17 +305,14 @@ static int launch_small(const nfc_groupby_args* a, const ColSet& cs, const OutSe
   constexpr int kState = 96 * 1024;
   constexpr int kMost = 200 * 1024;  // with the errors: 8,191 slots of one float64 sum are 160 KB
   const size_t slot = state_bytes_per_slot(cs);
-  int errs = 0;
+  const size_t errs = state_err_bytes_per_slot(cs);
   bool wide = false;  // 32-bit atomics alone keep up on few keys
-  for (int c = 0; c < cs.ncols; ++c) {
-    errs += cs.dtype[c] == NFC_F64 && (cs.aggs[c] & NFC_AGG_SUM);
-    wide |= cs.dtype[c] != NFC_I32 && cs.aggs[c] != 0;
-  }
-  const int smem = kState + errs * 8 * (int)(kState / slot);
+  for (int c = 0; c < cs.ncols; ++c) wide |= cs.dtype[c] != NFC_I32 && cs.aggs[c] != 0;
+  const int smem = kState + (int)(errs * (kState / slot));
   NFC_CUDA(cudaFuncSetAttribute(k_small<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
-  k_small<NC><<<1, SmallShape<NC>::threads, smem, s>>>(a->keys, bitmaps_of(a), cs, (int)a->n, inputs_aligned(a), o, a->out_cap,
-                                          kState, (uint32_t)slot, 8u * (uint32_t)errs, wide ? kSmCopies : 0, vmask, rec,
-                                                        res);
+  k_small<NC><<<1, SmallShape<NC>::threads, smem, s>>>(a->keys, bitmaps_of(a), cs, (int)a->n, inputs_aligned(a), o,
+                                                       a->out_cap, kState, (uint32_t)slot, (uint32_t)errs,
+                                                       wide ? kSmCopies : 0, vmask, rec, res);
   NFC_CUDA(cudaGetLastError());
   return NFC_OK;
 }

@@ -96,3 +96,13 @@ def test_small_sums_of_infinities_and_nan(cuda):
     with np.errstate(over="ignore", invalid="ignore"):
         want = v.reshape(-1, 300).sum(axis=0)
     np.testing.assert_array_equal(r.sums["f"].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("two_columns", [False, True])
+@pytest.mark.parametrize("n,card,strategy", [(1_000_000, 100, "dense_smem"), (1_000_000, 1500, "dense_smem"),
+                                             (4_000_000, 365, "dense_smem"), (1_000_000, 1500, "partition"),
+                                             (2_000_000, 20_000, "partition"), (4_000_000, 365, "partition")])
+def test_sums_of_many_ctas(cuda, n, card, strategy, two_columns):
+    """Keys whose rows are spread over many CTAs or slices."""
+    keys = np.random.default_rng(card).integers(0, card, n, dtype=np.int32)
+    assert _mean_error(keys, card, strategy, two_columns, strategy) <= MEAN_BOUND
