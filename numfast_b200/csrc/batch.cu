@@ -853,14 +853,12 @@ cudaError_t launch_batch(const BatchParams& P, int grid, size_t smem, cudaStream
   return cudaGetLastError();
 }
 
-// Dynamic shared memory limits are raised once per batch object, outside any
-// stream capture.
-cudaError_t set_batch_attributes(size_t smem) {
-  cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_batch<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_batch<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_batch<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_batch<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// Dynamic shared memory limits are raised outside any stream capture.
+cudaError_t set_batch_attributes() {
+  cudaError_t e = allow_dynamic_smem<k_batch<true, 1>>();
+  if (e == cudaSuccess) e = allow_dynamic_smem<k_batch<true, 2>>();
+  if (e == cudaSuccess) e = allow_dynamic_smem<k_batch<false, 1>>();
+  if (e == cudaSuccess) e = allow_dynamic_smem<k_batch<false, 2>>();
   return e;
 }
 
@@ -1097,7 +1095,7 @@ extern "C" nfc_batch* nfc_batch_create(int64_t nq, const int64_t* row_offsets, c
   if (e == cudaSuccess && b->n_items)
     e = cudaMemcpy(b->d_items, items.data(), sizeof(uint64_t) * b->n_items, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = set_batch_attributes((size_t)t.smem_slots * 8);
+  if (e == cudaSuccess) e = set_batch_attributes();
   if (e == cudaSuccess) num_sms();
   if (e != cudaSuccess) {
     cuda_fail(e, "nfc_batch_create");

@@ -360,7 +360,7 @@ int dp_spread(const nfc_groupby_args* g, const DpRule& rule, cudaStream_t s, Scr
   NFC_CUDA(sc.alloc(&d_ok, 4));
   const int samples = (int)std::min<int64_t>(kDpSampleThreads * kDpSamplesPerThread, g->n / 256);
   const size_t smem = kDpMaxBuckets * sizeof(uint16_t);
-  NFC_CUDA(cudaFuncSetAttribute(k_dp_sample, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NFC_CUDA(allow_dynamic_smem<k_dp_sample>());
   k_dp_sample<<<1, kDpSampleThreads, smem, s>>>(g->keys, g->key_validity, g->n, samples, rule, d_ok);
   NFC_CUDA(cudaGetLastError());
   NFC_CUDA(readback(ok, d_ok, sizeof(*ok), s));
@@ -438,7 +438,7 @@ int64_t unique_by_partition(const int32_t* keys, int64_t n, int32_t* uniq_out, i
   if (rc) return rc;
   most = (std::min<int64_t>(most, 1ll << a.wb) + 3) & ~3ll;
   const size_t smem = ((size_t)1 << a.wb) / 32 * 6 + (size_t)most * 6;
-  NFC_CUDA(cudaFuncSetAttribute(k_dp_unique, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NFC_CUDA(allow_dynamic_smem<k_dp_unique>());
   k_dp_unique<<<(unsigned)a.nb, kDpThreads, smem, s>>>(a, (int32_t)most, uniq_out, first_out, counts_out, inv_out);
   NFC_CUDA(cudaGetLastError());
   return dp_finish(a, s);
@@ -470,7 +470,7 @@ int64_t count_distinct_by_partition(const int32_t* keys, const uint8_t* key_vali
   int lg = 10;
   while ((4ll << lg) / 5 < most) ++lg;
   const size_t smem = ((size_t)8 << lg) + ((size_t)4 << a.wb);
-  NFC_CUDA(cudaFuncSetAttribute(k_dp_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NFC_CUDA(allow_dynamic_smem<k_dp_count>());
   k_dp_count<<<(unsigned)a.nb, kDpThreads, smem, s>>>(a, lg, ukeys_out, nunique_out);
   NFC_CUDA(cudaGetLastError());
   return dp_finish(a, s);

@@ -378,7 +378,7 @@ static int launch_dense_smem_t(const int32_t* keys, const uint32_t* vmask, const
   while (lg < 5 && ((size_t)m << (lg + 1)) * slot + 64 <= kDsState) ++lg;
   const size_t smem = ((size_t)m << lg) * slot + 64;
   const int per_sm = 2 * (smem + 2048) <= 227 * 1024 ? 2 : 1;
-  NFC_CUDA(cudaFuncSetAttribute(k_dense_smem_t<NC, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NFC_CUDA(allow_dynamic_smem<k_dense_smem_t<NC, SIG>>());
   // Whole waves of equal chunks (a multiple of a CTA's 2,048-row step).
   const int64_t slots = (int64_t)num_sms() * per_sm;
   const int64_t waves = std::max<int64_t>(1, (n + slots * kDsChunk - 1) / (slots * kDsChunk));

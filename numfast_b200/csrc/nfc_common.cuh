@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/numfast_cuda.h"
 
 #define NFC_DEV __device__ __forceinline__
@@ -30,14 +32,32 @@ constexpr uint32_t kSpinLimit = 1u << 24;
 void set_last_error(const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);
 
-#define NFC_CUDA(call)                                      \
-  do {                                                      \
-    cudaError_t _e = (call);                                \
-    if (_e != cudaSuccess) return nfc::cuda_fail(_e, #call); \
+#define NFC_CUDA(...)                                               \
+  do {                                                              \
+    cudaError_t _e = (__VA_ARGS__);                                 \
+    if (_e != cudaSuccess) return nfc::cuda_fail(_e, #__VA_ARGS__); \
   } while (0)
 
 int num_sms();
 void keep_pool_memory();
+
+// Raises a kernel's dynamic shared memory limit to the most a CTA of the current
+// device can have, once per device.  The limit belongs to the function, not to
+// the launch: set to each call's own size, a smaller call on another thread could
+// lower it between this thread's setting and its launch, which is then refused.
+cudaError_t raise_dynamic_smem(const void* kernel);
+template <auto Kernel>
+cudaError_t allow_dynamic_smem() {
+  static std::atomic<uint64_t> raised{0};  // bit per device
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0ull;
+  if (raised.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  const cudaError_t r = raise_dynamic_smem(reinterpret_cast<const void*>(Kernel));
+  if (r == cudaSuccess) raised.fetch_or(bit, std::memory_order_release);
+  return r;
+}
 
 // Per-thread pinned host buffer of kReadbackBytes for a call's small
 // device-to-host read-backs (allocated on the thread's first use and kept

@@ -1117,7 +1117,7 @@ static int launch_hist(const PartLaunch& q, uint32_t* ghist, cudaStream_t s, Sta
       hfull = q.a->n / kHistTile;
     if (hfull > 0) {
       const size_t smem = 128 + (size_t)kHistStages * kHistStageBytes + (size_t)q.nb * 4;
-      NFC_CUDA(cudaFuncSetAttribute(k_part_hist_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      NFC_CUDA(allow_dynamic_smem<k_part_hist_bulk>());
       const int per_sm = 2 * (smem + 1024) <= 228 * 1024 ? 2 : 1;
       const int64_t g = std::max<int64_t>(1, std::min<int64_t>(hfull, (int64_t)num_sms() * per_sm));
       k_part_hist_bulk<<<(unsigned)g, 512, smem, s>>>(q.a->keys, q.vmask, hfull, q.kmin, q.wb, q.nb, ghist, q.d_err);
@@ -1128,7 +1128,7 @@ static int launch_hist(const PartLaunch& q, uint32_t* ghist, cudaStream_t s, Sta
     if (q.a->n > r0) {
       const int64_t ntiles128 = (q.a->n - r0 + 127) / 128;
       const size_t smem = (size_t)q.nb * 4;
-      NFC_CUDA(cudaFuncSetAttribute(k_part_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      NFC_CUDA(allow_dynamic_smem<k_part_hist>());
       const int64_t g = std::max<int64_t>(1, std::min<int64_t>((ntiles128 + 15) / 16, (int64_t)num_sms() * 4));
       k_part_hist<<<(unsigned)g, 256, smem, s>>>(q.a->keys + r0, q.vmask ? q.vmask + (r0 >> 5) : nullptr, q.a->n - r0,
                                                   q.al, q.kmin, q.wb, q.nb, ghist);
@@ -1150,8 +1150,7 @@ static int launch_records(const PartLaunch& q, const int32_t* skew, cudaStream_t
     uint64_t* out1 = q.two_level ? q.rec_a : q.rec;
     if (q.nfull > 0) {
       const size_t smem = pass1_smem(q.L);
-      NFC_CUDA(cudaFuncSetAttribute(k_part_pass1<NC, PACK0, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
+      NFC_CUDA(allow_dynamic_smem<k_part_pass1<NC, PACK0, SIG>>());
       const int per_sm = 2 * smem <= kPass1SmemPerSm ? 2 : 1;
       const int64_t g = std::max<int64_t>(1, std::min<int64_t>(q.nfull, (int64_t)num_sms() * per_sm));
       k_part_pass1<NC, PACK0, SIG><<<(unsigned)g, kPartThreads, smem, s>>>(a->keys, q.vmask, q.cs, q.L, q.nfull,
@@ -1169,7 +1168,7 @@ static int launch_records(const PartLaunch& q, const int32_t* skew, cudaStream_t
     }
     if (q.two_level) {
       constexpr size_t smem2 = refine2_smem<NW>();
-      NFC_CUDA(cudaFuncSetAttribute(k_part_refine<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
+      NFC_CUDA(allow_dynamic_smem<k_part_refine<NW>>());
       const int64_t nt2 = (q.nv + refine2_tile<NW>() - 1) / refine2_tile<NW>();
       const int64_t g2 = std::max<int64_t>(1, std::min<int64_t>(nt2, (int64_t)num_sms() * 2));
       k_part_refine<NW><<<(unsigned)g2, kPartThreads, smem2, s>>>(q.rec_a, q.nv, q.wb, q.cursor, q.rec, q.d_err,
@@ -1179,8 +1178,7 @@ static int launch_records(const PartLaunch& q, const int32_t* skew, cudaStream_t
     }
   } else {
     const size_t smem = (size_t)q.nb * 8;
-    NFC_CUDA(cudaFuncSetAttribute(k_part_scatter<NC, PACK0, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem));
+    NFC_CUDA(allow_dynamic_smem<k_part_scatter<NC, PACK0, SIG>>());
     const int64_t ntiles = (a->n + kScatterTile - 1) / kScatterTile;
     const int64_t g = std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)num_sms() * 2));
     k_part_scatter<NC, PACK0, SIG><<<(unsigned)g, kPartThreads, smem, s>>>(a->keys, q.vmask, q.cs, a->n, q.al,
@@ -1198,8 +1196,7 @@ static int launch_part(const PartLaunch& q, PartAggArgs& pa, cudaStream_t s, Sta
   const int rc = launch_records<NC, PACK0, SIG>(q, pa.n_merge + 2, s, tm);
   if (rc) return rc;
   tm->mark(s);
-  NFC_CUDA(cudaFuncSetAttribute(k_part_agg<NC, PACK0, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)q.agg_smem));
+  NFC_CUDA(allow_dynamic_smem<k_part_agg<NC, PACK0, SIG>>());
   if (q.max_slices > 0) {
     const unsigned g = (unsigned)std::min<int64_t>(q.max_slices, 2 * (int64_t)num_sms());
     // 128 KB of counters at most; 32-bit aggregates alone keep up on hot keys.
@@ -1207,14 +1204,13 @@ static int launch_part(const PartLaunch& q, PartAggArgs& pa, cudaStream_t s, Sta
     for (int c = 0; c < NC; ++c) wide64 |= q.cs.dtype[c] != NFC_I32 && q.cs.aggs[c] != 0;
     const bool sample = wide64 && q.wb <= 15;
     const size_t cnt = sample ? (size_t)4 << q.wb : 0;
-    NFC_CUDA(cudaFuncSetAttribute(k_part_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cnt));
+    NFC_CUDA(allow_dynamic_smem<k_part_multi>());
     k_part_multi<<<g, kPartThreads, cnt, s>>>(q.cs, pa.gm, pa.rec, NW, pa.offs, q.wb, pa.n_merge, q.multi, sample,
                                               q.hot, pa.slice_done);
     NFC_CUDA(cudaGetLastError());
     tm->launched();
     if (sample) {
-      NFC_CUDA(cudaFuncSetAttribute(k_part_hot<NC, PACK0, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)q.agg_smem));
+      NFC_CUDA(allow_dynamic_smem<k_part_hot<NC, PACK0, SIG>>());
       k_part_hot<NC, PACK0, SIG><<<g, kPartThreads, q.agg_smem, s>>>(pa);
       NFC_CUDA(cudaGetLastError());
       tm->launched();
@@ -1327,7 +1323,7 @@ int run_partition(const nfc_groupby_args* a, const ColSet& cs_in, const OutSet& 
   q.multi = pl.multi;
   q.hot = reinterpret_cast<uint2*>(slices + 2 * max_slices);
   uint32_t* slice_done = reinterpret_cast<uint32_t*>(slices + 3 * max_slices);
-  NFC_CUDA(cudaFuncSetAttribute(k_part_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(nb * 4)));
+  NFC_CUDA(allow_dynamic_smem<k_part_plan>());
   k_part_plan<<<1, 1024, (size_t)nb * 4, s>>>(w.ghist, nb, slice, q.cshift, q.two_level ? q.ccursor : nullptr, pl);
   NFC_CUDA(cudaGetLastError());
   tm->launched();
@@ -1422,7 +1418,7 @@ int partition_records(const nfc_groupby_args* a, int32_t dtype, const void* valu
   StageTimer tm;
   int rc = launch_hist(q, ghist, s, &tm);
   if (rc) return rc;
-  NFC_CUDA(cudaFuncSetAttribute(k_part_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(nb * 4)));
+  NFC_CUDA(allow_dynamic_smem<k_part_plan>());
   // A slice longer than any bucket: nothing is split.
   k_part_plan<<<1, 1024, (size_t)nb * 4, s>>>(ghist, q.nb, INT32_MAX, q.cshift, q.two_level ? q.ccursor : nullptr, pl);
   NFC_CUDA(cudaGetLastError());

@@ -648,7 +648,7 @@ extern "C" int64_t nfc_unique(const int32_t* keys, int64_t n, int32_t* uniq_out,
     const int64_t nchunks = (n + 127) / 128;
     const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((nchunks + 15) / 16, (int64_t)num_sms() * 3));
     const int lc_smem = kLcSlots * 16;
-    NFC_CUDA(cudaFuncSetAttribute(k_unique_lowcard, cudaFuncAttributeMaxDynamicSharedMemorySize, lc_smem));
+    NFC_CUDA(allow_dynamic_smem<k_unique_lowcard>());
     k_unique_lowcard<<<g, 512, lc_smem, s>>>(keys, n, lc);
     NFC_CUDA(cudaGetLastError());
     int32_t over = 0;

@@ -406,8 +406,7 @@ template <class K, bool HAS_VALS, bool IOTA>
 static int launch_scatter(const K* kin, K* kout, const uint32_t* vin, uint32_t* vout, int64_t n, int shift,
                           uint32_t dmask, K xr, const RsCounts& rc, cudaStream_t s) {
   constexpr size_t smem = sizeof(RsSmem<K, HAS_VALS>);
-  NFC_CUDA(cudaFuncSetAttribute(k_rs_scatter<K, HAS_VALS, IOTA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem));
+  NFC_CUDA(allow_dynamic_smem<k_rs_scatter<K, HAS_VALS, IOTA>>());
   k_rs_scatter<K, HAS_VALS, IOTA><<<rc.ntiles, kRsThreads, smem, s>>>(kin, kout, vin, vout, n, shift, dmask, xr,
                                                                      rc.tcount, rc.gcount, rc.totals, rc.gtiles,
                                                                      rc.ngroups);

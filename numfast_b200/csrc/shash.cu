@@ -144,7 +144,7 @@ int launch_shash(const ShLaunch& L, size_t slot_bytes, cudaStream_t s) {
   int lgT = 12;
   while (lgT > 8 && ((size_t)8 + slot_bytes) * ((size_t)1 << lgT) > 110 * 1024) --lgT;
   const size_t smem = ((size_t)8 + slot_bytes) * ((size_t)1 << lgT) + 64;
-  NFC_CUDA(cudaFuncSetAttribute(k_shash_agg<NC, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NFC_CUDA(allow_dynamic_smem<k_shash_agg<NC, SIG>>());
   // Grid: one CTA per kShMinChunk rows, at most two per SM.  Equal chunk
   // counts per CTA: the chunk is shrunk (to a multiple of 512 rows, never
   // above kShChunk) until the chunks divide evenly over the grid, so no CTA

@@ -303,13 +303,12 @@ template <int NC>
 static int launch_small(const nfc_groupby_args* a, const ColSet& cs, const OutSet& o, uint32_t* vmask, ProbeRec* rec,
                         SmallResult* res, cudaStream_t s) {
   constexpr int kState = 96 * 1024;
-  constexpr int kMost = 200 * 1024;  // with the errors: 8,191 slots of one float64 sum are 160 KB
   const size_t slot = state_bytes_per_slot(cs);
   const size_t errs = state_err_bytes_per_slot(cs);
   bool wide = false;  // 32-bit atomics alone keep up on few keys
   for (int c = 0; c < cs.ncols; ++c) wide |= cs.dtype[c] != NFC_I32 && cs.aggs[c] != 0;
-  const int smem = kState + (int)(errs * (kState / slot));
-  NFC_CUDA(cudaFuncSetAttribute(k_small<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
+  const int smem = kState + (int)(errs * (kState / slot));  // 8,191 slots of one float64 sum: 160 KB
+  NFC_CUDA(allow_dynamic_smem<k_small<NC>>());
   k_small<NC><<<1, SmallShape<NC>::threads, smem, s>>>(a->keys, bitmaps_of(a), cs, (int)a->n, inputs_aligned(a), o,
                                                        a->out_cap, kState, (uint32_t)slot, (uint32_t)errs,
                                                        wide ? kSmCopies : 0, vmask, rec, res);

@@ -952,7 +952,7 @@ int launch_sorted(const nfc_groupby_args* a, const ColSet& cs, const OutSet& o, 
                   const uint64_t* prev, const Pieces& P, const Pieces& Q, int64_t ntiles, int64_t nchunks,
                   uint64_t* lb, uint32_t* ticket, int64_t* d_ng, int32_t* d_err, cudaStream_t s, StageTimer* tm) {
   const size_t smem = sizeof(SortedSmem<NC, SIG>);
-  NFC_CUDA(cudaFuncSetAttribute(k_sorted_agg<NC, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NFC_CUDA(allow_dynamic_smem<k_sorted_agg<NC, SIG>>());
   k_sorted_agg<NC, SIG><<<(unsigned)ntiles, kSoThreads + 32, smem, s>>>(a->keys, vmask, cs, a->n, inputs_aligned(a), prev, o,
                                                                    a->out_cap, P, lb, ticket, d_ng, d_err);
   NFC_CUDA(cudaGetLastError());

@@ -117,7 +117,7 @@ int launch_runs(const int32_t* keys, const uint32_t* perm, int64_t nv, const Col
                 int64_t* ukeys, uint64_t* lb, uint32_t* ticket, int64_t* d_ng, int32_t* d_err, size_t slot_bytes,
                 cudaStream_t s) {
   const size_t smem = slot_bytes * kSrTile + 64;
-  NFC_CUDA(cudaFuncSetAttribute(k_sort_runs<NC, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NFC_CUDA(allow_dynamic_smem<k_sort_runs<NC, SIG>>());
   const int64_t ntiles = (nv + kSrTile - 1) / kSrTile;
   k_sort_runs<NC, SIG><<<(unsigned)ntiles, kSrThreads, smem, s>>>(keys, perm, nv, cs, gst, ukeys, lb, ticket, d_ng,
                                                                   d_err);

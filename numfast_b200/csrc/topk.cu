@@ -686,7 +686,7 @@ int topk_sampled(const void* keys, const uint8_t* validity, int64_t n, bool desc
   k_tk_collect<DT><<<gc, kTkThreads, 0, s>>>(keys, validity, n, vec, desc, st, c_img, c_row);
   NFC_CUDA(cudaGetLastError());
   constexpr int smem = kTkCap * 12;
-  NFC_CUDA(cudaFuncSetAttribute(k_tk_final, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  NFC_CUDA(allow_dynamic_smem<k_tk_final>());
   k_tk_final<<<(unsigned)num_sms(), kTkFinalThreads, smem, s>>>(st, DT == NFC_F64 && desc, (uint32_t)k, c_img, c_row, perm_out);
   NFC_CUDA(cudaGetLastError());
   uint32_t status = 0;

@@ -36,6 +36,17 @@ int num_sms() {
   return cached[dev];
 }
 
+cudaError_t raise_dynamic_smem(const void* kernel) {
+  int dev = 0, most = 0;
+  cudaFuncAttributes fa;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kernel);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes);
+  return e;
+}
+
 // Stream-ordered scratch comes from the device's default memory pool.  By
 // default the pool returns memory to the OS at every synchronisation, which
 // would re-map gigabytes of scratch on every call; keep it instead (once per
