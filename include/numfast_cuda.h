@@ -563,6 +563,12 @@ int32_t nfc_selftest_bounded_waits(uint32_t spins, int32_t* status_out, void* st
  * then disarms itself; a negative value disarms.  Process-wide. */
 int32_t nfc_debug_fail_alloc(int64_t after);
 
+/* The same for bounded waits: of the points before the scatter passes and after
+ * them of PARTITION, unique and COUNT DISTINCT calls, `after` pass and the next one
+ * sets the call's status word on the stream, as a kernel whose wait ran out does
+ * (the call then returns NFC_ERR_TIMEOUT), and disarms. */
+int32_t nfc_debug_fail_wait(int64_t after);
+
 #ifdef __cplusplus
 }
 #endif

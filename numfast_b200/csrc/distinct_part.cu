@@ -101,10 +101,10 @@ NFC_DEV int64_t dp_base(const DpArgs& a, int32_t b, uint32_t total, DpWalk* sw) 
   return (int64_t)excl;
 }
 
+// The CTA's bucket; -1 when an earlier kernel gave up on a wait.
 NFC_DEV int32_t dp_claim(const DpArgs& a, int32_t* s_bucket) {
   if (threadIdx.x == 0) *s_bucket = (int32_t)atomicAdd(a.ticket, 1u);
-  __syncthreads();
-  return *s_bucket;
+  return sync_failed(a.err) ? -1 : *s_bucket;
 }
 
 // How the rows are cut up.  wb: the widest bucket (2^wb keys, lo <= wb <= hi) of
@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(kDpThreads, 3) k_dp_unique(DpArgs a, int32_t m
   __shared__ DpWalk s_walk;
   __shared__ int32_t s_bucket;
   const int32_t b = dp_claim(a, &s_bucket);
+  if (b < 0) return;
   const int32_t words = (1 << a.wb) >> 5;
   uint32_t* bits = dp_smem;
   uint32_t* first = bits + words;
@@ -286,6 +287,7 @@ __global__ void __launch_bounds__(kDpThreads, 3) k_dp_count(DpArgs a, int lg_slo
   __shared__ DpWalk s_walk;
   __shared__ int32_t s_bucket;
   const int32_t b = dp_claim(a, &s_bucket);
+  if (b < 0) return;
   const int32_t slots = 1 << lg_slots, W = 1 << a.wb;
   uint32_t* distinct = reinterpret_cast<uint32_t*>(dp_set + slots);
   const int64_t r0 = a.offs[b];

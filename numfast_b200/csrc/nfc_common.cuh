@@ -73,6 +73,9 @@ cudaError_t readback(void* dst, const void* src, size_t bytes, cudaStream_t s);
 // Host-side fault injection for tests (nfc_debug_fail_alloc): true when the
 // scratch allocation being made is the one armed to fail.
 bool alloc_fault();
+// The same for waits (nfc_debug_fail_wait): at the point armed, the status word is
+// set on the stream as by a kernel whose wait ran out.
+cudaError_t wait_fault(int32_t* status, cudaStream_t s);
 
 // Stream-ordered scratch allocation.  Scratch is freed on the same stream
 // by the RAII holder, so concurrent calls on different streams never share
@@ -178,6 +181,13 @@ NFC_DEV void f64_atomic_add_err(double* sum, double* err, double x) {
   double s = atomicAdd(sum, x);
   const double e = f64_two_sum(s, x);
   if (!(e == 0.0)) atomicAdd(err, e);
+}
+
+// Barrier that also tells the whole CTA whether the call's status word is set,
+// i.e. an earlier kernel of the call gave up on a wait: the records it leaves
+// behind are incomplete, and what comes next would index memory by them.
+NFC_DEV bool sync_failed(const int32_t* status) {
+  return __syncthreads_or(threadIdx.x == 0 && ld_volatile_u32(reinterpret_cast<const uint32_t*>(status)) != 0u) != 0;
 }
 
 // Bit i of an LSB-first validity bitmap (Arrow layout).

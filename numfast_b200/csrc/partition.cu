@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(kPartThreads, 2) k_part_pass1(const int32_t* _
     for (int i = 0; i < L.stages; ++i) mbar_init(&bars[i], 1);
     mbar_fence_init();
   }
-  __syncthreads();
+  if (sync_failed(err)) return;
   const int64_t my_tiles = nfull > blockIdx.x ? (nfull - 1 - blockIdx.x) / gridDim.x + 1 : 0;
   const uint64_t pol_in = l2_policy_evict_first();
   auto issue = [&](int64_t k) {
@@ -580,7 +580,9 @@ __global__ void __launch_bounds__(kPartThreads) k_part_pass1_tail(const int32_t*
                                                                  const uint32_t* __restrict__ vmask, ColSet cs,
                                                                  int64_t row_off, int64_t n, int32_t kmin, int shift,
                                                                  uint32_t keep_mask, uint32_t* __restrict__ gcursor,
-                                                                 uint64_t* __restrict__ out, uint32_t* gwide) {
+                                                                 uint64_t* __restrict__ out, const int32_t* err,
+                                                                 uint32_t* gwide) {
+  if (sync_failed(err)) return;
   constexpr int NW = Rec<NC, PACK0>::NW;
   uint32_t wide = 0;
   for (int64_t i = row_off + threadIdx.x; i < n; i += blockDim.x) {
@@ -649,7 +651,7 @@ __global__ void __launch_bounds__(kPartThreads, 2) k_part_refine(const uint64_t*
     for (int i = 0; i < kRefineStages; ++i) mbar_init(&bars[i], 1);
     mbar_fence_init();
   }
-  __syncthreads();
+  if (sync_failed(err)) return;
   const int64_t ntiles = (nv + T - 1) / T;
   const int64_t my_tiles = ntiles > blockIdx.x ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
   const uint64_t pol_in = l2_policy_evict_first();
@@ -877,9 +879,10 @@ __global__ void __launch_bounds__(kPartThreads) k_part_multi(ColSet cs, StateRef
                                                             const int32_t* __restrict__ n_merge,
                                                             const int2* __restrict__ multi, bool sample,
                                                             uint2* __restrict__ hot,
-                                                            uint32_t* __restrict__ slice_done) {
+                                                            uint32_t* __restrict__ slice_done, const int32_t* err) {
   extern __shared__ uint32_t s_cnt[];  // 2^wb counters (sample)
   __shared__ uint32_t s_red[33];
+  if (sync_failed(err)) return;
   const int32_t W = 1 << wb, n = n_merge[0];
   for (int32_t i = blockIdx.x; i < n; i += gridDim.x) {
     for (int32_t g = threadIdx.x; g < W; g += blockDim.x) {
@@ -910,6 +913,7 @@ __global__ void __launch_bounds__(kPartThreads) k_part_multi(ColSet cs, StateRef
 template <int NC, bool PACK0, uint32_t SIG>
 __global__ void __launch_bounds__(kPartThreads, SIG == 0 && NC >= 2 ? 1 : 2) k_part_hot(PartAggArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  if (sync_failed(a.err)) return;
   const int32_t W = 1 << a.wb;
   const int32_t nslices = a.n_merge[1];
   const AggState<NC> st = carve_agg<NC, SIG>(a.cs, smem_raw, W, ~__ldg(a.wide));
@@ -966,7 +970,7 @@ __global__ void __launch_bounds__(kPartThreads, 2) k_part_agg(PartAggArgs a) {
   __shared__ int64_t s_base;
   __shared__ int32_t s_item;
   if (threadIdx.x == 0) s_item = (int32_t)atomicAdd(a.ticket, 1u);
-  __syncthreads();
+  if (sync_failed(a.err)) return;
   const int32_t nslices = a.n_merge[1];
   const int32_t it = s_item;
   if (it >= nslices + a.nb) return;
@@ -1143,6 +1147,7 @@ template <int NC, bool PACK0, uint32_t SIG>
 static int launch_records(const PartLaunch& q, const int32_t* skew, cudaStream_t s, StageTimer* tm) {
   const nfc_groupby_args* a = q.a;
   constexpr int NW = Rec<NC, PACK0>::NW;
+  NFC_CUDA(wait_fault(q.d_err, s));
   if (q.coalesced) {
     const int shift = q.two_level ? q.wb + q.cshift : q.wb;
     const uint32_t keep = q.two_level ? 0xFFFFFFFFu : (1u << q.wb) - 1u;
@@ -1162,11 +1167,12 @@ static int launch_records(const PartLaunch& q, const int32_t* skew, cudaStream_t
     const int64_t row_off = q.nfull * kBulkTile;
     if (a->n > row_off) {
       k_part_pass1_tail<NC, PACK0, SIG><<<1, kPartThreads, 0, s>>>(a->keys, q.vmask, q.cs, row_off, a->n, q.kmin,
-                                                                   shift, keep, cur1, out1, q.wide);
+                                                                   shift, keep, cur1, out1, q.d_err, q.wide);
       NFC_CUDA(cudaGetLastError());
       tm->launched();
     }
     if (q.two_level) {
+      NFC_CUDA(wait_fault(q.d_err, s));
       constexpr size_t smem2 = refine2_smem<NW>();
       NFC_CUDA(allow_dynamic_smem<k_part_refine<NW>>());
       const int64_t nt2 = (q.nv + refine2_tile<NW>() - 1) / refine2_tile<NW>();
@@ -1187,6 +1193,7 @@ static int launch_records(const PartLaunch& q, const int32_t* skew, cudaStream_t
     NFC_CUDA(cudaGetLastError());
     tm->launched();
   }
+  NFC_CUDA(wait_fault(q.d_err, s));
   return NFC_OK;
 }
 
@@ -1206,7 +1213,7 @@ static int launch_part(const PartLaunch& q, PartAggArgs& pa, cudaStream_t s, Sta
     const size_t cnt = sample ? (size_t)4 << q.wb : 0;
     NFC_CUDA(allow_dynamic_smem<k_part_multi>());
     k_part_multi<<<g, kPartThreads, cnt, s>>>(q.cs, pa.gm, pa.rec, NW, pa.offs, q.wb, pa.n_merge, q.multi, sample,
-                                              q.hot, pa.slice_done);
+                                              q.hot, pa.slice_done, q.d_err);
     NFC_CUDA(cudaGetLastError());
     tm->launched();
     if (sample) {

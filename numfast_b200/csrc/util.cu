@@ -95,7 +95,24 @@ bool alloc_fault() {
   return false;
 }
 
+// Armed count for nfc_debug_fail_wait, counted down the same way.
+static std::atomic<int64_t> g_wait_fault{-1};
+
+cudaError_t wait_fault(int32_t* status, cudaStream_t s) {
+  static const int32_t timeout = NFC_ERR_TIMEOUT;
+  int64_t v = g_wait_fault.load(std::memory_order_relaxed);
+  while (v >= 0)
+    if (g_wait_fault.compare_exchange_weak(v, v - 1))
+      return v == 0 ? cudaMemcpyAsync(status, &timeout, sizeof(timeout), cudaMemcpyHostToDevice, s) : cudaSuccess;
+  return cudaSuccess;
+}
+
 }  // namespace nfc
+
+extern "C" int32_t nfc_debug_fail_wait(int64_t after) {
+  nfc::g_wait_fault.store(after < 0 ? -1 : after);
+  return NFC_OK;
+}
 
 extern "C" int32_t nfc_debug_fail_alloc(int64_t after) {
   nfc::g_alloc_fault.store(after < 0 ? -1 : after);
