@@ -447,6 +447,9 @@ __global__ void __launch_bounds__(kTkThreads) k_tk_sample(const void* __restrict
   __threadfence();
   constexpr int kPer = kTkBins / kTkThreads;
   uint32_t c[kPer], sum = 0;
+  // Read before the scan's barriers: the thread that holds the digit moves the
+  // state on after them, while others may still be on their way.
+  const uint32_t want = level ? st->target : target, before = level ? st->below : 0u;
 #pragma unroll
   for (int j = 0; j < kPer; ++j) {
     c[j] = __ldcg(&gh[threadIdx.x * kPer + j]);
@@ -454,7 +457,6 @@ __global__ void __launch_bounds__(kTkThreads) k_tk_sample(const void* __restrict
   }
   uint32_t total;
   uint32_t x = block_excl_scan(sum, s_scan, &total);
-  const uint32_t want = level ? st->target : target;
   // Fewer sampled valid rows than the target: no digit holds it, and the
   // levels that follow find nothing to count.
 #pragma unroll
@@ -463,7 +465,7 @@ __global__ void __launch_bounds__(kTkThreads) k_tk_sample(const void* __restrict
       st->prefix = prefix | ((uint64_t)(threadIdx.x * kPer + j) << shift);
       st->mask = mask | ((uint64_t)dmask << shift);
       st->target = want - x;
-      const uint32_t below = (level ? st->below : 0u) + x;
+      const uint32_t below = before + x;
       st->below = below;
       if ((uint64_t)(below + c[j]) * step <= (uint64_t)(kTkExpect + kTkExpect / 4)) st->ready = 1u;
     }
