@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(kRsCountThreads) k_rs_count(const K* __restric
   constexpr int VEC = 16 / sizeof(K);
   constexpr int U = kTile / (VEC * kRsCountThreads);
   static_assert(U * VEC * kRsCountThreads == kTile, "whole vectors per thread");
-  __shared__ uint32_t h[kRsDigits * kRsCopies];
+  __shared__ __align__(16) uint32_t h[kRsDigits * kRsCopies];
   for (int i = threadIdx.x; i < kRsDigits * kRsCopies; i += kRsCountThreads) h[i] = 0u;
   const uint32_t copy = threadIdx.x & (kRsCopies - 1);
   auto add = [&](K k) { atomicAdd(&h[(((uint32_t)((k ^ xr) >> shift) & dmask) * kRsCopies) + copy], 1u); };

@@ -1,5 +1,6 @@
 """Properties of the kernels that no run shows reliably, read from their sources."""
 
+import glob
 import os
 import re
 
@@ -25,3 +26,15 @@ def test_sample_state_is_read_before_it_is_moved_on():
     last_read = max(m.end() for f in ("target", "below") for m in re.finditer(r"st->%s\b(?!\s*=[^=])" % f, body))
     first_write = min(m.start() for f in ("target", "below") for m in re.finditer(r"st->%s\s*=[^=]" % f, body))
     assert "block_excl_scan" in body[last_read:first_write]
+
+
+def test_shared_arrays_read_as_vectors_are_aligned():
+    """A __shared__ array that is accessed by 16-byte vectors declares that alignment."""
+    loose = []
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+        text = _source(os.path.basename(path))
+        for name in set(re.findall(r"reinterpret_cast<(?:const )?(?:u?int4|ulonglong2|double2)\*>\(&?(\w+)\b", text)):
+            for decl in re.findall(r"[^;{}]*__shared__[^;{}]*\b%s\s*\[[^;{}]*;" % name, text):
+                if "__align__(16)" not in decl and "__align__(128)" not in decl:
+                    loose.append((os.path.basename(path), " ".join(decl.split())))
+    assert not loose, loose
