@@ -468,14 +468,29 @@ int64_t count_distinct_by_partition(const int32_t* keys, const uint8_t* key_vali
   int64_t most = 0, nv = 0;
   const int rc = dp_prepare(&g, NFC_I32, values, DpRule{6200, 512, 13000, 0, 13}, s, sc, &a, &most, &nv);
   if (rc) return rc;
-  if (out_cap < std::min<int64_t>(a.m, nv)) return NFC_ERR_UNSUPPORTED;
+  // Outputs that may not hold every key are written once they are known to.
+  const int64_t bound = std::min<int64_t>(a.m, nv);
+  int64_t *uk = ukeys_out, *nu = nunique_out;
+  if (out_cap < bound) {
+    NFC_CUDA(sc.alloc(&uk, (size_t)(2 * bound)));
+    nu = uk + bound;
+  }
   int lg = 10;
   while ((4ll << lg) / 5 < most) ++lg;
   const size_t smem = ((size_t)8 << lg) + ((size_t)4 << a.wb);
   NFC_CUDA(allow_dynamic_smem<k_dp_count>());
-  k_dp_count<<<(unsigned)a.nb, kDpThreads, smem, s>>>(a, lg, ukeys_out, nunique_out);
+  k_dp_count<<<(unsigned)a.nb, kDpThreads, smem, s>>>(a, lg, uk, nu);
   NFC_CUDA(cudaGetLastError());
-  return dp_finish(a, s);
+  const int64_t ng = dp_finish(a, s);
+  if (ng <= 0 || out_cap >= bound) return ng;
+  if (ng > out_cap) {
+    set_last_error("group_count_distinct: %lld groups > out_cap %lld", (long long)ng, (long long)out_cap);
+    return NFC_ERR_RANGE;
+  }
+  NFC_CUDA(cudaMemcpyAsync(ukeys_out, uk, sizeof(int64_t) * ng, cudaMemcpyDeviceToDevice, s));
+  NFC_CUDA(cudaMemcpyAsync(nunique_out, nu, sizeof(int64_t) * ng, cudaMemcpyDeviceToDevice, s));
+  NFC_CUDA(cudaStreamSynchronize(s));
+  return ng;
 }
 
 }  // namespace nfc
