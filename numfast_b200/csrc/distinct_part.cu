@@ -13,8 +13,8 @@
 // instead of four of pairs (or of one per eight bits of the pair), and no run
 // pass: 200M keys over the full int32 range 5.85 -> 3.89 ms, COUNT DISTINCT of
 // 50M rows over 1M keys 2.10 -> 1.28 ms.  Rows that do not spread over the
-// buckets (few keys, skew) and small inputs stay with the sort: a bucket has to
-// fit one CTA.
+// buckets (few keys, skew), small inputs and unaligned columns stay with the sort:
+// a bucket has to fit one CTA, the scatter passes copy 16-byte vectors.
 #include <algorithm>
 
 #include "groupby_host.h"
@@ -429,7 +429,7 @@ int64_t dp_finish(const DpArgs& a, cudaStream_t s) {
 // no longer fit one CTA, and a CTA's time would show as a tail.
 int64_t unique_by_partition(const int32_t* keys, int64_t n, int32_t* uniq_out, int32_t* first_out,
                             int64_t* counts_out, int32_t* inv_out, cudaStream_t s) {
-  if (n < kDpMinRows) return NFC_ERR_UNSUPPORTED;
+  if (n < kDpMinRows || !aligned16(keys)) return NFC_ERR_UNSUPPORTED;
   Scratch sc(s);
   nfc_groupby_args g{};
   g.n = n;
@@ -452,7 +452,7 @@ int64_t unique_by_partition(const int32_t* keys, int64_t n, int32_t* uniq_out, i
 int64_t count_distinct_by_partition(const int32_t* keys, const uint8_t* key_validity, const int32_t* values,
                                     const uint8_t* value_validity, int64_t n, int64_t out_cap, int64_t* ukeys_out,
                                     int64_t* nunique_out, cudaStream_t s) {
-  if (n < kDpMinRows) return NFC_ERR_UNSUPPORTED;
+  if (n < kDpMinRows || !aligned16(keys) || !aligned16(values)) return NFC_ERR_UNSUPPORTED;
   Scratch sc(s);
   nfc_value_col col{};
   col.dtype = NFC_I32;

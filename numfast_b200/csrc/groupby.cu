@@ -426,8 +426,6 @@ __global__ void __launch_bounds__(256) k_compact_dense(ColSet cs, StateRef st, i
 // =====================================================================
 // Host orchestration.
 // =====================================================================
-static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
-
 static int grid_stream(int64_t work_tiles, int per_sm) {
   int64_t g = std::min<int64_t>(work_tiles, (int64_t)num_sms() * per_sm);
   return (int)std::max<int64_t>(g, 1);

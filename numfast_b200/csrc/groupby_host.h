@@ -44,6 +44,7 @@ int64_t groupby_run(const nfc_groupby_args* a, int32_t strategy, PlanHook* hook,
                     nfc_groupby_stats* stats);
 
 int build_colset(const nfc_groupby_args* a, ColSet* cs, OutSet* o);
+inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 bool inputs_aligned(const nfc_groupby_args* a);
 // Probe records: k_probe writes one per block of kProbeBlockRows rows (in
 // row order): the first and last valid key, the valid key range and count,

@@ -39,3 +39,31 @@ def test_output_for_the_groups_only(cuda):
     _, want = torch.unique(pairs // 4, return_counts=True)
     assert torch.equal(out[0], torch.arange(groups, device="cuda") * 37 - 1000)
     assert torch.equal(out[1], want)
+
+
+def _allocations(call):
+    """Scratch allocations of a call: the first one whose failure the call does not see."""
+    lib = _lib.load()
+    for k in range(64):
+        lib.nfc_debug_fail_alloc(k)
+        try:
+            call()
+            return k
+        except _lib.NativeError as e:
+            assert e.code == _lib.ERR_NOMEM
+        finally:
+            lib.nfc_debug_fail_alloc(-1)
+    raise AssertionError("no end of allocations")
+
+
+@pytest.mark.parametrize("kind", ["unique", "count distinct"])
+def test_unaligned_columns_go_straight_to_the_sort(cuda, kind):
+    """The scatter passes need 16-byte aligned columns: an unaligned call allocates what a call
+    below the row limit does."""
+    def call(n, shift):
+        g = torch.Generator(device="cuda").manual_seed(n)
+        k = torch.randint(0, 50_000_000, (n + shift,), generator=g, device="cuda", dtype=torch.int32)[shift:]
+        if kind == "unique":
+            return lambda: D.unique(k)
+        return lambda: D.group_count_distinct(k, k)
+    assert _allocations(call(LIMIT + 40_000, 1)) == _allocations(call(LIMIT - 40_000, 0))
