@@ -44,7 +44,8 @@ constexpr int kBWarps = kBThreads / 32;
 constexpr int kBPer = 16;                    // rows per thread per sub-tile
 constexpr int kBSub = kBThreads * kBPer;     // 8192 rows per sub-tile
 constexpr int kBEmitRound = kBThreads * 4;   // slots per emit round
-constexpr int kSoloSlack = 16384;            // span a solo query may have above four slots per row
+constexpr int kSoloSlack = 16384;            // span a solo query may have above four slots per row, and span
+                                             // that needs no arena: the shared table or the CTA's own words
 
 enum : uint32_t { kItProbe = 0, kItSolo = 1, kItAgg = 2, kItEmit = 3 };
 
@@ -712,14 +713,14 @@ NFC_DEV void do_solo(const BatchParams& P, BSmem& S, uint32_t* s_cnt, int32_t* s
   }
   const int64_t kmin = (int32_t)((~mnc) ^ 0x80000000u);
   const int64_t span = (int64_t)(int32_t)(mx ^ 0x80000000u) - kmin + 1;
-  const bool in_smem = span <= P.smem_slots;
+  const bool in_smem = span <= P.smem_slots, own = !in_smem && span <= kSoloSlack;
   if (threadIdx.x == 0) {
-    int64_t ob = -1, off = 0;
-    if (in_smem) {
+    int64_t ob = -1, off = P.arena_words + (int64_t)blockIdx.x * kSoloSlack;
+    if (in_smem || own) {
       ob = reserve(&P.hdr->out_cursor, imin64(cnt, span), P.out_cap);
     } else if (span <= 4 * qd.rows + imax64(P.smem_slots, kSoloSlack)) {
-      // Too wide for the shared table: packed global state in the arena,
-      // still finished by this CTA alone.
+      // Too wide for those: packed global state in the arena, still finished by
+      // this CTA alone.
       off = reserve(&P.hdr->arena_cursor, (span + 3) & ~3ll, P.arena_words);
       if (off >= 0) ob = reserve(&P.hdr->out_cursor, imin64(cnt, span), P.out_cap);
     }
@@ -889,6 +890,7 @@ struct nfc_batch {
   int32_t* d_qstatus = nullptr;
   unsigned long long* d_arena = nullptr;
   int64_t arena_words = 0;
+  int64_t own_words = 0;  // after the arena: kSoloSlack per CTA, where the shared table has fewer slots
   bool arena_dirty = true;
   cudaStream_t cap_stream = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -909,6 +911,10 @@ void batch_free(nfc_batch* b) {
   cudaFree(b->d_rt);
   cudaFree(b->d_arena);
   delete b;
+}
+
+int batch_grid(const nfc_batch* b) {
+  return (int)std::min<int64_t>((int64_t)num_sms() * b->tune.ctas_per_sm, b->n_items);
 }
 
 // Picked on mixed batches of 40 to 512 queries of 1K..4M rows.  The emit items
@@ -1090,7 +1096,8 @@ extern "C" nfc_batch* nfc_batch_create(int64_t nq, const int64_t* row_offsets, c
   if (e == cudaSuccess) e = cudaMalloc(&b->d_qd, sizeof(QDesc) * nq);
   if (e == cudaSuccess) e = cudaMalloc(&b->d_items, sizeof(uint64_t) * std::max<int64_t>(b->n_items, 1));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_rt, b->rt_bytes);
-  if (e == cudaSuccess) e = cudaMalloc(&b->d_arena, sizeof(unsigned long long) * words);
+  if (t.smem_slots < kSoloSlack && b->counts_by_type[kItSolo]) b->own_words = (int64_t)batch_grid(b) * kSoloSlack;
+  if (e == cudaSuccess) e = cudaMalloc(&b->d_arena, sizeof(unsigned long long) * (words + b->own_words));
   if (e == cudaSuccess) e = cudaMemcpy(b->d_qd, b->hqd.data(), sizeof(QDesc) * nq, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && b->n_items)
     e = cudaMemcpy(b->d_items, items.data(), sizeof(uint64_t) * b->n_items, cudaMemcpyHostToDevice);
@@ -1138,7 +1145,7 @@ int enqueue_batch(nfc_batch* b, const BatchParams& P, bool vec, cudaStream_t s) 
   NFC_CUDA(cudaMemsetAsync(b->d_rt, 0, b->rt_bytes, s));
   if (P.n_items == 0) return NFC_OK;
   const int cps = b->tune.ctas_per_sm;
-  const int grid = (int)std::min<int64_t>((int64_t)num_sms() * cps, P.n_items);
+  const int grid = batch_grid(b);
   const size_t smem = (size_t)b->tune.smem_slots * 8;
   cudaError_t e;
   if (vec) e = cps == 2 ? launch_batch<true, 2>(P, grid, smem, s) : launch_batch<true, 1>(P, grid, smem, s);
@@ -1270,7 +1277,7 @@ extern "C" int64_t nfc_batch_run(nfc_batch* b, const int32_t* keys, const uint8_
   P.warp_agg = b->tune.warp_agg;
   const bool vec = ((uintptr_t)keys % 16 == 0) && ((uintptr_t)values % 16 == 0);
   if (b->arena_dirty) {
-    NFC_CUDA(cudaMemsetAsync(b->d_arena, 0, sizeof(unsigned long long) * b->arena_words, s));
+    NFC_CUDA(cudaMemsetAsync(b->d_arena, 0, sizeof(unsigned long long) * (b->arena_words + b->own_words), s));
     b->arena_dirty = false;
   }
   const bool use_graph = flags & NFC_BATCH_GRAPH;

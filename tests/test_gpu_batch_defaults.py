@@ -36,3 +36,28 @@ def test_spans_around_the_shared_table(cuda, rows, extra):
             np.testing.assert_array_equal(gs, su)
             np.testing.assert_array_equal(gc, ct)
     b.close()
+
+
+@pytest.mark.parametrize("rows", [2_500, 30_000])
+def test_small_arena(cuda, rows):
+    """A small explicit arena: queries of up to 16,384 keys never needed it; wider ones are deferred
+    and still right."""
+    rs = np.random.default_rng(rows)
+    spans = [100, 8_192, 8_193, 12_000, 16_383, 16_384] * 60 + [17_000]
+    keys = [np.concatenate([[0, s - 1], rs.integers(0, s, rows - 2)]).astype(np.int32) - 9 for s in spans]
+    vals = [rs.integers(-1000, 1001, rows).astype(np.int32) for _ in spans]
+    off = np.arange(len(spans) + 1, dtype=np.int64) * rows
+    k, v = np.concatenate(keys), np.concatenate(vals)
+    t = B.default_tuning()
+    t.arena_bytes = 64 * 1024
+    b = B.BatchGroupby(off, tuning=t)
+    assert b.info()["arena_bytes"] == 64 * 1024
+    for graph in (False, True, True):
+        r = b.run(to_dev(k), to_dev(v), graph=graph)
+        assert r.deferred == 1
+        for q, (uk, su, ct) in enumerate(O.batch_sum_count(k, v, off)):
+            gk, gs, gc = r.query(q)
+            np.testing.assert_array_equal(gk, uk)
+            np.testing.assert_array_equal(gs, su)
+            np.testing.assert_array_equal(gc, ct)
+    b.close()
