@@ -213,11 +213,8 @@ NFC_DEV int64_t agg_sum_bits(const ColSet& cs, const AggState<NC>& st, int c, in
 }
 
 // Merge shared slot g into the global merge state (StateRef layout) slot d.
-// ERR: that state keeps the rounding errors of its float64 sums.  The CTAs'
-// partial sums of a slot are one chain, and more CTAs make it longer (4M rows
-// over 365 keys, mean relative error of a sum: 62 CTAs 1.8e-16, 280 CTAs 3.5e-16,
-// with the errors 4.7e-17).
-template <int NC, uint32_t SIG, bool ERR = false>
+// LEAVE: without the float64 sums of which that state keeps the errors.
+template <int NC, uint32_t SIG, bool LEAVE = false>
 NFC_DEV void agg_merge(const ColSet& cs, const StateRef& dst, int64_t d, const AggState<NC>& st, int g) {
   const uint32_t k = st.cnt[g];
   if (k == 0u) return;
@@ -226,12 +223,13 @@ NFC_DEV void agg_merge(const ColSet& cs, const StateRef& dst, int64_t d, const A
   for (int c = 0; c < NC; ++c) {
     const int dt = col_dt<SIG>(cs, c), ag = col_ag<SIG>(cs, c);
     if (ag & NFC_AGG_SUM) {
-      if (dt == NFC_F64 && ERR)
-        f64_atomic_add_err(static_cast<double*>(dst.sum[c]) + d, dst.err[c] + d,
-                           __longlong_as_double((long long)st.s64[c][g]));
-      else if (dt == NFC_F64)
-        atomicAdd(static_cast<double*>(dst.sum[c]) + d, __longlong_as_double((long long)st.s64[c][g]));
-      else atomicAdd(static_cast<unsigned long long*>(dst.sum[c]) + d, (unsigned long long)agg_sum_bits<NC, SIG>(cs, st, c, g));
+      if (dt == NFC_F64) {
+        if (!(LEAVE && dst.err[c]))
+          atomicAdd(static_cast<double*>(dst.sum[c]) + d, __longlong_as_double((long long)st.s64[c][g]));
+      } else {
+        atomicAdd(static_cast<unsigned long long*>(dst.sum[c]) + d,
+                  (unsigned long long)agg_sum_bits<NC, SIG>(cs, st, c, g));
+      }
     }
     if (dt == NFC_I32) {
       if (ag & NFC_AGG_MIN) atomicMin(static_cast<int*>(dst.mn[c]) + d, static_cast<const int*>(st.mn[c])[g]);
@@ -248,54 +246,125 @@ NFC_DEV void agg_merge(const ColSet& cs, const StateRef& dst, int64_t d, const A
   }
 }
 
-// Entry e of an interleaved state (slot e >> lg of copy e & (2^lg - 1)): the
-// lanes of a group of 2^lg combine their copies and the first one folds the
-// slot into the global state, which keeps rounding errors.  Whole warp; lanes at or past `entries` add
-// nothing (entries is a multiple of the group).
+// Slots 0 .. w of a state into slots d0 on of the global one (whole block, after
+// a barrier); slot g is entry g << lg.  The CTAs' float64 partial sums of a slot
+// are one chain, and more CTAs make it longer (4M rows over 365 keys, mean relative
+// error of a sum: 62 CTAs 1.8e-16, 280 CTAs 3.5e-16), so the global state may keep
+// the rounding error of each addition (4.7e-17).  That needs the old value back
+// from the atomic; a thread has four of them under way.
 template <int NC, uint32_t SIG>
-NFC_DEV void agg_merge_copies(const ColSet& cs, const StateRef& dst, const AggState<NC>& st, int e, int entries,
-                              int lg) {
-  const bool in = e < entries;
-  uint32_t k = in ? st.cnt[e] : 0u;
-  for (int o = 1; o < (1 << lg); o <<= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
-  uint64_t sum[NC > 0 ? NC : 1], mn[NC > 0 ? NC : 1], mx[NC > 0 ? NC : 1];
+NFC_DEV void agg_merge_all(const ColSet& cs, const StateRef& dst, int64_t d0, const AggState<NC>& st, int w, int lg) {
+  for (int g = threadIdx.x; g < w; g += blockDim.x) agg_merge<NC, SIG, true>(cs, dst, d0 + g, st, g << lg);
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
-    const int dt = col_dt<SIG>(cs, c), ag = col_ag<SIG>(cs, c);
-    uint64_t s = 0, lo = 0, hi = 0;
-    if (ag & NFC_AGG_SUM) {
-      s = in ? (uint64_t)agg_sum_bits<NC, SIG>(cs, st, c, e) : 0ull;
-      for (int o = 1; o < (1 << lg); o <<= 1) {
-        const uint64_t t = __shfl_xor_sync(0xffffffffu, s, o);
-        s = dt == NFC_F64 ? (uint64_t)__double_as_longlong(__longlong_as_double((long long)s) +
-                                                           __longlong_as_double((long long)t))
-                          : s + t;
+    if (col_dt<SIG>(cs, c) != NFC_F64 || !(col_ag<SIG>(cs, c) & NFC_AGG_SUM) || !dst.err[c]) continue;
+    double* sum = static_cast<double*>(dst.sum[c]) + d0;
+    constexpr int K = 4;
+    for (int g0 = threadIdx.x; g0 < w; g0 += K * blockDim.x) {
+      double old[K], x[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int g = g0 + k * (int)blockDim.x;
+        old[k] = x[k] = 0.0;
+        if (g < w && st.cnt[g << lg]) {
+          x[k] = __longlong_as_double((long long)st.s64[c][g << lg]);
+          old[k] = atomicAdd(sum + g, x[k]);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const double e = f64_two_sum(old[k], x[k]);
+        if (!(e == 0.0)) atomicAdd(dst.err[c] + d0 + g0 + k * (int)blockDim.x, e);
       }
     }
-    // Minima and maxima as int64, float64 as the ordered encodings.
-    if (ag & NFC_AGG_MIN) {
-      lo = dt == NFC_F64 ? ~0ull : (uint64_t)LLONG_MAX;
-      if (in) lo = dt == NFC_I32 ? (uint64_t)(int64_t) static_cast<const int32_t*>(st.mn[c])[e]
-                                 : static_cast<const uint64_t*>(st.mn[c])[e];
-      for (int o = 1; o < (1 << lg); o <<= 1) {
-        const uint64_t t = __shfl_xor_sync(0xffffffffu, lo, o);
-        lo = dt == NFC_F64 ? min(lo, t) : (uint64_t)min((long long)lo, (long long)t);
-      }
-    }
-    if (ag & NFC_AGG_MAX) {
-      hi = dt == NFC_F64 ? 0ull : (uint64_t)LLONG_MIN;
-      if (in) hi = dt == NFC_I32 ? (uint64_t)(int64_t) static_cast<const int32_t*>(st.mx[c])[e]
-                                 : static_cast<const uint64_t*>(st.mx[c])[e];
-      for (int o = 1; o < (1 << lg); o <<= 1) {
-        const uint64_t t = __shfl_xor_sync(0xffffffffu, hi, o);
-        hi = dt == NFC_F64 ? max(hi, t) : (uint64_t)max((long long)hi, (long long)t);
-      }
-    }
-    sum[c] = s;
-    mn[c] = lo;
-    mx[c] = hi;
   }
-  if (in && k && (lane_id() & ((1u << lg) - 1u)) == 0u) state_apply_group<true>(cs, dst, e >> lg, k, sum, mn, mx);
+}
+
+// The 2^lg interleaved copies of every slot (slot g of copy r is entry
+// (g << lg) + r) combined into the first one (whole block).  As many lanes share
+// a slot as the block has to spare, each takes its copies one after the other,
+// turned by the slot so that the lanes of a warp meet no bank twice.  (32 lanes to
+// a slot and all of it by shuffles: 20 us a CTA for 365 slots of 32 copies.)
+// ERR: the state keeps the rounding errors of its float64 sums.
+template <int NC, uint32_t SIG, bool ERR = false>
+NFC_DEV void fold_copies(const ColSet& cs, const AggState<NC>& st, int slots, int lg) {
+  int lanes = 0;
+  while (lanes < min(lg, 5) && slots << (lanes + 1) <= (int)blockDim.x) ++lanes;
+  const int steps = 1 << (lg - lanes), all = (1 << lg) - 1;
+  const int part = lane_id() & ((1 << lanes) - 1);
+  for (int e0 = threadIdx.x & ~31; e0 < slots << lanes; e0 += (int)blockDim.x) {
+    const int g = (e0 + (int)lane_id()) >> lanes;
+    const bool in = g < slots, write = in && part == 0;
+    const int first = (in ? g : 0) << lg;
+    auto entry = [&](int r) { return first + ((((r + g) << lanes) + part) & all); };
+    uint32_t cnt = 0;
+    for (int r = 0; r < steps; ++r) cnt += st.cnt[entry(r)];
+    for (int o = 1; o < 1 << lanes; o <<= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    __syncwarp();
+    if (write) st.cnt[first] = cnt;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int dt = col_dt<SIG>(cs, c), ag = col_ag<SIG>(cs, c);
+      if ((ag & NFC_AGG_SUM) && dt == NFC_F64) {
+        const double* sum = reinterpret_cast<const double*>(st.s64[c]);
+        double s = 0.0, e = 0.0;
+        for (int r = 0; r < steps; ++r) {
+          if (ERR) e += st.err[c][entry(r)];
+          e += f64_two_sum(s, sum[entry(r)]);
+        }
+        for (int o = 1; o < 1 << lanes; o <<= 1) {
+          const double s2 = __shfl_xor_sync(0xffffffffu, s, o), e2 = __shfl_xor_sync(0xffffffffu, e, o);
+          e += e2;
+          e += f64_two_sum(s, s2);
+        }
+        if (write) {
+          st.s64[c][first] = (uint64_t)__double_as_longlong(ERR ? s : f64_close(s, e));
+          if (ERR) st.err[c][first] = e;
+        }
+      } else if (ag & NFC_AGG_SUM) {
+        uint64_t s = 0;
+        for (int r = 0; r < steps; ++r) s += (uint64_t)agg_sum_bits<NC, SIG>(cs, st, c, entry(r));
+        for (int o = 1; o < 1 << lanes; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (write) {
+          if (dt == NFC_I64) {
+            st.s64[c][first] = s;
+          } else {
+            st.slo[c][first] = (uint32_t)s & 0xFFFFu;
+            st.shi[c][first] = (int32_t)((int64_t)s >> 16);
+          }
+        }
+      }
+      if (!(ag & (NFC_AGG_MIN | NFC_AGG_MAX))) continue;
+      if (dt == NFC_I32) {
+        int32_t lo = INT_MAX, hi = INT_MIN;
+        for (int r = 0; r < steps; ++r) {
+          if (ag & NFC_AGG_MIN) lo = min(lo, static_cast<const int32_t*>(st.mn[c])[entry(r)]);
+          if (ag & NFC_AGG_MAX) hi = max(hi, static_cast<const int32_t*>(st.mx[c])[entry(r)]);
+        }
+        for (int o = 1; o < 1 << lanes; o <<= 1) {
+          lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+          hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        if (write && (ag & NFC_AGG_MIN)) static_cast<int32_t*>(st.mn[c])[first] = lo;
+        if (write && (ag & NFC_AGG_MAX)) static_cast<int32_t*>(st.mx[c])[first] = hi;
+      } else {
+        // As signed numbers; the float64 encodings with the top bit turned.
+        const uint64_t turn = dt == NFC_F64 ? 1ull << 63 : 0ull;
+        int64_t lo = LLONG_MAX, hi = LLONG_MIN;
+        for (int r = 0; r < steps; ++r) {
+          if (ag & NFC_AGG_MIN) lo = min(lo, (int64_t)(static_cast<const uint64_t*>(st.mn[c])[entry(r)] ^ turn));
+          if (ag & NFC_AGG_MAX) hi = max(hi, (int64_t)(static_cast<const uint64_t*>(st.mx[c])[entry(r)] ^ turn));
+        }
+        for (int o = 1; o < 1 << lanes; o <<= 1) {
+          lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+          hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        if (write && (ag & NFC_AGG_MIN)) static_cast<uint64_t*>(st.mn[c])[first] = (uint64_t)lo ^ turn;
+        if (write && (ag & NFC_AGG_MAX)) static_cast<uint64_t*>(st.mx[c])[first] = (uint64_t)hi ^ turn;
+      }
+    }
+    __syncwarp();
+  }
 }
 
 template <int NC, uint32_t SIG, bool ERR = false>

@@ -170,8 +170,7 @@ NFC_DEV void state_apply(const ColSet& cs, const StateRef& st, int64_t d, const 
 
 // Fold a combined row group -- k rows with the given per-column sums (int64
 // bits / float64 bits), minima and maxima (int64 / ordered float64 lanes) --
-// into slot d with one set of atomics.  ERR: the state keeps rounding errors.
-template <bool ERR = false>
+// into slot d with one set of atomics.
 NFC_DEV void state_apply_group(const ColSet& cs, const StateRef& st, int64_t d, uint32_t k, const uint64_t* sum,
                                const uint64_t* mn, const uint64_t* mx) {
   atomicAdd(&st.cnt[d], k);
@@ -180,11 +179,7 @@ NFC_DEV void state_apply_group(const ColSet& cs, const StateRef& st, int64_t d, 
     if (c >= cs.ncols) break;
     const int dt = cs.dtype[c], ag = cs.aggs[c];
     if (dt == NFC_F64) {
-      if (ag & NFC_AGG_SUM) {
-        const double x = __longlong_as_double((long long)sum[c]);
-        if (ERR) f64_atomic_add_err(static_cast<double*>(st.sum[c]) + d, st.err[c] + d, x);
-        else atomicAdd(static_cast<double*>(st.sum[c]) + d, x);
-      }
+      if (ag & NFC_AGG_SUM) atomicAdd(static_cast<double*>(st.sum[c]) + d, __longlong_as_double((long long)sum[c]));
       if (ag & NFC_AGG_MIN) atomicMin(static_cast<unsigned long long*>(st.mn[c]) + d, (unsigned long long)mn[c]);
       if (ag & NFC_AGG_MAX) atomicMax(static_cast<unsigned long long*>(st.mx[c]) + d, (unsigned long long)mx[c]);
     } else {

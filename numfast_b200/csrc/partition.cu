@@ -950,7 +950,7 @@ __global__ void __launch_bounds__(kPartThreads, SIG == 0 && NC >= 2 ? 1 : 2) k_p
       if (hot[h] != 0xFFFFFFFFu) hot_flush<NC, SIG>(a.cs, st, hot[h], acc[h]);
     __syncthreads();
     const int64_t m0 = (int64_t)ms * W;
-    for (int g = threadIdx.x; g < wbk; g += blockDim.x) agg_merge<NC, SIG, true>(a.cs, a.gm, m0 + g, st, g);
+    agg_merge_all<NC, SIG>(a.cs, a.gm, m0, st, wbk, 0);
     __syncthreads();  // the state is reused
   }
 }
@@ -1014,7 +1014,7 @@ __global__ void __launch_bounds__(kPartThreads, 2) k_part_agg(PartAggArgs a) {
                             [&](uint32_t g, const uint64_t* raw) { agg_apply<NC, SIG, false>(a.cs, st, g, raw); });
   __syncthreads();
   if (slice) {
-    for (int g = threadIdx.x; g < wbk; g += blockDim.x) agg_merge<NC, SIG, true>(a.cs, a.gm, m0 + g, st, g);
+    agg_merge_all<NC, SIG>(a.cs, a.gm, m0, st, wbk, 0);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) atomicAdd(a.slice_done + ms, 1u);
@@ -1344,7 +1344,9 @@ int run_partition(const nfc_groupby_args* a, const ColSet& cs_in, const OutSet& 
   const int64_t max_merge = nv / (slice + 1) + 1;
   unsigned char* gmb = nullptr;
   NFC_CUDA(sc.alloc(&gmb, (size_t)max_merge * W * (slot + state_err_bytes_per_slot(cs)) + 64));
-  const StateRef gm = carve_state(cs, gmb, max_merge * W, true);
+  // Slices of kSlice records add no more partial sums to a slot than ever; shorter
+  // ones do, and keep the errors (agg_merge_all).
+  const StateRef gm = carve_state(cs, gmb, max_merge * W, slice < kSlice);
 
   PartAggArgs pa;
   pa.cs = cs;

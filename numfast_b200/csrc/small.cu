@@ -38,82 +38,6 @@ struct SmallShape {
 static_assert(kSmallRows == kProbeBlockRows, "one probe record");
 constexpr int kSmCopies = 8;  // log2 of the most copies of the state
 
-// The 2^lg copies of every slot combined into the first one (whole block).
-template <int NC>
-NFC_DEV void fold_copies(const ColSet& cs, const AggState<NC>& st, int slots, int lg) {
-  const int lanes = min(lg, 5);
-  const int lane = lane_id(), part = lane & ((1 << lanes) - 1);
-  for (int e0 = threadIdx.x & ~31; e0 < slots << lanes; e0 += (int)blockDim.x) {
-    const int g = (e0 + lane) >> lanes;
-    const bool in = g < slots;
-    const int first = (in ? g : 0) << lg;
-    uint32_t cnt = 0;
-    for (int r = part; r < 1 << lg; r += 1 << lanes) cnt += st.cnt[first + r];
-    for (int o = 1; o < 1 << lanes; o <<= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    if (in && part == 0) st.cnt[first] = cnt;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const int dt = cs.dtype[c], ag = cs.aggs[c];
-      if (ag & NFC_AGG_SUM) {
-        if (dt == NFC_F64) {
-          double* sum = reinterpret_cast<double*>(st.s64[c]) + first;
-          double s = 0.0, e = 0.0;
-          for (int r = part; r < 1 << lg; r += 1 << lanes) {
-            e += st.err[c][first + r];
-            e += f64_two_sum(s, sum[r]);
-          }
-          for (int o = 1; o < 1 << lanes; o <<= 1) {
-            const double s2 = __shfl_xor_sync(0xffffffffu, s, o), e2 = __shfl_xor_sync(0xffffffffu, e, o);
-            e += e2;
-            e += f64_two_sum(s, s2);
-          }
-          if (in && part == 0) {
-            sum[0] = s;
-            st.err[c][first] = e;
-          }
-        } else {
-          uint64_t s = 0;
-          for (int r = part; r < 1 << lg; r += 1 << lanes) s += (uint64_t)agg_sum_bits<NC, 0>(cs, st, c, first + r);
-          for (int o = 1; o < 1 << lanes; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-          if (in && part == 0) {
-            if (dt == NFC_I64) {
-              st.s64[c][first] = s;
-            } else {
-              st.slo[c][first] = (uint32_t)s & 0xFFFFu;
-              st.shi[c][first] = (int32_t)((int64_t)s >> 16);
-            }
-          }
-        }
-      }
-      if (ag & (NFC_AGG_MIN | NFC_AGG_MAX)) {
-        // As signed 64-bit numbers; the float64 encodings with the top bit turned.
-        const uint64_t turn = dt == NFC_F64 ? 1ull << 63 : 0ull;
-        auto at = [&](const void* p, int i) {
-          return dt == NFC_I32 ? (int64_t) static_cast<const int32_t*>(p)[i]
-                               : (int64_t)(static_cast<const uint64_t*>(p)[i] ^ turn);
-        };
-        auto put = [&](void* p, int64_t v) {
-          if (dt == NFC_I32) static_cast<int32_t*>(p)[first] = (int32_t)v;
-          else static_cast<uint64_t*>(p)[first] = (uint64_t)v ^ turn;
-        };
-        int64_t lo = LLONG_MAX, hi = LLONG_MIN;
-        for (int r = part; r < 1 << lg; r += 1 << lanes) {
-          if (ag & NFC_AGG_MIN) lo = min(lo, at(st.mn[c], first + r));
-          if (ag & NFC_AGG_MAX) hi = max(hi, at(st.mx[c], first + r));
-        }
-        for (int o = 1; o < 1 << lanes; o <<= 1) {
-          lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-          hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-        }
-        if (in && part == 0) {
-          if (ag & NFC_AGG_MIN) put(st.mn[c], lo);
-          if (ag & NFC_AGG_MAX) put(st.mx[c], hi);
-        }
-      }
-    }
-  }
-}
-
 template <int NC>
 __global__ void __launch_bounds__(SmallShape<NC>::threads, 1) k_small(const int32_t* __restrict__ keys, BitmapSet bms, ColSet cs,
                                                          int n, bool aligned, OutSet o, int64_t out_cap,
@@ -273,7 +197,7 @@ __global__ void __launch_bounds__(SmallShape<NC>::threads, 1) k_small(const int3
   }
   __syncthreads();
   if (lg > 0) {
-    fold_copies(cs, st, w, lg);
+    fold_copies<NC, 0, true>(cs, st, w, lg);
     __syncthreads();
   }
   // ---- present groups in key order: warp w owns consecutive slots.
