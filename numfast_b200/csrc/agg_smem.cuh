@@ -406,10 +406,14 @@ struct HotAcc {
 
 // Keys held in registers: what two 512-thread CTAs per SM leave room for (the
 // slices of 69M Zipf(1.1) rows: four keys at one CTA per SM 1.04 ms, two keys at
-// two CTAs 0.76, four keys at two CTAs, spilled, 1.17).  Run-time column types
-// need room for every type.
+// two CTAs 0.76, four keys at two CTAs, spilled, 1.17).  Two and more columns of
+// run-time types would need one CTA per SM, and the rows of the other keys then
+// lose more than the hot keys gain (40M Zipf(1.1) rows over 30,000 keys, int64 and
+// float64 with all aggregates 1.54 ms without, 1.69 with; four columns 2.13 and
+// 2.55).
+constexpr int kHotKeys = 2;
 template <int NC, uint32_t SIG>
-constexpr int hot_keys() { return SIG != 0 || NC <= 1 ? 2 : 1; }
+constexpr bool hot_columns() { return SIG != 0 || NC == 1; }
 
 template <int NC, uint32_t SIG>
 NFC_DEV void hot_init(const ColSet& cs, HotAcc<NC>& a) {

@@ -911,14 +911,14 @@ __global__ void __launch_bounds__(kPartThreads) k_part_multi(ColSet cs, StateRef
 // The slices of buckets with hot keys, which collect in registers; a kernel of
 // its own, because the registers of this loop slow the plain one.
 template <int NC, bool PACK0, uint32_t SIG>
-__global__ void __launch_bounds__(kPartThreads, SIG == 0 && NC >= 2 ? 1 : 2) k_part_hot(PartAggArgs a) {
+__global__ void __launch_bounds__(kPartThreads, 2) k_part_hot(PartAggArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   if (sync_failed(a.err)) return;
   const int32_t W = 1 << a.wb;
   const int32_t nslices = a.n_merge[1];
   const AggState<NC> st = carve_agg<NC, SIG>(a.cs, smem_raw, W, ~__ldg(a.wide));
   constexpr int NW = Rec<NC, PACK0>::NW;
-  constexpr int H = hot_keys<NC, SIG>();
+  constexpr int H = kHotKeys;
   constexpr int U = 4;
   for (int32_t it = blockIdx.x; it < nslices; it += gridDim.x) {
     const int2 sl = a.slices[it];
@@ -1209,18 +1209,20 @@ static int launch_part(const PartLaunch& q, PartAggArgs& pa, cudaStream_t s, Sta
     // 128 KB of counters at most; 32-bit aggregates alone keep up on hot keys.
     bool wide64 = false;
     for (int c = 0; c < NC; ++c) wide64 |= q.cs.dtype[c] != NFC_I32 && q.cs.aggs[c] != 0;
-    const bool sample = wide64 && q.wb <= 15;
+    const bool sample = hot_columns<NC, SIG>() && wide64 && q.wb <= 15;
     const size_t cnt = sample ? (size_t)4 << q.wb : 0;
     NFC_CUDA(allow_dynamic_smem<k_part_multi>());
     k_part_multi<<<g, kPartThreads, cnt, s>>>(q.cs, pa.gm, pa.rec, NW, pa.offs, q.wb, pa.n_merge, q.multi, sample,
                                               q.hot, pa.slice_done, q.d_err);
     NFC_CUDA(cudaGetLastError());
     tm->launched();
-    if (sample) {
-      NFC_CUDA(allow_dynamic_smem<k_part_hot<NC, PACK0, SIG>>());
-      k_part_hot<NC, PACK0, SIG><<<g, kPartThreads, q.agg_smem, s>>>(pa);
-      NFC_CUDA(cudaGetLastError());
-      tm->launched();
+    if constexpr (hot_columns<NC, SIG>()) {
+      if (sample) {
+        NFC_CUDA(allow_dynamic_smem<k_part_hot<NC, PACK0, SIG>>());
+        k_part_hot<NC, PACK0, SIG><<<g, kPartThreads, q.agg_smem, s>>>(pa);
+        NFC_CUDA(cudaGetLastError());
+        tm->launched();
+      }
     }
   }
   k_part_agg<NC, PACK0, SIG><<<(unsigned)(q.nb + q.max_slices), kPartThreads, q.agg_smem, s>>>(pa);
