@@ -40,7 +40,11 @@ NFC_DEV int col_ag(const ColSet& cs, int c) {
   else if constexpr (SIG != 0) return (int)((SIG >> (5 * c + 2)) & 7u);
   else return cs.aggs[c];
 }
-// Column signatures with a dedicated instantiation .
+// Column c is the row number: only ever in a signature of its own, so run-time
+// types need not be asked.
+template <uint32_t SIG>
+constexpr bool is_row_id(int c) { return SIG != 0 && SIG != kSigSums && ((SIG >> (5 * c)) & 3u) == (uint32_t)kRowId; }
+// Column signatures with a dedicated instantiation.
 constexpr uint32_t kSigI32SumMinMax_F64SumMinMax =
     sig_col(0, NFC_I32, NFC_AGG_SUM | NFC_AGG_MIN | NFC_AGG_MAX) | sig_col(1, NFC_F64, NFC_AGG_SUM | NFC_AGG_MIN | NFC_AGG_MAX);
 constexpr uint32_t kSigI32Sum = sig_col(0, NFC_I32, NFC_AGG_SUM);
