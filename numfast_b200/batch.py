@@ -162,8 +162,8 @@ SEARCH_SPACE = [
     ("warp_agg", [{"warp_agg": 0}, {"warp_agg": 1}, {"warp_agg": 2}, {"warp_agg": 3}]),
     ("schedule", [{"schedule": v} for v in (0, 1, 2)]),
     ("probe_rows", [{"probe_rows": v} for v in (131072, 262144, 524288, 1048576)]),
-    ("emit", [{"emit_slice": 16384, "emit_max_items": 64}, {"emit_slice": 8192, "emit_max_items": 128},
-              {"emit_slice": 32768, "emit_max_items": 16}, {"emit_slice": 65536, "emit_max_items": 8}]),
+    ("emit", [{"emit_slice": 32768, "emit_max_items": 32}, {"emit_slice": 16384, "emit_max_items": 64},
+              {"emit_slice": 8192, "emit_max_items": 128}, {"emit_slice": 65536, "emit_max_items": 8}]),
 ]
 
 

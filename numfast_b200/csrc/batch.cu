@@ -39,11 +39,10 @@
 namespace nfc {
 namespace {
 
-constexpr int kBThreads = 512;
-constexpr int kBWarps = kBThreads / 32;
-constexpr int kBPer = 16;                    // rows per thread per sub-tile
-constexpr int kBSub = kBThreads * kBPer;     // 8192 rows per sub-tile
-constexpr int kBEmitRound = kBThreads * 4;   // slots per emit round
+// NT, the threads of a CTA, is a template parameter: 1,024 with one CTA per SM, 512
+// with two.  Either way an SM has 64 registers per thread.
+constexpr int kBSub = 8192;                  // rows per sub-tile, kBSub / NT per thread
+constexpr int kBEmitAlign = 2048;            // emit slices are multiples of this
 constexpr int kSoloSlack = 16384;            // span a solo query may have above four slots per row, and span
                                              // that needs no arena: the shared table or the CTA's own words
 
@@ -141,10 +140,11 @@ struct BSmem {
   int64_t a64[4];
   uint32_t u32[8];
   uint32_t scan[33];
-  uint32_t red[kBWarps];
-  uint32_t wv[kBWarps][32];
+  uint32_t red[32];
+  uint32_t wv[32][32];
 };
 
+template <int NT>
 NFC_DEV uint32_t block_max_u32(uint32_t v, BSmem& S) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -153,10 +153,11 @@ NFC_DEV uint32_t block_max_u32(uint32_t v, BSmem& S) {
   __syncthreads();
   uint32_t r = 0;
 #pragma unroll
-  for (int w = 0; w < kBWarps; ++w) r = max(r, S.red[w]);
+  for (int w = 0; w < NT / 32; ++w) r = max(r, S.red[w]);
   return r;
 }
 
+template <int NT>
 NFC_DEV uint32_t block_sum_u32(uint32_t v, BSmem& S) {
   v = warp_sum(v);
   __syncthreads();
@@ -164,20 +165,20 @@ NFC_DEV uint32_t block_sum_u32(uint32_t v, BSmem& S) {
   __syncthreads();
   uint32_t r = 0;
 #pragma unroll
-  for (int w = 0; w < kBWarps; ++w) r += S.red[w];
+  for (int w = 0; w < NT / 32; ++w) r += S.red[w];
   return r;
 }
 
 // Sub-tile of kBSub rows at 4-row aligned base g0 (rows g0 .. g0+8191 in
 // groups of 4 per thread per step), masked to [a, b).  Bit e of `mask` says
 // row e of the thread's 16 is in range and has valid key (and value).
-template <bool VEC, bool VALS>
-NFC_DEV void load_sub(const BatchParams& P, int64_t g0, int64_t a, int64_t b, int32_t (&k)[kBPer],
-                      int32_t (&v)[kBPer], uint32_t& mask) {
+template <bool VEC, bool VALS, int NT>
+NFC_DEV void load_sub(const BatchParams& P, int64_t g0, int64_t a, int64_t b, int32_t (&k)[kBSub / NT],
+                      int32_t (&v)[kBSub / NT], uint32_t& mask) {
   mask = 0;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int64_t r4 = g0 + ((int64_t)j * kBThreads + threadIdx.x) * 4;
+  for (int j = 0; j < kBSub / NT / 4; ++j) {
+    const int64_t r4 = g0 + ((int64_t)j * NT + threadIdx.x) * 4;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       k[4 * j + e] = 0;
@@ -292,19 +293,19 @@ NFC_DEV void plan_query(const BatchParams& P, const QDesc& qd, QRt* qr, int q) {
   atomicExch(&qr->plan_ready, 1u);
 }
 
-template <bool VEC>
+template <bool VEC, int NT>
 NFC_DEV void do_probe(const BatchParams& P, BSmem& S, int q, uint32_t idx) {
   const QDesc qd = P.qd[q];
   QRt* qr = P.qr + q;
   const int64_t a = qd.row_off + (int64_t)idx * P.probe_rows;
   const int64_t b = imin64(a + P.probe_rows, qd.row_off + qd.rows);
   uint32_t mx = 0, mnc = 0, cnt = 0;
-  int32_t k[kBPer], v[kBPer];
+  int32_t k[kBSub / NT], v[kBSub / NT];
   for (int64_t g0 = a & ~3ll; g0 < b; g0 += kBSub) {
     uint32_t m;
-    load_sub<VEC, false>(P, g0, a, b, k, v, m);
+    load_sub<VEC, false, NT>(P, g0, a, b, k, v, m);
 #pragma unroll
-    for (int e = 0; e < kBPer; ++e) {
+    for (int e = 0; e < kBSub / NT; ++e) {
       if (m & (1u << e)) {
         const uint32_t o = ord32(k[e]);
         mx = max(mx, o);
@@ -313,9 +314,9 @@ NFC_DEV void do_probe(const BatchParams& P, BSmem& S, int q, uint32_t idx) {
       }
     }
   }
-  mx = block_max_u32(mx, S);
-  mnc = block_max_u32(mnc, S);
-  cnt = block_sum_u32(cnt, S);
+  mx = block_max_u32<NT>(mx, S);
+  mnc = block_max_u32<NT>(mnc, S);
+  cnt = block_sum_u32<NT>(cnt, S);
   if (threadIdx.x == 0) {
     if (cnt) {
       atomicMax(&qr->kmax_o, mx);
@@ -332,13 +333,14 @@ NFC_DEV void do_probe(const BatchParams& P, BSmem& S, int q, uint32_t idx) {
 
 // Global packed reductions for one loaded sub-tile.  Returns false if a
 // value breaks the packed bound (the query is then flagged).
-NFC_DEV bool global_apply(const BatchParams& P, BSmem& S, const int32_t (&k)[kBPer], const int32_t (&v)[kBPer],
-                          uint32_t m, int64_t kmin, unsigned long long* st, uint32_t sh, uint64_t lim) {
+template <int NT>
+NFC_DEV bool global_apply(const BatchParams& P, BSmem& S, const int32_t (&k)[kBSub / NT],
+                          const int32_t (&v)[kBSub / NT], uint32_t m, int64_t kmin, unsigned long long* st, uint32_t sh, uint64_t lim) {
   bool ok = true;
   const uint64_t one = 1ull << sh;
   const int warp = threadIdx.x >> 5, lane = lane_id();
 #pragma unroll
-  for (int e = 0; e < kBPer; ++e) {
+  for (int e = 0; e < kBSub / NT; ++e) {
     const bool in = (m >> e) & 1u;
     if (in && absu(v[e]) > lim) ok = false;
     if (P.warp_agg == 2) {
@@ -382,16 +384,16 @@ NFC_DEV bool global_apply(const BatchParams& P, BSmem& S, const int32_t (&k)[kBP
   return ok;
 }
 
-template <bool VEC>
+template <bool VEC, int NT>
 NFC_DEV void global_chunk(const BatchParams& P, BSmem& S, const QDesc& qd, QRt* qr, int64_t a, int64_t b,
                           int64_t kmin, unsigned long long* st, uint32_t sh) {
   const uint64_t lim = packed_limit(qd.rows, sh);
-  int32_t k[kBPer], v[kBPer];
+  int32_t k[kBSub / NT], v[kBSub / NT];
   bool ok = true;
   for (int64_t g0 = a & ~3ll; g0 < b; g0 += kBSub) {
     uint32_t m;
-    load_sub<VEC, true>(P, g0, a, b, k, v, m);
-    ok &= global_apply(P, S, k, v, m, kmin, st, sh, lim);
+    load_sub<VEC, true, NT>(P, g0, a, b, k, v, m);
+    ok &= global_apply<NT>(P, S, k, v, m, kmin, st, sh, lim);
   }
   if (!ok) atomicOr(&qr->flags, kFlUnsafe);
 }
@@ -406,12 +408,12 @@ NFC_DEV void global_chunk(const BatchParams& P, BSmem& S, const QDesc& qd, QRt* 
 // reduction per row.
 constexpr int kCacheProbe = 8;
 
-template <bool VEC>
+template <bool VEC, int NT>
 NFC_DEV void cached_chunk(const BatchParams& P, BSmem& S, uint32_t* skey, uint32_t* s_cnt, int32_t* s_sum, int lgT,
                           const QDesc& qd, QRt* qr, int64_t a, int64_t b, int64_t kmin, unsigned long long* st,
                           uint32_t sh) {
   const int T = 1 << lgT;
-  for (int i = threadIdx.x; i < T; i += kBThreads) {
+  for (int i = threadIdx.x; i < T; i += NT) {
     skey[i] = 0u;
     s_cnt[i] = 0u;
     s_sum[i] = 0;
@@ -422,14 +424,14 @@ NFC_DEV void cached_chunk(const BatchParams& P, BSmem& S, uint32_t* skey, uint32
   const uint32_t lim_s = (uint32_t)(0x7FFFFFFFu / (uint32_t)imax64(b - a, 1));
   const uint64_t one = 1ull << sh;
   const uint32_t fill_cap = (uint32_t)(T - T / 4);
-  int32_t k[kBPer], v[kBPer];
+  int32_t k[kBSub / NT], v[kBSub / NT];
   bool ok = true;
   for (int64_t g0 = a & ~3ll; g0 < b; g0 += kBSub) {
     uint32_t m;
-    load_sub<VEC, true>(P, g0, a, b, k, v, m);
+    load_sub<VEC, true, NT>(P, g0, a, b, k, v, m);
     const bool can_insert = *reinterpret_cast<volatile uint32_t*>(&S.u32[4]) < fill_cap;
 #pragma unroll
-    for (int e = 0; e < kBPer; ++e) {
+    for (int e = 0; e < kBSub / NT; ++e) {
       if (!(m & (1u << e))) continue;
       const uint32_t av = absu(v[e]);
       ok &= av <= lim;
@@ -461,7 +463,7 @@ NFC_DEV void cached_chunk(const BatchParams& P, BSmem& S, uint32_t* skey, uint32
   }
   if (!ok) atomicOr(&qr->flags, kFlUnsafe);
   __syncthreads();
-  for (int i = threadIdx.x; i < T; i += kBThreads) {
+  for (int i = threadIdx.x; i < T; i += NT) {
     const uint32_t w = skey[i];
     const uint32_t c = s_cnt[i];
     if (w && c) atomicAdd(st + (w - 1u), (unsigned long long)c * one + (unsigned long long)(int64_t)s_sum[i]);
@@ -470,7 +472,7 @@ NFC_DEV void cached_chunk(const BatchParams& P, BSmem& S, uint32_t* skey, uint32
 
 // Shared-memory table: s_cnt[span], s_sum[span] (int32 partial sums, safe
 // while rows * |value| < 2^31 for the chunk).
-template <bool VEC>
+template <bool VEC, int NT>
 NFC_DEV uint32_t do_agg(const BatchParams& P, BSmem& S, uint32_t* s_cnt, int32_t* s_sum, int q, uint32_t idx) {
   const QDesc qd = P.qd[q];
   QRt* qr = P.qr + q;
@@ -496,12 +498,12 @@ NFC_DEV uint32_t do_agg(const BatchParams& P, BSmem& S, uint32_t* s_cnt, int32_t
     while ((2 << lgT) * 12 <= P.smem_slots * 8) ++lgT;
     const int T = 1 << lgT;
     uint32_t* base = s_cnt;
-    cached_chunk<VEC>(P, S, base + 2 * T, base, reinterpret_cast<int32_t*>(base + T), lgT, qd, qr, a, b, kmin, st,
+    cached_chunk<VEC, NT>(P, S, base + 2 * T, base, reinterpret_cast<int32_t*>(base + T), lgT, qd, qr, a, b, kmin, st,
                       sh);
   } else if (plan == kPlanGlobal) {
-    global_chunk<VEC>(P, S, qd, qr, a, b, kmin, st, sh);
+    global_chunk<VEC, NT>(P, S, qd, qr, a, b, kmin, st, sh);
   } else if (plan == kPlanSmem) {
-    for (int64_t i = threadIdx.x; i < span; i += kBThreads) {
+    for (int64_t i = threadIdx.x; i < span; i += NT) {
       s_cnt[i] = 0;
       s_sum[i] = 0;
     }
@@ -509,12 +511,12 @@ NFC_DEV uint32_t do_agg(const BatchParams& P, BSmem& S, uint32_t* s_cnt, int32_t
     const uint32_t lim_s = (uint32_t)(0x7FFFFFFFu / (uint32_t)imax64(b - a, 1));
     const uint64_t lim_q = packed_limit(qd.rows, sh);
     bool small = true, ok = true;
-    int32_t k[kBPer], v[kBPer];
+    int32_t k[kBSub / NT], v[kBSub / NT];
     for (int64_t g0 = a & ~3ll; g0 < b; g0 += kBSub) {
       uint32_t m;
-      load_sub<VEC, true>(P, g0, a, b, k, v, m);
+      load_sub<VEC, true, NT>(P, g0, a, b, k, v, m);
 #pragma unroll
-      for (int e = 0; e < kBPer; ++e) {
+      for (int e = 0; e < kBSub / NT; ++e) {
         if (m & (1u << e)) {
           const uint32_t av = absu(v[e]);
           small &= av <= lim_s;
@@ -528,14 +530,14 @@ NFC_DEV uint32_t do_agg(const BatchParams& P, BSmem& S, uint32_t* s_cnt, int32_t
     if (!ok) atomicOr(&qr->flags, kFlUnsafe);
     if (__syncthreads_and(small)) {
       const uint64_t one = 1ull << sh;
-      for (int64_t i = threadIdx.x; i < span; i += kBThreads) {
+      for (int64_t i = threadIdx.x; i < span; i += NT) {
         const uint32_t c = s_cnt[i];
         if (c) atomicAdd(st + i, (unsigned long long)c * one + (unsigned long long)(int64_t)s_sum[i]);
       }
     } else {
       // Some |value| could overflow the int32 partial sums: redo the chunk
       // with 64-bit global reductions.
-      global_chunk<VEC>(P, S, qd, qr, a, b, kmin, st, sh);
+      global_chunk<VEC, NT>(P, S, qd, qr, a, b, kmin, st, sh);
     }
   }
   __threadfence();
@@ -552,6 +554,7 @@ NFC_DEV void unpack(uint64_t w, uint32_t sh, int64_t& cnt, int64_t& sum) {
   cnt = (int64_t)((w - (uint64_t)s) >> sh);
 }
 
+template <int NT>
 NFC_DEV void do_emit(const BatchParams& P, BSmem& S, int q, uint32_t j) {
   const QDesc qd = P.qd[q];
   QRt* qr = P.qr + q;
@@ -577,14 +580,14 @@ NFC_DEV void do_emit(const BatchParams& P, BSmem& S, int q, uint32_t j) {
   if (lo >= span) return;
   const int64_t hi = imin64(lo + qd.emit_slice, span);
   if (unsafe) {
-    for (int64_t i = lo + threadIdx.x; i < hi; i += kBThreads) st[i] = 0ull;
+    for (int64_t i = lo + threadIdx.x; i < hi; i += NT) st[i] = 0ull;
     if (threadIdx.x == 0 && hi == span) P.qstatus[q] = 1;
     return;
   }
   // Pass 1: groups in the slice.
   uint32_t c = 0;
-  for (int64_t i = lo + threadIdx.x; i < hi; i += kBThreads) c += ldcg_u64(st + i) != 0ull;
-  const uint32_t total = block_sum_u32(c, S);
+  for (int64_t i = lo + threadIdx.x; i < hi; i += NT) c += ldcg_u64(st + i) != 0ull;
+  const uint32_t total = block_sum_u32<NT>(c, S);
   if (threadIdx.x < 32) {
     const int64_t lbx = lookback_exclusive(P.lb + qd.lb_base, j, total, &P.hdr->err);  // whole warp
     if (threadIdx.x == 0) {
@@ -598,7 +601,7 @@ NFC_DEV void do_emit(const BatchParams& P, BSmem& S, int q, uint32_t j) {
   __syncthreads();
   int64_t pos = out_base + S.a64[0];
   // Pass 2: compact in ascending slot order and clear.
-  for (int64_t r = lo; r < hi; r += kBEmitRound) {
+  for (int64_t r = lo; r < hi; r += 4 * NT) {
     const int64_t i0 = r + (int64_t)threadIdx.x * 4;
     uint64_t w[4];
     uint32_t cnt = 0;
@@ -628,22 +631,22 @@ NFC_DEV void do_emit(const BatchParams& P, BSmem& S, int q, uint32_t j) {
 
 // One CTA: packed reductions into an arena slice, then an ascending
 // compaction of the slice by the same CTA (which also clears it).
-template <bool VEC>
+template <bool VEC, int NT>
 NFC_DEV void solo_global(const BatchParams& P, BSmem& S, const QDesc& qd, int q, int64_t a, int64_t b,
                          int64_t kmin, int64_t span, unsigned long long* st, int64_t out_base) {
   const uint32_t sh = 64u - bitlen64((uint64_t)qd.rows);
   const uint64_t lim = packed_limit(qd.rows, sh);
-  int32_t k[kBPer], v[kBPer];
+  int32_t k[kBSub / NT], v[kBSub / NT];
   bool ok = true;
   for (int64_t g0 = a & ~3ll; g0 < b; g0 += kBSub) {
     uint32_t m;
-    load_sub<VEC, true>(P, g0, a, b, k, v, m);
-    ok &= global_apply(P, S, k, v, m, kmin, st, sh, lim);
+    load_sub<VEC, true, NT>(P, g0, a, b, k, v, m);
+    ok &= global_apply<NT>(P, S, k, v, m, kmin, st, sh, lim);
   }
   __threadfence();
   const bool all_ok = __syncthreads_and(ok);
   int64_t pos = out_base;
-  for (int64_t r = 0; r < span; r += kBEmitRound) {
+  for (int64_t r = 0; r < span; r += 4 * NT) {
     const int64_t i0 = r + (int64_t)threadIdx.x * 4;
     uint64_t w[4];
     uint32_t cnt = 0;
@@ -680,17 +683,17 @@ NFC_DEV void solo_global(const BatchParams& P, BSmem& S, const QDesc& qd, int q,
   }
 }
 
-template <bool VEC>
+template <bool VEC, int NT>
 NFC_DEV void do_solo(const BatchParams& P, BSmem& S, uint32_t* s_cnt, int32_t* s_sum, int q) {
   const QDesc qd = P.qd[q];
   const int64_t a = qd.row_off, b = qd.row_off + qd.rows;
   uint32_t mx = 0, mnc = 0, cnt = 0;
-  int32_t k[kBPer], v[kBPer];
+  int32_t k[kBSub / NT], v[kBSub / NT];
   for (int64_t g0 = a & ~3ll; g0 < b; g0 += kBSub) {
     uint32_t m;
-    load_sub<VEC, false>(P, g0, a, b, k, v, m);
+    load_sub<VEC, false, NT>(P, g0, a, b, k, v, m);
 #pragma unroll
-    for (int e = 0; e < kBPer; ++e) {
+    for (int e = 0; e < kBSub / NT; ++e) {
       if (m & (1u << e)) {
         const uint32_t o = ord32(k[e]);
         mx = max(mx, o);
@@ -699,9 +702,9 @@ NFC_DEV void do_solo(const BatchParams& P, BSmem& S, uint32_t* s_cnt, int32_t* s
       }
     }
   }
-  mx = block_max_u32(mx, S);
-  mnc = block_max_u32(mnc, S);
-  cnt = block_sum_u32(cnt, S);
+  mx = block_max_u32<NT>(mx, S);
+  mnc = block_max_u32<NT>(mnc, S);
+  cnt = block_sum_u32<NT>(cnt, S);
   QRt* qr = P.qr + q;
   if (cnt == 0) {
     if (threadIdx.x == 0) {
@@ -733,10 +736,10 @@ NFC_DEV void do_solo(const BatchParams& P, BSmem& S, uint32_t* s_cnt, int32_t* s
   const int64_t out_base = S.a64[0];
   if (out_base < 0) return;
   if (!in_smem) {
-    solo_global<VEC>(P, S, qd, q, a, b, kmin, span, P.arena + S.a64[1], out_base);
+    solo_global<VEC, NT>(P, S, qd, q, a, b, kmin, span, P.arena + S.a64[1], out_base);
     return;
   }
-  for (int64_t i = threadIdx.x; i < span; i += kBThreads) {
+  for (int64_t i = threadIdx.x; i < span; i += NT) {
     s_cnt[i] = 0;
     s_sum[i] = 0;
   }
@@ -745,9 +748,9 @@ NFC_DEV void do_solo(const BatchParams& P, BSmem& S, uint32_t* s_cnt, int32_t* s
   bool small = true;
   for (int64_t g0 = a & ~3ll; g0 < b; g0 += kBSub) {
     uint32_t m;
-    load_sub<VEC, true>(P, g0, a, b, k, v, m);
+    load_sub<VEC, true, NT>(P, g0, a, b, k, v, m);
 #pragma unroll
-    for (int e = 0; e < kBPer; ++e) {
+    for (int e = 0; e < kBSub / NT; ++e) {
       if (m & (1u << e)) {
         small &= absu(v[e]) <= lim_s;
         const int64_t slot = (int64_t)k[e] - kmin;
@@ -765,7 +768,7 @@ NFC_DEV void do_solo(const BatchParams& P, BSmem& S, uint32_t* s_cnt, int32_t* s
     return;
   }
   int64_t pos = out_base;
-  for (int64_t r = 0; r < span; r += kBEmitRound) {
+  for (int64_t r = 0; r < span; r += 4 * NT) {
     const int64_t i0 = r + (int64_t)threadIdx.x * 4;
     uint32_t c4[4];
     uint32_t n = 0;
@@ -794,8 +797,8 @@ NFC_DEV void do_solo(const BatchParams& P, BSmem& S, uint32_t* s_cnt, int32_t* s
   }
 }
 
-template <bool VEC, int MINB>
-__global__ void __launch_bounds__(kBThreads, MINB) k_batch(const BatchParams P) {
+template <bool VEC, int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_batch(const BatchParams P) {
   extern __shared__ __align__(16) unsigned char bsm[];
   __shared__ BSmem S;
   uint32_t* s_cnt = reinterpret_cast<uint32_t*>(bsm);
@@ -817,10 +820,10 @@ __global__ void __launch_bounds__(kBThreads, MINB) k_batch(const BatchParams P) 
     const long long t0 = clock64();
     uint32_t plan = 0;
     switch (type) {
-      case kItProbe: do_probe<VEC>(P, S, q, idx); break;
-      case kItSolo: do_solo<VEC>(P, S, s_cnt, s_sum, q); break;
-      case kItAgg: plan = do_agg<VEC>(P, S, s_cnt, s_sum, q, idx); break;
-      default: do_emit(P, S, q, idx); break;
+      case kItProbe: do_probe<VEC, NT>(P, S, q, idx); break;
+      case kItSolo: do_solo<VEC, NT>(P, S, s_cnt, s_sum, q); break;
+      case kItAgg: plan = do_agg<VEC, NT>(P, S, s_cnt, s_sum, q, idx); break;
+      default: do_emit<NT>(P, S, q, idx); break;
     }
     if (threadIdx.x == 0) {
       const unsigned long long dt = (unsigned long long)(clock64() - t0);
@@ -848,18 +851,18 @@ __global__ void k_bitmap_slice(const uint8_t* __restrict__ src, int64_t off, int
   }
 }
 
-template <bool VEC, int MINB>
+template <bool VEC, int NT>
 cudaError_t launch_batch(const BatchParams& P, int grid, size_t smem, cudaStream_t s) {
-  k_batch<VEC, MINB><<<grid, kBThreads, smem, s>>>(P);
+  k_batch<VEC, NT><<<grid, NT, smem, s>>>(P);
   return cudaGetLastError();
 }
 
 // Dynamic shared memory limits are raised outside any stream capture.
 cudaError_t set_batch_attributes() {
-  cudaError_t e = allow_dynamic_smem<k_batch<true, 1>>();
-  if (e == cudaSuccess) e = allow_dynamic_smem<k_batch<true, 2>>();
-  if (e == cudaSuccess) e = allow_dynamic_smem<k_batch<false, 1>>();
-  if (e == cudaSuccess) e = allow_dynamic_smem<k_batch<false, 2>>();
+  cudaError_t e = allow_dynamic_smem<k_batch<true, 1024>>();
+  if (e == cudaSuccess) e = allow_dynamic_smem<k_batch<true, 512>>();
+  if (e == cudaSuccess) e = allow_dynamic_smem<k_batch<false, 1024>>();
+  if (e == cudaSuccess) e = allow_dynamic_smem<k_batch<false, 512>>();
   return e;
 }
 
@@ -917,23 +920,25 @@ int batch_grid(const nfc_batch* b) {
   return (int)std::min<int64_t>((int64_t)num_sms() * b->tune.ctas_per_sm, b->n_items);
 }
 
-// Picked on mixed batches of 40 to 512 queries of 1K..4M rows.  The emit items
-// come last and a large query's eight slices of up to 512K slots left most of
-// the chip idle; slices of 16K slots halve the launch (512 queries, 253M rows:
-// 2.75 -> 1.58 ms; 40 queries: 0.76 -> 0.37).  Two CTAs per SM with the
-// shared-memory cache in front of the global state (warp_agg 3) take 3.1 ms of
-// the one-CTA, match_any form to 2.75.  Finer slices lose on large batches
-// (4K slots: 2.02 ms).
+// One CTA per SM, so that its table holds 16,384 keys: in the global state 64
+// queries of 4M rows over 12,000 keys take 2,420 us instead of 970, and any batch
+// of such queries 1.5 to 2.4 times as long.  1,024 threads, because 512 leave the SM
+// half empty (512 mixed queries of 1K..4M rows, 253M rows: 2,120 -> 1,610 us; two
+// CTAs of 512 threads and 8,192 slots each: 1,570).  The shared-memory cache in
+// front of the global state (warp_agg 3) takes the skewed queries of a mixed batch
+// from 2,350 to 1,680 us.  Emit items come last: a large query's eight slices of up
+// to 512K slots left most of the chip idle (3,340 us), 64 slices of 16K cost few-key
+// queries a tenth (64 of 1M rows over ten keys: 311 us, 276 with 32 slices of 32K).
 void default_tuning(nfc_batch_tuning* t) {
   t->solo_rows = 32768;
   t->chunk_rows = 65536;
   t->probe_rows = 262144;
-  t->emit_slice = 16384;
-  t->emit_max_items = 64;
-  t->smem_slots = 8192;
+  t->emit_slice = 32768;
+  t->emit_max_items = 32;
+  t->smem_slots = 16384;
   t->smem_span_div = 2;
   t->warp_agg = 3;
-  t->ctas_per_sm = 2;
+  t->ctas_per_sm = 1;
   t->schedule = 2;
   t->agg_split = 0;
   t->arena_bytes = 0;
@@ -943,7 +948,7 @@ int check_tuning(const nfc_batch_tuning& t) {
   auto pow2ok = [](int32_t x, int32_t lo, int32_t hi) { return x >= lo && x <= hi && x % kBSub == 0; };
   if (t.solo_rows < 0 || t.solo_rows > (1 << 20)) return 0;
   if (!pow2ok(t.chunk_rows, kBSub, 1 << 24) || !pow2ok(t.probe_rows, kBSub, 1 << 26)) return 0;
-  if (t.emit_slice < kBEmitRound || t.emit_slice % kBEmitRound) return 0;
+  if (t.emit_slice < kBEmitAlign || t.emit_slice % kBEmitAlign) return 0;
   if (t.emit_max_items < 1 || t.emit_max_items > 4096) return 0;
   if (t.ctas_per_sm != 1 && t.ctas_per_sm != 2) return 0;
   if (t.smem_slots < 1024 || t.smem_slots % 1024) return 0;
@@ -978,7 +983,7 @@ extern "C" nfc_batch* nfc_batch_create(int64_t nq, const int64_t* row_offsets, c
   if (!check_tuning(t)) {
     set_last_error("nfc_batch_create: invalid tuning (chunk/probe rows multiples of %d, emit_slice multiple of %d, "
                    "smem_slots multiple of 1024 within the per-CTA shared memory, ctas_per_sm 1 or 2)",
-                   kBSub, kBEmitRound);
+                   kBSub, kBEmitAlign);
     return nullptr;
   }
   if (row_offsets[0] != 0) {
@@ -1026,7 +1031,7 @@ extern "C" nfc_batch* nfc_batch_create(int64_t nq, const int64_t* row_offsets, c
       const int64_t cap = std::max<int64_t>(d.rows, t.smem_slots);
       int64_t ne = std::min<int64_t>((cap + t.emit_slice - 1) / t.emit_slice, t.emit_max_items);
       int64_t slice = (cap + ne - 1) / ne;
-      slice = (slice + kBEmitRound - 1) / kBEmitRound * kBEmitRound;
+      slice = (slice + kBEmitAlign - 1) / kBEmitAlign * kBEmitAlign;
       d.n_emit = (uint32_t)ne;
       d.emit_slice = (uint32_t)slice;
       d.lb_base = lb;
@@ -1148,8 +1153,8 @@ int enqueue_batch(nfc_batch* b, const BatchParams& P, bool vec, cudaStream_t s) 
   const int grid = batch_grid(b);
   const size_t smem = (size_t)b->tune.smem_slots * 8;
   cudaError_t e;
-  if (vec) e = cps == 2 ? launch_batch<true, 2>(P, grid, smem, s) : launch_batch<true, 1>(P, grid, smem, s);
-  else e = cps == 2 ? launch_batch<false, 2>(P, grid, smem, s) : launch_batch<false, 1>(P, grid, smem, s);
+  if (vec) e = cps == 2 ? launch_batch<true, 512>(P, grid, smem, s) : launch_batch<true, 1024>(P, grid, smem, s);
+  else e = cps == 2 ? launch_batch<false, 512>(P, grid, smem, s) : launch_batch<false, 1024>(P, grid, smem, s);
   NFC_CUDA(e);
   return NFC_OK;
 }

@@ -38,8 +38,9 @@ def test_spans_around_the_shared_table(cuda, rows, extra):
     b.close()
 
 
+@pytest.mark.parametrize("slots,ctas", [(16_384, 1), (8_192, 2), (1_024, 1)])
 @pytest.mark.parametrize("rows", [2_500, 30_000])
-def test_small_arena(cuda, rows):
+def test_small_arena(cuda, rows, slots, ctas):
     """A small explicit arena: queries of up to 16,384 keys never needed it; wider ones are deferred
     and still right."""
     rs = np.random.default_rng(rows)
@@ -49,7 +50,7 @@ def test_small_arena(cuda, rows):
     off = np.arange(len(spans) + 1, dtype=np.int64) * rows
     k, v = np.concatenate(keys), np.concatenate(vals)
     t = B.default_tuning()
-    t.arena_bytes = 64 * 1024
+    t.arena_bytes, t.smem_slots, t.ctas_per_sm = 64 * 1024, slots, ctas
     b = B.BatchGroupby(off, tuning=t)
     assert b.info()["arena_bytes"] == 64 * 1024
     for graph in (False, True, True):
