@@ -16,22 +16,22 @@
 //                       order, a thread per 8 or 16 consecutive rows.  A thread finds its
 //                       run heads (valid rows whose key differs from the
 //                       previous valid row's), sums the rows before its first
-//                       head and after its last one into shared memory, and a
-//                       decoupled look-back gives the tile its first run
+//                       head and after its last one and each run in between,
+//                       and a decoupled look-back gives the tile its first run
 //                       number.  The thread that holds a run's head then adds
 //                       what the threads after it have of that run (a whole
-//                       warp without heads is one step) and writes the run.
+//                       warp without heads is one step); the runs are staged
+//                       in shared memory and written out column by column.
 //                       The tile's first run (continued from earlier tiles) and
 //                       last run (possibly continued by later ones) leave as
 //                       two partial "pieces";
 //   3. k_sorted_fix     the pieces are merged in order (segmented scan by run
-//                       number): chunks of 1,024 in parallel CTAs, then the
+//                       number): chunks of a CTA each, then the
 //                       chunks' own edge runs in one CTA.
 // Output keys are written by the thread holding each run's head.  float64 sums
 // differ from the reference's row loop in the order of their additions (mean
 // relative error of a run's sum below 2^-53); everything else is exact.
 #include <algorithm>
-#include <type_traits>
 
 #include "groupby_host.h"
 
@@ -42,10 +42,14 @@ constexpr int kSoThreads = 256;                    // threads with rows; one mor
 constexpr int kSoWarps = kSoThreads / 32;
 // Consecutive rows per thread and rows per tile: more where a row is little work.
 constexpr int so_rows(int nc) { return nc <= 1 ? 16 : 8; }
+// float64 rows added in fours (Seg); three and more columns lack the registers.
+constexpr bool so_fours(int nc) { return nc <= 2; }
 constexpr int so_tile(int nc) { return kSoThreads * so_rows(nc); }
 static_assert(kProbeBlockRows % so_tile(0) == 0 && kProbeBlockRows % so_tile(4) == 0,
               "tiles do not straddle probe records");
-constexpr int kFixThreads = 1024;
+// Pieces of a chunk in k_sorted_fix; with three and more columns a thread needs more
+// than the 64 registers that 1,024 leave it.
+constexpr int fix_threads(int nc) { return nc <= 2 ? 1024 : 512; }
 
 // ---------------------------------------------------------------- run aggregate
 // Integers are kept as int64 bits (sums wrap like the other strategies' int64
@@ -53,13 +57,12 @@ constexpr int kFixThreads = 1024;
 // int32 min/max use int32 identities and 32-bit compares.  A count never
 // exceeds the row count (< 2^31).
 //
-// A float64 sum of rows added one after the other loses with the root of their
-// number.  So a thread adds its rows in fours (`rest`, added to the sum by
-// seg_add_four), and combining two run aggregates keeps the rounding error of the
-// float64 addition in `rest` (seg_close adds it).  Mean relative error of a sum,
-// 20M rows in runs of 200: 1.2e-16 with plain chains, 7e-17 as a tree over the
-// rows, 4.5e-17 this way; the errors of every single row as well: 4.4e-17, but
-// 5-12% of the time.
+// A float64 sum of many terms added one after the other loses with the root of
+// their number.  So a thread adds its rows in fours (from the second four on in
+// `rest`, which seg_add_four adds to the sum), and the aggregates of threads, warps and tiles are
+// added up with the rounding errors of the additions (in `rest`; seg_close adds
+// them).  Mean relative error of a sum, 20M rows in runs of 200: 1.2e-16 with plain
+// chains, 7e-17 as a tree over the rows, 4.5e-17 this way.
 template <int NC>
 struct Seg {
   uint32_t cnt;
@@ -140,16 +143,20 @@ NFC_DEV void seg_combine(const ColSet& cs, Seg<NC>& a, const Seg<NC>& b) {
   }
 }
 
-// Fold one row: int32 values as their 32-bit word, 8-byte values as bits.
+// Fold one row: int32 values as their 32-bit word, 8-byte values as bits.  first:
+// one of the thread's first four rows.
 template <int NC, uint32_t SIG>
-NFC_DEV void seg_add_row(const ColSet& cs, Seg<NC>& a, const uint64_t* raw) {
+NFC_DEV void seg_add_row(const ColSet& cs, Seg<NC>& a, const uint64_t* raw, bool first) {
   a.cnt += 1;
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     const int dt = col_dt<SIG>(cs, c), ag = col_ag<SIG>(cs, c);
     const uint64_t r = raw[c];
     if (dt == NFC_F64) {
-      if (ag & NFC_AGG_SUM) a.rest[c] += __longlong_as_double((long long)r);
+      if (ag & NFC_AGG_SUM) {
+        if (first) a.sum[c] = f64_add_bits(a.sum[c], r);
+        else a.rest[c] += __longlong_as_double((long long)r);
+      }
       if (ag & (NFC_AGG_MIN | NFC_AGG_MAX)) {
         // One order-preserving word for both lanes (the encodings of
         // nfc_common.cuh); NaN wins both.
@@ -451,35 +458,6 @@ NFC_DEV void load_rows4(const ColSet& cs, int64_t n, bool aligned, int64_t row, 
   }
 }
 
-// A thread's rows of column c (load_rows4's conventions).
-template <int kSoRows, uint32_t SIG>
-NFC_DEV void load_rows(const ColSet& cs, int c, int64_t n, bool aligned, int64_t row, uint64_t (&v)[kSoRows]) {
-  if (aligned && row + kSoRows <= n) {
-    if (col_dt<SIG>(cs, c) == NFC_I32) {
-      const int4* q = reinterpret_cast<const int4*>(static_cast<const int32_t*>(cs.data[c]) + row);
-#pragma unroll
-      for (int e = 0; e < kSoRows / 4; ++e) {
-        const int4 x = __ldg(q + e);
-        v[4 * e] = (uint32_t)x.x; v[4 * e + 1] = (uint32_t)x.y; v[4 * e + 2] = (uint32_t)x.z; v[4 * e + 3] = (uint32_t)x.w;
-      }
-    } else {
-      const ulonglong2* q = reinterpret_cast<const ulonglong2*>(static_cast<const uint64_t*>(cs.data[c]) + row);
-#pragma unroll
-      for (int e = 0; e < kSoRows / 2; ++e) {
-        const ulonglong2 x = __ldg(q + e);
-        v[2 * e] = x.x;
-        v[2 * e + 1] = x.y;
-      }
-    }
-  } else {
-#pragma unroll
-    for (int r = 0; r < kSoRows; ++r)
-      v[r] = row + r >= n                       ? 0ull
-             : col_dt<SIG>(cs, c) == NFC_I32 ? (uint64_t)(uint32_t) static_cast<const int32_t*>(cs.data[c])[row + r]
-                                             : static_cast<const uint64_t*>(cs.data[c])[row + r];
-  }
-}
-
 // Partial runs of the tile's threads, one array per field so that neighbouring
 // threads touch neighbouring words.
 template <int NC>
@@ -503,19 +481,122 @@ NFC_DEV void part_store(const ColSet& cs, Partials<NC>& p, int t, const Seg<NC>&
 }
 
 template <int NC, uint32_t SIG>
-NFC_DEV void part_add(const ColSet& cs, Seg<NC>& a, const Partials<NC>& p, int t) {
-  Seg<NC> b;
-  b.cnt = p.cnt[t];
+NFC_DEV void part_load(const ColSet& cs, Seg<NC>& a, const Partials<NC>& p, int t) {
+  a.cnt = p.cnt[t];
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     const int ag = col_ag<SIG>(cs, c);
-    b.sum[c] = ag & NFC_AGG_SUM ? p.sum[c][t] : 0ull;
-    b.rest[c] = 0.0;
-    b.mn[c] = ag & NFC_AGG_MIN ? p.mn[c][t] : 0ull;
-    b.mx[c] = ag & NFC_AGG_MAX ? p.mx[c][t] : 0ull;
+    a.sum[c] = ag & NFC_AGG_SUM ? p.sum[c][t] : 0ull;
+    a.rest[c] = 0.0;
+    a.mn[c] = ag & NFC_AGG_MIN ? p.mn[c][t] : 0ull;
+    a.mx[c] = ag & NFC_AGG_MAX ? p.mx[c][t] : 0ull;
   }
+}
+
+template <int NC, uint32_t SIG>
+NFC_DEV void part_add(const ColSet& cs, Seg<NC>& a, const Partials<NC>& p, int t) {
+  Seg<NC> b;
+  part_load<NC, SIG>(cs, b, p, t);
   seg_combine<NC, SIG>(cs, a, b);
 }
+
+// The tile's runs on their way out: arrays of `cap` 8-byte entries, key << 32 | count
+// first, then every aggregate (with run-time types room for all of a column's;
+// with known ones an int32 column's minimum and maximum share an array).  Array f
+// starts at f * cap, f known at compile time: a pointer per array would be 26
+// registers for four columns, which the rows' loads then lack.
+enum { kFSum, kFMin, kFMax };
+template <uint32_t SIG>
+constexpr bool stage_packs(int c) {
+  return SIG != 0 && SIG != kSigSums && ((SIG >> (5 * c)) & 3u) == (uint32_t)NFC_I32 && ((SIG >> (5 * c + 3)) & 3u) == 3u;
+}
+template <int NC, uint32_t SIG>
+constexpr int stage_field(int c, int which) {
+  if (SIG == 0) return 1 + 3 * c + which;
+  if (SIG == kSigSums) return 1 + c;
+  int f = 1;
+  for (int i = 0; i < c; ++i) {
+    for (int a = 0; a < 3; ++a) f += (SIG >> (5 * i + 2 + a)) & 1u;
+    f -= stage_packs<SIG>(i);
+  }
+  for (int a = 0; a < which; ++a) f += (SIG >> (5 * c + 2 + a)) & 1u;
+  return which == kFMax ? f - stage_packs<SIG>(c) : f;
+}
+static_assert(NFC_AGG_SUM == 1 && NFC_AGG_MIN == 2 && NFC_AGG_MAX == 4, "bit order of the fields");
+template <int NC, uint32_t SIG>
+constexpr int stage_fields() { return stage_field<NC, SIG>(NC, 0); }
+
+struct Stage {
+  uint64_t* base;
+  int cap;
+  NFC_DEV uint64_t& at(int f, int e) const { return base[f * cap + e]; }
+};
+
+template <int NC, uint32_t SIG>
+NFC_DEV void stage_put(const ColSet& cs, const Stage& st, int e, const Seg<NC>& a, int32_t key) {
+  st.at(0, e) = (uint64_t)(uint32_t)key << 32 | a.cnt;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int ag = col_ag<SIG>(cs, c);
+    if (ag & NFC_AGG_SUM) st.at(stage_field<NC, SIG>(c, kFSum), e) = a.sum[c];
+    if (stage_packs<SIG>(c)) {
+      st.at(stage_field<NC, SIG>(c, kFMin), e) = a.mx[c] << 32 | (uint32_t)a.mn[c];
+      continue;
+    }
+    if (ag & NFC_AGG_MIN) st.at(stage_field<NC, SIG>(c, kFMin), e) = a.mn[c];
+    if (ag & NFC_AGG_MAX) st.at(stage_field<NC, SIG>(c, kFMax), e) = a.mx[c];
+  }
+}
+
+// Entries 0 .. n of the stage to output rows g0 on, the keys of nk.
+template <int NC, uint32_t SIG>
+NFC_DEV void stage_write(const ColSet& cs, const Stage& st, const OutSet& o, int64_t g0, int nk, int n) {
+  const int t = threadIdx.x;
+  for (int i = t; i < nk; i += kSoThreads) {
+    const uint64_t x = st.at(0, i);
+    o.ukeys[g0 + i] = (int64_t)(int32_t)(x >> 32);
+    if (i < n) o.counts[g0 + i] = (int64_t)(uint32_t)x;
+  }
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int dt = col_dt<SIG>(cs, c), ag = col_ag<SIG>(cs, c);
+    if (ag & NFC_AGG_SUM) {
+      uint64_t* d = static_cast<uint64_t*>(o.sum[c]) + g0;
+      for (int i = t; i < n; i += kSoThreads) d[i] = st.at(stage_field<NC, SIG>(c, kFSum), i);
+    }
+    if (dt == NFC_I32) {
+      if (ag & NFC_AGG_MIN) {
+        int32_t* d = static_cast<int32_t*>(o.mn[c]) + g0;
+        for (int i = t; i < n; i += kSoThreads) d[i] = (int32_t)st.at(stage_field<NC, SIG>(c, kFMin), i);
+      }
+      if (ag & NFC_AGG_MAX) {
+        int32_t* d = static_cast<int32_t*>(o.mx[c]) + g0;
+        for (int i = t; i < n; i += kSoThreads)
+          d[i] = (int32_t)(st.at(stage_field<NC, SIG>(c, kFMax), i) >> (stage_packs<SIG>(c) ? 32 : 0));
+      }
+      continue;
+    }
+    if (ag & NFC_AGG_MIN) {
+      uint64_t* d = static_cast<uint64_t*>(o.mn[c]) + g0;
+      for (int i = t; i < n; i += kSoThreads) {
+        const uint64_t x = st.at(stage_field<NC, SIG>(c, kFMin), i);
+        d[i] = dt == NFC_F64 ? f64_min_dec(x) : x;
+      }
+    }
+    if (ag & NFC_AGG_MAX) {
+      uint64_t* d = static_cast<uint64_t*>(o.mx[c]) + g0;
+      for (int i = t; i < n; i += kSoThreads) {
+        const uint64_t x = st.at(stage_field<NC, SIG>(c, kFMax), i);
+        d[i] = dt == NFC_F64 ? f64_max_dec(x) : x;
+      }
+    }
+  }
+}
+
+// Shared memory of a CTA.  More stage, fewer turns for short runs, but less L1 for the
+// rows' loads: one float64 sum over 20M rows in long runs 254 us at 40 KB, 278 at
+// 75; two columns with all aggregates in runs of two 445 us at 40 KB, 392 at 60.
+constexpr size_t so_smem(int nc) { return (nc <= 1 ? 44 : nc == 2 ? 60 : 80) * 1024; }
 
 // CTAs per SM that the registers of the run aggregates leave room for.
 template <int NC, uint32_t SIG>
@@ -523,10 +604,7 @@ constexpr int so_ctas() { return NC == 0 ? 4 : NC <= 2 ? 3 : 2; }
 
 template <int NC, uint32_t SIG>
 struct SortedSmem {
-  union {
-    Partials<NC> lead;             // rows before the thread's first head; all its rows when it has none
-    uint64_t stage[so_tile(NC)];  // short runs: one output column of the tile's runs
-  };
+  Partials<NC> lead;  // rows before the thread's first head; all its rows when it has none
   Seg<NC> wsum[kSoWarps];  // all rows of a warp without heads
   uint64_t wlast[kSoWarps];  // last valid key of the warp (1 << 32 | key), 0 none
   uint32_t wheads[kSoWarps];
@@ -538,12 +616,15 @@ struct SortedSmem {
 // What bounds it: 40M rows of one int64 and one float64 sum in runs of 16 are
 // 0.88 GB (135 us); the form with a segmented warp scan per 128 rows, four rows
 // per lane, was issue bound at 1,145 us (and 16,384-row tiles left most SMs
-// without work below 2M rows).
+// without work below 2M rows).  Runs leave through a stage in one pass over the
+// rows: writing the runs between two heads in a second pass, and output column
+// by output column where runs are short, took 60M rows in runs of 2.3 with six
+// aggregates 1,160 us, 935 this way; runs of 8 850 and 790.
 template <int NC, uint32_t SIG>
 __global__ void __launch_bounds__(kSoThreads + 32, so_ctas<NC, SIG>())
     k_sorted_agg(const int32_t* __restrict__ keys, const uint32_t* __restrict__ vmask, ColSet cs, int64_t n,
-                 bool aligned, const uint64_t* __restrict__ prev, OutSet o, int64_t cap, Pieces P, uint64_t* lb,
-                 uint32_t* ticket, int64_t* ng_out, int32_t* err) {
+                 bool aligned, const uint64_t* __restrict__ prev, OutSet o, int64_t out_cap, int cap, Pieces P,
+                 uint64_t* lb, uint32_t* ticket, int64_t* ng_out, int32_t* err) {
   extern __shared__ __align__(128) unsigned char sm_raw[];
   SortedSmem<NC, SIG>& sm = *reinterpret_cast<SortedSmem<NC, SIG>*>(sm_raw);
   constexpr int kSoRows = so_rows(NC), kSoTile = so_tile(NC);
@@ -647,239 +728,106 @@ __global__ void __launch_bounds__(kSoThreads + 32, so_ctas<NC, SIG>())
   if (lane == 0) sm.wany[warp] = any;
   __syncthreads();
 
-  // ---- partial sums before the first and from the last head.
-  Seg<NC> cur, lead;
-  seg_identity<NC, SIG>(cs, cur);
-  seg_identity<NC, SIG>(cs, lead);
-#pragma unroll
-  for (int q = 0; q < kSoRows / 4; ++q) {
-    if (((vb >> (4 * q)) & 0xFu) == 0u) continue;
-    uint64_t v[4][NC > 0 ? NC : 1];
-    load_rows4<NC, SIG>(cs, n, aligned, row0 + 4 * q, v);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const uint32_t bit = 1u << (4 * q + r);
-      if (hb & bit) {
-        if ((hb & (bit - 1u)) == 0u) {
-          seg_add_four<NC, SIG>(cs, cur);
-          lead = cur;
-        }
-        seg_identity<NC, SIG>(cs, cur);
-      }
-      if (vb & bit) seg_add_row<NC, SIG>(cs, cur, v[r]);
-    }
-    seg_add_four<NC, SIG>(cs, cur);
-  }
-  part_store<NC, SIG>(cs, sm.lead, tid, hb ? lead : cur);
-  if (any == 0u) {
-    Seg<NC> w;
-    seg_warp_reduce<NC, SIG>(cs, cur, w);
-    if (lane == 0) sm.wsum[warp] = w;
-  }
-  __syncthreads();
   uint32_t total = 0, mine = 0;
   for (int w = 0; w < kSoWarps; ++w) {
     if (w < warp) mine += sm.wheads[w];
     total += sm.wheads[w];
   }
-  const int64_t excl = sm.excl;
+  const int l0 = (int)(mine + hi - hc);  // the thread's first run, in the tile
+  const Stage st{reinterpret_cast<uint64_t*>(sm_raw + ((sizeof(sm) + 15) & ~(size_t)15)), cap};
 
   // Adds to `a` what the threads from t on hold of an open run, and closes it;
   // true when the run ends inside the tile.
   auto follow = [&](Seg<NC>& a, int t) {
     bool ends = false;
-    while (t < kSoThreads) {
+    while (t < kSoThreads && !ends) {
       const uint32_t rest = sm.wany[t >> 5] >> (t & 31);
       if (rest == 0u && (t & 31) == 0) {
         seg_combine<NC, SIG>(cs, a, sm.wsum[t >> 5]);
         t += 32;
-        continue;
+      } else {
+        part_add<NC, SIG>(cs, a, sm.lead, t);
+        ends = rest & 1u;
+        ++t;
       }
-      part_add<NC, SIG>(cs, a, sm.lead, t);
-      if (rest & 1u) {
-        ends = true;
-        break;
-      }
-      ++t;
     }
     seg_close<NC, SIG>(cs, a);
     return ends;
   };
-  // The run that the tile continues (its rows before the first head).
-  if (tid == 0) {
-    Seg<NC> run = hb ? lead : any ? cur : sm.wsum[0];
-    if (!hb) follow(run, any ? 1 : 32);
-    if (run.cnt > 0) piece_store<NC>(P, 2 * tile, excl - 1, run);
-    else P.idx[2 * tile] = -1;
-    if (total == 0) P.idx[2 * tile + 1] = -1;
-  }
-  // The run of the thread's last head; the tile's last run stays open.
-  const int64_t g = excl + mine + hi - hc;
-  Seg<NC> run = cur;
-  bool ended = false;
-  if (hb) {
-    ended = follow(run, tid + 1);
-    if (!ended) piece_store<NC>(P, 2 * tile + 1, g + hc - 1, run);
-  }
-  // Runs never outnumber min(span, valid rows) <= cap for sorted keys; the
-  // checks only keep a broken sortedness flag in bounds.
-  if (excl + total > cap) {
-    if (tid == 0) atomicExch(err, NFC_ERR_RANGE);
-    return;
-  }
-  const uint32_t last_head = hb ? 31u - (uint32_t)__clz(hb) : 0u;
-  if (total < kSoTile / 4) {
-    // Few runs: every thread writes its own.
-    if (hb == 0u) return;
-    if (ended) seg_emit<NC, SIG>(cs, o, g + hc - 1, run);
-    int64_t gi = g;
+
+  // The tile's runs leave through the stage.  Where there are more of them than fit
+  // (runs of one or two rows), the threads of the later ones take another turn
+  // over their rows.
+  for (int w0 = 0;; w0 += cap) {
+    // The rows before the thread's first head, the runs between two heads, and in
+    // `cur` the rows from its last head on (all of them without one).
+    Seg<NC> cur;
+    seg_identity<NC, SIG>(cs, cur);
+    uint32_t e = (uint32_t)(l0 - 1 - w0);  // entry of the open run
+    int32_t key = 0;
+    const bool turn = w0 == 0 || (hb && l0 + (int)hc > w0 && l0 < w0 + cap);
+    if (turn) {
 #pragma unroll
-    for (int r = 0; r < kSoRows; ++r)
-      if (hb & (1u << r)) o.ukeys[gi++] = (int64_t)k[r];
-    if ((hb & (hb - 1u)) == 0u) return;
-    // Runs inside the thread: from each head to the next.
-    seg_identity<NC, SIG>(cs, run);
-    gi = g - 1;
+      for (int q = 0; q < kSoRows / 4; ++q) {
+        if (((vb >> (4 * q)) & 0xFu) == 0u) continue;
+        uint64_t v[4][NC > 0 ? NC : 1];
+        load_rows4<NC, SIG>(cs, n, aligned, row0 + 4 * q, v);
 #pragma unroll
-    for (int q = 0; q < kSoRows / 4; ++q) {
-      if (4u * q > last_head) continue;
-      uint64_t v[4][NC > 0 ? NC : 1];
-      load_rows4<NC, SIG>(cs, n, aligned, row0 + 4 * q, v);
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const uint32_t bit = 1u << (4 * q + r);
-        if (hb & bit) {
-          if (gi >= g) {
-            seg_add_four<NC, SIG>(cs, run);
-            seg_emit<NC, SIG>(cs, o, gi, run);
+        for (int r = 0; r < 4; ++r) {
+          const uint32_t bit = 1u << (4 * q + r);
+          if (hb & bit) {
+            if (q > 0 && so_fours(NC)) seg_add_four<NC, SIG>(cs, cur);
+            if (hb & (bit - 1u)) {
+              if (e < (uint32_t)cap) stage_put<NC, SIG>(cs, st, (int)e, cur, key);
+            } else if (w0 == 0) {
+              part_store<NC, SIG>(cs, sm.lead, tid, cur);
+            }
+            seg_identity<NC, SIG>(cs, cur);
+            key = k[4 * q + r];
+            ++e;
           }
-          ++gi;
-          seg_identity<NC, SIG>(cs, run);
+          if (vb & bit) seg_add_row<NC, SIG>(cs, cur, v[r], q == 0 || !so_fours(NC));
         }
-        if (vb & bit) seg_add_row<NC, SIG>(cs, run, v[r]);
+        if (q > 0 && so_fours(NC)) seg_add_four<NC, SIG>(cs, cur);
       }
-      seg_add_four<NC, SIG>(cs, run);
     }
-    return;
-  }
-  // Many short runs: threads writing several runs each would scatter 8-byte
-  // stores (20M rows in runs of 1.6, six aggregates: 763 us), so the outputs
-  // leave column by column through shared memory.
-  const uint32_t l0 = mine + hi - hc;
-  uint32_t last_key = 0u;  // of the thread's last head
-#pragma unroll
-  for (int r = 0; r < kSoRows; ++r)
-    if (hb & (1u << r)) last_key = (uint32_t)k[r];
-  // fill() sets the thread's entries of the stage, store(i, x) writes entry i.
-  auto put = [&](auto fill, auto store) {
-    __syncthreads();  // the stage is free
-    fill();
+    if (w0 == 0) {
+      if (hb == 0u) part_store<NC, SIG>(cs, sm.lead, tid, cur);
+      if (any == 0u) {
+        Seg<NC> w;
+        seg_warp_reduce<NC, SIG>(cs, cur, w);
+        if (lane == 0) sm.wsum[warp] = w;
+      }
+      __syncthreads();
+      // The run that the tile continues (its rows before the first head).
+      if (tid == 0) {
+        Seg<NC> run;
+        if (any) part_load<NC, SIG>(cs, run, sm.lead, 0);
+        else run = sm.wsum[0];
+        if (!hb) follow(run, any ? 1 : 32);
+        if (run.cnt > 0) piece_store<NC>(P, 2 * tile, sm.excl - 1, run);
+        else P.idx[2 * tile] = -1;
+        if (total == 0) P.idx[2 * tile + 1] = -1;
+      }
+      if (total == 0) return;
+    }
+    // The run of the thread's last head; the tile's last run stays open.
+    if (hb && turn) {
+      const bool ended = follow(cur, tid + 1);
+      if (e < (uint32_t)cap) stage_put<NC, SIG>(cs, st, (int)e, cur, key);
+      if (!ended && w0 == 0) piece_store<NC>(P, 2 * tile + 1, sm.excl + total - 1, cur);
+    }
+    // Runs never outnumber min(span, valid rows) <= out_cap for sorted keys; the
+    // check only keeps a broken sortedness flag in bounds.
+    if (sm.excl + total > out_cap) {
+      if (tid == 0) atomicExch(err, NFC_ERR_RANGE);
+      return;
+    }
     __syncthreads();
-    for (uint32_t i = tid; i < total; i += kSoThreads) store(i, sm.stage[i]);
-  };
-  // One aggregate of every run: `first` starts a run's value, `add` folds a
-  // row's, `dec` gives what is staged of it, `fin` is that of the thread's last
-  // run.  The tile's last run is open; its entry is not written out.
-  auto runs_of = [&](uint64_t first, uint64_t fin, auto add, auto dec) {
-    uint32_t l = l0;
-    uint64_t x = first;
-    bool open = false;
-#pragma unroll
-    for (int r = 0; r < kSoRows; ++r) {
-      if (hb & (1u << r)) {
-        if (open) sm.stage[l++] = dec(x);
-        open = true;
-        x = first;
-      }
-      if (vb & (1u << r)) x = add(x, r);
-    }
-    if (hb) sm.stage[l] = fin;
-  };
-  auto same = [](uint64_t x) { return x; };
-  // Keys and counts in one go: a run's key is any of its rows' keys.
-  put([&] {
-        runs_of(0, (uint64_t)run.cnt << 32 | last_key,
-                [&](uint64_t x, int r) { return ((x >> 32) + 1) << 32 | (uint32_t)k[r]; }, same);
-      },
-      [&](uint32_t i, uint64_t x) {
-        o.ukeys[excl + i] = (int64_t)(int32_t)(uint32_t)x;
-        if (i + 1 < total) o.counts[excl + i] = (int64_t)(x >> 32);
-      });
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const int dt = col_dt<SIG>(cs, c), ag = col_ag<SIG>(cs, c);
-    if (ag == 0) continue;
-    uint64_t v[kSoRows];
-    load_rows<kSoRows, SIG>(cs, c, n, aligned, row0, v);
-    auto to64 = [&](void* dst) {
-      uint64_t* d = static_cast<uint64_t*>(dst) + excl;
-      return [d, total](uint32_t i, uint64_t x) {
-        if (i + 1 < total) d[i] = x;
-      };
-    };
-    if ((ag & NFC_AGG_SUM) && dt == NFC_F64)
-      put([&] {
-            // In fours, as above.
-            double four = 0.0;
-            runs_of(0, run.sum[c],
-                    [&](uint64_t x, int r) {
-                      if ((hb >> r) & 1u) four = 0.0;  // a run starts
-                      if ((r & 3) == 0) {
-                        x = f64_add_bits(x, (uint64_t)__double_as_longlong(four));
-                        four = 0.0;
-                      }
-                      four += __longlong_as_double((long long)v[r]);
-                      return x;
-                    },
-                    [&](uint64_t x) { return f64_add_bits(x, (uint64_t)__double_as_longlong(four)); });
-          },
-          to64(o.sum[c]));
-    else if (ag & NFC_AGG_SUM)
-      put([&] {
-            runs_of(0, run.sum[c],
-                    [&](uint64_t x, int r) { return x + (dt == NFC_I32 ? (uint64_t)(int64_t)(int32_t)v[r] : v[r]); },
-                    same);
-          },
-          to64(o.sum[c]));
-    if (dt == NFC_I32) {
-      if (ag & (NFC_AGG_MIN | NFC_AGG_MAX))  // both in one word: maximum above minimum
-        put([&] {
-              runs_of((uint64_t)0x80000000u << 32 | 0x7FFFFFFFu,
-                      (uint64_t)(uint32_t)run.mx[c] << 32 | (uint32_t)run.mn[c],
-                      [&](uint64_t x, int r) {
-                        const int32_t y = (int32_t)v[r];
-                        const int32_t lo = min((int32_t)(uint32_t)x, y), hi = max((int32_t)(x >> 32), y);
-                        return (uint64_t)(uint32_t)hi << 32 | (uint32_t)lo;
-                      },
-                      same);
-            },
-            [&](uint32_t i, uint64_t x) {
-              if (i + 1 >= total) return;
-              if (ag & NFC_AGG_MIN) static_cast<int32_t*>(o.mn[c])[excl + i] = (int32_t)(uint32_t)x;
-              if (ag & NFC_AGG_MAX) static_cast<int32_t*>(o.mx[c])[excl + i] = (int32_t)(x >> 32);
-            });
-      continue;
-    }
-    if (ag & NFC_AGG_MIN)
-      put([&] {
-            if (dt == NFC_F64)
-              runs_of(~0ull, f64_min_dec(run.mn[c]), [&](uint64_t x, int r) { return min(x, f64_min_enc(v[r])); },
-                      [](uint64_t x) { return f64_min_dec(x); });
-            else
-              runs_of((uint64_t)LLONG_MAX, run.mn[c],
-                      [&](uint64_t x, int r) { return (uint64_t)min((long long)x, (long long)v[r]); }, same);
-          },
-          to64(o.mn[c]));
-    if (ag & NFC_AGG_MAX)
-      put([&] {
-            if (dt == NFC_F64)
-              runs_of(0ull, f64_max_dec(run.mx[c]), [&](uint64_t x, int r) { return max(x, f64_max_enc(v[r])); },
-                      [](uint64_t x) { return f64_max_dec(x); });
-            else
-              runs_of((uint64_t)LLONG_MIN, run.mx[c],
-                      [&](uint64_t x, int r) { return (uint64_t)max((long long)x, (long long)v[r]); }, same);
-          },
-          to64(o.mx[c]));
+    const int nk = min((int)total - w0, cap);
+    if (warp * 32 < nk) stage_write<NC, SIG>(cs, st, o, sm.excl + w0, nk, min((int)total - 1 - w0, cap));
+    if (w0 + cap >= (int)total) return;
+    __syncthreads();  // the stage is free
   }
 }
 
@@ -889,7 +837,7 @@ __global__ void __launch_bounds__(kSoThreads + 32, so_ctas<NC, SIG>())
 // it are written, and its first and last runs -- which may continue in the
 // neighbouring chunks -- become pieces 2b and 2b+1 of Q for a second pass.
 template <int NC, uint32_t SIG>
-__global__ void __launch_bounds__(kFixThreads) k_sorted_fix(ColSet cs, Pieces P, int64_t npieces, OutSet o,
+__global__ void __launch_bounds__(fix_threads(NC), 1) k_sorted_fix(ColSet cs, Pieces P, int64_t npieces, OutSet o,
                                                             int64_t cap, Pieces Q) {
   __shared__ SegScanSmem<NC, SIG> sm;
   __shared__ int64_t s_wmax[32];
@@ -951,21 +899,25 @@ template <int NC, uint32_t SIG>
 int launch_sorted(const nfc_groupby_args* a, const ColSet& cs, const OutSet& o, const uint32_t* vmask,
                   const uint64_t* prev, const Pieces& P, const Pieces& Q, int64_t ntiles, int64_t nchunks,
                   uint64_t* lb, uint32_t* ticket, int64_t* d_ng, int32_t* d_err, cudaStream_t s, StageTimer* tm) {
-  const size_t smem = sizeof(SortedSmem<NC, SIG>);
+  // The stage: what leaves the loads some L1 (runs of one row need several turns).
+  const size_t base = (sizeof(SortedSmem<NC, SIG>) + 15) & ~(size_t)15, entry = 8 * (size_t)stage_fields<NC, SIG>();
+  const size_t room = so_smem(NC) - base;
+  const int cap = (int)std::min<size_t>(so_tile(NC), room / entry);
+  const size_t smem = base + (size_t)cap * entry;
   NFC_CUDA(allow_dynamic_smem<k_sorted_agg<NC, SIG>>());
-  k_sorted_agg<NC, SIG><<<(unsigned)ntiles, kSoThreads + 32, smem, s>>>(a->keys, vmask, cs, a->n, inputs_aligned(a), prev, o,
-                                                                   a->out_cap, P, lb, ticket, d_ng, d_err);
+  k_sorted_agg<NC, SIG><<<(unsigned)ntiles, kSoThreads + 32, smem, s>>>(a->keys, vmask, cs, a->n, inputs_aligned(a), prev,
+                                                                      o, a->out_cap, cap, P, lb, ticket, d_ng, d_err);
   NFC_CUDA(cudaGetLastError());
   tm->launched();
   tm->mark(s);
   Pieces none{};
   if (nchunks > 1) {
-    k_sorted_fix<NC, SIG><<<(unsigned)nchunks, kFixThreads, 0, s>>>(cs, P, 2 * ntiles, o, a->out_cap, Q);
+    k_sorted_fix<NC, SIG><<<(unsigned)nchunks, fix_threads(NC), 0, s>>>(cs, P, 2 * ntiles, o, a->out_cap, Q);
     NFC_CUDA(cudaGetLastError());
-    k_sorted_fix<NC, SIG><<<1, kFixThreads, 0, s>>>(cs, Q, 2 * nchunks, o, a->out_cap, none);
+    k_sorted_fix<NC, SIG><<<1, fix_threads(NC), 0, s>>>(cs, Q, 2 * nchunks, o, a->out_cap, none);
     tm->launched(2);
   } else {
-    k_sorted_fix<NC, SIG><<<1, kFixThreads, 0, s>>>(cs, P, 2 * ntiles, o, a->out_cap, none);
+    k_sorted_fix<NC, SIG><<<1, fix_threads(NC), 0, s>>>(cs, P, 2 * ntiles, o, a->out_cap, none);
     tm->launched();
   }
   NFC_CUDA(cudaGetLastError());
@@ -995,7 +947,7 @@ int run_sorted(const nfc_groupby_args* a, const ColSet& cs, const OutSet& o, con
   const int64_t ntiles = (n + so_tile(a->ncols) - 1) / so_tile(a->ncols);
   const int64_t nrec = (n + kProbeBlockRows - 1) / kProbeBlockRows;  // <= ntiles
   const int64_t np = 2 * ntiles;
-  const int64_t nchunks = (np + kFixThreads - 1) / kFixThreads;
+  const int64_t nchunks = (np + fix_threads(a->ncols) - 1) / fix_threads(a->ncols);
   const int64_t nq = 2 * nchunks;
   // One allocation: prev[ntiles], lb[ntiles], ticket, tile pieces, chunk pieces.
   const size_t per_piece = 2 + 3 * NFC_MAX_COLS;
