@@ -391,7 +391,7 @@ struct TkSample {
   uint32_t ready;         // the threshold lets few enough rows through
   uint32_t count;         // rows collected
   uint32_t status;        // 1: the exact passes have to run
-  uint32_t pad;
+  uint32_t failed;        // fewer valid rows in the sample than the target
   uint32_t done[kTkLevels];  // CTAs that have finished each level
   uint32_t hist[kTkLevels][kTkBins];
 };
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(kTkThreads) k_tk_sample(const void* __restrict
   __shared__ uint32_t h[2][kTkBins];
   __shared__ uint32_t s_scan[33];
   __shared__ int s_last;
-  if (level && st->ready) return;
+  if (level && (st->ready || st->failed)) return;
   const uint64_t prefix = level ? st->prefix : 0ull, mask = level ? st->mask : 0ull;
   uint32_t* hs = h[(threadIdx.x >> 5) & 1];
   for (int i = threadIdx.x; i < 2 * kTkBins; i += kTkThreads) (&h[0][0])[i] = 0u;
@@ -457,8 +457,8 @@ __global__ void __launch_bounds__(kTkThreads) k_tk_sample(const void* __restrict
   }
   uint32_t total;
   uint32_t x = block_excl_scan(sum, s_scan, &total);
-  // Fewer sampled valid rows than the target: no digit holds it, and the
-  // levels that follow find nothing to count.
+  // Fewer sampled valid rows than the target: no digit holds it.
+  if (total < want && threadIdx.x == 0) st->failed = 1u;
 #pragma unroll
   for (int j = 0; j < kPer; ++j) {
     if (x < want && want <= x + c[j]) {
