@@ -162,6 +162,42 @@ __global__ void __launch_bounds__(kTkThreads) k_tk_hist(const void* __restrict__
   }
 }
 
+// Valid rows, rows below the prefix and rows on it -> cnt[0..2].
+template <int DT>
+__global__ void __launch_bounds__(kTkThreads) k_tk_below(const void* __restrict__ keys,
+                                                        const uint8_t* __restrict__ validity, int64_t n, bool vec,
+                                                        bool desc, uint64_t mask, uint64_t prefix,
+                                                        unsigned long long* __restrict__ cnt) {
+  const int64_t ngroups = (n + 3) >> 2;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  constexpr int U = 2;
+  uint32_t c[3] = {0u, 0u, 0u};
+  for (int64_t g0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g0 < ngroups; g0 += U * stride) {
+    uint64_t img[U][4];
+    uint32_t ok[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t g = g0 + u * stride;
+      ok[u] = g < ngroups ? tk_load4<DT>(keys, validity, g * 4, n, vec, desc, img[u]) : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if ((ok[u] >> r) & 1u) {
+          const uint64_t m = img[u][r] & mask;
+          c[0] += 1u;
+          c[1] += m < prefix;
+          c[2] += m == prefix;
+        }
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const uint32_t w = warp_sum(c[k]);
+    if (lane_id() == 0 && w) atomicAdd(&cnt[k], (unsigned long long)w);
+  }
+}
+
 // Row class: 0 taken (below the prefix), 1 tie (on the prefix), 2 NULL,
 // 3 neither.
 template <int DT>
@@ -384,7 +420,7 @@ constexpr int64_t kTkExpect = 5000;   // most rows expected under the threshold
 constexpr int kTkFinalThreads = 512;
 constexpr int kTkLevels = 4;          // digits of the threshold at most
 
-struct TkSample {
+struct TkSampleHead {
   uint64_t prefix, mask;  // threshold: rows with (image & mask) <= prefix
   uint32_t target;        // rank in the sample still to find on the prefix
   uint32_t below;         // sampled rows under the prefix
@@ -392,6 +428,8 @@ struct TkSample {
   uint32_t count;         // rows collected
   uint32_t status;        // 1: the exact passes have to run
   uint32_t failed;        // fewer valid rows in the sample than the target
+};
+struct TkSample : TkSampleHead {
   uint32_t done[kTkLevels];  // CTAs that have finished each level
   uint32_t hist[kTkLevels][kTkBins];
 };
@@ -653,10 +691,17 @@ int64_t tk_target(int64_t k, int64_t step) {
 }
 
 // The sampled form, for k small enough that its rows fit one CTA's sort.
-// *done = 0: not tried, or the threshold did not hold.
+// *done = 0: not tried, or the threshold did not hold.  Where the sample went
+// through all its digits and many rows were still on the prefix (ties),
+// hint->mask is set: the k-th image is very likely on hint->prefix.
+struct TkHint {
+  uint64_t prefix, mask;
+  int shift;  // bits below the prefix
+};
+
 template <int DT>
 int topk_sampled(const void* keys, const uint8_t* validity, int64_t n, bool desc, int64_t k, int32_t* perm_out,
-                 cudaStream_t s, int* done) {
+                 cudaStream_t s, int* done, TkHint* hint) {
   *done = 0;
   // About a million sampled rows at 64M (their histograms take a tenth of the
   // pass), fewer groups skipped where k needs a sharper threshold.
@@ -691,9 +736,10 @@ int topk_sampled(const void* keys, const uint8_t* validity, int64_t n, bool desc
   NFC_CUDA(allow_dynamic_smem<k_tk_final>());
   k_tk_final<<<(unsigned)num_sms(), kTkFinalThreads, smem, s>>>(st, DT == NFC_F64 && desc, (uint32_t)k, c_img, c_row, perm_out);
   NFC_CUDA(cudaGetLastError());
-  uint32_t status = 0;
-  NFC_CUDA(readback(&status, &st->status, sizeof(status), s));
-  *done = status == 0;
+  TkSampleHead h;
+  NFC_CUDA(readback(&h, static_cast<TkSampleHead*>(st), sizeof(h), s));
+  *done = h.status == 0;
+  if (h.status && !h.ready && !h.failed) *hint = TkHint{h.prefix, h.mask, std::max(0, bits - kTkLevels * kTkDigitBits)};
   return NFC_OK;
 }
 
@@ -701,9 +747,10 @@ template <int DT>
 int topk_impl(const void* keys, const uint8_t* validity, int64_t n, bool desc, int64_t k, int32_t* perm_out,
               cudaStream_t s) {
   using K = typename std::conditional<DT == NFC_I32, uint32_t, uint64_t>::type;
+  TkHint hint{};
   {
     int done = 0;
-    const int rc = topk_sampled<DT>(keys, validity, n, desc, k, perm_out, s, &done);
+    const int rc = topk_sampled<DT>(keys, validity, n, desc, k, perm_out, s, &done, &hint);
     if (rc || done) return rc;
   }
   Scratch sc(s);
@@ -720,8 +767,32 @@ int topk_impl(const void* keys, const uint8_t* validity, int64_t n, bool desc, i
   int64_t nv = 0, ksel = 0, need = 0, on_prefix = 0;
   uint32_t hh[kTkBins];
   bool first = true;
-  bool use_cand = false;
-  while (shift > 0) {
+  bool use_cand = false, found = false;
+  if (hint.mask) {
+    // One count over the column in place of its digit histograms, if the k-th
+    // image is where the sample says (100M int32 of 1,000 values: three of them).
+    unsigned long long* d_cnt = nullptr;
+    unsigned long long c[3] = {0, 0, 0};  // valid, below, on the prefix
+    NFC_CUDA(sc.alloc(&d_cnt, 3));
+    NFC_CUDA(cudaMemsetAsync(d_cnt, 0, sizeof(c), s));
+    k_tk_below<DT><<<tk_grid((n + 3) / 4), kTkThreads, 0, s>>>(keys, validity, n, vec, desc, hint.mask, hint.prefix,
+                                                               d_cnt);
+    NFC_CUDA(cudaGetLastError());
+    NFC_CUDA(readback(c, d_cnt, sizeof(c), s));
+    if (k < (int64_t)c[0] && (int64_t)c[1] < k && k <= (int64_t)(c[1] + c[2])) {
+      first = false;
+      nv = (int64_t)c[0];
+      ksel = k;
+      need = k - (int64_t)c[1];
+      on_prefix = (int64_t)c[2];
+      prefix = hint.prefix;
+      mask = hint.mask;
+      shift = hint.shift;
+      use_cand = on_prefix != need && on_prefix <= kTkCandCap && shift > 0;
+      found = on_prefix == need || use_cand;
+    }
+  }
+  while (shift > 0 && !found) {
     const int dbits = std::min(kTkDigitBits, shift);
     shift -= dbits;
     const uint32_t dmask = (1u << dbits) - 1u;
