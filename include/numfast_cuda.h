@@ -212,7 +212,9 @@ typedef struct nfc_probe {
 #define NFC_MAX_STAGES 8
 
 typedef struct nfc_groupby_stats {
-  int32_t strategy; /* strategy that ran                          */
+  int32_t strategy; /* strategy that ran; AUTO inputs of at most 16,384 rows
+                       whose keys span little are grouped by one kernel
+                       (launches 1), and this is the rule's pick */
   int32_t status;   /* device status word (0 ok)                  */
   int64_t ng;       /* groups written                             */
   nfc_probe probe;

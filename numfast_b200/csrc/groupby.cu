@@ -666,6 +666,7 @@ int64_t nfc::groupby_run(const nfc_groupby_args* a, int32_t strategy, PlanHook* 
     stats->status = 0;
     stats->ng = 0;
     stats->buckets = 0;
+    stats->overflowed = 0;
     stats->launches = tm.launches;
     stats->nstages = 0;
   }
