@@ -614,7 +614,9 @@ extern "C" int32_t nfc_plan_strategy(const nfc_groupby_args* args, const nfc_pro
   OutSet o;
   const int rc = build_colset(args, &cs, &o);
   if (rc) return rc;
-  return plan_strategy(cs, *probe);
+  nfc_probe p = *probe;
+  p.pad = 0;  // only a probe of the library's own has a sampled count there
+  return plan_strategy(cs, p);
 }
 
 extern "C" int64_t nfc_groupby(const nfc_groupby_args* a, int32_t strategy, void* stream,
