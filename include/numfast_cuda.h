@@ -206,7 +206,7 @@ typedef struct nfc_probe {
   int64_t kmin;    /* over valid rows (0 when n_valid == 0)       */
   int64_t kmax;
   int32_t sorted;  /* valid keys nondecreasing in row order        */
-  int32_t pad;     /* nfc_groupby, large inputs: most sampled rows (of 1,024) in one key slot; else 0 */
+  int32_t pad;     /* AUTO, large inputs: most sampled rows (of 1,024) in one key slot; else 0 */
 } nfc_probe;
 
 #define NFC_MAX_STAGES 8

@@ -475,7 +475,7 @@ constexpr int64_t kSkewMinRows = 1 << 20;
 constexpr int32_t kSkewHot = 16;
 
 int run_probe(const nfc_groupby_args* a, cudaStream_t s, Scratch& sc, uint32_t** vmask_out,
-              nfc_probe* host_probe, StageTimer* tm, const ProbeRec** recs_out) {
+              nfc_probe* host_probe, StageTimer* tm, const ProbeRec** recs_out, bool sample) {
   const int64_t n = a->n;
   const BitmapSet bms = bitmaps_of(a);
   uint32_t* vmask = nullptr;
@@ -492,7 +492,8 @@ int run_probe(const nfc_groupby_args* a, cudaStream_t s, Scratch& sc, uint32_t**
     NFC_CUDA(cudaGetLastError());
     tm->launched();
   }
-  k_probe_finalize<<<1, 1024, 0, s>>>(recs, (nspans + 7) / 8, dprobe, n >= kSkewMinRows ? a->keys : nullptr, vmask, n);
+  k_probe_finalize<<<1, 1024, 0, s>>>(recs, (nspans + 7) / 8, dprobe, sample && n >= kSkewMinRows ? a->keys : nullptr,
+                                      vmask, n);
   NFC_CUDA(cudaGetLastError());
   tm->launched();
   tm->mark(s);
@@ -654,7 +655,10 @@ int64_t nfc::groupby_run(const nfc_groupby_args* a, int32_t strategy, PlanHook* 
     rc = run_small(a, cs, o, s, sc, &vmask, &recs, &small, &tm);
     p = small.probe;
   }
-  if (rc == NFC_ERR_UNSUPPORTED) rc = run_probe(a, s, sc, &vmask, &p, &tm, &recs);
+  // The hot-key sample is for the library's own rule (also as a planner's and in
+  // place of SORTED on unsorted keys).
+  const bool sample = strategy == NFC_STRAT_AUTO || strategy == NFC_STRAT_SORTED;
+  if (rc == NFC_ERR_UNSUPPORTED) rc = run_probe(a, s, sc, &vmask, &p, &tm, &recs, sample);
   if (rc) return rc;
   int strat = strategy == NFC_STRAT_AUTO ? plan_strategy(cs, p) : strategy;
   int64_t hint = stats ? stats->distinct_hint : 0;

@@ -59,9 +59,10 @@ struct ProbeRec {
 
 // Probe of the call's rows: *host_probe (read back), the combined validity
 // bitmap (*vmask_out, null when no input has a bitmap) and, when recs_out is
-// given, the device array of ceil(n / kProbeBlockRows) probe records.
+// given, the device array of ceil(n / kProbeBlockRows) probe records.  sample:
+// with the sampled count of the hottest key (pad) for large inputs.
 int run_probe(const nfc_groupby_args* a, cudaStream_t s, Scratch& sc, uint32_t** vmask_out,
-              nfc_probe* host_probe, StageTimer* tm, const ProbeRec** recs_out = nullptr);
+              nfc_probe* host_probe, StageTimer* tm, const ProbeRec** recs_out = nullptr, bool sample = false);
 int plan_strategy(const ColSet& cs, const nfc_probe& p);
 
 // Small inputs (small.cu), n in [1, kSmallRows]: the probe and, if the key

@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 def groupby(n, strategy, stats, span=50):
-    k = torch.randint(0, span, (n,), device="cuda", dtype=torch.int32)
+    k = (torch.arange(n, device="cuda", dtype=torch.int32) * 7919) % span
     out = torch.empty((2, max(n, 1)), dtype=torch.int64, device="cuda")
     a = _lib.GroupbyArgs()
     a.n, a.keys, a.ncols, a.out_cap = n, k.data_ptr(), 0, n
@@ -27,3 +27,13 @@ def test_reused_stats(cuda, n):
     s.overflowed, s.buckets, s.status, s.ng, s.nstages = 2, 77, -7, 99, 5
     assert groupby(n, _lib.STRAT_AUTO, s) == 50
     assert (s.overflowed, s.buckets, s.status, s.ng, s.nstages) == (0, 0, 0, 50, 0)
+
+
+@pytest.mark.parametrize("strategy", [_lib.STRAT_AUTO, _lib.STRAT_PARTITION])
+def test_hot_key_sample(cuda, strategy):
+    """The library's own rule samples for hot keys on large inputs; a named strategy does not."""
+    s = _lib.GroupbyStats()
+    assert groupby(1_200_000, strategy, s, span=3) == 3
+    assert (s.probe.pad >= 200) == (strategy == _lib.STRAT_AUTO)
+    assert groupby(100_000, strategy, s, span=3) == 3
+    assert s.probe.pad == 0
