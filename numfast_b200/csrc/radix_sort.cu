@@ -178,27 +178,23 @@ struct RsSmem {
   uint32_t wt[2][kRsWarps];
 };
 
-// Lanes whose digit equals this lane's, from one vote per digit bit: a fixed
-// cost for any digits, where __match_any_sync goes through the distinct values
-// (200M u32 pairs sorted in 6.9 against 5.6 ms).  In PTX because the predicate
-// that feeds the vote also selects the complement, which keeps a bit at three
-// to four ALU operations (the same loop in C++: 3-8% slower sorts).
 NFC_DEV unsigned match_digit8(uint32_t d) {
-  unsigned m = 0xffffffffu;
+  uint32_t differ = 0u;
 #pragma unroll
   for (int b = 0; b < 8; ++b)
-    asm volatile("{\n"
-        " .reg .pred p;\n"
-        " .reg .b32 t;\n"
-        " and.b32 t, %1, %2;\n"
-        " setp.ne.u32 p, t, 0;\n"
-        " vote.sync.ballot.b32 t, p, 0xffffffff;\n"
-        " @!p not.b32 t, t;\n"
-        " and.b32 %0, %0, t;\n"
+    asm volatile(
+        "{\n"
+        " .reg .pred set;\n"
+        " .reg .b32 mine, all;\n"
+        " and.b32 mine, %1, %2;\n"
+        " setp.ne.u32 set, mine, 0;\n"
+        " selp.b32 mine, 0xffffffff, 0, set;\n"
+        " vote.sync.ballot.b32 all, set, 0xffffffff;\n"
+        " lop3.b32 %0, %0, all, mine, 0xF6;\n"
         "}"
-        : "+r"(m)
+        : "+r"(differ)
         : "r"(d), "r"(1u << b));
-  return m;
+  return ~differ;
 }
 
 // 4 bytes from global straight to shared memory, no register held meanwhile.
