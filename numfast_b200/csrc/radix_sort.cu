@@ -178,6 +178,12 @@ struct RsSmem {
   uint32_t wt[2][kRsWarps];
 };
 
+// Lanes whose digit equals this lane's: a vote per digit bit, as GPU radix sorts
+// commonly rank (CUB's among them), and the lanes whose bit is not this lane's
+// collected with one three-input operation on the vote and this lane's bit as a
+// mask.  A fixed cost for any digits, where __match_any_sync goes through the
+// distinct values (200M u32 pairs sorted in 6.9 against 5.6 ms).  In PTX because
+// the compiler's own choice for the same steps takes 2-4% longer sorts.
 NFC_DEV unsigned match_digit8(uint32_t d) {
   uint32_t differ = 0u;
 #pragma unroll
