@@ -26,22 +26,10 @@ NFC_DEV void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 
-NFC_DEV void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-}
-
-// L2 eviction-priority policies (createpolicy) for cache-hinted accesses.
+// L2 eviction-priority policy (createpolicy) for cache-hinted accesses.
 NFC_DEV uint64_t l2_policy_evict_first() {
   uint64_t p;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-NFC_DEV uint64_t l2_policy_evict_last() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
 
@@ -52,19 +40,6 @@ NFC_DEV void bulk_g2s_hint(void* dst, const void* src, uint32_t bytes, uint64_t*
           smem_u32(dst)),
       "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
       : "memory");
-}
-
-// Bring [p, p + bytes) into L2 (p and bytes multiples of 16).
-NFC_DEV void prefetch_l2(const void* p, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
-// 16- and 8-byte global stores with an L2 eviction policy.
-NFC_DEV void st_v2_u64_hint(uint64_t* p, uint64_t a, uint64_t b, uint64_t policy) {
-  asm volatile("st.global.L2::cache_hint.v2.u64 [%0], {%1, %2}, %3;" ::"l"(p), "l"(a), "l"(b), "l"(policy) : "memory");
-}
-NFC_DEV void st_u64_hint(uint64_t* p, uint64_t a, uint64_t policy) {
-  asm volatile("st.global.L2::cache_hint.u64 [%0], %1, %2;" ::"l"(p), "l"(a), "l"(policy) : "memory");
 }
 
 NFC_DEV bool mbar_try_wait(uint64_t* bar, uint32_t parity) {

@@ -296,35 +296,6 @@ NFC_DEV void warp_agg_apply(const ColSet& cs, const StateRef& st, bool active, i
       });
 }
 
-// Merge slot s of `src` into slot d of `dst` (dst shared by many CTAs).
-NFC_DEV void state_merge(const ColSet& cs, const StateRef& dst, int64_t d, const StateRef& src, int64_t s) {
-  const uint32_t k = src.cnt[s];
-  if (k == 0u) return;
-  atomicAdd(&dst.cnt[d], k);
-#pragma unroll
-  for (int c = 0; c < NFC_MAX_COLS; ++c) {
-    if (c >= cs.ncols) break;
-    const int dt = cs.dtype[c], ag = cs.aggs[c];
-    if (dt == NFC_F64) {
-      if (ag & NFC_AGG_SUM) atomicAdd(static_cast<double*>(dst.sum[c]) + d, static_cast<const double*>(src.sum[c])[s]);
-      if (ag & NFC_AGG_MIN)
-        atomicMin(static_cast<unsigned long long*>(dst.mn[c]) + d, static_cast<const unsigned long long*>(src.mn[c])[s]);
-      if (ag & NFC_AGG_MAX)
-        atomicMax(static_cast<unsigned long long*>(dst.mx[c]) + d, static_cast<const unsigned long long*>(src.mx[c])[s]);
-    } else {
-      if (ag & NFC_AGG_SUM)
-        atomicAdd(static_cast<unsigned long long*>(dst.sum[c]) + d, static_cast<const unsigned long long*>(src.sum[c])[s]);
-      if (dt == NFC_I32) {
-        if (ag & NFC_AGG_MIN) atomicMin(static_cast<int*>(dst.mn[c]) + d, static_cast<const int*>(src.mn[c])[s]);
-        if (ag & NFC_AGG_MAX) atomicMax(static_cast<int*>(dst.mx[c]) + d, static_cast<const int*>(src.mx[c])[s]);
-      } else {
-        if (ag & NFC_AGG_MIN) atomicMin(static_cast<long long*>(dst.mn[c]) + d, static_cast<const long long*>(src.mn[c])[s]);
-        if (ag & NFC_AGG_MAX) atomicMax(static_cast<long long*>(dst.mx[c]) + d, static_cast<const long long*>(src.mx[c])[s]);
-      }
-    }
-  }
-}
-
 // Output pointers of one group-by call.
 struct OutSet {
   int64_t* ukeys;

@@ -33,7 +33,6 @@
 // 64-bit min/max on an order-preserving encoding; float64 sums use the
 // 64-bit float add.
 #include <algorithm>
-#include <type_traits>
 
 #include "agg_smem.cuh"
 #include "bulk.cuh"
@@ -236,8 +235,8 @@ struct Rec {
   static constexpr int word(int c) { return PACK0 ? (c == 0 ? 0 : c) : c + 1; }
 };
 
-template <int NC, bool PACK0, bool HINT = false>
-NFC_DEV void rec_store(uint64_t* __restrict__ dst, uint32_t klow, const uint64_t* raw, uint64_t policy = 0) {
+template <int NC, bool PACK0>
+NFC_DEV void rec_store(uint64_t* __restrict__ dst, uint32_t klow, const uint64_t* raw) {
   // (raw[0] of a packed column is a sign-extended int32; only its low 32 bits are kept)
   uint64_t w[Rec<NC, PACK0>::NW];
   w[0] = klow;
@@ -249,16 +248,10 @@ NFC_DEV void rec_store(uint64_t* __restrict__ dst, uint32_t klow, const uint64_t
   constexpr int NW = Rec<NC, PACK0>::NW;
   if (NW % 2 == 0) {
 #pragma unroll
-    for (int i = 0; i < NW; i += 2) {
-      if (HINT) st_v2_u64_hint(dst + i, w[i], w[i + 1], policy);
-      else *reinterpret_cast<ulonglong2*>(dst + i) = make_ulonglong2(w[i], w[i + 1]);
-    }
+    for (int i = 0; i < NW; i += 2) *reinterpret_cast<ulonglong2*>(dst + i) = make_ulonglong2(w[i], w[i + 1]);
   } else {
 #pragma unroll
-    for (int i = 0; i < NW; ++i) {
-      if (HINT) st_u64_hint(dst + i, w[i], policy);
-      else dst[i] = w[i];
-    }
+    for (int i = 0; i < NW; ++i) dst[i] = w[i];
   }
 }
 
