@@ -240,8 +240,9 @@ typedef struct nfc_groupby_stats {
  * ng.  Stages (stats->stage_ms when stats->timing is set):
  *   DENSE_*:   probe, state init, aggregate, compact
  *   PARTITION: probe, histogram+plan, scatter, merge-init+aggregate
- *   HASH:      probe, table init, aggregate, extract+sort+emit  Returns ng >= 0, or a negative NFC_ERR_* code.  out_cap must be >=
- * ng (n is always enough).  stream may be NULL (legacy default stream). */
+ *   HASH:      probe, table init, aggregate, extract+sort+emit
+ * Returns ng >= 0, or a negative NFC_ERR_* code.  out_cap must be >= ng (n is
+ * always enough).  stream may be NULL (legacy default stream). */
 int64_t nfc_groupby(const nfc_groupby_args* args, int32_t strategy,
                     void* stream, nfc_groupby_stats* stats);
 
@@ -476,7 +477,7 @@ typedef struct nfc_batch_tuning {
   int32_t warp_agg;       /* global-plan reductions: 0 one per row; 1 equal keys of a warp
                              combined (match_any); 2 the warp's leading key combined (ballot +
                              reduce); 3 a per-CTA shared-memory hash cache in front of them */
-  int32_t ctas_per_sm;    /* resident CTAs per SM: 1 or 2 */
+  int32_t ctas_per_sm;    /* resident CTAs per SM: 1 (of 1,024 threads) or 2 (of 512) */
   int32_t schedule;       /* item order: 0 phase-major, 1 emits interleaved two queries behind, 2 solo queries last */
   int32_t agg_split;      /* 0, or cut every query into at least this many aggregate items */
   int32_t pad;

@@ -313,9 +313,11 @@ __global__ void __launch_bounds__(256) k_dense_global(const int32_t* __restrict_
 //
 // What bounds it is the shared atomics: with few keys the lanes of a warp meet
 // on the same addresses, and a float64 sum is a compare-and-swap loop there.  So
-// the state has as many copies as fit (a power of two up to 32), interleaved:
-// slot g of copy r is entry g * R + r, lane l uses copy l mod R, and with 32
-// copies no two lanes of a warp share an address or a bank.  The chunk is
+// the state has as many copies as fit 100 KB (a power of two up to 32: all 32 for
+// at most 72 keys of 44-byte state), interleaved: slot g of copy r is entry
+// g * R + r, lane l uses copy l mod R, and with 32 copies no two lanes of a warp
+// share an address or a bank.  Before the merge the CTA folds its copies into the
+// first (fold_copies), so that a slot is merged once per CTA.  The chunk is
 // chosen so that the CTAs fill whole waves: fixed chunks of 65,536 rows left ten
 // CTAs of 20M rows for a second wave and most SMs idle below 10M rows.
 constexpr int64_t kDsChunk = 65536;

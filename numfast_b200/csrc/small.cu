@@ -39,11 +39,10 @@ static_assert(kSmallRows == kProbeBlockRows, "one probe record");
 constexpr int kSmCopies = 8;  // log2 of the most copies of the state
 
 template <int NC>
-__global__ void __launch_bounds__(SmallShape<NC>::threads, 1) k_small(const int32_t* __restrict__ keys, BitmapSet bms, ColSet cs,
-                                                         int n, bool aligned, OutSet o, int64_t out_cap,
-                                                         uint32_t state_bytes, uint32_t slot_bytes, uint32_t err_bytes, int max_copies,
-                                                         uint32_t* __restrict__ vmask, ProbeRec* __restrict__ rec,
-                                                         SmallResult* __restrict__ res) {
+__global__ void __launch_bounds__(SmallShape<NC>::threads, 1)
+    k_small(const int32_t* __restrict__ keys, BitmapSet bms, ColSet cs, int n, bool aligned, OutSet o, int64_t out_cap,
+            uint32_t state_bytes, uint32_t slot_bytes, uint32_t err_bytes, int max_copies,
+            uint32_t* __restrict__ vmask, ProbeRec* __restrict__ rec, SmallResult* __restrict__ res) {
   constexpr int kSmThreads = SmallShape<NC>::threads, kSmWarps = SmallShape<NC>::warps;
   constexpr int kSmSteps = SmallShape<NC>::steps, kSmParts = SmallShape<NC>::parts;
   extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -13,9 +13,9 @@
 //                       key before every tile (an exclusive "last non-empty"
 //                       scan over the 16,384-row blocks the probe summarised);
 //   2. k_sorted_agg     one CTA per tile of 2,048 or 4,096 rows, claimed in
-//                       order, a thread per 8 or 16 consecutive rows.  A thread finds its
-//                       run heads (valid rows whose key differs from the
-//                       previous valid row's), sums the rows before its first
+//                       order, a thread per 8 or 16 consecutive rows.  A
+//                       thread finds its run heads (valid rows whose key
+//                       differs from the previous valid row's), sums the rows before its first
 //                       head and after its last one and each run in between,
 //                       and a decoupled look-back gives the tile its first run
 //                       number.  The thread that holds a run's head then adds
@@ -26,11 +26,12 @@
 //                       last run (possibly continued by later ones) leave as
 //                       two partial "pieces";
 //   3. k_sorted_fix     the pieces are merged in order (segmented scan by run
-//                       number): chunks of a CTA each, then the
-//                       chunks' own edge runs in one CTA.
-// Output keys are written by the thread holding each run's head.  float64 sums
-// differ from the reference's row loop in the order of their additions (mean
-// relative error of a run's sum below 2^-53); everything else is exact.
+//                       number): chunks of a CTA each, then the chunks' own
+//                       edge runs in one CTA.
+// Every run's output key is staged by the thread holding its head, the last run's
+// too, whose values leave as a piece.  float64 sums differ from the reference's
+// row loop in the order of their additions (mean relative error of a run's sum
+// below 2^-53); everything else is exact.
 #include <algorithm>
 
 #include "groupby_host.h"
@@ -508,7 +509,8 @@ NFC_DEV void part_add(const ColSet& cs, Seg<NC>& a, const Partials<NC>& p, int t
 enum { kFSum, kFMin, kFMax };
 template <uint32_t SIG>
 constexpr bool stage_packs(int c) {
-  return SIG != 0 && SIG != kSigSums && ((SIG >> (5 * c)) & 3u) == (uint32_t)NFC_I32 && ((SIG >> (5 * c + 3)) & 3u) == 3u;
+  return SIG != 0 && SIG != kSigSums && ((SIG >> (5 * c)) & 3u) == (uint32_t)NFC_I32 &&
+         ((SIG >> (5 * c + 3)) & 3u) == 3u;
 }
 template <int NC, uint32_t SIG>
 constexpr int stage_field(int c, int which) {

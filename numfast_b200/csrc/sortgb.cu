@@ -5,7 +5,7 @@
 // bincounts (src/Drivers/CPU/_lib/groupindex.py:178-211; planner.py:254-262).
 // Here:
 //   1. positions of the valid rows, sorted stably by key (radix
-//      sort of (key, row) pairs, radix.cu)
+//      sort of (key, row) pairs, radix_sort.cu)
 //   2. k_sort_runs: tiles of 1024 sorted positions; run heads by comparing
 //      neighbouring keys, run ids by a block scan plus a decoupled look-back
 //      across tiles; rows fold into a shared-memory state indexed by the

@@ -34,9 +34,11 @@
 //
 // Small k (topk_sampled) needs one pass over the column: the histograms run on
 // a sample of the rows, the rows up to a threshold that holds the k-th smallest
-// image with near certainty are collected in any order, and one CTA sorts them
-// by (image, row).  If the count shows the threshold too low, or too many rows
-// are on it (ties), the passes above run instead.
+// image with near certainty are collected in any order, and every one's place is
+// counted against all of them, by (image, row), over the whole chip.  If the
+// count shows the threshold too low, or too many rows are on it (ties), the
+// passes above run instead; what the sample learned (TkHint) spares them the
+// histograms where the k-th image is on its prefix.
 //
 // Descending float64: every NaN is its own group in the reference's
 // _stable_desc_idx, so the NaN block comes first in REVERSE input order: the
@@ -414,7 +416,7 @@ __global__ void k_tk_reverse(int32_t* p, int64_t m) {
 // and one ordered split, both over the whole column, and 50,000 candidates are
 // then sorted.  A threshold from a sample costs two small histograms; what is
 // left is one pass that reads the column and writes a few thousand rows.
-constexpr int kTkCap = 8192;          // rows one CTA sorts
+constexpr int kTkCap = 8192;          // rows collected at most (96 KB of shared memory in k_tk_final)
 constexpr int64_t kTkExpect = 5000;   // most rows expected under the threshold
 
 constexpr int kTkFinalThreads = 512;
@@ -681,16 +683,17 @@ int tk_status(cudaStream_t s, const int32_t* d_err) {
   return h;
 }
 
-// Sample rank of the threshold when one group in `step` is sampled: it gets six standard deviations and 16 rows more
-// than k / step, so that the k-th row is missed about once in 1e8 calls on
-// rows that the sample represents (and the exact passes then run).
+// Sample rank of the threshold when one group in `step` is sampled: it gets six
+// standard deviations and 16 rows more than k / step, so that the k-th row is
+// missed about once in 1e8 calls on rows that the sample represents (and the
+// exact passes then run).
 int64_t tk_target(int64_t k, int64_t step) {
   if (step == 1) return k;
   const double q = (double)k / (double)step;
   return (int64_t)(q + 6.0 * std::sqrt(q) + 16.0) + 1;
 }
 
-// The sampled form, for k small enough that its rows fit one CTA's sort.
+// The sampled form, for k small enough that its rows fit k_tk_final's list.
 // *done = 0: not tried, or the threshold did not hold.  Where the sample went
 // through all its digits and many rows were still on the prefix (ties),
 // hint->mask is set: the k-th image is very likely on hint->prefix.  Where the
